@@ -232,11 +232,19 @@ __device__ __forceinline__ void prefetch_block(const DPlane& p, int x0, int x1, 
   }
 }
 
+// The frame of an item: base[f] <= item < base[f + 1].  Each round probes 32
+// evenly spaced entries of what is left, one a lane, so a batch of up to 32
+// frames takes one load's latency and one of up to 1,024 takes two, where a
+// binary search waits for a load at every halving.  Called by whole warps.
 __device__ __forceinline__ int find_frame(const int* base, int n, int item) {
-  int lo = 0, hi = n;  // base[lo] <= item < base[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(&base[mid]) <= item) lo = mid; else hi = mid;
+  const int lane = threadIdx.x & 31;
+  int lo = 0, span = n;  // base[lo] <= item < base[lo + span]
+  while (span > 1) {
+    const int step = (span + 31) >> 5;
+    const bool le = lane * step < span && __ldg(&base[lo + lane * step]) <= item;
+    const int k = __popc(__ballot_sync(0xffffffffu, le)) - 1;  // lane 0's always is
+    lo += k * step;
+    span = imin(step, span - k * step);
   }
   return lo;
 }
