@@ -16,310 +16,518 @@
 // boundary that falls inside the unit (tile/restoration_boundary.go:192-255):
 // the boundary-line save is fused into the CDEF pass instead of a separate
 // frame sweep.
+//
+// Bound by instruction issue (72 % of the slots at 32 warps per SM; the
+// half-rate fp16 and integer pipes are both half busy, DRAM 3 %).  Hence the
+// packed pairs of pf_cdef_dev.cuh (7 instructions a tap for two samples,
+// where one sample's constrain() from a shared-memory table took 5 with two
+// shared reads) and the three 4:2:0 planes staged and filtered in one pass.
+// Per frame, 60 x 1080p 8-bit: 22.4 us before, 12.0 now (5.6 of it the taps,
+// 1.5 the directions, 1.0 the staging); 8 x 4K 10-bit: 103.2 and 49.4; one
+// 1080p frame alone: 44.8 and 24.3.  64 registers and 4 CTAs per SM: 48 (5
+// CTAs, with spills) and 80 (3 CTAs) measured 4 % slower.
 #include "pf_cdef_dev.cuh"
 
 namespace pf {
 
-// 8-bit units without sentinels read constrain() from tables: one per
-// primary strength used in the unit (8-bit strengths are 1..15) and one for
-// the secondary strength, 511 entries each (differences -255..255).
-constexpr int kTabLen = 512;
-constexpr int kSecTab = 16;
-
-struct CdefSmem {
-  alignas(16) uint16_t in[kSH * kSW];
-  int32_t cost[64 * 8];
-  int32_t var[64];
-  int32_t blk[64];   // per block: filter flag << 16 | priShift << 12 | strength << 4 | dir
-  int2 ofs[12];      // direction tap offsets in smem units (cdef/filter.go:53-66)
-  uint8_t dir[64];
-  alignas(16) int16_t tab[kSecTab + 1][kTabLen];
-  uint32_t strengths;    // bit k: a block of the plane filters with primary strength k
-  int8_t slot[16];       // table of each primary strength
-  int8_t slot_str[16];   // strength of each table
+// What a luma block's filter needs, made once per block: the primary tap's
+// constants (PairTap; plain strength and shift for samples staged as
+// integers) and flags: bit 31 filtered, bit 4 odd strength (weights 3, 3
+// instead of 4, 2), low bits the direction.
+struct CdefBlk {
+  PairTap pri;
+  uint32_t flags;
 };
 
-// One 64x64 filter unit (uc, ur), all planes.  aw/ah: MI-aligned extents
-// (frameWorkCDEFAlignedPlane).
+// Pitch of a 4:2:0 chroma unit's 32 + 8 words; other chroma units are staged
+// where luma was, with its pitch.
+constexpr int kPC = 40;
+
+struct CdefSmem {
+  alignas(16) uint32_t y[kPH * kPW];
+  alignas(16) uint32_t c[2][36 * kPC];
+  alignas(16) int32_t cost[64 * 8];
+  alignas(16) CdefBlk blk[64];
+  int32_t var[64];
+  int2 ofs[2][12];  // direction tap offsets in words (cdef/filter.go:53-66), pitch kPW and kPC
+  uint8_t dir[64];
+};
+
+// Four samples of a row as they lie in memory.
 template <typename T>
-__device__ void cdef_unit(const DFrame& in, const DFrame& out, const CdefArgs& a, const int* aw, const int* ah,
-                          int uc, int ur, CdefSmem& sm) {
-  uint16_t* s_in = sm.in;
-  uint8_t* s_dir = sm.dir;
-  int32_t* s_var = sm.var;
-  int32_t* s_cost = sm.cost;
+struct Quad;
+template <>
+struct Quad<uint8_t> {
+  typedef uint32_t W;
+  static __device__ __forceinline__ W zero() { return 0; }
+  static __device__ __forceinline__ W load(const uint8_t* p, bool words) {
+    if (words) return *reinterpret_cast<const uint32_t*>(p);
+    return p[0] | (uint32_t)p[1] << 8 | (uint32_t)p[2] << 16 | (uint32_t)p[3] << 24;
+  }
+  // Column k's samples of two rows as a pair of plain integers.
+  template <int k>
+  static __device__ __forceinline__ uint32_t pair(W a, W b) {
+    return __byte_perm(a, b, 0x0400 + 0x0101 * k) & 0x00ff00ffu;
+  }
+  static __device__ __forceinline__ uint32_t over(W) { return 0; }
+};
+template <>
+struct Quad<uint16_t> {
+  typedef uint2 W;
+  static __device__ __forceinline__ W zero() { return make_uint2(0, 0); }
+  static __device__ __forceinline__ W load(const uint16_t* p, bool words) {
+    if (words) return *reinterpret_cast<const uint2*>(p);
+    return make_uint2(p[0] | (uint32_t)p[1] << 16, p[2] | (uint32_t)p[3] << 16);
+  }
+  template <int k>
+  static __device__ __forceinline__ uint32_t pair(W a, W b) {
+    return __byte_perm(k < 2 ? a.x : a.y, k < 2 ? b.x : b.y, k & 1 ? 0x7632 : 0x5410);
+  }
+  // Bits that a sample of 10 bits does not have.
+  static __device__ __forceinline__ uint32_t over(W a) { return (a.x | a.y) & 0xfc00fc00u; }
+};
+
+// One plane of a unit: where its samples are and what of them there is.
+struct CdefPlane {
+  const uint8_t* src;
+  int64_t stride;
+  int x, y, w, h;  // the unit in the plane
+  int Wa, Ha;      // the plane's MI-aligned extent
+  bool words;      // rows on 4-sample boundaries
+  bool inside;     // the whole halo is frame data
+};
+
+__device__ __forceinline__ CdefPlane cdef_plane(const DPlane& p, int bytes, int x, int y, int wmax, int hmax, int Wa,
+                                                int Ha) {
+  CdefPlane q;
+  q.src = p.ptr;
+  q.stride = p.stride;
+  q.x = x;
+  q.y = y;
+  q.w = imin(wmax, Wa - x);
+  q.h = imin(hmax, Ha - y);
+  q.Wa = Wa;
+  q.Ha = Ha;
+  q.words = ((reinterpret_cast<uintptr_t>(p.ptr) | (uintptr_t)p.stride) & (4 * bytes - 1)) == 0;
+  q.inside = x >= 4 && x + q.w + 4 <= Wa && y >= 2 && y + q.h + 3 <= Ha;
+  return q;
+}
+
+// Staging of a unit with its 2-row / 4-column halo as pair words
+// (frameWorkFillCDEFInputSentinels / frameWorkCopyCDEFInput; planes end on
+// 4-sample boundaries and the taps reach two samples, so the reference's row
+// and column replication past a plane's end is never read).  A task is four
+// columns (group cg, from the unit's column -4) of two word rows (2d,
+// 2d + 1): three 4-sample loads, eight words.  Loads and stores are apart so
+// that a thread's tasks are all in flight together.
+// kIn: the unit's whole halo is frame data in rows on 4-sample boundaries.
+template <typename T, bool kIn>
+__device__ __forceinline__ void stage_load(const CdefPlane& p, const uint8_t* src, int d, int cg,
+                                           typename Quad<T>::W (&v)[3]) {
+  const int x = p.x - 4 + 4 * cg, y = p.y - 2 + 2 * d;
+  const uint8_t* s = src + (int64_t)y * p.stride + (int64_t)x * (int)sizeof(T);
+  const bool cin = x >= 0 && x < p.Wa;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    if (!kIn) v[j] = Quad<T>::zero();
+    if (kIn || (cin && y + j >= 0 && y + j < p.Ha))
+      v[j] = Quad<T>::load(reinterpret_cast<const T*>(s + j * p.stride), kIn || p.words);
+  }
+}
+
+// kRaw: plain integers instead of biased fp16 values.
+template <typename T, bool kIn, bool kRaw, int kPitch>
+__device__ __forceinline__ void stage_store(const CdefPlane& p, int d, int cg, const typename Quad<T>::W (&v)[3],
+                                            uint32_t* buf) {
+  constexpr uint32_t kBias = kRaw ? 0u : kPairBias, kNone = kRaw ? kPairRawNone : kPairNone;
+  uint32_t* o = buf + 2 * d * kPitch + 4 * cg;
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    uint4 w = make_uint4(Quad<T>::template pair<0>(v[j], v[j + 1]) | kBias,
+                         Quad<T>::template pair<1>(v[j], v[j + 1]) | kBias,
+                         Quad<T>::template pair<2>(v[j], v[j + 1]) | kBias,
+                         Quad<T>::template pair<3>(v[j], v[j + 1]) | kBias);
+    if (!kIn) {
+      const int x = p.x - 4 + 4 * cg, y = p.y - 2 + 2 * d + j;
+      const bool cin = x >= 0 && x < p.Wa;
+      const uint32_t keep =
+          (cin && y >= 0 && y < p.Ha ? 0xffffu : 0u) | (cin && y + 1 >= 0 && y + 1 < p.Ha ? 0xffff0000u : 0u);
+      const uint32_t fill = kNone & ~keep;
+      w = make_uint4((w.x & keep) | fill, (w.y & keep) | fill, (w.z & keep) | fill, (w.w & keep) | fill);
+    }
+    *reinterpret_cast<uint4*>(o + j * kPitch) = w;
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ uint32_t stage_over(const typename Quad<T>::W (&v)[3]) {
+  return Quad<T>::over(v[0]) | Quad<T>::over(v[1]) | Quad<T>::over(v[2]);
+}
+
+// One plane's tasks one by one, any unit.
+template <typename T, bool kRaw, int kPitch>
+__device__ __forceinline__ uint32_t stage_any(const CdefPlane& p, const uint8_t* src, uint32_t* buf) {
+  const int cgs = (p.w + 8) >> 2;
+  const uint32_t inv = (65536u + (uint32_t)cgs - 1) / (uint32_t)cgs;  // i / cgs for i < 612
+  const int total = cgs * ((p.h + 4) >> 1);
+  uint32_t over = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < total; i += 256) {
+    typename Quad<T>::W t[3];
+    const int d = (int)((i * inv) >> 16), cg = i - d * cgs;
+    stage_load<T, false>(p, src, d, cg, t);
+    if (!kRaw) over |= stage_over<T>(t);
+    stage_store<T, false, kRaw, kPitch>(p, d, cg, t, buf);
+  }
+  return over;
+}
+
+// The three planes of a 4:2:0 unit.  Luma's 18 x 34 tasks fill two rounds of
+// the CTA and warps 0-3 of the third; 2 x (10 x 18) chroma tasks follow on
+// warps 4-7 and in a fourth.  All of a thread's loads are in flight together.
+// kIn: a whole 64x64 unit with its halo inside the frame.
+template <typename T, bool kIn>
+__device__ __forceinline__ uint32_t stage_420(const CdefPlane& P, const CdefPlane& Q, const uint8_t* vsrc, bool y,
+                                              bool c, CdefSmem& sm) {
   const int tid = threadIdx.x;
-  if (tid < 12) sm.ofs[tid] = make_int2(dir_off(tid, 0), dir_off(tid, 1));
-  const int coeffShift = sizeof(T) == 1 ? 0 : in.bd - 8;
+  const bool c2 = tid >= 128;  // the third round is chroma's
+  typename Quad<T>::W t[4][3];
+  int d[4], cg[4], i[4];
+  bool on[4];
+  uint32_t over = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const bool chroma = k == 3 || (k == 2 && c2);
+    i[k] = chroma ? (k == 2 ? tid - 128 : tid + 128) : tid + 256 * k;
+    const bool second = chroma && i[k] >= 180;
+    const int j = i[k] - (second ? 180 : 0);
+    d[k] = chroma ? j / 10 : j / 18;
+    cg[k] = j - (chroma ? 10 : 18) * d[k];
+    on[k] = i[k] < (chroma ? 360 : 612);
+    if (!kIn) {
+      const CdefPlane& p = chroma ? Q : P;
+      on[k] = on[k] && (chroma ? c : y) && 4 * cg[k] < p.w + 8 && 2 * d[k] < p.h + 4;
+    }
+    if (on[k]) {
+      if (chroma)
+        stage_load<T, kIn>(Q, second ? vsrc : Q.src, d[k], cg[k], t[k]);
+      else
+        stage_load<T, kIn>(P, P.src, d[k], cg[k], t[k]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (!on[k]) continue;
+    over |= stage_over<T>(t[k]);
+    if (k == 3 || (k == 2 && c2))
+      stage_store<T, kIn, false, kPC>(Q, d[k], cg[k], t[k], sm.c[i[k] >= 180]);
+    else
+      stage_store<T, kIn, false, kPW>(P, d[k], cg[k], t[k], sm.y);
+  }
+  return over;
+}
+
+// Filters a run of `rows` rows (whole blocks of kBh) of one column, two rows
+// at a time, so that a block's parameters are read once per block.  c: the
+// run's first word; o: its first output sample; blk(k): the run's k-th
+// block's parameters.
+template <typename T, bool kRaw, bool kPri, bool kSec, int kBh, class B>
+__device__ __forceinline__ void filter_run(const uint32_t* c, int pitch, const int2* ofs, uint8_t* o, int64_t os,
+                                           int rows, const PairTap& st, int sec, int secShift, int coeffShift, B blk) {
+#pragma unroll 1
+  for (int k = 0; k * kBh < rows; k++) {
+    const CdefBlk b = blk(k);
+    const int dir = b.flags & 7;
+    const bool filt = b.flags >> 31, odd = b.flags & 16;
+    const int2 po = ofs[dir + 2], s0 = ofs[dir + 4], s1 = ofs[dir];
+    const __half2 w0 = __float2half2_rn(odd ? 3.f : 4.f), w1 = __float2half2_rn(odd ? 3.f : 2.f);
+#pragma unroll 1
+    for (int y = 0; y < kBh; y += 2, c += 2 * pitch, o += 2 * os) {
+      uint32_t v = c[0];
+      if (filt) {
+        if (!kRaw) {
+          v = pair_filter<kPri, kSec>(c, b.pri, w0, w1, st, po, s0, s1);
+        } else {
+          const uint16_t* e = reinterpret_cast<const uint16_t*>(c);
+          const int2 p2 = make_int2(2 * po.x, 2 * po.y), q0 = make_int2(2 * s0.x, 2 * s0.y),
+                     q1 = make_int2(2 * s1.x, 2 * s1.y);
+          v = 0;
+#pragma unroll 1
+          for (int h = 1; h >= 0; h--)
+            v = v << 16 |
+                (cdef_filter_px(e + h, (int)b.pri.k, (int)b.pri.m, sec, secShift, p2, q0, q1, coeffShift) & 0xffff);
+        }
+      }
+      if (sizeof(T) == 2 && !kRaw) v &= 0x03ff03ffu;
+      *reinterpret_cast<T*>(o) = (T)v;
+      *reinterpret_cast<T*>(o + os) = (T)(v >> 16);
+    }
+  }
+}
+
+template <typename T, bool kRaw, int kBh, class B>
+__device__ __forceinline__ void filter_plane(const uint32_t* c, int pitch, const int2* ofs, uint8_t* o, int64_t os,
+                                             int rows, int pri, int sec, int damping, int coeffShift, B blk) {
+  const int secShift = constrain_shift(sec, damping);
+  const PairTap st = pair_tap(sec, secShift);
+  if (kRaw || (pri && sec))
+    filter_run<T, kRaw, true, true, kBh>(c, pitch, ofs, o, os, rows, st, sec, secShift, coeffShift, blk);
+  else if (pri)
+    filter_run<T, kRaw, true, false, kBh>(c, pitch, ofs, o, os, rows, st, sec, secShift, coeffShift, blk);
+  else
+    filter_run<T, kRaw, false, true, kBh>(c, pitch, ofs, o, os, rows, st, sec, secShift, coeffShift, blk);
+}
+
+// The four rows b-2 .. b+1 around the restoration stripe boundary
+// b = k*SH - off (k >= 1) that lies inside the unit (stripes are as high as
+// units, so a unit of row ur has the one of k = ur + 1), saved from the
+// pre-CDEF samples (tile/restoration_boundary.go:192-255): from the staged
+// words (`staged` points at the unit's first one) or, where the plane was not
+// staged, from the frame.  Thread `t` of a group saves sample t of the
+// 4 x (64 >> xdec).
+template <typename T>
+__device__ __forceinline__ void cdef_save_lines(const CdefArgs& a, const DPlane& ip, const CdefPlane& p, int plane,
+                                                int xdec, int ydec, int ur, const uint32_t* staged, int pitch,
+                                                uint32_t mask, int t) {
+  const int Hc = ip.h;
+  const int k = ur + 1, b = (k << (6 - ydec)) - (8 >> ydec);
+  const int j = t >> (6 - xdec), c = t & ((64 >> xdec) - 1);
+  const int y = b - 2 + j, x = p.x + c;
+  if (b < Hc && j < 4 && y < imin(p.y + p.h, Hc) && c < p.w && x < ip.w) {
+    const T v = staged ? (T)(staged[(y - p.y) * pitch + c] & mask) : row_ptr<T>(ip, y)[x];
+    uint8_t* line = a.lines[plane] + (int64_t)(k * 4 + j) * a.line_stride[plane];
+    reinterpret_cast<T*>(line)[x] = v;
+    if (j == 2 && b + 1 >= Hc) reinterpret_cast<T*>(line + a.line_stride[plane])[x] = v;
+  }
+}
+
+// One 64x64 filter unit (uc, ur) of all planes.  4:2:0 units (k420) stage the
+// three planes at once and go through the steps together: one wait for the
+// frame's samples and four barriers a unit, where plane after plane took
+// three waits and thirteen barriers, which is what a unit of few
+// instructions spends its time on.  Other layouts' chroma is as large as
+// luma or half of it and takes luma's place in shared memory, plane by
+// plane.  Starts at plane `plane` (0 for k420) and returns 3, or the plane it
+// stopped at, before writing it, because a 10-bit sample there has more than
+// 10 bits (kRaw off); the raw form takes over from that plane.
+template <typename T, bool kRaw, bool k420>
+__device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int plane, CdefSmem& sm) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const CdefArgs& a = J.cdef;
+  const int ssx = k420 ? 1 : J.io.ssx, ssy = k420 ? 1 : J.io.ssy;
+  const int coeffShift = sizeof(T) == 1 ? 0 : (kRaw ? J.io.bd - 8 : 2);
+  constexpr uint32_t kSample = kRaw ? 0xffffu : 0x3ffu;
+  if (tid < 24) sm.ofs[tid / 12][tid % 12] = make_int2(pair_off(tid % 12, 0, tid < 12 ? kPW : kPC),
+                                                       pair_off(tid % 12, 1, tid < 12 ? kPW : kPC));
+  // ---- what the unit filters, postfilter_cdef.go:936-956 ----
   // The index map is only present when CDEF filters; the copy-only pass (CDEF
   // off, loop restoration on) reads no side information.
-  const int mapOff = ur * a.index_stride + uc;
-  const bool rd = a.filter && a.read[mapOff] != 0;
-  const int idx = a.filter ? a.index[mapOff] : 0;
-  uint64_t word = ~0ull;
-  if (a.filter && a.noskip) {
-    const uint8_t* w = a.noskip + (size_t)(ur * a.ucols + uc) * 8;
-    word = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) word |= (uint64_t)w[i] << (8 * i);
-  }
-  const int nplanes = in.mono ? 1 : 3;
-  for (int plane = 0; plane < nplanes; plane++) {
-    const int xdec = plane ? in.ssx : 0, ydec = plane ? in.ssy : 0;
-    const int Wa = aw[plane], Ha = ah[plane];
-    const int unitX = (uc * 64) >> xdec, unitY = (ur * 64) >> ydec;
-    const int unitW = imin(64 >> xdec, Wa - unitX), unitH = imin(64 >> ydec, Ha - unitY);
-    if (unitW <= 0 || unitH <= 0) continue;
-    const DPlane& ip = in.pl[plane];
-    const DPlane& op = out.pl[plane];
-    // ---- activity of this (unit, plane), postfilter_cdef.go:936-956 ----
-    bool active = false, needPrimary = false, directionOnly = false;
-    int packed = 0;
-    if (a.filter && a.plane_process[plane] && rd && idx < a.strength_count) {
-      packed = plane == 0 ? a.y_strength[idx] : a.uv_strength[idx];
-      if (plane == 0)
-        needPrimary = (a.y_strength[idx] >> 2) != 0 || (a.chroma_filtering && (a.uv_strength[idx] >> 2) != 0);
-      else
-        needPrimary = (a.uv_strength[idx] >> 2) != 0;
-      directionOnly = plane == 0 && a.chroma_filtering && packed == 0 && (a.uv_strength[idx] >> 2) != 0;
-      active = packed != 0 || directionOnly;
-    }
-    const int bwLog2 = 3 - xdec, bhLog2 = 3 - ydec;
-    const int bcols = (unitW + (1 << bwLog2) - 1) >> bwLog2, brows = (unitH + (1 << bhLog2) - 1) >> bhLog2;
-    uint64_t listed = 0;
-    if (active) {
-      const uint64_t colMask = (1ull << bcols) - 1;
-      for (int by = 0; by < brows; by++) listed |= ((word >> (by * 8)) & colMask) << (by * 8);
-      if (listed == 0) active = false;
-    }
-    const int uwMax = 64 >> xdec;
-    const int rowStep = 256 / uwMax;
-    const int tx = tid % uwMax, ty0 = tid / uwMax;
-    if (!active) {
-      // Copy-through (inactive unit / plane or the CDEF stage is off).
-      copy_block<T>(ip, op, unitX, unitX + unitW, unitY, unitY + unitH);
-    } else {
-      // ---- stage the unit + halo (frameWorkFillCDEFInputSentinels /
-      //      frameWorkCopyCDEFInput with the replicate quirk) ----
-      const int srcX0 = imax(unitX - 8, 0), srcY0 = imax(unitY - 2, 0);
-      const int srcX1 = imin(unitX + unitW + 8, Wa), srcY1 = imin(unitY + unitH + 2, Ha);
-      const int wantY1 = unitY + unitH + 2, wantX1 = unitX + unitW + 8;
-      const bool rowExt = srcY1 < wantY1 && srcY1 > 0 && unitY + unitH < Ha;
-      const bool colExt = srcX1 < wantX1 && srcX1 > 0 && unitX + unitW < Wa;
-      const int extRowsEnd = srcY0 + (rowExt ? wantY1 - srcY0 : srcY1 - srcY0);
-      const int fillW = unitW + 16, fillH = unitH + 4;
-      const int warp = tid >> 5, lane = tid & 31;
-      const bool interior = srcX0 == unitX - 8 && srcX1 == wantX1 && srcY0 == unitY - 2 && srcY1 == wantY1;
-      const uint8_t* tile0 = reinterpret_cast<const uint8_t*>(row_ptr<T>(ip, unitY - 2) + (unitX - 8));
-      // Words of 8 samples: 8 bytes (8-bit, rows start 8 bytes before a
-      // 64-sample unit) or 16 bytes (10/12-bit).
-      constexpr int kWord = 8 * sizeof(T);
-      if (interior && fillW % 8 == 0 &&
-          ((reinterpret_cast<uintptr_t>(tile0) | (uintptr_t)ip.stride) & (kWord - 1)) == 0) {
-        // Interior unit with aligned rows: the whole halo is frame data, a
-        // thread's few words unrolled so their loads are in flight together.
-        const int wpr = fillW / 8, total = fillH * wpr;
-        constexpr int kMaxItems = (kSH * (kSW / 8) + 255) / 256;
-#pragma unroll
-        for (int k = 0; k < kMaxItems; k++) {
-          const int i = tid + 256 * k;
-          if (i < total) {
-            const int r = i / wpr, cw = i - r * wpr;
-            const uint8_t* src = tile0 + (int64_t)r * ip.stride + cw * kWord;
-            uint4 v;
-            if (sizeof(T) == 1) {
-              const uint2 w = *reinterpret_cast<const uint2*>(src);
-              v = make_uint4(__byte_perm(w.x, 0, 0x4140), __byte_perm(w.x, 0, 0x4342), __byte_perm(w.y, 0, 0x4140),
-                             __byte_perm(w.y, 0, 0x4342));
-            } else {
-              v = *reinterpret_cast<const uint4*>(src);
-            }
-            *reinterpret_cast<uint4*>(&s_in[r * kSW + cw * 8]) = v;
-          }
-        }
-      } else if (interior) {
-        // Interior unit: the whole halo is frame data.
-        for (int r = warp; r < fillH; r += 8) {
-          const T* src = row_ptr<T>(ip, unitY - 2 + r) + (unitX - 8);
-          uint16_t* dst = &s_in[r * kSW];
-          for (int c = lane; c < fillW; c += 32) dst[c] = src[c];
-        }
+  int ystr = 0, uvstr = 0;
+  uint64_t listed = 0;
+  if (a.filter) {
+    const int mapOff = ur * a.index_stride + uc;
+    const int rd = a.read[mapOff], idx = a.index[mapOff];
+    uint64_t word = ~0ull;
+    if (a.noskip) {
+      const uint8_t* w = a.noskip + (size_t)(ur * a.ucols + uc) * 8;
+      if ((reinterpret_cast<uintptr_t>(w) & 7) == 0) {
+        word = *reinterpret_cast<const uint64_t*>(w);
       } else {
-        for (int r = warp; r < fillH; r += 8) {
-          const int sy = unitY - 2 + r;
-          int ry = -1;
-          if (sy >= srcY0 && sy < srcY1) ry = sy;
-          else if (rowExt && sy >= srcY1 && sy < wantY1) ry = srcY1 - 1;
-          const bool extRow = colExt && sy >= srcY0 && sy < extRowsEnd;
-          const int ryExt = ry < 0 ? srcY1 - 1 : ry;
-          uint16_t* dst = &s_in[r * kSW];
-          for (int c = lane; c < fillW; c += 32) {
-            const int sx = unitX - 8 + c;
-            int v = kVeryLarge;
-            if (sx >= srcX0 && sx < srcX1) {
-              if (ry >= 0) v = row_ptr<T>(ip, ry)[sx];
-            } else if (extRow && sx >= srcX1 && sx < wantX1) {
-              v = row_ptr<T>(ip, ryExt)[srcX1 - 1];
-            }
-            dst[c] = (uint16_t)v;
-          }
-        }
+        word = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) word |= (uint64_t)w[i] << (8 * i);
       }
-      __syncthreads();
-      // ---- luma direction search on listed blocks (needPrimary) ----
-      if (plane == 0 && needPrimary) {
-        // A warp takes one direction for 32 blocks, so the direction's
-        // template runs without divergence.
-        for (int w = tid; w < 64 * 8; w += 256) {
-          const int d = w >> 6, b = w & 63;
-          const int by = b >> 3, bx = b & 7;
-          if ((listed >> b) & 1)
-            s_cost[b * 8 + d] = dir_cost_any(d, &s_in[(2 + by * 8) * kSW + 8 + bx * 8], coeffShift);
-        }
-        __syncthreads();
-        if (tid < 64 && ((listed >> tid) & 1)) {
-          int best = 0;
-          int32_t bestCost = s_cost[tid * 8];
-          for (int d = 1; d < 8; d++) {
-            const int32_t c = s_cost[tid * 8 + d];
-            if (c > bestCost) {
-              best = d;
-              bestCost = c;
-            }
-          }
-          s_dir[tid] = (uint8_t)best;
-          s_var[tid] = (bestCost - s_cost[tid * 8 + ((best + 4) & 7)]) >> 10;
-        }
-        __syncthreads();
-      }
-      if (plane == 1 && needPrimary && xdec != ydec) {
-        // cdef/filter.go:614-633: U converts the shared grid in place (V reuses it).
-        if (tid < 64 && ((listed >> tid) & 1)) {
-          const uint8_t conv422[8] = {7, 0, 2, 4, 5, 6, 6, 6};
-          const uint8_t conv440[8] = {1, 2, 2, 2, 3, 4, 6, 0};
-          s_dir[tid] = xdec ? conv422[s_dir[tid]] : conv440[s_dir[tid]];
-        }
-        __syncthreads();
-      }
-      // ---- filter ----
-      int lvl = packed >> 2, sec = packed & 3;
-      if (sec == 3) sec = 4;
-      const int pri = lvl << coeffShift;
-      sec <<= coeffShift;
-      int damping = a.damping + coeffShift;
-      if (plane != 0) damping--;
-      const bool lumaAdjust = plane == 0 && (needPrimary || pri != 0);
-      // Per-block parameters once (cdef/filter.go:490-543): adjusted luma
-      // strength, direction (0 when the primary strength is zero), shift.
-      // 8-bit units whose halo is all frame data: constrain() from tables.
-      const bool useTab = sizeof(T) == 1 && interior;
-      if (tid == 0) sm.strengths = 0;
-      __syncthreads();
-      if (tid < 64) {
-        const int b = tid;
-        int pk = 0;
-        if (!directionOnly && ((listed >> b) & 1)) {
-          const int strength = lumaAdjust ? adjust_strength(pri, s_var[b]) : pri;
-          const int dir = pri != 0 ? s_dir[b] : 0;
-          pk = (1 << 16) | (constrain_shift(strength, damping) << 12) | (strength << 4) | dir;
-          if (useTab && strength) atomicOr(&sm.strengths, 1u << strength);
-        }
-        sm.blk[b] = pk;
-      }
-      __syncthreads();
-      const int secShift = constrain_shift(sec, damping);
-      // The output row base in registers: the plane descriptor sits in the
-      // job table, which the compiler would re-read after every store.
-      uint8_t* const obase = op.ptr;
-      const int64_t ostride = op.stride;
-      if (useTab) {
-        const uint32_t used = sm.strengths;
-        const int ntab = __popc(used);
-        if (tid < 16) {
-          const bool on = (used >> tid) & 1;
-          const int k = __popc(used & ((1u << tid) - 1));
-          sm.slot[tid] = on ? (int8_t)k : (int8_t)-1;
-          if (on) sm.slot_str[k] = (int8_t)tid;
-        }
-        __syncthreads();
-        // Each table is a copy of the context's precomputed one for its
-        // strength and shift (64 16-byte words; zeros for no secondary).
-        for (int i = tid; i < (ntab + 1) * (kTabLen / 8); i += 256) {
-          const int t = i / (kTabLen / 8), wd = i - t * (kTabLen / 8);
-          const int st = t < ntab ? sm.slot_str[t] : sec;
-          const int sh = t < ntab ? constrain_shift(st, damping) : secShift;
-          uint4 v = make_uint4(0, 0, 0, 0);
-          if (st) v = reinterpret_cast<const uint4*>(a.ctab + (size_t)(st * 8 + sh) * kTabLen)[wd];
-          reinterpret_cast<uint4*>(&sm.tab[t < ntab ? t : kSecTab][0])[wd] = v;
-        }
-        __syncthreads();
-      }
-      if (tx < unitW) {
-        // A thread takes one column over a run of whole block rows (16 or
-        // 8 luma rows, 4 or 8 chroma rows), so each block's parameters
-        // (strength, direction taps, table) are read once per block, not
-        // once per sample; a warp still covers 32 adjacent columns of one
-        // row at a time.
-        const int rpt = (64 >> ydec) / rowStep;
-        const int ya = ty0 * rpt, yb = imin(unitH, ya + rpt);
-        const int bh = 1 << bhLog2;
-        for (int yblk = ya; yblk < yb; yblk += bh) {
-          const int b = ((yblk >> bhLog2) << 3) + (tx >> bwLog2);
-          const int pk = sm.blk[b];
-          const int yend = imin(yblk + bh, yb);
-          const int strength = (pk >> 4) & 255, dir = pk & 7;
-          const bool filt = (pk >> 16) && (strength | sec);
-          const int2 po = sm.ofs[dir + 2], s0 = sm.ofs[dir + 4], s1 = sm.ofs[dir];
-          const int16_t* tp = (useTab && strength) ? &sm.tab[sm.slot[strength]][255] : nullptr;
-          const int16_t* ts = &sm.tab[kSecTab][255];
-          const int priShift = (pk >> 12) & 15;
-          for (int y = yblk; y < yend; y++) {
-            const uint16_t* c = &s_in[(2 + y) * kSW + 8 + tx];
-            int v = c[0];
-            if (filt) {
-              if (useTab)
-                v = cdef_filter_px_tab(c, strength, tp, sec, ts, po, s0, s1);
-              else if (interior)  // no VeryLarge sentinel anywhere in the halo
-                v = cdef_filter_px<false>(c, strength, priShift, sec, secShift, po, s0, s1, coeffShift);
-              else
-                v = cdef_filter_px<true>(c, strength, priShift, sec, secShift, po, s0, s1, coeffShift);
-            }
-            reinterpret_cast<T*>(obase + (int64_t)(unitY + y) * ostride)[unitX + tx] = (T)v;
-          }
-        }
-      }
-      __syncthreads();
     }
-    // ---- fused loop-restoration boundary-line save (pre-CDEF rows) ----
-    // Rows b-2 .. b+1 around each stripe boundary b = k*SH - off (k >= 1)
-    // inside the unit; the rows of one boundary are spread over the CTA.
-    if (a.save_lines[plane]) {
-      const int Hc = ip.h, Wc = ip.w;
-      const int SHs = 64 >> ydec, off = 8 >> ydec;
-      const int yEnd = imin(unitY + unitH, Hc);
-      if (unitY < yEnd) {
-        const int k0 = imax((unitY + off + 2) / SHs, 1), k1 = (yEnd - 1 + off + 2) / SHs;
-        for (int k = k0; k <= k1; k++) {
-          const int b = k * SHs - off;
-          if (b >= Hc) break;
-          const int ya = imax(unitY, b - 2), yb = imin(yEnd - 1, b + 1);
-          // At most 4 rows of at most 64 samples: one sample per thread,
-          // from the staged unit when this plane was staged (the rows lie
-          // inside the unit, so they are frame samples there too).
-          const int r = tid >> (6 - xdec), c = tid & (uwMax - 1);
-          const int y = ya + r, x = unitX + c;
-          if (y <= yb && c < unitW && x < Wc) {
-            const int j = y - (b - 2);
-            const T v = active ? (T)s_in[(y - unitY + 2) * kSW + 8 + c] : row_ptr<T>(ip, y)[x];
-            reinterpret_cast<T*>(a.lines[plane] + (int64_t)(k * 4 + j) * a.line_stride[plane])[x] = v;
-            if (j == 2 && b + 1 >= Hc)
-              reinterpret_cast<T*>(a.lines[plane] + (int64_t)(k * 4 + 3) * a.line_stride[plane])[x] = v;
-          }
-        }
-      }
-      if (active) __syncthreads();  // the next plane restages s_in
+    if (rd && idx < a.strength_count) {
+      ystr = a.y_strength[idx];
+      uvstr = a.uv_strength[idx];
+      // The unit's 8x8 blocks inside the MI-aligned plane (the same in every plane).
+      const int bcols = imin(8, (J.aw[0] - uc * 64) >> 3), brows = imin(8, (J.ah[0] - ur * 64) >> 3);
+      const uint64_t cols = 0x0101010101010101ull * ((1u << bcols) - 1);
+      listed = word & cols & (brows == 8 ? ~0ull : (1ull << (8 * brows)) - 1);
     }
   }
+  const bool chromaPri = a.chroma_filtering && (uvstr >> 2) != 0;
+  const bool actY = listed && a.plane_process[0] && (ystr || chromaPri);
+  const bool actC = listed && a.plane_process[1] && uvstr;
+  const bool needDir = actY && ((ystr >> 2) || chromaPri);
+  const int nplanes = J.io.mono ? 1 : 3;
+  for (; plane < nplanes; plane += k420 ? 3 : 1) {
+    const int p1 = k420 ? nplanes : plane + 1;  // this pass: planes [plane, p1)
+    // ---- stage ----
+    uint32_t over = 0;
+    CdefPlane P, Q;  // luma (or the one plane of the pass); k420: chroma
+    const int xd = plane ? ssx : 0, yd = plane ? ssy : 0;
+    const bool actP = plane ? actC : actY;
+    P = cdef_plane(J.io.pl[plane], sizeof(T), (uc * 64) >> xd, (ur * 64) >> yd, 64 >> xd, 64 >> yd, J.aw[plane],
+                   J.ah[plane]);
+    if (P.w <= 0 || P.h <= 0) continue;
+    if (k420) {
+      Q = cdef_plane(J.io.pl[1], sizeof(T), uc * 32, ur * 32, 32, 32, J.aw[1], J.ah[1]);
+      const uint8_t* const vsrc = J.io.pl[2].ptr;
+      Q.words &= ((reinterpret_cast<uintptr_t>(vsrc) | (uintptr_t)J.io.pl[2].stride) & (4 * sizeof(T) - 1)) == 0;
+      Q.words &= J.io.pl[2].stride == Q.stride;
+      if (P.inside && P.words && Q.inside && Q.words && P.w == 64 && P.h == 64 && actY && actC) {
+        over = stage_420<T, true>(P, Q, vsrc, true, true, sm);
+      } else if (J.io.pl[2].stride == Q.stride) {
+        over = stage_420<T, false>(P, Q, vsrc, actY, actC, sm);
+      } else {
+        if (actY) over |= stage_any<T, kRaw, kPW>(P, P.src, sm.y);
+        if (actC) {
+          over |= stage_any<T, kRaw, kPC>(Q, Q.src, sm.c[0]);
+          CdefPlane V = Q;
+          V.stride = J.io.pl[2].stride;
+          over |= stage_any<T, kRaw, kPC>(V, vsrc, sm.c[1]);
+        }
+      }
+    } else if (actP) {
+      over = stage_any<T, kRaw, kPW>(P, P.src, sm.y);
+    }
+    if (sizeof(T) == 1 || kRaw)
+      __syncthreads();
+    else if (__syncthreads_or((int)(over != 0)))
+      return plane;
+    // ---- luma direction search on listed blocks ----
+    if (plane == 0 && needDir) {
+      // A pair of warps takes two directions of the 64 blocks, so a warp
+      // runs one code without divergence.
+      const int b = tid & 63;
+      if ((listed >> b) & 1)
+        dir_costs_vert(tid >> 6, &sm.y[(2 + (b >> 3) * 8) * kPW + kPX + (b & 7) * 8], kRaw ? coeffShift : (sizeof(T) == 1 ? 0 : 2),
+                       kRaw ? (0xffffu >> coeffShift) * 0x10001u : 0x00ff00ffu, &sm.cost[b * 8]);
+      __syncthreads();
+    }
+    // ---- block parameters (cdef/filter.go:490-543): the adjusted luma
+    // strength, the direction (0 when the primary strength is zero) ----
+    int ypri = ystr >> 2, ysec = ystr & 3, cpri = uvstr >> 2, csec = uvstr & 3;
+    ypri <<= coeffShift;
+    cpri <<= coeffShift;
+    ysec = (ysec + (ysec == 3)) << coeffShift;
+    csec = (csec + (csec == 3)) << coeffShift;
+    const int ydamp = a.damping + coeffShift, cdamp = ydamp - 1;
+    if (plane == 0 && actY && tid < 64 && ((listed >> tid) & 1)) {
+      int best = 0, var = 0;
+      if (needDir) {
+        const int4 c0 = *reinterpret_cast<const int4*>(&sm.cost[tid * 8]);
+        const int4 c1 = *reinterpret_cast<const int4*>(&sm.cost[tid * 8 + 4]);
+        const int32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        int32_t top = c[0], across = c[4];  // the best direction's cost and that across it
+#pragma unroll
+        for (int d = 1; d < 8; d++)
+          if (c[d] > top) {
+            best = d;
+            top = c[d];
+            across = c[(d + 4) & 7];
+          }
+        var = (top - across) >> 10;
+      }
+      sm.dir[tid] = (uint8_t)best;
+      // lumaAdjust holds whenever ypri is not zero: needDir does then.
+      const int strength = ypri ? adjust_strength(ypri, var) : 0;
+      const int shift = constrain_shift(strength, ydamp);
+      CdefBlk blk;
+      blk.pri = kRaw ? PairTap{(uint32_t)strength, (uint32_t)shift, 0} : pair_tap(strength, shift);
+      blk.flags = (strength | ysec ? 1u << 31 : 0u) | (((strength >> coeffShift) & 1) << 4) | (ypri ? best : 0);
+      sm.blk[tid] = blk;
+    } else if (!k420 && plane == 1 && actC && cpri && ssx != ssy && tid < 64 && ((listed >> tid) & 1)) {
+      // cdef/filter.go:614-633: U converts the shared grid in place (V reuses
+      // it): {7, 0, 2, 4, 5, 6, 6, 6} (4:2:2), {1, 2, 2, 2, 3, 4, 6, 0}
+      // (4:4:0), four bits an entry.
+      sm.dir[tid] = (uint8_t)(((ssx ? 0x66654207u : 0x06432221u) >> (4 * sm.dir[tid])) & 15);
+    }
+    __syncthreads();
+    // ---- filter ----
+    // The descriptors of the output in registers: they sit in the job table,
+    // which the compiler would re-read after every store.
+    if (plane == 0) {
+      if (actY && ystr) {
+        uint8_t* const ob = J.scr.pl[0].ptr;
+        const int64_t os = J.scr.pl[0].stride;
+        const int tx = tid & 63, ya = (tid >> 6) * 16, rows = imin(16, P.h - ya);
+        if (tx < P.w && rows > 0)
+          filter_plane<T, kRaw, 8>(&sm.y[(2 + ya) * kPW + kPX + tx], kPW, sm.ofs[0],
+                                   ob + (int64_t)(P.y + ya) * os + (int64_t)(P.x + tx) * (int)sizeof(T), os, rows, ypri,
+                                   ysec, ydamp, coeffShift, [&](int k) {
+                                     const int b = ((ya >> 3) + k) * 8 + (tx >> 3);
+                                     CdefBlk r = sm.blk[b];
+                                     if (!((listed >> b) & 1)) r.flags = 0;
+                                     return r;
+                                   });
+      } else {
+        copy_block<T>(J.io.pl[0], J.scr.pl[0], P.x, P.x + P.w, P.y, P.y + P.h);
+      }
+    }
+    if (k420 ? nplanes > 1 : plane > 0) {
+      const int cshift = constrain_shift(cpri, cdamp);
+      CdefBlk cb;
+      cb.pri = kRaw ? PairTap{(uint32_t)cpri, (uint32_t)cshift, 0} : pair_tap(cpri, cshift);
+      cb.flags = 1u << 31 | (((cpri >> coeffShift) & 1) << 4);
+      auto chroma_blk = [&](int b) {
+        CdefBlk r = cb;
+        r.flags = (listed >> b) & 1 ? cb.flags | (cpri ? sm.dir[b] : 0) : 0;
+        return r;
+      };
+      if (k420) {
+        // Warps 0-3 take U, 4-7 V: 32 columns by 8 rows (two blocks) each.
+        const int pl = 1 + (warp >> 2);
+        uint8_t* const ob = J.scr.pl[pl].ptr;
+        const int64_t os = J.scr.pl[pl].stride;
+        const int ya = (warp & 3) * 8, rows = imin(8, Q.h - ya);
+        if (!actC) {
+          copy_block<T>(J.io.pl[1], J.scr.pl[1], Q.x, Q.x + Q.w, Q.y, Q.y + Q.h);
+          copy_block<T>(J.io.pl[2], J.scr.pl[2], Q.x, Q.x + Q.w, Q.y, Q.y + Q.h);
+        } else if (lane < Q.w && rows > 0) {
+          filter_plane<T, kRaw, 4>(&sm.c[pl - 1][(2 + ya) * kPC + kPX + lane], kPC, sm.ofs[1],
+                                   ob + (int64_t)(Q.y + ya) * os + (int64_t)(Q.x + lane) * (int)sizeof(T), os, rows,
+                                   cpri, csec, cdamp, coeffShift,
+                                   [&](int k) { return chroma_blk(((ya >> 2) + k) * 8 + (lane >> 2)); });
+        }
+      } else if (!actC) {
+        copy_block<T>(J.io.pl[plane], J.scr.pl[plane], P.x, P.x + P.w, P.y, P.y + P.h);
+      } else {
+        uint8_t* const ob = J.scr.pl[plane].ptr;
+        const int64_t os = J.scr.pl[plane].stride;
+        const int lw = 6 - ssx, tx = tid & ((1 << lw) - 1), rpt = (64 >> ssy) >> (8 - lw);
+        const int ya = (tid >> lw) * rpt, rows = imin(rpt, P.h - ya);
+        const uint32_t* c = &sm.y[(2 + ya) * kPW + kPX + tx];
+        uint8_t* o = ob + (int64_t)(P.y + ya) * os + (int64_t)(P.x + tx) * (int)sizeof(T);
+        if (tx < P.w && rows > 0) {
+          auto at = [&](int k) { return chroma_blk(((ya >> (3 - ssy)) + k) * 8 + (tx >> (3 - ssx))); };
+          if (ssy)
+            filter_plane<T, kRaw, 4>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, coeffShift, at);
+          else
+            filter_plane<T, kRaw, 8>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, coeffShift, at);
+        }
+      }
+    }
+    // ---- fused loop-restoration boundary-line save ----
+    if (k420) {
+      if (a.save_lines[0])
+        cdef_save_lines<T>(a, J.io.pl[0], P, 0, 0, 0, ur, actY ? &sm.y[2 * kPW + kPX] : nullptr, kPW, kSample, tid);
+      if (nplanes > 1) {
+        const int pl = 1 + (tid >> 7);
+        if (a.save_lines[pl])
+          cdef_save_lines<T>(a, J.io.pl[pl], Q, pl, 1, 1, ur, actC ? &sm.c[pl - 1][2 * kPC + kPX] : nullptr, kPC, kSample,
+                             tid & 127);
+      }
+    } else if (a.save_lines[plane]) {
+      cdef_save_lines<T>(a, J.io.pl[plane], P, plane, xd, yd, ur, actP ? &sm.y[2 * kPW + kPX] : nullptr, kPW, kSample, tid);
+    }
+    if (p1 < nplanes) __syncthreads();  // the next plane restages sm.y
+  }
+  return 3;
+}
+
+// The unit from plane `plane` on, with samples staged as integers: 12-bit
+// frames, and 10-bit ones that hold longer samples.
+__device__ __noinline__ void cdef_unit_raw(const FrameJob* J, int uc, int ur, int plane, CdefSmem* sm) {
+  cdef_unit<uint16_t, true, false>(*J, uc, ur, plane, *sm);
+}
+
+// 4:2:2, 4:4:4 and 4:4:0.
+template <typename T>
+__device__ __noinline__ int cdef_unit_planes(const FrameJob* J, int uc, int ur, CdefSmem* sm) {
+  return cdef_unit<T, false, false>(*J, uc, ur, 0, *sm);
 }
 
 // Batched CDEF: each work item is one 64x64 unit of one frame.
@@ -334,10 +542,19 @@ __global__ void __launch_bounds__(256, 4) k_cdef_batch(BatchArgs b) {
         const FrameJob& J = b.jobs[fi];
         const int local = item - base[fi];
         const int uc = local % J.cdef.ucols, ur = local / J.cdef.ucols;
-        if (J.io.bd == 8)
-          cdef_unit<uint8_t>(J.io, J.scr, J.cdef, J.aw, J.ah, uc, ur, sm);
-        else
-          cdef_unit<uint16_t>(J.io, J.scr, J.cdef, J.aw, J.ah, uc, ur, sm);
+        const bool c420 = J.io.ssx && J.io.ssy;
+        if (J.io.bd == 8) {
+          if (c420)
+            cdef_unit<uint8_t, false, true>(J, uc, ur, 0, sm);
+          else
+            cdef_unit_planes<uint8_t>(&J, uc, ur, &sm);
+        } else {
+          int from = 0;
+          if (J.io.bd == 10)
+            from = c420 ? cdef_unit<uint16_t, false, true>(J, uc, ur, 0, sm)
+                        : cdef_unit_planes<uint16_t>(&J, uc, ur, &sm);
+          if (from < 3) cdef_unit_raw(&J, uc, ur, from, &sm);
+        }
       },
       [&](int item) {
         // Every plane's unit with its 8-column / 2-row halo.
@@ -358,6 +575,8 @@ __global__ void __launch_bounds__(256, 4) k_cdef_batch(BatchArgs b) {
 
 // The constrain() tables of CdefArgs.ctab, from constrain() itself: one
 // CTA per (strength, shift).
+constexpr int kTabLen = 512;
+
 __global__ void __launch_bounds__(kTabLen) k_cdef_tables(int16_t* t) {
   const int st = blockIdx.x >> 3, sh = blockIdx.x & 7, i = threadIdx.x;
   t[(size_t)blockIdx.x * kTabLen + i] = (int16_t)(i < 511 ? constrain(i - 255, st, sh) : 0);

@@ -4,6 +4,8 @@
 // cdef/filter.go:79-191, :603-612.
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "pf_common.cuh"
 
 namespace pf {
@@ -11,6 +13,110 @@ namespace pf {
 constexpr int kVeryLarge = 0x4000;
 constexpr int kSW = 80;   // smem row stride (64 + 2*8)
 constexpr int kSH = 68;   // smem rows (64 + 2*2)
+
+// ---- CDEF on vertical sample pairs ----
+//
+// A staged unit is an array of 32-bit words: word (r, c) holds the samples of
+// rows r and r + 1 of column c, so every tap of two vertically adjacent
+// samples is one aligned word whatever its offset, and both are filtered by
+// the same packed instructions.  A sample n of 8 or 10 bits is held as the
+// fp16 value 1 + n / 1024 (bits 0x3c00 | n), an absent one as -3 (kPairNone):
+// below every sample in a signed 16-bit maximum, above every one in an
+// unsigned minimum, and too far from any for a tap to count, so it drops out
+// of the filter by itself.  Everything the filter forms from samples is a
+// whole or half multiple of 2^-10 below 2^11 of them, which fp16 holds
+// exactly: the result is the same integer as the reference's
+// (tests/test_cdef_pair_arithmetic.py runs through every difference,
+// strength and shift).  12-bit samples do not fit: they are staged as plain
+// integers (absent: kVeryLarge) and filtered one by one.
+constexpr int kPH = 68;  // rows -2 .. 65 of a unit
+constexpr int kPX = 4;   // words left of the unit's first column
+constexpr int kPW = 96;  // words a row: a multiple of the 32 banks, so a tap's row offset moves no lane's bank
+constexpr uint32_t kPairBias = 0x3c003c00u;
+constexpr uint32_t kPairNone = 0xc200c200u;
+constexpr uint32_t kPairRawNone = 0x40004000u;
+
+__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+
+// constrain() of one threshold and shift on pairs (cdef/filter.go:603-612):
+// min(|d|, max(0, thr - (|d| >> shift))) with d's sign.
+// thr - floor(|d| / 2^shift) is the fp16 rounding of
+//   1 + (thr - (|d| + 1/2 - 2^(shift-1)) / 2^shift) / 1024,
+// whose last place in [1, 2) is 2^-10: the sum is at least 2^-(shift+1) off
+// every tie, and below 1 only where the threshold has run out, which the
+// saturating subtraction turns into 0.
+struct PairTap {
+  uint32_t k, m, o;  // 1 + thr / 1024; -2^-shift; (1/2 - 2^(shift-1)) / 1024, each in both halves
+};
+
+// The constants from their bits: 1 + thr / 1024 is 0x3c00 + thr, -2^-shift has
+// the exponent 15 - shift, and 2^(shift-1) - 1/2 is shift ones in binary
+// (thr at most 1023, shift at most 8).
+__host__ __device__ __forceinline__ PairTap pair_tap(int thr, int shift) {
+  const uint32_t m = 0xbc00u - ((uint32_t)shift << 10);
+  const uint32_t o = shift ? 0x8000u + (((uint32_t)shift + 3) << 10) + 1024u - (2048u >> shift) : 0u;
+  return PairTap{kPairBias + (uint32_t)thr * 0x10001u, m * 0x10001u, o * 0x10001u};
+}
+
+__device__ __forceinline__ __half2 pair_constrain(__half2 d, const PairTap& t) {
+  const __half2 a = __habs2(d);
+  const __half2 v = __hfma2(__hadd2(a, bits_h2(t.o)), bits_h2(t.m), bits_h2(t.k));
+  const __half2 c = __hmin2(__hadd2_sat(v, __float2half2_rn(-1.f)), a);
+  return bits_h2(h2_bits(c) | (h2_bits(d) & 0x80008000u));
+}
+
+// x + (8 + sum - (sum < 0) >> 4): sum / 16 rounded half away from zero, by
+// moving the sum half a step away from zero and letting the addition to the
+// sample (last place 2^-10 in [1, 2)) round.  A value below sample 0 or above
+// 1023 is not a whole one; the clamp that follows takes it to the range.
+__device__ __forceinline__ __half2 pair_round(__half2 x, __half2 sum) {
+  const __half2 h = bits_h2((h2_bits(sum) & 0x80008000u) | 0x10001000u);  // +-1/2048
+  return __hfma2(__hadd2(sum, h), __float2half2_rn(0.0625f), x);
+}
+
+// One pair through the filter (cdef/filter.go:79-169); c points at its word.
+// po: the primary taps' word offsets (entry dir + 2), s0 / s1 the secondary
+// ones' (dir + 4, dir).  w0, w1: the primary weights (4, 2 or 3, 3).  The
+// clamp applies with both filters on; where a block's own primary strength is
+// zero it changes nothing (the secondary taps alone stay inside their own
+// range), so it needs no per-block test.
+template <bool kPri, bool kSec>
+__device__ __forceinline__ uint32_t pair_filter(const uint32_t* c, const PairTap& pri, __half2 w0, __half2 w1,
+                                                const PairTap& sec, int2 po, int2 s0, int2 s1) {
+  const uint32_t xb = c[0];
+  const __half2 x = bits_h2(xb);
+  uint32_t hi = xb, lo = xb;
+  auto range = [&](uint32_t a, uint32_t b) {
+    if (kPri && kSec) {
+      lo = __vimin3_u16x2(lo, a, b);
+      hi = __vimax3_s16x2(hi, a, b);
+    }
+  };
+  auto tap = [&](uint32_t a, const PairTap& t) { return pair_constrain(__hsub2(bits_h2(a), x), t); };
+  __half2 sum = __float2half2_rn(0.f);
+  if (kPri) {
+    const uint32_t a0 = c[po.x], a1 = c[-po.x], a2 = c[po.y], a3 = c[-po.y];
+    sum = __hmul2(w0, __hadd2(tap(a0, pri), tap(a1, pri)));
+    sum = __hfma2(w1, __hadd2(tap(a2, pri), tap(a3, pri)), sum);
+    range(a0, a1);
+    range(a2, a3);
+  }
+  if (kSec) {
+    const uint32_t b0 = c[s0.x], b1 = c[-s0.x], b2 = c[s1.x], b3 = c[-s1.x];
+    const __half2 n = __hadd2(__hadd2(tap(b0, sec), tap(b1, sec)), __hadd2(tap(b2, sec), tap(b3, sec)));
+    range(b0, b1);
+    range(b2, b3);
+    const uint32_t b4 = c[s0.y], b5 = c[-s0.y], b6 = c[s1.y], b7 = c[-s1.y];
+    const __half2 f = __hadd2(__hadd2(tap(b4, sec), tap(b5, sec)), __hadd2(tap(b6, sec), tap(b7, sec)));
+    range(b4, b5);
+    range(b6, b7);
+    sum = __hadd2(sum, __hfma2(n, __float2half2_rn(2.f), f));
+  }
+  uint32_t y = h2_bits(pair_round(x, sum));
+  if (kPri && kSec) y = __vminu2(__vmaxu2(y, lo), hi);
+  return y;
+}
 
 // (dy, dx) of the two taps of each CDEF direction entry, cdef/filter.go:53-66.
 static __constant__ int8_t c_cdef_dir[12][2][2] = {
@@ -20,6 +126,7 @@ static __constant__ int8_t c_cdef_dir[12][2][2] = {
 };
 
 __device__ __forceinline__ int dir_off(int e, int k) { return c_cdef_dir[e][k][0] * kSW + c_cdef_dir[e][k][1]; }
+__device__ __forceinline__ int pair_off(int e, int k, int pitch) { return c_cdef_dir[e][k][0] * pitch + c_cdef_dir[e][k][1]; }
 
 // Direction cost over one 8x8 block (cdef/direction.go:37-79 partial sums,
 // :469-501 cost): for direction D the samples (i, j), shifted to 8 bits
@@ -38,7 +145,7 @@ __host__ __device__ constexpr int dir_count(int D, int k) {
 }
 
 // The direction cost on packed sample pairs: w[i][m] holds samples (i, 2m) and
-// (i, 2m + 1) of the block in its low and high halves, raw.  Each pair is
+// (i, 2m + 1) of the block in its low and high halves, shifted to 8 bits.  Each pair is
 // added as one 32-bit word into the accumulator of its even sample's index
 // (the odd sample's index differs from it by the same -1, 0 or +1 for every
 // pair of a direction), with the samples shifted to 8 bits and left biased
@@ -48,16 +155,15 @@ __host__ __device__ constexpr int dir_count(int D, int k) {
 // them (direction.go:469-501), so the result is the same integer as summing
 // the shifted, unbiased samples one by one.
 template <int D>
-__host__ __device__ __forceinline__ int32_t dir_cost_pairs(const uint32_t (&w)[8][4], int shift) {
+__host__ __device__ __forceinline__ int32_t dir_cost_pairs(const uint32_t (&w)[8][4]) {
   constexpr int kDelta = dir_k(D, 0, 1) - dir_k(D, 0, 0);
-  const uint32_t mask = (0xffffu >> shift) * 0x10001u;
   uint32_t acc[15];
 #pragma unroll
   for (int k = 0; k < 15; k++) acc[k] = 0;
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int m = 0; m < 4; m++) acc[dir_k(D, i, 2 * m)] += (w[i][m] >> shift) & mask;
+    for (int m = 0; m < 4; m++) acc[dir_k(D, i, 2 * m)] += w[i][m];
   int32_t p[15];
 #pragma unroll
   for (int k = 0; k < 15; k++) {
@@ -83,27 +189,40 @@ __host__ __device__ __forceinline__ int32_t dir_cost_pairs(const uint32_t (&w)[8
          (p[2] * p[2] + p[8] * p[8]) * 140;
 }
 
-template <int D>
-__device__ __forceinline__ int32_t dir_cost_packed(const uint16_t* blk, int shift) {
+// Two of the eight direction costs of a block staged as vertical pairs (blk:
+// its first word), for group g of 0..3, into cost[0..7]: the block is read
+// and masked once for both, and a light direction goes with a heavy one.  The
+// words (2m, i) are the pairs (i, 2m), (i, 2m + 1) of the transposed block,
+// and transposing a block turns direction D's lines into those of
+// (8 - D) & 7 (dir_k(D, i, j) = dir_k((8 - D) & 7, j, i), for D = 4 read
+// backwards, which its symmetric weights do not see).  mask: the sample bits
+// that remain after the shift to 8 bits.
+__device__ __forceinline__ void dir_costs_vert(int g, const uint32_t* blk, int shift, uint32_t mask, int32_t* cost) {
   uint32_t w[8][4];
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint4 row = *reinterpret_cast<const uint4*>(blk + i * kSW);
-    w[i][0] = row.x, w[i][1] = row.y, w[i][2] = row.z, w[i][3] = row.w;
-  }
-  return dir_cost_pairs<D>(w, shift);
-}
-
-__device__ __forceinline__ int32_t dir_cost_any(int d, const uint16_t* blk, int shift) {
-  switch (d) {
-    case 0: return dir_cost_packed<0>(blk, shift);
-    case 1: return dir_cost_packed<1>(blk, shift);
-    case 2: return dir_cost_packed<2>(blk, shift);
-    case 3: return dir_cost_packed<3>(blk, shift);
-    case 4: return dir_cost_packed<4>(blk, shift);
-    case 5: return dir_cost_packed<5>(blk, shift);
-    case 6: return dir_cost_packed<6>(blk, shift);
-    default: return dir_cost_packed<7>(blk, shift);
+  for (int m = 0; m < 4; m++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint4 q = *reinterpret_cast<const uint4*>(blk + 2 * m * kPW + 4 * h);
+      w[4 * h][m] = (q.x >> shift) & mask, w[4 * h + 1][m] = (q.y >> shift) & mask;
+      w[4 * h + 2][m] = (q.z >> shift) & mask, w[4 * h + 3][m] = (q.w >> shift) & mask;
+    }
+  switch (g) {
+    case 0:
+      cost[0] = dir_cost_pairs<0>(w);
+      cost[2] = dir_cost_pairs<6>(w);
+      break;
+    case 1:
+      cost[4] = dir_cost_pairs<4>(w);
+      cost[6] = dir_cost_pairs<2>(w);
+      break;
+    case 2:
+      cost[1] = dir_cost_pairs<7>(w);
+      cost[3] = dir_cost_pairs<5>(w);
+      break;
+    default:
+      cost[5] = dir_cost_pairs<3>(w);
+      cost[7] = dir_cost_pairs<1>(w);
   }
 }
 
@@ -160,40 +279,6 @@ __device__ __forceinline__ int cdef_filter_px(const uint16_t* c, int pri, int pr
       const int m = kMask ? kVeryLarge - 1 : 0xffff;
       hi = __vimax3_s32(__vimax3_s32(hi, b0 & m, b1 & m), __vimax3_s32(b2 & m, b3 & m, b4 & m),
                         __vimax3_s32(b5 & m, b6 & m, b7 & m));
-      lo = __vimin3_s32(__vimin3_s32(lo, b0, b1), __vimin3_s32(b2, b3, b4), __vimin3_s32(b5, b6, b7));
-    }
-  }
-  int y = x + ((8 + sum - (sum < 0)) >> 4);
-  if (pri && sec) y = imin(imax(y, lo), hi);
-  return y;
-}
-
-// cdef_filter_px for 8-bit input without sentinels, with constrain() read
-// from tables: tp (primary, the block's strength) and ts (secondary) point at
-// the entry for a difference of 0 of 511-entry tables covering -255..255,
-// built from constrain() itself, so the result is the same sample.
-__device__ __forceinline__ int cdef_filter_px_tab(const uint16_t* c, int pri, const int16_t* tp, int sec,
-                                                  const int16_t* ts, int2 po, int2 s0, int2 s1) {
-  const int x = c[0];
-  int sum = 0;
-  int hi = x, lo = x;
-  if (pri) {
-    const int odd = pri & 1;
-    const int t0 = odd ? 3 : 4, t1 = odd ? 3 : 2;
-    const int a0 = c[po.x], a1 = c[-po.x], a2 = c[po.y], a3 = c[-po.y];
-    sum += t0 * (tp[a0 - x] + tp[a1 - x]) + t1 * (tp[a2 - x] + tp[a3 - x]);
-    if (sec) {
-      hi = __vimax3_s32(__vimax3_s32(hi, a0, a1), a2, a3);
-      lo = __vimin3_s32(__vimin3_s32(lo, a0, a1), a2, a3);
-    }
-  }
-  if (sec) {
-    const int b0 = c[s0.x], b1 = c[-s0.x], b2 = c[s1.x], b3 = c[-s1.x];
-    const int b4 = c[s0.y], b5 = c[-s0.y], b6 = c[s1.y], b7 = c[-s1.y];
-    sum += 2 * (ts[b0 - x] + ts[b1 - x] + ts[b2 - x] + ts[b3 - x]) + ts[b4 - x] + ts[b5 - x] + ts[b6 - x] +
-           ts[b7 - x];
-    if (pri) {
-      hi = __vimax3_s32(__vimax3_s32(hi, b0, b1), __vimax3_s32(b2, b3, b4), __vimax3_s32(b5, b6, b7));
       lo = __vimin3_s32(__vimin3_s32(lo, b0, b1), __vimin3_s32(b2, b3, b4), __vimin3_s32(b5, b6, b7));
     }
   }

@@ -122,7 +122,7 @@ __device__ __forceinline__ int32_t dir_cost8(const uint8_t* blk, int64_t stride)
 #pragma unroll
       for (int m = 0; m < 4; m++) w[i][m] = blk[i * stride + 2 * m] | ((uint32_t)blk[i * stride + 2 * m + 1] << 16);
   }
-  return dir_cost_pairs<D>(w, 0);
+  return dir_cost_pairs<D>(w);
 }
 
 __device__ __forceinline__ int32_t dir_cost8_dev(int d, const uint8_t* blk, int64_t stride) {
