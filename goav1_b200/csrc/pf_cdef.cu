@@ -573,22 +573,6 @@ __global__ void __launch_bounds__(256, 4) k_cdef_batch(BatchArgs b) {
       });
 }
 
-// The constrain() tables of CdefArgs.ctab, from constrain() itself: one
-// CTA per (strength, shift).
-constexpr int kTabLen = 512;
-
-__global__ void __launch_bounds__(kTabLen) k_cdef_tables(int16_t* t) {
-  const int st = blockIdx.x >> 3, sh = blockIdx.x & 7, i = threadIdx.x;
-  t[(size_t)blockIdx.x * kTabLen + i] = (int16_t)(i < 511 ? constrain(i - 255, st, sh) : 0);
-}
-
-size_t cdef_tables_bytes() { return (size_t)16 * 8 * kTabLen * sizeof(int16_t); }
-
-cudaError_t launch_cdef_tables(int16_t* dst, cudaStream_t st) {
-  k_cdef_tables<<<16 * 8, kTabLen, 0, st>>>(dst);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_cdef_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
   if (total <= 0) return cudaSuccess;
   static int wave = 0;

@@ -8,16 +8,13 @@
 // back).  Trial indices past the list hold kNotATrial, which no selection
 // step picks, so the selection over all 64 indices equals finish's over the
 // list (:892-899: endGI = len(filterMap)):
-//   k_cdef_search   one CTA per 64x64 filter block: the noskip 8x8 list
-//                   (computeCDEFList, :410-447), the VeryLarge-padded input
-//                   (loadCDEFInput, :479-506), luma directions from the
-//                   reconstruction, then for each tested trial the SSE of
-//                   the filtered block against the source (searchRow,
-//                   :649-745; FilterBlocksU8SubsampledTrusted with row step 1,
-//                   cdef/filter_search.go:20-74).  The work is split into
-//                   (trial, 8-row group) tasks spread over the warps, so a
-//                   block that tests few trials (the learned search) still
-//                   keeps every warp busy.  An untested trial gets the
+//   k_cdef_search   a cluster of three CTAs per 64x64 filter block: the noskip
+//                   8x8 list (computeCDEFList, :410-447), the VeryLarge-padded
+//                   input (loadCDEFInput, :479-506), luma directions from the
+//                   reconstruction, then for each tested trial the SSE of the
+//                   filtered block against the source (searchRow, :649-745;
+//                   FilterBlocksU8SubsampledTrusted with row step 1,
+//                   cdef/filter_search.go:20-74).  An untested trial gets the
 //                   reference's untested-chroma figure (cdefDefaultMSEUV*64,
 //                   :669-672) in both planes.
 //   k_sel_greedy    finish (:886-945): jointStrengthSearchDual /
@@ -41,246 +38,393 @@ namespace cg = cooperative_groups;
 
 namespace pf {
 
-constexpr int kLearnedSlices = 4;
-constexpr int kTrialsPerSlice = 16;
+// ---- the trial search ----
+//
+// One cluster of three CTAs per 64x64 filter block: rank 0 the block's upper
+// 32 luma rows, rank 1 the lower ones, rank 2 both chroma planes, which is
+// the same number of samples each.  A warp takes 32 columns by 8 rows: a lane
+// has one column as four pair words (pf_cdef_dev.cuh).
+//
+// What a trial's filter adds to a sample is the sum of a part that depends
+// only on the primary strength (4 taps) and one that depends only on the
+// secondary strength (8 taps), and the clamp range depends on neither.  So
+// the 64 trials of a block need 15 primary sums and 3 secondary ones (and 3
+// more with the direction that a zero primary strength implies) a sample, 108
+// taps instead of 64 x 12, and the rest of a trial is one addition, the
+// rounding, the clamp and the squared error of four samples at a time.
+// Bound by the packed instructions themselves.  1080p: all 64 luma and 64
+// chroma trials 113 us, trial by trial with constrain() tables about 1,500;
+// the learned search's few trials a block 54 us, then 178.
+//
+// What a sample does not count for is settled once, before the trials: an
+// unlisted block's, a skipped row's (subsampled search) has its clamp range,
+// source and reconstruction set to the sample itself, so that every trial's
+// error there is 0; one below or right of the crop, which the reference
+// stages as VeryLarge and whose filtered 8-bit value is 0
+// (cdef/filter_u8.go:151), has the range {-3}, whose low byte is 0.
 
-__global__ void __launch_bounds__(256) k_cdef_search(SearchArgs a) {
-  __shared__ uint16_t s_in[kSH * kSW];
-  __shared__ __align__(16) uint8_t s_src[64 * 64];
-  __shared__ __align__(16) uint8_t s_rec[64 * 64];  // the reconstruction itself (unfiltered trials measure it)
-  __shared__ int32_t s_cost[64 * 8];
-  __shared__ uint8_t s_dir[64];
-  __shared__ int8_t s_ai[64];   // adjustStrength index, -1 for zero variance
-  __shared__ int2 s_ofs[12];
-  __shared__ uint32_t s_sse[2][64];  // luma; U+V
-  __shared__ uint8_t s_list[2][64];  // tested trials, ascending
-  __shared__ int s_cnt[2];
-  // constrain() of the plane's damping: primary strength k at row k (0..15),
-  // secondary strengths 1, 2, 4 at rows 16..18; entry kTab0 is a difference
-  // of 0, entries kTab0 -/+ 256 stand for every difference beyond +/-255
-  // (both 0).  A row is a copy of the context's table for its strength and
-  // shift, two entries in, so its 32-bit words stay aligned.
-  constexpr int kTabStride = 520, kTab0 = 257;
-  __shared__ __align__(16) int16_t s_tab[19][kTabStride];
+constexpr int kSrchTab = 14;  // entries of a luma primary strength: zero variance, adjust index 0..12
+
+struct SearchSmem {
+  alignas(16) uint32_t w[36 * kPW];  // 36 rows of half a luma unit, or two chroma units (pitch kSrchPC)
+  alignas(16) uint4 pri[16 * kSrchTab];  // PairTap; bit 0 odd strength, bit 1 zero strength
+  alignas(16) uint4 sec[3];
+  alignas(16) int32_t cost[64 * 8];
+  uint32_t tested[2];  // strengths that some tested trial has (bit: packed strength)
+  uint32_t sse[64];    // by packed strength
+  int2 ofs[12];
+  uint8_t dir[64];
+  int8_t ai[64];  // adjustStrength index, -1 for zero variance
+};
+constexpr int kSrchPC = 40;
+static_assert(2 * 36 * kSrchPC <= 36 * kPW, "chroma units fit the luma buffer");
+
+// Stages pair words (four columns from x, two word rows from y) of a plane:
+// frame samples inside the crop, absent ones outside it (loadCDEFInput,
+// cdef_search.go:479-506).
+__device__ __forceinline__ void search_stage(const DPlane& p, bool inside, int x, int y, uint32_t* o, int pitch) {
+  uint32_t v[3], ok[3];
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const uint8_t* r = p.ptr + (int64_t)(y + j) * p.stride + x;
+    if (inside) {
+      v[j] = *reinterpret_cast<const uint32_t*>(r);
+    } else {
+      v[j] = 0;
+      ok[j] = 0;
+      if (y + j >= 0 && y + j < p.h)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (x + k >= 0 && x + k < p.w) {
+            v[j] |= (uint32_t)r[k] << (8 * k);
+            ok[j] |= 1u << k;
+          }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      w[k] = (__byte_perm(v[j], v[j + 1], 0x0400 + 0x0101 * k) & 0x00ff00ffu) | kPairBias;
+      if (!inside) {
+        const uint32_t keep = ((ok[j] >> k) & 1 ? 0xffffu : 0u) | ((ok[j + 1] >> k) & 1 ? 0xffff0000u : 0u);
+        w[k] = (w[k] & keep) | (kPairNone & ~keep);
+      }
+    }
+    *reinterpret_cast<uint4*>(o + j * pitch) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// The secondary sum of one pair at one strength from its eight differences
+// (0..3: weight 2, 4..7: weight 1).
+__device__ __forceinline__ __half2 search_sec(const __half2 (&d)[8], const uint4& c) {
+  const PairTap t{c.x, c.y, c.z};
+  const __half2 n = __hadd2(__hadd2(pair_constrain(d[0], t), pair_constrain(d[1], t)),
+                            __hadd2(pair_constrain(d[2], t), pair_constrain(d[3], t)));
+  const __half2 f = __hadd2(__hadd2(pair_constrain(d[4], t), pair_constrain(d[5], t)),
+                            __hadd2(pair_constrain(d[6], t), pair_constrain(d[7], t)));
+  return __hfma2(n, __float2half2_rn(2.f), f);
+}
+
+__device__ __forceinline__ uint32_t search_y(__half2 x, __half2 sum, uint32_t lo, uint32_t hi) {
+  return __vminu2(__vmaxu2(h2_bits(pair_round(x, sum)), lo), hi);
+}
+
+// Adds the squared errors of the eight samples of two quads: ys, the four
+// pairs' outcomes (8-bit samples in their low bytes), against the sources.
+__device__ __forceinline__ uint32_t search_err(uint32_t y4, uint32_t s4, uint32_t acc) {
+  const uint32_t d = __vabsdiffu4(y4, s4);
+  return __dp4a(d, d, acc);
+}
+
+__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(256, 3) k_cdef_search(SearchArgs a) {
+  __shared__ SearchSmem sm;
+  cg::cluster_group cl = cg::this_cluster();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int slices = a.slices > 1 ? a.slices : 1;
-  const int fb = blockIdx.x / slices, slice = blockIdx.x - fb * slices;
+  const int fb = blockIdx.x / 3, rank = blockIdx.x - 3 * fb;
+  const bool chroma = rank == 2;
   const int fbr = fb / a.nhfb, fbc = fb - fbr * a.nhfb;
-  const int lr = 16 * fbr, lc = 16 * fbc;
-  const int nhb = imin(16, a.miCols - lc), nvb = imin(16, a.miRows - lr);
   const int nfb = a.nhfb * a.nvfb;
-  uint64_t* m0 = a.mse + (size_t)fb * 64;
-  uint64_t* m1 = a.mse + (size_t)nfb * 64 + (size_t)fb * 64;
-  const uint64_t listed = fb_listed(a, fb, lr, lc);
+  uint64_t* const m = a.mse + (size_t)(chroma ? nfb + fb : fb) * 64;
+  const uint64_t listed = fb_listed(a, fb, 16 * fbr, 16 * fbc);
   const int count = a.trials.count;
   if (listed == 0) {
-    if (tid < 64 && slice == 0) {
-      m0[tid] = tid < count ? 0 : (uint64_t)kNotATrial;
-      m1[tid] = tid < count ? 0 : (uint64_t)kNotATrial;
-    }
-    if (tid == 0 && slice == 0) a.skip[fb] = 1;
+    // The whole cluster leaves before any barrier.
+    if (tid < 64 && rank != 1) m[tid] = tid < count ? 0 : (uint64_t)kNotATrial;
+    if (tid == 0 && rank == 0) a.skip[fb] = 1;
     return;
   }
+  if (tid == 0 && rank == 0) a.skip[fb] = 0;
   const uint64_t listMask = count >= 64 ? ~0ull : (1ull << count) - 1;
-  const uint64_t mask0 = a.tmask ? a.tmask[2 * fb] : listMask;
-  const uint64_t mask1 = a.tmask ? a.tmask[2 * fb + 1] : a.trials.uvMask;
-  const int ssY = a.trials.ss;
-  // The slices this block uses: one per kTrialsPerSlice tested trials (a
-  // block with a handful of trials is measured by one CTA, a fallback block
-  // by all of its CTAs); the others have nothing to do.
-  const int used = imin(slices, 1 + (__popcll(mask0) + __popcll(mask1)) / kTrialsPerSlice);
-  if (slice >= used) return;
-  if (tid == 0) {
-    if (slice == 0) a.skip[fb] = 0;
-    // This slice's share of the tested trials: list positions slice,
-    // slice + used, ...
-    int c0 = 0, c1 = 0, n0 = 0, n1 = 0;
-    for (int g = 0; g < 64; g++) {
-      if ((mask0 >> g) & 1) {
-        if (n0 % used == slice) s_list[0][c0++] = (uint8_t)g;
-        n0++;
-      }
-      if ((mask1 >> g) & 1) {
-        if (n1 % used == slice) s_list[1][c1++] = (uint8_t)g;
-        n1++;
-      }
-    }
-    s_cnt[0] = c0;
-    s_cnt[1] = c1;
+  const uint64_t mask = a.tmask ? a.tmask[2 * fb + (chroma ? 1 : 0)] : (chroma ? a.trials.uvMask : listMask);
+  // ---- stage, strengths, tap constants ----
+  if (tid < 2) sm.tested[tid] = 0;
+  if (tid < 64) sm.sse[tid] = 0;
+  if (tid < 12) sm.ofs[tid] = make_int2(pair_off(tid, 0, chroma ? kSrchPC : kPW), pair_off(tid, 1, chroma ? kSrchPC : kPW));
+  const int damping = chroma ? a.damping - 1 : a.damping;
+  if (tid < 16 * kSrchTab) {
+    const int p = tid / kSrchTab, e = tid - p * kSrchTab;
+    const int strength = chroma ? p : (e == 0 ? 0 : (p * (3 + e) + 8) >> 4);
+    const PairTap t = pair_tap(strength, constrain_shift(strength, damping));
+    sm.pri[tid] = make_uint4(t.k, t.m, t.o, (uint32_t)(strength & 1) | (strength == 0 ? 2u : 0u));
+  } else if (tid < 16 * kSrchTab + 3) {
+    const int s = 1 << (tid - 16 * kSrchTab);
+    const PairTap t = pair_tap(s, constrain_shift(s, damping));
+    sm.sec[tid - 16 * kSrchTab] = make_uint4(t.k, t.m, t.o, 0);
   }
-  if (tid < 12) s_ofs[tid] = make_int2(dir_off(tid, 0), dir_off(tid, 1));
-  if (tid < 128) s_sse[tid >> 6][tid & 63] = 0;
-  const int damping = a.damping;
-  for (int pli = 0; pli < 3; pli++) {
-    const int dec = pli ? 1 : 0;
-    const int P = pli ? 1 : 0;
-    const int x0 = (lc * 4) >> dec, y0 = (lr * 4) >> dec;
-    const int w = (nhb * 4) >> dec, h = (nvb * 4) >> dec;
-    const DPlane& rp = a.rec.pl[pli];
-    const DPlane& sp = a.src.pl[pli];
-    const int planeW = rp.w, planeH = rp.h;
-    __syncthreads();  // the previous plane's tasks are done with the buffers
-    // A slice with none of the block's tested trials in this plane skips it
-    // (the chroma planes share one count); the chroma trials still need the
-    // luma directions, which the features kernel left in a.dirs.
-    if (s_cnt[P] == 0 && !(pli == 0 && s_cnt[1] > 0 && !a.dirs)) {
-      if (pli == 0 && s_cnt[1] > 0 && tid < 64 && ((listed >> tid) & 1)) {
-        s_dir[tid] = a.dirs[(size_t)fb * 64 + tid];
-        s_ai[tid] = a.ais[(size_t)fb * 64 + tid];
-      }
-      continue;
+  if (!chroma) {
+    const DPlane& rp = a.rec.pl[0];
+    const int x = 64 * fbc - 4, y = 64 * fbr + 32 * rank - 2;
+    const bool in = x >= 0 && x + 72 <= rp.w && y >= 0 && y + 37 <= rp.h &&
+                    ((reinterpret_cast<uintptr_t>(rp.ptr) | (uintptr_t)rp.stride) & 3) == 0;
+    for (int i = tid; i < 18 * 18; i += 256) {
+      const int d = i / 18, cg4 = i - 18 * d;
+      search_stage(rp, in, x + 4 * cg4, y + 2 * d, &sm.w[2 * d * kPW + 4 * cg4], kPW);
     }
-    // loadCDEFInput: frame samples where they exist, VeryLarge elsewhere.
-    // A row wholly inside the plane whose start is 4-byte aligned is read
-    // four samples at a time (w + 16 is a multiple of 4).
-    for (int r = warp; r < h + 4; r += 8) {
-      const int yy = y0 - 2 + r;
-      const bool rowIn = yy >= 0 && yy < planeH;
-      const uint8_t* srow = rowIn ? row_ptr<uint8_t>(rp, yy) : nullptr;
-      const int xs = x0 - 8;
-      if (rowIn && xs >= 0 && xs + w + 16 <= planeW && (((uintptr_t)(srow + xs)) & 3) == 0) {
-        const uint32_t* q = reinterpret_cast<const uint32_t*>(srow + xs);
-        for (int c4 = lane; c4 < (w + 16) >> 2; c4 += 32) {
-          const uint32_t v = q[c4];
-          uint16_t* d = &s_in[r * kSW + 4 * c4];
-          d[0] = v & 0xff;
-          d[1] = (v >> 8) & 0xff;
-          d[2] = (v >> 16) & 0xff;
-          d[3] = v >> 24;
-        }
+  } else {
+    for (int i = tid; i < 2 * 180; i += 256) {
+      const int pl = i >= 180, j = i - (pl ? 180 : 0), d = j / 10, cg4 = j - 10 * d;
+      const DPlane& rp = a.rec.pl[1 + pl];
+      const int x = 32 * fbc - 4, y = 32 * fbr - 2;
+      const bool in = x >= 0 && x + 40 <= rp.w && y >= 0 && y + 37 <= rp.h &&
+                      ((reinterpret_cast<uintptr_t>(rp.ptr) | (uintptr_t)rp.stride) & 3) == 0;
+      search_stage(rp, in, x + 4 * cg4, y + 2 * d, &sm.w[(pl * 36 + 2 * d) * kSrchPC + 4 * cg4], kSrchPC);
+    }
+  }
+  __syncthreads();
+  if (tid < 64 && ((mask >> tid) & 1)) {
+    const int s = chroma ? a.trials.uv[tid] : a.trials.y[tid];
+    atomicOr(&sm.tested[s >> 5], 1u << (s & 31));
+  }
+  // ---- luma directions of the listed blocks, from the reconstruction ----
+  if (a.dirs) {
+    // Found by the features kernel (same arithmetic).
+    if (tid < 64 && ((listed >> tid) & 1)) {
+      sm.dir[tid] = a.dirs[(size_t)fb * 64 + tid];
+      sm.ai[tid] = a.ais[(size_t)fb * 64 + tid];
+    }
+    cl.sync();  // rank 0's sums are cleared before rank 1 can add to them
+  } else {
+    if (!chroma) {
+      const DPlane& rp = a.rec.pl[0];
+      const int x0 = 64 * fbc, y0 = 64 * fbr;
+      const bool whole = x0 + 64 <= rp.w && y0 + 32 * rank + 32 <= rp.h;
+      if (whole) {
+        // A warp has two directions of the half's 32 blocks.
+        const int b = rank * 32 + lane;
+        if (warp < 4 && ((listed >> b) & 1))
+          dir_costs_vert(warp, &sm.w[(2 + (lane >> 3) * 8) * kPW + kPX + (lane & 7) * 8], 0, 0x00ff00ffu,
+                         &sm.cost[b * 8]);
       } else {
-        for (int c = lane; c < w + 16; c += 32) {
-          const int xx = xs + c;
-          s_in[r * kSW + c] = (rowIn && xx >= 0 && xx < planeW) ? srow[xx] : (uint16_t)kVeryLarge;
-        }
-      }
-    }
-    for (int r = warp; r < h; r += 8) {
-      const uint8_t* srow = row_ptr<uint8_t>(sp, y0 + r) + x0;
-      const uint8_t* rrow = row_ptr<uint8_t>(rp, y0 + r) + x0;
-      if ((((uintptr_t)srow | (uintptr_t)rrow) & 3) == 0) {
-        for (int c4 = lane; c4 < w >> 2; c4 += 32) {
-          reinterpret_cast<uint32_t*>(&s_src[r * 64])[c4] = reinterpret_cast<const uint32_t*>(srow)[c4];
-          reinterpret_cast<uint32_t*>(&s_rec[r * 64])[c4] = reinterpret_cast<const uint32_t*>(rrow)[c4];
-        }
-      } else {
-        for (int c = lane; c < w; c += 32) {
-          s_src[r * 64 + c] = srow[c];
-          s_rec[r * 64 + c] = rrow[c];
-        }
-      }
-    }
-    if (pli == 0 && a.dirs) {
-      // Directions already found by the features kernel (same arithmetic).
-      if (tid < 64 && ((listed >> tid) & 1)) {
-        s_dir[tid] = a.dirs[(size_t)fb * 64 + tid];
-        s_ai[tid] = a.ais[(size_t)fb * 64 + tid];
-      }
-    } else if (pli == 0) {
-      // Luma directions of the listed blocks, from the reconstruction.
-      // A warp takes one direction for 32 blocks (no divergence between
-      // the eight direction templates).
-      for (int wi = tid; wi < 64 * 8; wi += 256) {
-        const int d = wi >> 6, b = wi & 63;
+        // Blocks past the crop take their directions from the padding too.
+        const int b = rank * 32 + lane;
         if ((listed >> b) & 1)
-          s_cost[b * 8 + d] = dir_cost8_dev(d, row_ptr<uint8_t>(rp, y0 + (b >> 3) * 8) + x0 + (b & 7) * 8, rp.stride);
+          sm.cost[b * 8 + warp] =
+              dir_cost8_dev(warp, rp.ptr + (int64_t)(y0 + (b >> 3) * 8) * rp.stride + x0 + (b & 7) * 8, rp.stride);
       }
       __syncthreads();
-      if (tid < 64 && ((listed >> tid) & 1)) {
+      const int b = rank * 32 + tid;
+      if (tid < 32 && ((listed >> b) & 1)) {
         int best = 0;
-        int32_t bc = s_cost[tid * 8];
+        int32_t bc = sm.cost[b * 8];
         for (int d = 1; d < 8; d++)
-          if (s_cost[tid * 8 + d] > bc) {
+          if (sm.cost[b * 8 + d] > bc) {
             best = d;
-            bc = s_cost[tid * 8 + d];
+            bc = sm.cost[b * 8 + d];
           }
-        const int32_t var = (bc - s_cost[tid * 8 + ((best + 4) & 7)]) >> 10;
-        s_dir[tid] = (uint8_t)best;
+        const int32_t var = (bc - sm.cost[b * 8 + ((best + 4) & 7)]) >> 10;
+        sm.dir[b] = (uint8_t)best;
         int ai = -1;
         if (var != 0) {
           ai = 0;
           const int32_t v = var >> 6;
           if (v) ai = imin(31 - __clz(v), 12);
         }
-        s_ai[tid] = (int8_t)ai;
+        sm.ai[b] = (int8_t)ai;
       }
     }
-    const int bl = 3 - dec;
-    const int dmp = pli ? damping - 1 : damping;
-    if (pli < 2) {  // chroma planes share one damping
-      // Rows of 256 32-bit words (entries -255 .. 256 at kTab0 - 255 ..),
-      // then entry kTab0 - 256 (a difference below -255) set to 0.
-      for (int i = tid; i < 19 * 256; i += 256) {
-        const int t = i >> 8, wd = i & 255;
-        const int k = t < 16 ? t : (t == 16 ? 1 : (t == 17 ? 2 : 4));
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(a.ctab + (size_t)(k * 8 + constrain_shift(k, dmp)) * 512);
-        reinterpret_cast<uint32_t*>(&s_tab[t][kTab0 - 255])[wd] = src[wd];
-      }
-      if (tid < 19) s_tab[tid][kTab0 - 256] = 0;
-    }
-    __syncthreads();
-    const int ngrp = (h + 7) >> 3;
-    const int ntask = s_cnt[P] * ngrp;
-    // Luma rows every ssY-th (the subsampled search), chroma every row.
-    const int step = P ? 1 : ssY;
-    for (int task = warp; task < ntask; task += 8) {
-      const int g = s_list[P][task / ngrp];
-      const int grp = task - (task / ngrp) * ngrp;
-      const int packed = P ? a.trials.uv[g] : a.trials.y[g];
-      const int pri = packed >> 2;
-      int sec = packed & 3;
-      if (sec == 3) sec = 4;
-      const int16_t* ts = &s_tab[sec == 1 ? 16 : (sec == 2 ? 17 : 18)][kTab0];
-      uint32_t sse = 0;
-      for (int xx = lane; xx < w; xx += 32) {
-        for (int yb = grp * 8; yb < imin(grp * 8 + 8, h); yb += 1 << bl) {
-          const int b = ((yb >> bl) << 3) + (xx >> bl);
-          if (!((listed >> b) & 1)) continue;
-          int strength = pri;
-          if (pli == 0 && pri != 0) {
-            const int ai = s_ai[b];
-            strength = ai < 0 ? 0 : (pri * (4 + ai) + 8) >> 4;
-          }
-          const bool filt = (strength | sec) != 0;
-          const int dir = pri != 0 ? s_dir[b] : 0;
-          const int16_t* tp = &s_tab[strength][kTab0];
-          const int2 po = s_ofs[dir + 2], q0 = s_ofs[dir + 4], q1 = s_ofs[dir];
-          for (int yy = yb; yy < yb + (1 << bl); yy += step) {
-            // An unfiltered block keeps the reconstruction (cdefDist8 against
-            // recon / the copyFB trial buffer), which below the crop is not
-            // the VeryLarge-padded input.
-            int v = s_rec[yy * 64 + xx];
-            if (filt)
-              // The 8-bit trial buffer keeps the low byte (cdef/filter_u8.go:151),
-              // which matters only below the crop where the centre is VeryLarge.
-              v = (uint8_t)cdef_filter_px_tab8(&s_in[(2 + yy) * kSW + 8 + xx], strength, tp, sec, ts, po, q0, q1);
-            const int e = (int)s_src[yy * 64 + xx] - v;
-            sse += (uint32_t)(e * e);
-          }
-        }
+    cl.sync();
+    // The chroma CTA takes the directions from the two luma ones.
+    if (chroma && tid < 64) sm.dir[tid] = cl.map_shared_rank(&sm.dir[0], tid >> 5)[tid];
+    cl.sync();  // and they stay until it has
+  }
+  // ---- trials ----
+  const uint64_t tested = sm.tested[0] | (uint64_t)sm.tested[1] << 32;
+  if (tested) {
+    const int pl = chroma ? 1 + (warp >> 2) : 0;
+    const int pitch = chroma ? kSrchPC : kPW;
+    // The lane's column and first row in the unit, and its word there.
+    const int col = chroma ? lane : 32 * (warp & 1) + lane;
+    const int row = chroma ? 8 * (warp & 3) : 32 * rank + 8 * (warp >> 1);
+    const uint32_t* c = chroma ? &sm.w[((pl - 1) * 36 + 2 + row) * kSrchPC + kPX + col]
+                               : &sm.w[(2 + row - 32 * rank) * kPW + kPX + col];
+    const DPlane& sp = a.src.pl[pl];
+    const int64_t at = (int64_t)((chroma ? 32 * fbr : 64 * fbr) + row);
+    const int px = (chroma ? 32 * fbc : 64 * fbc) + col;
+    // Per quad (four rows): its block, source and reconstruction samples; per
+    // pair: the sample, the clamp range.
+    int dir[2];
+    uint32_t s4[2], r4[2], x[4], lo[4], hi[4], fix[4];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int b = chroma ? ((row >> 2) + q) * 8 + (col >> 2) : (row >> 3) * 8 + (col >> 3);
+      const bool on = (listed >> b) & 1;
+      dir[q] = on ? sm.dir[b] : 0;
+      // Rows that count: every ss-th of a luma block, all of a chroma one.
+      uint32_t rows = on ? 0xffffffffu : 0u;
+      if (!chroma && a.trials.ss > 1)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if ((4 * q + k) % a.trials.ss) rows &= ~(0xffu << (8 * k));
+      x[2 * q] = c[4 * q * pitch];
+      x[2 * q + 1] = c[(4 * q + 2) * pitch];
+      const uint32_t x4 = __byte_perm(x[2 * q], x[2 * q + 1], 0x6420);
+      s4[q] = r4[q] = x4;
+      if (on) {
+        uint32_t s = 0;
+        const uint8_t* sr = sp.ptr + (at + 4 * q) * sp.stride + px;
+#pragma unroll
+        for (int k = 0; k < 4; k++) s |= (uint32_t)sr[k * sp.stride] << (8 * k);
+        s4[q] = (s & rows) | (x4 & ~rows);
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sse += __shfl_xor_sync(0xffffffffu, sse, o);
-      if (lane == 0) atomicAdd(&s_sse[P][g], sse);
+      for (int h = 0; h < 2; h++) {
+        const uint32_t xv = x[2 * q + h], rb = rows >> (16 * h);
+        // Halves whose outcome is the sample itself whatever the trial:
+        // those that do not count, and absent ones.
+        uint32_t f = (rb & 1 ? 0u : 0xffffu) | (rb & 0x100 ? 0u : 0xffff0000u);
+        if ((xv & 0xffffu) == (kPairNone & 0xffffu)) f |= 0xffffu;
+        if ((xv >> 16) == (kPairNone >> 16)) f |= 0xffff0000u;
+        fix[2 * q + h] = f;
+      }
+      if (on && ((fix[2 * q] | fix[2 * q + 1]) & (((x[2 * q] | x[2 * q + 1]) & 0x80008000u) >> 15)) != 0) {
+        // Absent samples that count: the unfiltered trial measures the
+        // reconstruction's padding.
+        const DPlane& rp = a.rec.pl[pl];
+        const uint8_t* rr = rp.ptr + (at + 4 * q) * rp.stride + px;
+        uint32_t r = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) r |= (uint32_t)rr[k * rp.stride] << (8 * k);
+        r4[q] = (r & rows) | (x4 & ~rows);
+      }
+    }
+    auto put = [&](int strength, uint32_t e) {
+      e = __reduce_add_sync(0xffffffffu, e);
+      if (lane == 0) atomicAdd(&sm.sse[strength], e);
+    };
+    auto taps8 = [&](int j, const int2& s0, const int2& s1, uint32_t (&t)[8]) {
+      const uint32_t* w = c + 2 * j * pitch;
+      t[0] = w[s0.x], t[1] = w[-s0.x], t[2] = w[s1.x], t[3] = w[-s1.x];
+      t[4] = w[s0.y], t[5] = w[-s0.y], t[6] = w[s1.y], t[7] = w[-s1.y];
+    };
+    // Primary strength 0: direction 0 whatever the block's, no clamp.
+    if (tested & 1) put(0, search_err(r4[1], s4[1], search_err(r4[0], s4[0], 0)));
+    if (tested & 14) {
+      const int2 s0 = sm.ofs[4], s1 = sm.ofs[0];
+      uint32_t y[3][4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        uint32_t t[8];
+        __half2 d[8];
+        taps8(j, s0, s1, t);
+#pragma unroll
+        for (int k = 0; k < 8; k++) d[k] = __hsub2(bits_h2(t[k]), bits_h2(x[j]));
+        const uint32_t l = (fix[j] & x[j]) | (~fix[j] & 0x3c003c00u), h = (fix[j] & x[j]) | (~fix[j] & 0x3cff3cffu);
+#pragma unroll
+        for (int s = 0; s < 3; s++)
+          if ((tested >> (s + 1)) & 1) y[s][j] = search_y(bits_h2(x[j]), search_sec(d, sm.sec[s]), l, h);
+      }
+#pragma unroll
+      for (int s = 0; s < 3; s++)
+        if ((tested >> (s + 1)) & 1)
+          put(s + 1, search_err(__byte_perm(y[s][2], y[s][3], 0x6420), s4[1],
+                                search_err(__byte_perm(y[s][0], y[s][1], 0x6420), s4[0], 0)));
+    }
+    if (tested >> 4) {
+      // Some primary strength: the differences of its taps, the secondary
+      // sums that any trial needs, the clamp range.
+      __half2 d[4][4], sec[3][4];
+      const uint64_t any = tested >> 4;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int2 po = sm.ofs[dir[j >> 1] + 2], s0 = sm.ofs[dir[j >> 1] + 4], s1 = sm.ofs[dir[j >> 1]];
+        const uint32_t* w = c + 2 * j * pitch;
+        const uint32_t p[4] = {w[po.x], w[-po.x], w[po.y], w[-po.y]};
+        uint32_t t[8];
+        taps8(j, s0, s1, t);
+        uint32_t l = x[j], h = x[j];
+        __half2 e[8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) d[j][k] = __hsub2(bits_h2(p[k]), bits_h2(x[j]));
+#pragma unroll
+        for (int k = 0; k < 8; k++) e[k] = __hsub2(bits_h2(t[k]), bits_h2(x[j]));
+        l = __vimin3_u16x2(__vimin3_u16x2(l, p[0], p[1]), p[2], p[3]);
+        h = __vimax3_s16x2(__vimax3_s16x2(h, p[0], p[1]), p[2], p[3]);
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          l = __vimin3_u16x2(l, t[k], t[k + 1]);
+          h = __vimax3_s16x2(h, t[k], t[k + 1]);
+        }
+        lo[j] = (l & ~fix[j]) | (x[j] & fix[j]);
+        hi[j] = (h & ~fix[j]) | (x[j] & fix[j]);
+#pragma unroll
+        for (int s = 0; s < 3; s++) {
+          sec[s][j] = __float2half2_rn(0.f);
+          if (any & (0x1111111111111111ull << (s + 1))) sec[s][j] = search_sec(e, sm.sec[s]);
+        }
+      }
+      const int e0 = chroma ? 0 : ((listed >> ((row >> 3) * 8 + (col >> 3))) & 1 ? sm.ai[(row >> 3) * 8 + (col >> 3)] + 1 : 0);
+#pragma unroll 1
+      for (int p = 1; p < 16; p++) {
+        const uint32_t t4 = (uint32_t)(tested >> (4 * p)) & 15u;
+        if (t4 == 0) continue;
+        const uint4 k = sm.pri[p * kSrchTab + e0];
+        const PairTap pt{k.x, k.y, k.z};
+        const __half2 w0 = bits_h2(k.w & 1 ? 0x42004200u : 0x44004400u), w1 = bits_h2(k.w & 1 ? 0x42004200u : 0x40004000u);
+        __half2 sum[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          sum[j] = __hmul2(w0, __hadd2(pair_constrain(d[j][0], pt), pair_constrain(d[j][1], pt)));
+          sum[j] = __hfma2(w1, __hadd2(pair_constrain(d[j][2], pt), pair_constrain(d[j][3], pt)), sum[j]);
+        }
+        if (t4 & 1) {
+          uint32_t y[4], e = 0;
+#pragma unroll
+          for (int j = 0; j < 4; j++) y[j] = search_y(bits_h2(x[j]), sum[j], lo[j], hi[j]);
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            const uint32_t y4 = __byte_perm(y[2 * q], y[2 * q + 1], 0x6420);
+            e = search_err(k.w & 2 ? r4[q] : y4, s4[q], e);  // a zero strength leaves the block unfiltered
+          }
+          put(4 * p, e);
+        }
+#pragma unroll
+        for (int s = 0; s < 3; s++)
+          if (t4 & (2u << s)) {
+            uint32_t y[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) y[j] = search_y(bits_h2(x[j]), __hadd2(sum[j], sec[s][j]), lo[j], hi[j]);
+            put(4 * p + s + 1, search_err(__byte_perm(y[2], y[3], 0x6420), s4[1],
+                                          search_err(__byte_perm(y[0], y[1], 0x6420), s4[0], 0)));
+          }
+      }
     }
   }
   __syncthreads();
-  if (tid < 64) {
-    // Each entry written once: a tested trial by the slice that measured
-    // it, the rest by slice 0.
-    const uint64_t below = (1ull << tid) - 1;
-    const bool t0 = (mask0 >> tid) & 1, t1 = (mask1 >> tid) & 1;
-    const bool own0 = t0 && __popcll(mask0 & below) % used == slice;
-    const bool own1 = t1 && __popcll(mask1 & below) % used == slice;
-    if (tid >= count) {
-      if (slice == 0) m0[tid] = m1[tid] = kNotATrial;
-    } else {
+  // ---- the table: rank 0 has luma's sums (rank 1 adds its own), rank 2 chroma's ----
+  if (rank == 1 && tid < 64 && ((tested >> tid) & 1)) atomicAdd(&cl.map_shared_rank(&sm.sse[0], 0)[tid], sm.sse[tid]);
+  cl.sync();
+  if (rank != 1 && tid < 64) {
+    uint64_t v;
+    if (tid >= count)
+      v = kNotATrial;
+    else if ((mask >> tid) & 1)
       // A subsampled luma SSE is scaled back by the row step (searchRow, :722-734).
-      if (own0) m0[tid] = (uint64_t)s_sse[0][tid] * (uint64_t)ssY;
-      else if (!t0 && slice == 0) m0[tid] = (uint64_t)kUntestedMSE;
-      if (own1) m1[tid] = (uint64_t)s_sse[1][tid];
-      else if (!t1 && slice == 0) m1[tid] = (uint64_t)kUntestedMSE;
-    }
+      v = (uint64_t)sm.sse[chroma ? a.trials.uv[tid] : a.trials.y[tid]] * (uint64_t)(chroma ? 1 : a.trials.ss);
+    else
+      v = (uint64_t)kUntestedMSE;
+    m[tid] = v;
   }
 }
 
@@ -615,7 +759,7 @@ size_t sel_smem_bytes(int nfb, bool rows) {
 }
 
 cudaError_t launch_search(const SearchArgs& a, cudaStream_t st) {
-  k_cdef_search<<<a.nhfb * a.nvfb * (a.slices > 1 ? a.slices : 1), 256, 0, st>>>(a);
+  k_cdef_search<<<3 * a.nhfb * a.nvfb, 256, 0, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -700,7 +844,6 @@ using namespace pf;
 void* pf_internal_search_scratch(pf_ctx* c, size_t bytes);  // pf_api.cu
 void* pf_internal_stream(pf_ctx* c);
 cudaEvent_t* pf_internal_events(pf_ctx* c);  // pf_api.cu: null unless the context times stages
-const int16_t* pf_internal_ctab(pf_ctx* c);  // pf_api.cu
 void* pf_internal_pinned(pf_ctx* c, size_t bytes);
 void* pf_internal_cached_upload(pf_ctx* c, const void* host, size_t bytes, size_t extra, cudaStream_t st,
                                 int* changed);
@@ -864,8 +1007,6 @@ static int stage_search(pf_ctx* ctx, const pf_frame* source, const pf_frame* rec
   a.skip = base + oSkip;
   a.dirs = nullptr;
   a.ais = nullptr;
-  a.ctab = pf_internal_ctab(ctx);
-  a.slices = 1;
   level1_trials(&a.trials);
   SelArgs& s = S->s;
   s.mse = a.mse;
@@ -1236,10 +1377,6 @@ extern "C" int pf_cdef_search_learned(pf_ctx* ctx, const pf_frame* source, const
     return PF_ERR_DEVICE;
   if (ev && cudaEventRecord(ev[2], S.st) != cudaSuccess) return PF_ERR_DEVICE;
   S.a.tmask = masks;
-  // A block's tested trials vary from a few to all 64 (a fallback head):
-  // four CTAs share each block's list, so the fallback blocks do not set
-  // the launch's length alone.
-  S.a.slices = kLearnedSlices;
   S.s.refine = (flags & PF_LEARNED_REFINE) ? 1 : 0;
   const int r = search_finish(S, params, mse_out, fb_index_out, result, ev);
   if (r != PF_OK) return r;

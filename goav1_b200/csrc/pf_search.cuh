@@ -54,12 +54,6 @@ struct SearchArgs {
   uint8_t* dirs;            // [nfb][64]
   int8_t* ais;              // [nfb][64]
   TrialList trials;         // tmask searches use the level-1 list
-  // constrain() tables of the context ([strength 16][shift 8][512], entry
-  // 255 + d for a difference d, entry 511 = 0: CdefArgs.ctab).
-  const int16_t* ctab;
-  // CTAs per filter block: slice s of a block measures the tested trials at
-  // positions s, s + slices, ... of its list (1: one CTA measures them all).
-  int slices;
 };
 
 struct SelOut {

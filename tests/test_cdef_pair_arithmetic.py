@@ -38,7 +38,7 @@ def pair_constrain(d, tap):
 
 
 def pair_round(x, s):
-    return f16(f16(s + np.copysign(2.0 ** -11, s)) * 0.0625 + x)
+    return f16(s * from_bits(0x2C01) + x)
 
 
 def constrain_shift(thr, damping):
