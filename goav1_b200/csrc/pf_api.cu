@@ -130,7 +130,7 @@ struct pf_ctx {
   int persistent[ST_COUNT] = {};
   int chunk[ST_COUNT] = {1, 1, 1, 1, 1, 1, 1, 1};
   int ahead[ST_COUNT] = {};
-  int tile[ST_COUNT] = {};  // launch-level tile setting (grain apply: rows per load group)
+  int tile[ST_COUNT] = {};  // launch-level tile setting (grain apply: rows loaded together)
   int db_tile = 0;          // deblocking tile shape (per job: it sets the tile counts)
   // Frame groups (pf_set_frame_groups): 2 runs the batch's two halves on the
   // main stream and stream2.
@@ -658,7 +658,8 @@ static size_t frame_scratch(const pf_frame* f, const pf_frame_side* s) {
   }
   int act[3];
   if (fg_active(f, s, act)) {
-    n += align256(3 * 82 * 73 * sizeof(int16_t));
+    n += align256(3 * kGrainLen * sizeof(int16_t));
+    if (bps == 2) n += 3 * kFgScaleLen;
     n += align256((size_t)((f->height + 31) / 32) * ((f->width + 31) / 32));
   }
   return n;
@@ -845,11 +846,12 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
     FgArgs& a = J.fg;
     if (on) {
       const pf_film_grain& g = s->fg;
-      int16_t* gbase = (int16_t*)arena.take(3 * 82 * 73 * sizeof(int16_t));
+      int16_t* gbase = (int16_t*)arena.take(3 * kGrainLen * sizeof(int16_t));
+      if (bps == 2) a.scale = (uint8_t*)arena.take(3 * kFgScaleLen);
       const int rows = (f->height + 31) / 32, cols = (f->width + 31) / 32;
       a.offsets = (const uint8_t*)arena.take((size_t)rows * cols);
       for (int p = 0; p < 3; p++) {
-        a.grain[p] = gbase + p * 82 * 73;
+        a.grain[p] = gbase + p * kGrainLen + kGrainShift(p && f->ss_x);
         a.active[p] = act[p];
       }
       a.off_rows = rows;
@@ -888,7 +890,7 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
       t.ssx = f->ss_x;
       t.ssy = f->ss_y;
       counts[ST_FG_TEMPLATES] = 1;
-      counts[ST_FG_OFFSETS] = (rows + 63) / 64;
+      counts[ST_FG_OFFSETS] = (rows + 63) / 64 + (bps == 2 ? 3 << (f->bit_depth - 8) : 0);
     }
     int tiles = 0;
     for (int p = 0; p < (f->mono ? 1 : 3); p++) {
@@ -1145,7 +1147,7 @@ static void add_stats(const pf_ctx* c, int n, uint32_t done, pf_stats* stats) {
   stats->completed |= done;
   stats->cdef_units += total(ST_CDEF);
   stats->lr_units += total(ST_LR);
-  stats->fg_rows += total(ST_FG_OFFSETS);
+  for (int i = 0; i < n; i++) stats->fg_rows += (c->hjobs[i].fg.off_rows + 63) / 64;
 }
 
 // Builds the job table for n validated frames and queues every stage.

@@ -123,8 +123,17 @@ struct LrArgs {
   int64_t line_stride[3];
 };
 
+// Grain templates in memory: 73 rows of 82 samples a plane, kGrainLen samples
+// apart; planes that are not horizontally subsampled start one sample in
+// (kGrainShift), which puts the odd columns their blocks start at on word
+// boundaries.
+constexpr int kGrainLen = 82 * 73 + 2;
+__host__ __device__ constexpr int kGrainShift(int subsampled) { return subsampled ? 0 : 1; }
+constexpr int kFgScaleLen = 4096;
+
 struct FgArgs {
   int16_t* grain[3];      // 73*82 templates
+  uint8_t* scale;         // [3][kFgScaleLen] scaling by sample value (more than 8 bits)
   const uint8_t* offsets; // [rows][blocks] offsets of the stripe LFSRs
   int off_rows, off_cols;
   uint8_t lut[3][256];

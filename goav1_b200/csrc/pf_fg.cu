@@ -15,7 +15,7 @@
 // wavefront over t = x + 4y (every AR input of sample (y, x) has a smaller
 // t), one warp per template, rows in lanes, neighbours passed between lanes
 // by shuffles.  Offsets come from one thread per 32-row stripe.  The apply
-// is one thread per output sample, 64x16-sample tiles per CTA.
+// is a thread per 4x4 samples, 64x64-sample tiles per CTA.
 #include <atomic>
 
 #include "pf_common.cuh"
@@ -279,17 +279,34 @@ __device__ __forceinline__ void fg_templates(const FgTemplateArgs& p, int16_t* g
       ar_warp_lag<false>(S.g[warp], nullptr, p, warp, cw, ch);
   }
   __syncthreads();
-  // Two samples per 32-bit store (rows of 82 samples keep pairs aligned).
+  // Two samples per 32-bit store (rows of 82 samples keep pairs aligned),
+  // one sample each where the plane starts on an odd one (kGrainShift).
   for (int pl = 0; pl < 3; pl++) {
     if (!outs[pl]) continue;
-    uint32_t* o = reinterpret_cast<uint32_t*>(outs[pl]);
-    for (int i = threadIdx.x; i < kGH * kGW / 2; i += blockDim.x) {
-      const int y = i / (kGW / 2), x = 2 * (i - y * (kGW / 2));
-      const uint32_t s = *reinterpret_cast<const uint32_t*>(&S.g[pl][tpl_at(y, x)]);
-      const int lo = tpl_decode((int16_t)(s & 0xffff)), hi = tpl_decode((int16_t)(s >> 16));
-      o[i] = (uint32_t)(uint16_t)lo | ((uint32_t)(uint16_t)hi << 16);
+    if (pl && p.ssx) {
+      uint32_t* o = reinterpret_cast<uint32_t*>(outs[pl]);
+      for (int i = threadIdx.x; i < kGH * kGW / 2; i += blockDim.x) {
+        const int y = i / (kGW / 2), x = 2 * (i - y * (kGW / 2));
+        const uint32_t s = *reinterpret_cast<const uint32_t*>(&S.g[pl][tpl_at(y, x)]);
+        const int lo = tpl_decode((int16_t)(s & 0xffff)), hi = tpl_decode((int16_t)(s >> 16));
+        o[i] = (uint32_t)(uint16_t)lo | ((uint32_t)(uint16_t)hi << 16);
+      }
+    } else {
+      for (int i = threadIdx.x; i < kGH * kGW; i += blockDim.x) {
+        const int y = i / kGW;
+        outs[pl][i] = (int16_t)tpl_decode(S.g[pl][tpl_at(y, i - y * kGW)]);
+      }
     }
   }
+}
+
+// The scaling function of 10- and 12-bit samples (scaling.go:88-121) at every
+// sample value: entries [0, 1 << bd) of each plane's 4,096.
+__device__ __forceinline__ int scale_at(const uint8_t* lut, int index, int bd) {
+  const int shift = bd - 8, x = index >> shift;
+  if (x == 255) return lut[x];
+  const int rem = index - (x << shift), start = lut[x], end = lut[x + 1];
+  return (uint8_t)(start + rpow2((end - start) * rem, shift));
 }
 
 // Offsets of every 32x32 block: row r uses the LFSR seeded by stripe r
@@ -302,310 +319,263 @@ __device__ __forceinline__ void fg_offsets_row(uint16_t seed, int r, int cols, u
   for (int b = 0; b < cols; b++) out[r * cols + b] = (uint8_t)lfsr(reg, 8);
 }
 
-__device__ __forceinline__ int scale_lut(const uint8_t* lut, int index, int bd) {
-  index = iclip(index, 0, (1 << bd) - 1);
-  const int shift = bd - 8;
-  const int x = index >> shift;
-  if (bd == 8 || x == 255) return lut[x];
-  const int rem = index - (x << shift);
-  const int start = lut[x], end = lut[x + 1];
-  return (uint8_t)(start + rpow2((end - start) * rem, shift));
-}
+// ---- grain application ----
+//
+// Display = reference with grain added on the cropped area of active planes;
+// every allocated sample of the display frame is written.
+//
+// A thread takes four adjacent columns by four rows of one plane (always
+// inside one grain block): the four samples of a row move as one word, the
+// block's set-up (offsets, template positions, blend weights) is shared by
+// sixteen samples, and nothing else is done per sample but the scaling
+// lookup, the multiply-add and one fused add-and-clamp.  10- and 12-bit
+// planes look the scaling up in a table of every sample value, built once a
+// frame beside the block offsets, instead of interpolating per sample.  The
+// quads on a block's left edge, which blend with the block to the left, are
+// gathered in warps of their own, so the others' warps never wait for that
+// path.
+//
+// Bound by integer issue (57 % of the slots) and the wait for the grain
+// behind the block offset.  us per frame: 60 x 1080p 8-bit 12.6 before (one
+// column by 16 rows a thread, every sample by itself), 7.1 now, at 2.2 warp
+// instructions per luma sample instead of 5.0; 8 x 4K 10-bit 62.9 and 30.2;
+// one 1080p frame 25.6 and 17.  Two rows' or one row's loads at a time
+// measured 7.3 and 7.8; 5 or 6 CTAs per SM (48, 40 registers) 7.6 and 7.5.
+
+template <typename T>
+struct FgQuad;
+template <>
+struct FgQuad<uint8_t> {
+  typedef uint32_t W;
+  static __device__ __forceinline__ W load(const uint8_t* p, bool word, int n) {
+    if (word) return *reinterpret_cast<const uint32_t*>(p);
+    uint32_t v = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k < n) v |= (uint32_t)p[k] << (8 * k);
+    return v;
+  }
+  static __device__ __forceinline__ void store(uint8_t* p, W v, bool word, int n) {
+    if (word) {
+      *reinterpret_cast<uint32_t*>(p) = v;
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k < n) p[k] = (uint8_t)(v >> (8 * k));
+  }
+  static __device__ __forceinline__ int get(W v, int k) { return (v >> (8 * k)) & 0xff; }
+  static __device__ __forceinline__ W pack(int a, int b, int c, int d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+  }
+};
+template <>
+struct FgQuad<uint16_t> {
+  typedef uint2 W;
+  static __device__ __forceinline__ W load(const uint16_t* p, bool word, int n) {
+    if (word) return *reinterpret_cast<const uint2*>(p);
+    uint2 v = make_uint2(0, 0);
+    if (n > 0) v.x = p[0];
+    if (n > 1) v.x |= (uint32_t)p[1] << 16;
+    if (n > 2) v.y = p[2];
+    if (n > 3) v.y |= (uint32_t)p[3] << 16;
+    return v;
+  }
+  static __device__ __forceinline__ void store(uint16_t* p, W v, bool word, int n) {
+    if (word) {
+      *reinterpret_cast<uint2*>(p) = v;
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k < n) p[k] = (uint16_t)get(v, k);
+  }
+  static __device__ __forceinline__ int get(W v, int k) {
+    const uint32_t h = k < 2 ? v.x : v.y;
+    return k & 1 ? h >> 16 : h & 0xffff;
+  }
+  static __device__ __forceinline__ W pack(int a, int b, int c, int d) {
+    return make_uint2(__byte_perm(a, b, 0x5410), __byte_perm(c, d, 0x5410));
+  }
+};
 
 __device__ __forceinline__ int blend_w(int prev, int cur, int pw, int cw, int bd) {
   return iclip(rpow2(prev * pw + cur * cw, 5), -(1 << (bd - 1)), (1 << (bd - 1)) - 1);
 }
 
-// Display = reference with grain added on the cropped area of active planes;
-// every allocated sample of the display frame is written.
-// One column x of up to 4 rows y0.. of one display plane (all inside one
-// 32-row grain block row): per-block values once, then per sample.
-// kFgRowGroup: rows of the column whose loads go out together (1, 2 or 4,
-// the grain group's tile setting).
-template <typename T, int kFgRowGroup>
-__device__ __forceinline__ void fg_apply_col(const DFrame& ref, const DFrame& disp, const FgArgs& a, const uint8_t* lut,
-                                             int plane, int x, int y0, int nrows) {
-  // Plane descriptors and parameters by value: they live in the job table in
-  // global memory, which the compiler would re-read after every store.
+// Four grains of a template row from column c: the plane's templates start
+// so that unsubsampled planes' columns (always odd) fall on word boundaries
+// (kGrainShift); subsampled ones are taken from three words by the parity.
+template <bool kSx>
+__device__ __forceinline__ uint2 grain4(const int16_t* row, int c) {
+  if (!kSx) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(row + c);
+    return make_uint2(w[0], w[1]);
+  }
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(row + (c & ~1));
+  const uint32_t a = w[0], b = w[1], d = w[2];
+  const int sh = (c & 1) * 16;
+  return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, d, sh));
+}
+
+__device__ __forceinline__ int grain_of(uint2 g, int k) {
+  const uint32_t h = k < 2 ? g.x : g.y;
+  return k & 1 ? (int)h >> 16 : (int)(int16_t)(h & 0xffff);
+}
+
+// Columns x .. x + 3, rows y0 .. y0 + 3 of one display plane (x and y0
+// multiples of 4).  kLuma / kSx: the plane is luma / horizontally subsampled
+// chroma.  kRows rows' loads are issued before their first store.  word: four
+// samples of a row move as one word.
+template <typename T, bool kLuma, bool kSx, int kRows>
+__device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& disp, const FgArgs& a,
+                                              const uint8_t* lut, int plane, int x, int y0, const bool word) {
+  typedef FgQuad<T> Q;
+  // Plane descriptors by value: they live in the job table in global memory,
+  // which the compiler would re-read after every store.
   const DPlane sp = ref.pl[plane];
   const DPlane dp = disp.pl[plane];
-  if (x >= sp.aw) return;
-  const int yend = imin(y0 + nrows, sp.ah);
-  if (!a.active[plane] || x >= sp.w) {
-    if (kFgRowGroup == 1) {
-      for (int y = y0; y < yend; y++) row_ptr<T>(dp, y)[x] = row_ptr<T>(sp, y)[x];
-      return;
-    }
-    // Loads of a group of rows before its stores (the compiler may not move
-    // a load of the frame above a store to the display frame).
-    for (int yg = y0; yg < yend; yg += kFgRowGroup) {
-      T v[kFgRowGroup];
+  const DPlane lp = ref.pl[0];
+  const int n = word ? 4 : imin(4, sp.aw - x), yend = imin(y0 + 4, sp.ah);
+  const bool on = a.active[plane] && x < sp.w;
+  const int sx = kSx ? 1 : 0, sy = kLuma ? 0 : ref.ssy;
+  const int yclip = on ? imin(yend, sp.h) : 0;
+  const uint8_t* srow = sp.ptr + (int64_t)y0 * sp.stride + (int64_t)x * (int)sizeof(T);
+  uint8_t* drow = dp.ptr + (int64_t)y0 * dp.stride + (int64_t)x * (int)sizeof(T);
+  if (!on) {
+    typename Q::W v[4];
 #pragma unroll
-      for (int k = 0; k < kFgRowGroup; k++)
-        if (yg + k < yend) v[k] = row_ptr<T>(sp, yg + k)[x];
+    for (int k = 0; k < 4; k++)
+      if (y0 + k < yend) v[k] = Q::load(reinterpret_cast<const T*>(srow + k * sp.stride), word, n);
 #pragma unroll
-      for (int k = 0; k < kFgRowGroup; k++)
-        if (yg + k < yend) row_ptr<T>(dp, yg + k)[x] = v[k];
-    }
+    for (int k = 0; k < 4; k++)
+      if (y0 + k < yend) Q::store(reinterpret_cast<T*>(drow + k * dp.stride), v[k], word, n);
     return;
   }
   const int bd = sizeof(T) == 1 ? 8 : ref.bd;  // a constant for 8-bit: the depth shifts fold
-  const int sx = plane ? ref.ssx : 0, sy = plane ? ref.ssy : 0;
   const int bwl = 5 - sx, bhl = 5 - sy;
   const int bw = 1 << bwl, bh = 1 << bhl;
   const int row = y0 >> bhl, bcol = x >> bwl;
-  const int xi = x - (bcol << bwl);
-  const int ovl = 2;
-  const int xStart = (a.overlap && bcol > 0) ? imin(sp.w - (bcol << bwl), ovl >> sx) : 0;
-  const int yStart = (a.overlap && row > 0) ? imin(sp.h - (row << bhl), ovl >> sy) : 0;
+  const int xi = x - (bcol << bwl), yi0 = y0 - (row << bhl);
+  constexpr int ovl = 2;
+  const int xStart = (a.overlap && bcol > 0 && xi == 0) ? imin(sp.w - x, ovl >> sx) : 0;
+  const int yStart = (a.overlap && row > 0 && yi0 == 0) ? imin(sp.h - y0, ovl >> sy) : 0;
   const uint8_t* offs = a.offsets + row * a.off_cols + bcol;
   const int16_t* gr = a.grain[plane];
   // Template column / row origins of the current, left, top and top-left blocks.
   auto gcol = [&](int offset, int bc) { return 3 + (ovl >> sx) * (3 + (offset >> 4)) + xi + bw * bc; };
-  auto grow = [&](int offset, int br) { return 3 + (ovl >> sy) * (3 + (offset & 15)) + bh * br; };
+  auto grow = [&](int offset, int br) { return 3 + (ovl >> sy) * (3 + (offset & 15)) + yi0 + bh * br; };
   const int o00 = offs[0];
-  const int c00 = gcol(o00, 0), r00 = grow(o00, 0);
-  const bool left = xi < xStart;
-  int c10 = 0, r10 = 0, c01 = 0, r01 = 0, c11 = 0, r11 = 0;
-  if (left) {
-    const int o10 = offs[-1];
-    c10 = gcol(o10, 1);
-    r10 = grow(o10, 0);
-  }
-  if (yStart > 0) {
-    const int o01 = offs[-a.off_cols];
-    c01 = gcol(o01, 0);
-    r01 = grow(o01, 1);
-    if (left) {
-      const int o11 = offs[-a.off_cols - 1];
-      c11 = gcol(o11, 1);
-      r11 = grow(o11, 1);
-    }
-  }
-  // Horizontal blend weights: luma 27/17 then 17/27; subsampled chroma 23/22.
-  const int hpw = sx ? 23 : (xi == 1 ? 17 : 27), hcw = sx ? 22 : (xi == 1 ? 27 : 17);
-  const int shift = a.scaling_shift;
+  const int c00 = gcol(o00, 0);
+  const int16_t* g00 = gr + grow(o00, 0) * kGW;
+  const int shift = a.scaling_shift, rnd = 1 << (shift - 1);
   int minV = 0, maxV = (256 << (bd - 8)) - 1;
   if (a.clip_restricted) {
     minV = 16 << (bd - 8);
-    maxV = (plane == 0 ? 235 : (a.matrix_identity ? 235 : 240)) << (bd - 8);
+    maxV = (kLuma ? 235 : (a.matrix_identity ? 235 : 240)) << (bd - 8);
   }
-  const int yclip = imin(yend, sp.h);
-  const DPlane lp = ref.pl[0];
-  const bool cfl = a.cfl, oddLuma = a.odd_luma;
+  const bool cfl = a.cfl, edge = x + 4 > sp.w;
+  const int oddCol = a.odd_luma ? sp.w - 1 - x : -1;  // the column whose luma has no right neighbour
   const int lumaMult = a.luma_mult[plane] - 128, mult = a.mult[plane] - 128;
   const int offs0 = (a.offset[plane] << (bd - 8)) - (1 << bd);
-  if (kFgRowGroup == 1) {
-    // One row at a time (40 registers, 6 CTAs per SM).
-    for (int y = y0; y < yend; y++) {
-      const int s = row_ptr<T>(sp, y)[x];
-      if (y >= yclip) {
-        row_ptr<T>(dp, y)[x] = (T)s;
-        continue;
-      }
-      const int yi = y - (row << bhl);
-      int g = gr[(r00 + yi) * kGW + c00];
-      if (left) g = blend_w(gr[(r10 + yi) * kGW + c10], g, hpw, hcw, bd);
-      if (yi < yStart) {
-        int top = gr[(r01 + yi) * kGW + c01];
-        if (left) top = blend_w(gr[(r11 + yi) * kGW + c11], top, hpw, hcw, bd);
-        const int vpw = sy ? 23 : (yi == 1 ? 17 : 27), vcw = sy ? 22 : (yi == 1 ? 27 : 17);
-        g = blend_w(top, g, vpw, vcw, bd);
-      }
-      int idx;
-      if (plane == 0) {
-        idx = s;
-      } else {
-        // chromaScalingIndex (apply.go:501-520) on the un-grained luma.
-        const T* lrow = row_ptr<T>(lp, y << sy);
-        const int lx = x << sx;
-        int avg = lrow[lx];
-        if (sx && !(oddLuma && x == sp.w - 1)) avg = (avg + lrow[lx + 1] + 1) >> 1;
-        if (cfl) {
-          idx = avg;
-        } else {
-          const int combined = avg * lumaMult + s * mult;
-          idx = iclip((combined >> 6) + offs0, 0, (1 << bd) - 1);
+  const int top = (1 << bd) - 1;
+#pragma unroll
+  for (int k0 = 0; k0 < 4; k0 += kRows) {
+    typename Q::W s[kRows], l[kRows][2];
+    uint2 g[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+      const int k = k0 + r, y = y0 + k;
+      if (y < yend) s[r] = Q::load(reinterpret_cast<const T*>(srow + k * sp.stride), word, n);
+      if (y < yclip) {
+        g[r] = grain4<kSx>(g00 + k * kGW, c00);
+        if (!kLuma) {
+          // The co-located luma row; a subsampled quad's eight samples are
+          // inside the 8-aligned luma allocation.
+          const T* lrow = reinterpret_cast<const T*>(lp.ptr + (int64_t)(y << sy) * lp.stride) + (x << sx);
+          l[r][0] = Q::load(lrow, word, kSx ? 4 : n);
+          if (kSx) l[r][1] = Q::load(lrow + 4, word, 4);
         }
       }
-      const int scale = scale_lut(lut, idx, bd);
-      const int noise = rpow2(scale * g, shift);
-      row_ptr<T>(dp, y)[x] = (T)iclip(s + noise, minV, maxV);
     }
-    return;
-  }
-  // Groups of rows: every load of a group (frame sample, grain, co-located
-  // luma) is issued before the group's first store to the display frame.
-  for (int yg = y0; yg < yend; yg += kFgRowGroup) {
-    int sv[kFgRowGroup], gv[kFgRowGroup], lv[kFgRowGroup];
 #pragma unroll
-    for (int k = 0; k < kFgRowGroup; k++) {
-      const int y = yg + k;
-      sv[k] = gv[k] = lv[k] = 0;
+    for (int r = 0; r < kRows; r++) {
+      const int k = k0 + r, y = y0 + k;
       if (y >= yend) continue;
-      sv[k] = row_ptr<T>(sp, y)[x];
-      if (y >= yclip) continue;
-      const int yi = y - (row << bhl);
-      int g = gr[(r00 + yi) * kGW + c00];
-      if (left) g = blend_w(gr[(r10 + yi) * kGW + c10], g, hpw, hcw, bd);
-      if (yi < yStart) {
-        int top = gr[(r01 + yi) * kGW + c01];
-        if (left) top = blend_w(gr[(r11 + yi) * kGW + c11], top, hpw, hcw, bd);
-        const int vpw = sy ? 23 : (yi == 1 ? 17 : 27), vcw = sy ? 22 : (yi == 1 ? 27 : 17);
-        g = blend_w(top, g, vpw, vcw, bd);
-      }
-      gv[k] = g;
-      if (plane != 0) {
-        // chromaScalingIndex (apply.go:501-520) on the un-grained luma.
-        const T* lrow = row_ptr<T>(lp, y << sy);
-        const int lx = x << sx;
-        int avg = lrow[lx];
-        if (sx && !(oddLuma && x == sp.w - 1)) avg = (avg + lrow[lx + 1] + 1) >> 1;
-        lv[k] = avg;
-      }
-    }
+      typename Q::W out = s[r];
+      if (y < yclip) {
+        int gv[4];
 #pragma unroll
-    for (int k = 0; k < kFgRowGroup; k++) {
-      const int y = yg + k;
-      if (y >= yend) break;
-      const int s = sv[k];
-      if (y >= yclip) {
-        row_ptr<T>(dp, y)[x] = (T)s;
-        continue;
-      }
-      int idx;
-      if (plane == 0 || cfl) {
-        idx = plane == 0 ? s : lv[k];
-      } else {
-        const int combined = lv[k] * lumaMult + s * mult;
-        idx = iclip((combined >> 6) + offs0, 0, (1 << bd) - 1);
-      }
-      const int scale = scale_lut(lut, idx, bd);
-      const int noise = rpow2(scale * gv[k], shift);
-      row_ptr<T>(dp, y)[x] = (T)iclip(s + noise, minV, maxV);
-    }
-  }
-}
-
-// fg_apply_col for four adjacent columns x .. x + 3 (x a multiple of 4,
-// 8-bit planes): the four samples of a row are read and written as one
-// 32-bit word, and the block set-up (offsets, template positions, blend
-// weights) is shared by the four columns, which always lie in one grain
-// block.  Planes whose rows are not 4-byte aligned, or a quad reaching past
-// the allocated width, go column by column.
-__device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& disp, const FgArgs& a,
-                                              const uint8_t* lut, int plane, int x, int y0, int nrows) {
-  const DPlane sp = ref.pl[plane];
-  const DPlane dp = disp.pl[plane];
-  if (x >= sp.aw) return;
-  const DPlane lp = ref.pl[0];
-  const uintptr_t al = reinterpret_cast<uintptr_t>(sp.ptr) | (uintptr_t)sp.stride |
-                       reinterpret_cast<uintptr_t>(dp.ptr) | (uintptr_t)dp.stride |
-                       reinterpret_cast<uintptr_t>(lp.ptr) | (uintptr_t)lp.stride;
-  if (x + 4 > sp.aw || (al & 3)) {
+        for (int j = 0; j < 4; j++) gv[j] = grain_of(g[r], j);
+        if (xStart | yStart) {
+          // Overlap (apply.go:301-343): horizontal weights 27/17 then 17/27
+          // (subsampled 23/22), vertical ones the same by row.
+          if (xStart) {
+            const int o10 = offs[-1];
+            const int c10 = gcol(o10, 1), r10 = grow(o10, 0) + k;
 #pragma unroll
-    for (int k = 0; k < 4; k++) fg_apply_col<uint8_t, 1>(ref, disp, a, lut, plane, x + k, y0, nrows);
-    return;
-  }
-  const int yend = imin(y0 + nrows, sp.ah);
-  auto word = [](const DPlane& p, int y, int xx) { return reinterpret_cast<uint32_t*>(row_ptr<uint8_t>(p, y) + xx); };
-  if (!a.active[plane] || x >= sp.w) {
-    for (int y = y0; y < yend; y++) *word(dp, y, x) = *word(sp, y, x);
-    return;
-  }
-  const int sx = plane ? ref.ssx : 0, sy = plane ? ref.ssy : 0;
-  const int bwl = 5 - sx, bhl = 5 - sy;
-  const int bw = 1 << bwl, bh = 1 << bhl;
-  const int row = y0 >> bhl, bcol = x >> bwl;
-  const int xi = x - (bcol << bwl);
-  const int ovl = 2;
-  const int xStart = (a.overlap && bcol > 0) ? imin(sp.w - (bcol << bwl), ovl >> sx) : 0;
-  const int yStart = (a.overlap && row > 0) ? imin(sp.h - (row << bhl), ovl >> sy) : 0;
-  const uint8_t* offs = a.offsets + row * a.off_cols + bcol;
-  const int16_t* gr = a.grain[plane];
-  auto gcol = [&](int offset, int bc) { return 3 + (ovl >> sx) * (3 + (offset >> 4)) + xi + bw * bc; };
-  auto grow = [&](int offset, int br) { return 3 + (ovl >> sy) * (3 + (offset & 15)) + bh * br; };
-  const int o00 = offs[0];
-  const int c00 = gcol(o00, 0), r00 = grow(o00, 0);
-  const bool left = xi < xStart;  // only column xi (and xi + 1 for luma) of the first quad of a block
-  int c10 = 0, r10 = 0, c01 = 0, r01 = 0, c11 = 0, r11 = 0;
-  if (left) {
-    const int o10 = offs[-1];
-    c10 = gcol(o10, 1);
-    r10 = grow(o10, 0);
-  }
-  if (yStart > 0) {
-    const int o01 = offs[-a.off_cols];
-    c01 = gcol(o01, 0);
-    r01 = grow(o01, 1);
-    if (left) {
-      const int o11 = offs[-a.off_cols - 1];
-      c11 = gcol(o11, 1);
-      r11 = grow(o11, 1);
-    }
-  }
-  const int shift = a.scaling_shift;
-  int minV = 0, maxV = 255;
-  if (a.clip_restricted) {
-    minV = 16;
-    maxV = plane == 0 ? 235 : (a.matrix_identity ? 235 : 240);
-  }
-  const int yclip = imin(yend, sp.h);
-  const bool cfl = a.cfl, oddLuma = a.odd_luma;
-  const int lumaMult = a.luma_mult[plane] - 128, mult = a.mult[plane] - 128;
-  const int offs0 = a.offset[plane] - 256;
-  for (int y = y0; y < yend; y++) {
-    const uint32_t s4 = *word(sp, y, x);
-    if (y >= yclip) {
-      *word(dp, y, x) = s4;
-      continue;
-    }
-    const int yi = y - (row << bhl);
-    // The co-located luma of the four chroma samples: 8 bytes (4:2:x) or 4,
-    // the second word only when a column it serves is inside the crop.
-    uint32_t l0 = 0, l1 = 0;
-    if (plane != 0) {
-      l0 = *word(lp, y << sy, x << sx);
-      if (sx && x + 2 < sp.w) l1 = *word(lp, y << sy, (x << sx) + 4);
-    }
-    const int16_t* g00 = gr + (r00 + yi) * kGW + c00;
-    uint32_t out = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int s = (s4 >> (8 * k)) & 0xff;
-      int o = s;
-      if (x + k < sp.w) {
-        const bool lk = xi + k < xStart;
-        const int hpw = sx ? 23 : (xi + k == 1 ? 17 : 27), hcw = sx ? 22 : (xi + k == 1 ? 27 : 17);
-        int g = g00[k];
-        if (lk) g = blend_w(gr[(r10 + yi) * kGW + c10 + k], g, hpw, hcw, 8);
-        if (yi < yStart) {
-          int top = gr[(r01 + yi) * kGW + c01 + k];
-          if (lk) top = blend_w(gr[(r11 + yi) * kGW + c11 + k], top, hpw, hcw, 8);
-          const int vpw = sy ? 23 : (yi == 1 ? 17 : 27), vcw = sy ? 22 : (yi == 1 ? 27 : 17);
-          g = blend_w(top, g, vpw, vcw, 8);
-        }
-        int idx;
-        if (plane == 0) {
-          idx = s;
-        } else {
-          // chromaScalingIndex (apply.go:501-520) on the un-grained luma.
-          int avg;
-          if (sx) {
-            const uint32_t lw = k < 2 ? l0 : l1;
-            const int b0 = (lw >> (16 * (k & 1))) & 0xff, b1 = (lw >> (16 * (k & 1) + 8)) & 0xff;
-            avg = (oddLuma && x + k == sp.w - 1) ? b0 : (b0 + b1 + 1) >> 1;
-          } else {
-            avg = (l0 >> (8 * k)) & 0xff;
+            for (int j = 0; j < ovl; j++)
+              if (j < xStart) {
+                const int hpw = sx ? 23 : (j == 1 ? 17 : 27), hcw = sx ? 22 : (j == 1 ? 27 : 17);
+                gv[j] = blend_w(gr[r10 * kGW + c10 + j], gv[j], hpw, hcw, bd);
+              }
           }
-          idx = cfl ? avg : iclip(((avg * lumaMult + s * mult) >> 6) + offs0, 0, 255);
+          if (k < yStart) {
+            const int vpw = sy ? 23 : (k == 1 ? 17 : 27), vcw = sy ? 22 : (k == 1 ? 27 : 17);
+            const int o01 = offs[-a.off_cols];
+            const uint2 t = grain4<kSx>(gr + (grow(o01, 1) + k) * kGW, gcol(o01, 0));
+            int tv[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) tv[j] = grain_of(t, j);
+            if (xStart) {
+              const int o11 = offs[-a.off_cols - 1];
+              const int c11 = gcol(o11, 1), r11 = grow(o11, 1) + k;
+#pragma unroll
+              for (int j = 0; j < ovl; j++)
+                if (j < xStart) {
+                  const int hpw = sx ? 23 : (j == 1 ? 17 : 27), hcw = sx ? 22 : (j == 1 ? 27 : 17);
+                  tv[j] = blend_w(gr[r11 * kGW + c11 + j], tv[j], hpw, hcw, bd);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) gv[j] = blend_w(tv[j], gv[j], vpw, vcw, bd);
+          }
         }
-        const int noise = rpow2(lut[idx] * g, shift);
-        o = iclip(s + noise, minV, maxV);
+        int o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int v = Q::get(s[r], j);
+          int idx = v;
+          if (!kLuma) {
+            // chromaScalingIndex (apply.go:501-520) on the un-grained luma.
+            int avg;
+            if (kSx) {
+              const typename Q::W& lw = l[r][j >> 1];
+              const int b0 = Q::get(lw, 2 * (j & 1)), b1 = Q::get(lw, 2 * (j & 1) + 1);
+              avg = (b0 + b1 + 1) >> 1;
+              if (edge && j == oddCol) avg = b0;
+            } else {
+              avg = Q::get(l[r][0], j);
+            }
+            idx = cfl ? avg : __viaddmin_s32_relu((avg * lumaMult + v * mult) >> 6, offs0, top);
+          }
+          if (sizeof(T) == 2) idx = imin(idx, top);
+          const int noise = (int)(lut[idx] * gv[j] + rnd) >> shift;
+          o[j] = __viaddmin_s32_relu(v, noise, maxV);
+        }
+        if (minV) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) o[j] = imax(o[j], minV);
+        }
+        if (edge) {
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (x + j >= sp.w) o[j] = Q::get(s[r], j);
+        }
+        out = Q::pack(o[0], o[1], o[2], o[3]);
       }
-      out |= (uint32_t)o << (8 * k);
+      Q::store(reinterpret_cast<T*>(drow + k * dp.stride), out, word, n);
     }
-    *word(dp, y, x) = out;
   }
 }
 
@@ -637,15 +607,27 @@ __global__ void __launch_bounds__(64) k_fg_offsets_batch(BatchArgs b) {
   for_each_item(b, ST_FG_OFFSETS, [&](int item) {
     const int fi = find_frame(base, b.n, item);
     const FrameJob& J = b.jobs[fi];
-    const int r = (item - base[fi]) * 64 + threadIdx.x;
+    int local = item - base[fi];
+    if (J.io.bd > 8) {
+      // The first items of a frame of more than 8 bits build its scaling
+      // tables, 256 entries each.
+      const int per = 1 << (J.io.bd - 8);
+      if (local < 3 * per) {
+        const int pl = local / per, i0 = (local - pl * per) * 256;
+        for (int i = threadIdx.x; i < 256; i += 64)
+          J.fg.scale[pl * kFgScaleLen + i0 + i] = (uint8_t)scale_at(J.fg.lut[pl], i0 + i, J.io.bd);
+        return;
+      }
+      local -= 3 * per;
+    }
+    const int r = local * 64 + threadIdx.x;
     if (r < J.fg.off_rows) fg_offsets_row(J.fgt.seed, r, J.fg.off_cols, const_cast<uint8_t*>(J.fg.offsets));
   });
 }
 
-// Display frame: 64x64-sample tiles of each plane, 256 threads x 16 rows (a
-// thread's rows stay inside one grain block: blocks are 32 or 16 rows high,
-// and a thread's per-column set-up is spread over 16 samples).
-// The plane's scaling table is staged in shared memory per tile.
+// Display frame: 64x64-sample tiles of each plane, 256 threads of four
+// columns by four rows.  The plane's scaling table is staged in shared memory
+// per tile.
 struct FgTile {
   const FrameJob* J;
   int plane, tx, ty;
@@ -663,39 +645,75 @@ __device__ __forceinline__ FgTile fg_locate(const BatchArgs& b, const int* base,
   return FgTile{&J, plane, local % J.fg_tx[plane], local / J.fg_tx[plane]};
 }
 
-// kGroup rows per load group (fg_apply_col); one row at a time keeps 40
-// registers (6 CTAs per SM), groups of 2 or 4 need 64 (4 CTAs per SM).
-// kGroup 0: four columns by four rows a thread (fg_apply_quad, 8-bit).
-template <bool kLoop, int kGroup>
-__global__ void __launch_bounds__(256, kGroup == 1 ? 6 : 4) k_fg_apply_batch(BatchArgs b) {
-  __shared__ uint8_t s_lut[256];
+// A quad of a plane whose rows are not on word boundaries, or one that
+// reaches past the allocated width.
+template <typename T, bool kLuma, bool kSx>
+__device__ __noinline__ void fg_apply_any(const FrameJob* J, const uint8_t* lut, int plane, int x, int y0) {
+  fg_apply_quad<T, kLuma, kSx, 1>(J->io, J->disp, J->fg, lut, plane, x, y0, false);
+}
+
+template <typename T, bool kLuma, bool kSx, int kRows>
+__device__ __forceinline__ void fg_apply_plane(const FrameJob& J, const uint8_t* lut, int plane, int x, int y0) {
+  const DPlane &sp = J.io.pl[plane], &dp = J.disp.pl[plane], &lp = J.io.pl[0];
+  if (x >= sp.aw || y0 >= sp.ah) return;
+  if (x + 4 <= sp.aw &&
+      ((reinterpret_cast<uintptr_t>(sp.ptr) | (uintptr_t)sp.stride | reinterpret_cast<uintptr_t>(dp.ptr) |
+        (uintptr_t)dp.stride | reinterpret_cast<uintptr_t>(lp.ptr) | (uintptr_t)lp.stride) &
+       (4 * sizeof(T) - 1)) == 0)
+    fg_apply_quad<T, kLuma, kSx, kRows>(J.io, J.disp, J.fg, lut, plane, x, y0, true);
+  else
+    fg_apply_any<T, kLuma, kSx>(&J, lut, plane, x, y0);
+}
+
+template <typename T, int kRows>
+__device__ __forceinline__ void fg_tile(const FgTile& t, uint8_t* lut) {
+  const FrameJob& J = *t.J;
+  const int tid = threadIdx.x;
+  if (sizeof(T) == 1) {
+    lut[tid] = J.fg.lut[t.plane][tid];
+  } else if (J.fg.active[t.plane]) {
+    const uint4* src = reinterpret_cast<const uint4*>(J.fg.scale + t.plane * kFgScaleLen);
+    if (tid < 1 << (J.io.bd - 4)) reinterpret_cast<uint4*>(lut)[tid] = src[tid];
+  }
+  __syncthreads();
+  // Quads of the tile: first those inside their blocks, four rows at a
+  // time, then (the last one or two warps) those on a block's left edge.
+  const bool sx = t.plane && J.io.ssx;
+  const int per = sx ? 12 : 14;  // inside quads a row: 3 of 4 or 7 of 8
+  int q, rg;
+  if (tid < per * 16) {
+    rg = sx ? tid / 12 : tid / 14;
+    const int i = tid - rg * per;
+    q = sx ? i + i / 3 + 1 : i + i / 7 + 1;
+  } else {
+    const int i = tid - per * 16;
+    rg = sx ? i >> 2 : i >> 1;
+    q = sx ? (i & 3) * 4 : (i & 1) * 8;
+  }
+  const int x = t.tx * 64 + 4 * q, y0 = t.ty * 64 + 4 * rg;
+  if (t.plane == 0)
+    fg_apply_plane<T, true, false, kRows>(J, lut, 0, x, y0);
+  else if (sx)
+    fg_apply_plane<T, false, true, kRows>(J, lut, t.plane, x, y0);
+  else
+    fg_apply_plane<T, false, false, kRows>(J, lut, t.plane, x, y0);
+}
+
+// kRows: rows of a thread's four whose loads go out together (the grain
+// group's tile setting).
+template <bool kLoop, int kRows>
+__global__ void __launch_bounds__(256, 4) k_fg_apply_batch(BatchArgs b) {
+  __shared__ __align__(16) uint8_t s_lut[kFgScaleLen];
   const int* base = b.base + ST_FG_APPLY * (b.n + 1);
   for_each_item<kLoop>(
       b, ST_FG_APPLY,
       [&](int item) {
         const FgTile t = fg_locate(b, base, item);
-        const FrameJob& J = *t.J;
-        s_lut[threadIdx.x] = J.fg.lut[t.plane][threadIdx.x];
-        __syncthreads();
-        if constexpr (kGroup == 0) {
-          // Four columns by four rows a thread.
-          const int x = t.tx * 64 + (threadIdx.x & 15) * 4;
-          const int y0 = t.ty * 64 + (threadIdx.x >> 4) * 4;
-          if (J.io.bd == 8) {
-            fg_apply_quad(J.io, J.disp, J.fg, s_lut, t.plane, x, y0, 4);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++) fg_apply_col<uint16_t, 1>(J.io, J.disp, J.fg, s_lut, t.plane, x + k, y0, 4);
-          }
-        } else {
-          const int x = t.tx * 64 + (threadIdx.x & 63);
-          const int y0 = t.ty * 64 + (threadIdx.x >> 6) * 16;
-          if (J.io.bd == 8)
-            fg_apply_col<uint8_t, kGroup>(J.io, J.disp, J.fg, s_lut, t.plane, x, y0, 16);
-          else
-            fg_apply_col<uint16_t, kGroup>(J.io, J.disp, J.fg, s_lut, t.plane, x, y0, 16);
-        }
-        __syncthreads();  // the table is rewritten by the next tile
+        if (t.J->io.bd == 8)
+          fg_tile<uint8_t, kRows>(t, s_lut);
+        else
+          fg_tile<uint16_t, kRows>(t, s_lut);
+        if (kLoop) __syncthreads();  // the table is rewritten by the next tile
       },
       [&](int item) {
         // The tile of the filtered frame (the grain's input).
@@ -796,26 +814,21 @@ cudaError_t launch_fg_offsets_batch(const BatchArgs& b, int total, int grid, cud
   return cudaGetLastError();
 }
 
+template <int kRows>
+static void launch_fg_apply_rows(const BatchArgs& b, int grid, cudaStream_t st) {
+  static int wave = 0;
+  if (batch_loops(b))
+    k_fg_apply_batch<true, kRows><<<grid, 256, 0, st>>>(b);
+  else
+    k_fg_apply_batch<false, kRows><<<grid, 256, 0, st>>>(with_wave(b, k_fg_apply_batch<false, kRows>, 256, 0, wave));
+}
+
 cudaError_t launch_fg_apply_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
   if (total <= 0) return cudaSuccess;
-  const bool loop = batch_loops(b);
-  static int w0 = 0, w1 = 0, w2 = 0, w4 = 0;
   switch (b.tile) {
-    case 3:
-      loop ? k_fg_apply_batch<true, 0><<<grid, 256, 0, st>>>(b)
-           : k_fg_apply_batch<false, 0><<<grid, 256, 0, st>>>(with_wave(b, k_fg_apply_batch<false, 0>, 256, 0, w0));
-      break;
-    case 1:
-      loop ? k_fg_apply_batch<true, 2><<<grid, 256, 0, st>>>(b)
-           : k_fg_apply_batch<false, 2><<<grid, 256, 0, st>>>(with_wave(b, k_fg_apply_batch<false, 2>, 256, 0, w2));
-      break;
-    case 2:
-      loop ? k_fg_apply_batch<true, 4><<<grid, 256, 0, st>>>(b)
-           : k_fg_apply_batch<false, 4><<<grid, 256, 0, st>>>(with_wave(b, k_fg_apply_batch<false, 4>, 256, 0, w4));
-      break;
-    default:
-      loop ? k_fg_apply_batch<true, 1><<<grid, 256, 0, st>>>(b)
-           : k_fg_apply_batch<false, 1><<<grid, 256, 0, st>>>(with_wave(b, k_fg_apply_batch<false, 1>, 256, 0, w1));
+    case 1: launch_fg_apply_rows<2>(b, grid, st); break;
+    case 2: launch_fg_apply_rows<1>(b, grid, st); break;
+    default: launch_fg_apply_rows<4>(b, grid, st);
   }
   return cudaGetLastError();
 }

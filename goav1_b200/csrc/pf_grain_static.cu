@@ -38,12 +38,14 @@ using namespace pf;
 
 namespace {
 
-// Scratch layout (bytes): [job record | stage table | 3 grain templates | offsets].
+// Scratch layout (bytes): [job record | stage table | 3 grain templates |
+// scaling tables | offsets].
 constexpr size_t kJobBytes = 8192;
 constexpr size_t kBaseOff = kJobBytes;
 constexpr size_t kGrainOff = kBaseOff + 256;
-constexpr size_t kGrainBytes = 36096;  // 3 * 82 * 73 int16, rounded up to 256
-constexpr size_t kOffsetsOff = kGrainOff + kGrainBytes;
+constexpr size_t kGrainBytes = (3 * kGrainLen * sizeof(int16_t) + 255) / 256 * 256;
+constexpr size_t kScaleOff = kGrainOff + kGrainBytes;
+constexpr size_t kOffsetsOff = kScaleOff + 3 * kFgScaleLen;
 static_assert(sizeof(FrameJob) <= kJobBytes, "job record does not fit its scratch slot");
 static_assert(kOffsetsOff + PF_GRAIN_STATIC_MAX_BLOCKS <= PF_GRAIN_STATIC_SCRATCH_BYTES, "scratch too small");
 
@@ -149,9 +151,10 @@ extern "C" int pf_film_grain_static(const pf_frame* ref, const pf_film_grain* fg
   if (on) {
     int16_t* grain = (int16_t*)(scratch + kGrainOff);
     for (int p = 0; p < 3; p++) {
-      a.grain[p] = grain + p * 82 * 73;
+      a.grain[p] = grain + p * kGrainLen + kGrainShift(p && ref->ss_x);
       a.active[p] = act[p];
     }
+    a.scale = scratch + kScaleOff;
     a.offsets = scratch + kOffsetsOff;
     a.off_rows = rows;
     a.off_cols = cols;
@@ -189,7 +192,7 @@ extern "C" int pf_film_grain_static(const pf_frame* ref, const pf_film_grain* fg
     t.ssx = ref->ss_x;
     t.ssy = ref->ss_y;
     counts[ST_FG_TEMPLATES] = 1;
-    counts[ST_FG_OFFSETS] = (rows + 63) / 64;
+    counts[ST_FG_OFFSETS] = (rows + 63) / 64 + (ref->bit_depth > 8 ? 3 << (ref->bit_depth - 8) : 0);
   }
   int tiles = 0;
   for (int p = 0; p < (ref->mono ? 1 : 3); p++) {

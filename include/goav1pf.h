@@ -328,11 +328,9 @@ int pf_batch_apply(pf_ctx* ctx, const pf_batch_item* items, int32_t n, pf_stats*
  *                      inside the chunk (then below units_per_cta);
  *       tile           deblocking: the tile shape, 0 = 32x8, 1 = 64x4,
  *                      2 = 16x16, 3 = 8x32 edge units a tile (one thread
- *                      each); grain apply: rows of a column whose loads are
- *                      issued together, 0 = 1 (40 registers, 6 CTAs per SM),
- *                      1 = 2, 2 = 4 (64 registers, 4 CTAs per SM), 3 = four
- *                      columns by four rows a thread, 8-bit samples moved as
- *                      32-bit words (64 registers); 0 for the other groups.
+ *                      each); grain apply: how many of a thread's four rows
+ *                      have their loads issued together, 0 and 3 = four,
+ *                      1 = two, 2 = one; 0 for the other groups.
  *     Work items are independent, so every schedule gives the same samples.
  * pf_autotune searches the schedule of each group on a given batch, one
  * dimension at a time (tile setting, units per CTA, staging depth, persistent
