@@ -816,7 +816,11 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
     int tiles = 0;
     for (int p = 0; p < (f->mono ? 1 : 3); p++) {
       const int sx = p ? f->ss_x : 0, sy = p ? f->ss_y : 0;
-      const int PW = 64 >> sx, SH = 64 >> sy, off = 8 >> sy;
+      // Units are powers of two and tiles start at multiples of their width,
+      // so a tile no wider than a unit has one unit.
+      const int SH = 64 >> sy, off = 8 >> sy;
+      const int PW = lrOn && s->lr.type[p] != PF_LR_NONE && J.lr.unit_size[p] < 64 ? 64 >> sx : 64;
+      J.lr.tile_w[p] = PW;
       J.lr_cols[p] = (J.aw[p] + PW - 1) / PW;
       J.lr_rows[p] = (J.ah[p] + off + SH - 1) / SH;
       tiles += J.lr_cols[p] * J.lr_rows[p];
@@ -1146,7 +1150,15 @@ static void add_stats(const pf_ctx* c, int n, uint32_t done, pf_stats* stats) {
   auto total = [&](int k) { return c->hbase[(size_t)k * (n + 1) + n]; };
   stats->completed |= done;
   stats->cdef_units += total(ST_CDEF);
-  stats->lr_units += total(ST_LR);
+  // Restoration units are counted as the reference's processing units (64
+  // luma samples wide), whatever the tiles' width.
+  for (int i = 0; i < n; i++) {
+    const FrameJob& J = c->hjobs[i];
+    for (int p = 0; p < 3; p++) {
+      const int pw = 64 >> (p ? J.io.ssx : 0);
+      stats->lr_units += (J.aw[p] + pw - 1) / pw * J.lr_rows[p];
+    }
+  }
   for (int i = 0; i < n; i++) stats->fg_rows += (c->hjobs[i].fg.off_rows + 63) / 64;
 }
 

@@ -119,6 +119,7 @@ struct LrArgs {
   int type[3];          // frame type per plane
   int unit_size[3];
   int horz[3], vert[3];
+  int tile_w[3];        // width of a tile: 64 where a 64-wide one lies in one unit, else the processing width
   const uint8_t* lines[3];
   int64_t line_stride[3];
 };

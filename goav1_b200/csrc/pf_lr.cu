@@ -1,6 +1,6 @@
 // pf_lr.cu - loop restoration (Wiener / SGRproj) on the GPU.
 //
-// One CTA per (64-wide processing column, restoration stripe, plane).  The
+// One CTA per (64-wide column, restoration stripe, plane).  The
 // geometry is goav1's: tile/restoration_schedule.go:61-109, :400-409 (unit
 // grid), tile/restoration_geometry.go:54-236 (unit rects shifted up by 8/4
 // rows, stripes of 64/32 rows with the first one 8/4 rows shorter, 64-wide
@@ -18,55 +18,110 @@
 // Every sample of the tile inside the MI-aligned plane is written to the
 // destination: restored samples where a Wiener/SGR unit covers the cropped
 // plane, the post-CDEF sample everywhere else.
+//
+// Bound by instruction issue (76 % of the slots; both integer pipes about 60 %
+// busy, DRAM 4 %), so the filters work on whole words: sample pairs for the
+// sums and products (dp4a squares of 8-bit samples, dp2a for two Wiener
+// taps), one word for an SGR box's a and b, two output columns a thread; and
+// chroma tiles are as wide as luma's where their unit is, since a 32x32 tile
+// cost a CTA's set-up for a quarter of the samples.  us per frame: 60 x 1080p
+// 8-bit, a third of the units of each kind, 18.9 before, 10.4 now (7.6 and
+// 4.4 warp instructions per luma sample); 8 x 4K 10-bit 78.9 and 44.9; one
+// 1080p frame 28.7 and 20.6.  The encoder's search at 1080p: 144 and 68 us.
 #include "pf_common.cuh"
 #include "pf_tables.h"
 
 namespace pf {
 
 __constant__ int16_t c_sgr_params[16][4];
-__constant__ uint16_t c_x_by_xplus1[256];
-__constant__ uint16_t c_one_by_x[25];
+__constant__ uint8_t c_xbx[256];  // a - 1 by z: x / (x + 1) in 1/256, less one
 
-constexpr int kWin = 70;  // 64 + 2*3
-constexpr int kLrMaxRun = 16;  // rows of one thread's output run (see lr_wiener_window)
+// ---- the staged window and the two filters ----
+//
+// The window holds a tile (at most 64x64) with its 3-sample halo as 16-bit
+// samples: sample (x, y) of the tile at row y + 3, column x + 4, so that a
+// sample pair starting on an even x is one word, four samples of the frame
+// are two, and every table below is built from whole words.
+constexpr int kWinRows = 70;
+constexpr int kWinWords = 36;  // 72 columns: x = -4 .. 67
+constexpr int kTabPitch = 68;  // SGR tables: column x at x + 1, x = -1 .. 64
 
 struct LrSmem {
-  uint16_t win[kWin * kWin];
+  alignas(16) uint32_t win[kWinRows * kWinWords];
   union {
-    // SGR a (<= 256) / b tables: radius 1 for rows -1..h, radius 2 for the
-    // rows -1, 1, 3, ... it is computed on; columns -1..w.
+    // SGR a and b of one box in one word, (a - 1) << 22 | b (a - 1 <= 255, b
+    // <= 256 * 4095), so that the sum of three neighbours is one addition
+    // chain: radius 1 for rows -1..h, radius 2 for the rows -1, 1, 3, ... it
+    // is computed on.
     struct {
-      uint16_t A1[66 * 66];
-      int32_t B1[66 * 66];
-      uint16_t A2[33 * 66];
-      int32_t B2[33 * 66];
+      uint32_t t1[66 * kTabPitch];
+      uint32_t t2[33 * kTabPitch];
     } sgr;
-    uint16_t wtemp[kWin * 64];  // Wiener row-pass output, (h+6) x 64
+    uint32_t wt[35 * 64];  // Wiener row-pass output as vertical pairs: rows 2k and 2k + 1 of a column
   };
-  uint16_t x_by_xplus1[256];  // data-dependent lookup: smem, not constant memory
+  uint8_t xbx[256];  // a - 1 by z: data-dependent lookup, so shared memory and not constant
 };
 
 __device__ __forceinline__ int32_t rpot(int32_t v, int bits) {
   return bits <= 0 ? v : (v + (int32_t)(1 << (bits - 1))) >> bits;
 }
-__device__ __forceinline__ uint32_t rpotu(uint32_t v, int bits) {
-  return bits <= 0 ? v : (v + (1u << (bits - 1))) >> bits;
+
+// How a CTA shares a tile's output: thread tid has the column pair
+// x = 2 * (tid % (PW / 2)) over a run of an even number of rows.
+struct LrRun {
+  int x, ya, yb;
+};
+__device__ __forceinline__ LrRun lr_run(int h, int PW) {
+  const int lg = PW == 64 ? 5 : 4, segs = 256 >> lg;
+  const int rows = ((h + segs - 1) / segs + 1) & ~1;
+  const int ya = (threadIdx.x >> lg) * rows;
+  return LrRun{2 * (int)(threadIdx.x & ((1 << lg) - 1)), ya, imin(h, ya + rows)};
 }
 
-// Wiener filter of the staged window (restoration/wiener.go:132-211): the
-// block's sample (0,0) sits at sm.win[3 * kWin + 3], w x h <= 64 x 64, with
-// the 3-sample halo around it.  hf/vf are the 7 horizontal / vertical taps.
-// out(y, x, v) receives every output sample; thread tid produces column
-// x = tid % PW over a run of consecutive rows (the h rows split into 256 / PW
-// runs).  Every thread of the CTA calls it; it leaves the window untouched
-// and ends without a barrier.
+// The symmetric 7-tap filter of a pair of neighbours from packed sample
+// pairs: `in` holds the eight samples s0..s7 as four words when kEven (the
+// first output is s0..s6's, the second s1..s7's), and s-1..s8 as five
+// otherwise (s0 in the first word's upper half).  Two taps are one dp2a; the
+// centre tap can exceed its 8-bit operand and is a multiplication of its own.
+struct WienerTaps {
+  int t01, t12, t2, t0, t0h, t2h, t21, t10, c;
+};
+__device__ __forceinline__ WienerTaps wiener_taps(int f0, int f1, int f2) {
+  auto two = [](int lo, int hi) { return (lo & 0xff) | (hi & 0xff) << 8; };
+  return WienerTaps{two(f0, f1), two(f1, f2), two(f2, 0), two(f0, 0), two(0, f0),
+                    two(0, f2),  two(f2, f1), two(f1, f0), 128 - 2 * (f0 + f1 + f2)};
+}
+// Two unsigned 16-bit samples times two signed 8-bit taps, added to c.
+__device__ __forceinline__ int dp2a_us(uint32_t a, int b, int c) {
+  int d;
+  asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+// Samples s0..s6 with s0 in a word's lower half: words (s0 s1)(s2 s3)(s4 s5)(s6 -).
+__device__ __forceinline__ int wiener_low(const WienerTaps& f, uint32_t a, uint32_t b, uint32_t c, uint32_t d, int init) {
+  int s = dp2a_us(a, f.t01, init);
+  s = dp2a_us(b, f.t2, s);
+  s = dp2a_us(c, f.t21, s);
+  s = dp2a_us(d, f.t0, s);
+  return s + (int)(b >> 16) * f.c;
+}
+// Samples s0..s6 with s0 in a word's upper half: (- s0)(s1 s2)(s3 s4)(s5 s6).
+__device__ __forceinline__ int wiener_high(const WienerTaps& f, uint32_t a, uint32_t b, uint32_t c, uint32_t d, int init) {
+  int s = dp2a_us(a, f.t0h, init);
+  s = dp2a_us(b, f.t12, s);
+  s = dp2a_us(c, f.t2h, s);
+  s = dp2a_us(d, f.t10, s);
+  return s + (int)(c & 0xffffu) * f.c;
+}
+
+// Wiener filter of the staged window (restoration/wiener.go:132-211), w x h
+// <= 64 x 64; h and v are the first three horizontal / vertical taps.
+// out(y, x, v0, v1) receives the outputs of columns x and x + 1 (x even; the
+// second is past the tile when x + 1 == w).  Every thread of the CTA calls
+// it; it leaves the window untouched and ends without a barrier.
 template <class Out>
-__device__ __forceinline__ void lr_wiener_window(LrSmem& sm, int w, int h, int bd, const int* hf, const int* vf, int PW,
-                                 Out&& out) {
-  const uint16_t* s_win = sm.win;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tid = threadIdx.x, tx = tid % PW, ty0 = tid / PW, rpg = (h + 256 / PW - 1) / (256 / PW);
-  const int wh = h + 6;
+__device__ __forceinline__ void lr_wiener_window(LrSmem& sm, int w, int h, int bd, const int8_t* hf, const int8_t* vf,
+                                                 int PW, Out&& out) {
   const int maxv = (1 << bd) - 1;
   // restoration/wiener.go:202-211 (wienerRounds), :132-196.
   int round0 = 3, round1 = 11;
@@ -75,222 +130,262 @@ __device__ __forceinline__ void lr_wiener_window(LrSmem& sm, int w, int h, int b
     round0 += range - 16;
     round1 -= range - 16;
   }
-  const int32_t limit = 1 << (bd + 1 + 7 - round0);
-  const int32_t offH = 1 << (bd + 7 - 1);
-  uint16_t* temp = sm.wtemp;  // (h+6) x 64
-  // Row pass: a lane takes the column pair (2 lane, 2 lane + 1) of a row,
-  // its eight window samples read as four aligned 32-bit words (kWin and
-  // the column are even); the taps are symmetric (hf[k] == hf[6 - k]), so
-  // the mirrored samples are summed first.
-  const int hc = hf[3] + 128;
-  for (int r = warp; r < wh; r += 8) {
-    const int c = 2 * lane;
-    if (c < w) {
-      const uint32_t* sw = reinterpret_cast<const uint32_t*>(&s_win[r * kWin + c]);
-      const uint32_t p01 = sw[0], p23 = sw[1], p45 = sw[2], p67 = sw[3];
-      const int32_t v0 = p01 & 0xffff, v1 = p01 >> 16, v2 = p23 & 0xffff, v3 = p23 >> 16;
-      const int32_t v4 = p45 & 0xffff, v5 = p45 >> 16, v6 = p67 & 0xffff, v7 = p67 >> 16;
-      const int32_t s0 = offH + v3 * hc + (v0 + v6) * hf[0] + (v1 + v5) * hf[1] + (v2 + v4) * hf[2];
-      const int32_t s1 = offH + v4 * hc + (v1 + v7) * hf[0] + (v2 + v6) * hf[1] + (v3 + v5) * hf[2];
-      const uint32_t o0 = (uint32_t)imin(imax(rpot(s0, round0), 0), limit - 1);
-      const uint32_t o1 = (uint32_t)imin(imax(rpot(s1, round0), 0), limit - 1);
-      *reinterpret_cast<uint32_t*>(&temp[r * 64 + c]) = o0 | (o1 << 16);
-    }
+  const int top = (1 << (bd + 1 + 7 - round0)) - 1;
+  // Row pass: a thread takes two rows of a column pair and leaves each
+  // column's two results as one word.
+  {
+    const WienerTaps f = wiener_taps(hf[0], hf[1], hf[2]);
+    const int init = (1 << (bd + 6)) + (1 << (round0 - 1));
+    const int lg = PW == 64 ? 5 : 4;
+    const int xw = threadIdx.x & ((1 << lg) - 1), step = 256 >> lg;
+    if (2 * xw < w)
+      for (int k = threadIdx.x >> lg; 2 * k < h + 6; k += step) {
+        int o[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          const uint32_t* p = &sm.win[(2 * k + r) * kWinWords + xw];
+          const uint32_t a = p[0], b = p[1], c = p[2], d = p[3], e = p[4];
+          o[r][0] = __vimin_s32_relu(wiener_high(f, a, b, c, d, init) >> round0, top);
+          o[r][1] = __vimin_s32_relu(wiener_low(f, b, c, d, e, init) >> round0, top);
+        }
+        *reinterpret_cast<uint2*>(&sm.wt[k * 64 + 2 * xw]) =
+            make_uint2(__byte_perm(o[0][0], o[1][0], 0x5410), __byte_perm(o[0][1], o[1][1], 0x5410));
+      }
   }
   __syncthreads();
-  const int32_t offV = 1 << (bd + round1 - 1);
-  // Each thread a run of consecutive output rows of column tx: the seven
-  // vertical taps slide down in registers, one new row read per output.  A
-  // run is at most kLrMaxRun rows (h <= 64 over 4 runs per column at PW 64,
-  // over 8 at PW 32), and the loop is unrolled to that bound so that the
-  // slide is register renaming.
-  const int ya = ty0 * rpg, yb = imin(h, ya + rpg);
-  if (tx < w && ya < yb) {
-    int32_t t[7];
-#pragma unroll
-    for (int k = 0; k < 6; k++) t[k] = temp[(ya + k) * 64 + tx];
-#pragma unroll
-    for (int i = 0; i < kLrMaxRun; i++) {
-      const int y = ya + i;
-      if (y >= yb) break;
-      t[6] = temp[(y + 6) * 64 + tx];
-      int32_t sum = (t[3] << 7) - offV + t[3] * vf[3];
-#pragma unroll
-      for (int k = 0; k < 3; k++) sum += (t[k] + t[6 - k]) * vf[k];
-      out(y, tx, imin(imax(rpot(sum, round1), 0), maxv));
-#pragma unroll
-      for (int k = 0; k < 6; k++) t[k] = t[k + 1];
+  // Column pass: two rows of the column pair at a time from four rows' worth
+  // of words, one of them new.
+  const LrRun t = lr_run(h, PW);
+  if (t.x < w && t.ya < t.yb) {
+    const WienerTaps f = wiener_taps(vf[0], vf[1], vf[2]);
+    const int init = (1 << (round1 - 1)) - (1 << (bd + round1 - 1));
+    const uint32_t* p = &sm.wt[(t.ya >> 1) * 64 + t.x];
+    uint2 a = *reinterpret_cast<const uint2*>(p), b = *reinterpret_cast<const uint2*>(p + 64),
+          c = *reinterpret_cast<const uint2*>(p + 128);
+#pragma unroll 4
+    for (int y = t.ya; y < t.yb; y += 2) {
+      p += 64;
+      const uint2 d = *reinterpret_cast<const uint2*>(p + 128);
+      out(y, t.x, __vimin_s32_relu(wiener_low(f, a.x, b.x, c.x, d.x, init) >> round1, maxv),
+          __vimin_s32_relu(wiener_low(f, a.y, b.y, c.y, d.y, init) >> round1, maxv));
+      if (y + 1 < t.yb)
+        out(y + 1, t.x, __vimin_s32_relu(wiener_high(f, a.x, b.x, c.x, d.x, init) >> round1, maxv),
+            __vimin_s32_relu(wiener_high(f, a.y, b.y, c.y, d.y, init) >> round1, maxv));
+      a = b;
+      b = c;
+      c = d;
     }
   }
 }
 
-// a and b of one SGR box (restoration/selfguided.go:132-231): the box's sum
-// and sum of squares, area N (9 or 25), strength sv.
-template <int N>
-__device__ __forceinline__ void sgr_ab(uint32_t bs, uint32_t bq, int bd, int sv, const uint16_t* xbx, uint16_t* A,
-                                       int32_t* B) {
-  const int32_t sum = (int32_t)bs, sq = (int32_t)bq;
-  const uint32_t av = (uint32_t)rpot(sq, 2 * (bd - 8));
-  const uint32_t bv = (uint32_t)rpot(sum, bd - 8);
-  uint32_t p = 0;
-  if (av * N >= bv * bv) p = av * N - bv * bv;
-  uint32_t z = rpotu(p * (uint32_t)sv, 20);
-  if (z > 255) z = 255;
-  const int32_t a = xbx[z];
-  *A = (uint16_t)a;
-  *B = (int32_t)rpotu((uint32_t)(256 - a) * (uint32_t)sum * (uint32_t)c_one_by_x[N - 1], 12);
+// a and b of one SGR box (restoration/selfguided.go:132-231), packed as in
+// LrSmem: the box's sum and sum of squares, area N (9 or 25), strength sv.
+// 8-bit variances are never negative; deeper ones are rounded first and can be.
+template <int N, bool k8>
+__device__ __forceinline__ uint32_t sgr_ab(uint32_t sum, uint32_t sq, int bd, uint32_t sv, const uint8_t* xbx) {
+  constexpr uint32_t kOneByN = (4096 + N / 2) / N;
+  uint32_t p;
+  if (k8) {
+    p = sq * N - sum * sum;
+  } else {
+    const int32_t av = rpot((int32_t)sq, 2 * (bd - 8)), bv = rpot((int32_t)sum, bd - 8);
+    p = (uint32_t)imax(av * N - bv * bv, 0);
+  }
+  uint32_t z = (p * sv + (1u << 19)) >> 20;
+  z = z < 255u ? z : 255u;
+  const uint32_t a1 = xbx[z];  // a - 1
+  const uint32_t b = ((255u - a1) * sum * kOneByN + 2048u) >> 12;
+  return (a1 << 22) + b;
+}
+
+// Sums over three (h3, q3) and five (h5, q5) columns of one window row around
+// a column pair, of the samples and of their squares: .x of the first column,
+// .y of the second.  8-bit sample sums stay packed in .x (five rows of five
+// fit a half); deeper ones do not fit.
+struct BoxRow {
+  uint2 h3, h5, q3, q5;
+};
+
+template <bool R2, bool k8>
+__device__ __forceinline__ BoxRow box_row(const uint32_t* p) {
+  const uint32_t A = p[0], B = p[1], C = p[2];  // samples x-2 .. x+3
+  BoxRow o;
+  if (k8) {
+    o.h3.x = __byte_perm(A, B, 0x5432) + B + __byte_perm(B, C, 0x5432);
+    o.h5.x = o.h3.x + A + C;
+    // Bytes of a word squared and summed by one dp4a (the upper byte of an
+    // 8-bit sample is a zero to fill with).
+    const uint32_t a3 = __byte_perm(A, B, 0x1642), b3 = __byte_perm(B, C, 0x1420);
+    o.q3 = make_uint2(__dp4a(a3, a3, 0u), __dp4a(b3, b3, 0u));
+    if (R2) {
+      const uint32_t a5 = __byte_perm(A, C, 0x1140), b5 = __byte_perm(A, C, 0x1162);
+      o.q5 = make_uint2(__dp4a(a5, a5, o.q3.x), __dp4a(b5, b5, o.q3.y));
+    }
+  } else {
+    const uint32_t x0 = A & 0xffff, x1 = A >> 16, x2 = B & 0xffff, x3 = B >> 16, x4 = C & 0xffff, x5 = C >> 16;
+    const uint32_t m = x2 * x2 + x3 * x3;
+    o.h3 = make_uint2(x1 + x2 + x3, x2 + x3 + x4);
+    o.q3 = make_uint2(x1 * x1 + m, x4 * x4 + m);
+    if (R2) {
+      o.h5 = make_uint2(x0 + x4 + o.h3.x, x1 + x5 + o.h3.y);
+      o.q5 = make_uint2(x0 * x0 + (x4 * x4 + o.q3.x), x1 * x1 + (x5 * x5 + o.q3.y));
+    }
+  }
+  return o;
+}
+
+// Sums of three rows' pairs, unpacked.
+template <bool k8>
+__device__ __forceinline__ uint2 pair_sum(uint2 a, uint2 b, uint2 c) {
+  const uint32_t x = a.x + b.x + c.x;
+  return k8 ? make_uint2(x & 0xffff, x >> 16) : make_uint2(x, a.y + b.y + c.y);
 }
 
 // Self-guided filter of the staged window (restoration/selfguided.go:111-390)
-// for a parameter set whose radius-2 (R2) and radius-1 (R1) filters are on
-// or off, with the decoded projection weights xq0 / xq1; same window,
-// thread mapping and out() contract as lr_wiener_window.  sm.x_by_xplus1
-// must hold the table.  Ends with a barrier.
+// for a parameter set whose radius-2 (R2) and radius-1 (R1) filters are on or
+// off, with the decoded projection weights xq0 / xq1; the same contract as
+// lr_wiener_window, with a barrier at its end.  sm.xbx must hold the table.
 //
-// Box sums: one sweep down the window for both radii.  A warp takes a chunk
-// of 32 - 2*halo box columns and a segment of box rows; each lane slides the
-// 3-row and 5-row column sums of its window column down the segment (two
-// window loads a row: the rows entering the 5-row sum and leaving the 3-row
-// one; the other two moves reuse the previous row's), and the row sums come
-// from the neighbouring lanes by shuffles.  Radius 1 has a box on every row,
-// radius 2 on the rows -1, 1, 3, ....  Filters: one pass, each thread a run
-// of rows of one column, the a/b neighbourhoods of both radii sliding down
-// in registers, projected straight to out().
-template <bool R2, bool R1, class Out>
-__device__ __forceinline__ void lr_sgr_window_t(LrSmem& sm, int w, int h, int bd, int s2, int s1, int xq0, int xq1,
-                                                int PW, Out&& out) {
-  const uint16_t* s_win = sm.win;
-  uint16_t* A1 = sm.sgr.A1;
-  int32_t* B1 = sm.sgr.B1;
-  uint16_t* A2 = sm.sgr.A2;
-  int32_t* B2 = sm.sgr.B2;
-  const uint16_t* xbx = sm.x_by_xplus1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tid = threadIdx.x, tx = tid % PW, ty0 = tid / PW, rpg = (h + 256 / PW - 1) / (256 / PW);
-  const int ya = ty0 * rpg, yb = imin(h, ya + rpg);
-  const int ww = w + 6;
-  const int maxv = (1 << bd) - 1;
-  constexpr int kHalo = R2 ? 2 : 1;
-  constexpr int kOutPer = 32 - 2 * kHalo;
-  constexpr unsigned kAll = 0xffffffffu;
-  const int nrows = h + 2, ncols = w + 2;
-  const int nch = (ncols + kOutPer - 1) / kOutPer;
-  const int segLen = (nrows + 7) >> 3;  // 8 row segments per column chunk
-  for (int item = warp; item < nch * 8; item += 8) {
-    const int seg = item / nch, q = item - seg * nch;
-    const int cc = q * kOutPer + lane - kHalo;  // box column + 1 of this lane
-    const int wc = cc + 2;                      // its window column
-    const bool colIn = wc >= 0 && wc < ww;
-    const bool store = lane >= kHalo && lane < 32 - kHalo && cc < ncols;
-    const int rs = seg * segLen, re = imin(rs + segLen, nrows);
-    if (rs >= re) continue;
-    auto ld = [&](int r) -> uint32_t { return colIn ? (uint32_t)s_win[r * kWin + wc] : 0u; };
-    // Box row rr (= row + 1) covers window rows rr+1 .. rr+3 (radius 1) and
-    // rr .. rr+4 (radius 2).
-    const uint32_t v0 = ld(rs), v1 = ld(rs + 1), v2 = ld(rs + 2), v3 = ld(rs + 3), v4 = ld(rs + 4);
-    uint32_t c3s = v1 + v2 + v3, c3q = v1 * v1 + v2 * v2 + v3 * v3;
-    uint32_t c5s = c3s + v0 + v4, c5q = c3q + v0 * v0 + v4 * v4;
-    uint32_t enter3 = v4, leave5 = v0;  // window rows rr+4 (enters the 3-row sum) and rr (leaves the 5-row one)
-    for (int rr = rs; rr < re; rr++) {
-      if (R1) {
-        const uint32_t bs = c3s + __shfl_up_sync(kAll, c3s, 1) + __shfl_down_sync(kAll, c3s, 1);
-        const uint32_t bq = c3q + __shfl_up_sync(kAll, c3q, 1) + __shfl_down_sync(kAll, c3q, 1);
-        if (store) sgr_ab<9>(bs, bq, bd, s1, xbx, &A1[rr * 66 + cc], &B1[rr * 66 + cc]);
+// Tables: a thread has a column pair and slides down it two box rows at a
+// time (radius 1 has a box on every row, radius 2 on the rows -1, 1, 3, ...),
+// each window row's 3- and 5-column sums made once for both radii and both
+// columns, the row sums added up from the last few rows' registers.
+// Filters: a thread has a column pair over a run of rows; the three-column
+// sums of a table row are two additions for both columns, and the rows' terms
+// slide down in registers: 6 C + 5 (S - C) = 5 S + C for radius 2, and
+// 4 S(y+1) + 3 (S(y) + S(y+2)) + C(y) + C(y+2) for radius 1.  The tables' a
+// is one less than a; the missing weights (32, or 16 on radius 2's odd rows)
+// and the rounding ride on constants that the additions have room for.
+template <bool R2, bool R1, bool k8, class Out>
+__device__ __forceinline__ void lr_sgr_window_t(LrSmem& sm, int w, int h, int bd, uint32_t s2, uint32_t s1, int xq0,
+                                                int xq1, int PW, Out&& out) {
+  const int tid = threadIdx.x;
+  {
+    const int npairs = (w + 2) / 2 + 1;  // column pairs x = -2, 0, ..
+    const int segs = 256 / npairs, n2 = (h + 3) >> 1, per = (n2 + segs - 1) / segs;
+    const int seg = tid / npairs, p = tid - seg * npairs;
+    const int k0 = seg * per, k1 = imin(n2, k0 + per);
+    if (seg < segs && k0 < k1) {
+      const int c = 2 * p - 1;  // table column of the pair's first
+      const bool c0in = c >= 0 && c <= w + 1, c1 = c + 1 <= w + 1;
+      const uint32_t* win = &sm.win[2 * k0 * kWinWords + p];
+      uint32_t* o1 = &sm.sgr.t1[2 * k0 * kTabPitch + c];
+      uint32_t* o2 = &sm.sgr.t2[k0 * kTabPitch + c];
+      const BoxRow r0 = box_row<R2, k8>(win), r1 = box_row<R2, k8>(win + kWinWords);
+      BoxRow rc = box_row<R2, k8>(win + 2 * kWinWords), rb = r1;
+      auto add2 = [](uint2 a, uint2 b) { return make_uint2(a.x + b.x, a.y + b.y); };
+      uint2 t0{}, u0{};
+      if (R2) {
+        t0 = add2(r0.h5, r1.h5);
+        u0 = add2(r0.q5, r1.q5);
       }
-      if (R2 && (rr & 1) == 0) {
-        const uint32_t bs = c5s + __shfl_up_sync(kAll, c5s, 1) + __shfl_down_sync(kAll, c5s, 1) +
-                            __shfl_up_sync(kAll, c5s, 2) + __shfl_down_sync(kAll, c5s, 2);
-        const uint32_t bq = c5q + __shfl_up_sync(kAll, c5q, 1) + __shfl_down_sync(kAll, c5q, 1) +
-                            __shfl_up_sync(kAll, c5q, 2) + __shfl_down_sync(kAll, c5q, 2);
-        if (store) sgr_ab<25>(bs, bq, bd, s2, xbx, &A2[(rr >> 1) * 66 + cc], &B2[(rr >> 1) * 66 + cc]);
-      }
-      if (rr + 1 < re) {
-        const uint32_t l3 = ld(rr + 1);
+      win += 3 * kWinWords;
+#pragma unroll 1
+      for (int k = k0; k < k1; k++, win += 2 * kWinWords, o1 += 2 * kTabPitch, o2 += kTabPitch) {
+        // Box rows 2k and 2k + 1: window rows 2k .. 2k + 4 are r0, rb, rc, rd, re.
+        const BoxRow rd = box_row<R2, k8>(win), re = box_row<R2, k8>(win + kWinWords);
         if (R1) {
-          c3s += enter3 - l3;
-          c3q += enter3 * enter3 - l3 * l3;
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            const BoxRow &a = r ? rc : rb, &b = r ? rd : rc, &d = r ? re : rd;
+            if (r == 1 && 2 * k + 1 > h + 1) break;
+            const uint2 s = pair_sum<k8>(a.h3, b.h3, d.h3);
+            if (c0in) o1[r * kTabPitch] = sgr_ab<9, k8>(s.x, a.q3.x + b.q3.x + d.q3.x, bd, s1, sm.xbx);
+            if (c1) o1[r * kTabPitch + 1] = sgr_ab<9, k8>(s.y, a.q3.y + b.q3.y + d.q3.y, bd, s1, sm.xbx);
+          }
         }
         if (R2) {
-          const uint32_t e5 = ld(rr + 5);
-          c5s += e5 - leave5;
-          c5q += e5 * e5 - leave5 * leave5;
-          enter3 = e5;
-        } else {
-          enter3 = ld(rr + 4 + 1);
+          const uint2 t1 = add2(rc.h5, rd.h5), u1 = add2(rc.q5, rd.q5);
+          const uint2 s = pair_sum<k8>(t0, t1, re.h5);
+          if (c0in) o2[0] = sgr_ab<25, k8>(s.x, u0.x + u1.x + re.q5.x, bd, s2, sm.xbx);
+          if (c1) o2[1] = sgr_ab<25, k8>(s.y, u0.y + u1.y + re.q5.y, bd, s2, sm.xbx);
+          t0 = t1;
+          u0 = u1;
         }
-        leave5 = l3;
+        rb = rd;
+        rc = re;
       }
     }
   }
   __syncthreads();
-  if (tx < w && ya < yb) {
-    // Radius 2: even y weighs table rows y and y + 2 (6 centre / 5 corners,
-    // shift 9), odd y row y + 1 (6 / 5, shift 8); the tables hold the even
-    // rows k at k / 2.  Radius 1: rows y, y + 1, y + 2 (4 cross / 3
-    // corners).  A table row enters as its 3-sum S and centre C over columns
-    // tx .. tx + 2: 6 C + 5 (S - C) = 5 S + C, and the radius-1 weights sum
-    // to 4 S(y+1) + 3 (S(y) + S(y+2)) + C(y) + C(y+2).
-    struct SC {
-      int32_t sa, ca, sb, cb;
+  const LrRun t = lr_run(h, PW);
+  if (t.x < w && t.ya < t.yb) {
+    const int maxv = (1 << bd) - 1;
+    // Projection (selfguided.go:233-247): (v + 1024) >> 11 as a 16-bit
+    // integer is the upper half of 32 v + 32768.
+    const int kd = 32 * (2048 - 16 * (xq0 + xq1)), k0 = 32 * xq0, k1 = 32 * xq1;
+    constexpr uint32_t kB = (1u << 22) - 1;
+    struct Term {
+      int a[2], b[2];
     };
-    auto row2 = [&](int i) {
-      const int o = i * 66 + tx;
-      const int32_t a0 = A2[o], a1 = A2[o + 1], a2 = A2[o + 2];
-      const int32_t b0 = B2[o], b1 = B2[o + 1], b2 = B2[o + 2];
-      return SC{a0 + a1 + a2, a1, b0 + b1 + b2, b1};
+    // Three-column sums S and centres C of a table row for the pair.
+    auto row = [&](const uint32_t* p, Term& s, Term& c) {
+      const uint2 e = *reinterpret_cast<const uint2*>(p), f = *reinterpret_cast<const uint2*>(p + 2);
+      const uint32_t m = e.y + f.x, s0 = e.x + m, s1 = m + f.y;
+      s.a[0] = s0 >> 22, s.b[0] = s0 & kB, s.a[1] = s1 >> 22, s.b[1] = s1 & kB;
+      c.a[0] = e.y >> 22, c.b[0] = e.y & kB, c.a[1] = f.x >> 22, c.b[1] = f.x & kB;
     };
-    auto row1 = [&](int k) {
-      const int o = k * 66 + tx;
-      const int32_t a0 = A1[o], a1 = A1[o + 1], a2 = A1[o + 2];
-      const int32_t b0 = B1[o], b1 = B1[o + 1], b2 = B1[o + 2];
-      return SC{a0 + a1 + a2, a1, b0 + b1 + b2, b1};
-    };
-    // For y = ya: the pair (ya / 2, ya / 2 + 1) when ya is even, the one
-    // row (ya + 1) / 2 in d2 when it is odd.
-    SC u2{}, d2{}, u1{}, m1{};
-    if (R2) {
-      u2 = row2(ya >> 1);
-      d2 = row2((ya >> 1) + 1);
-    }
-    if (R1) {
-      u1 = row1(ya);
-      m1 = row1(ya + 1);
-    }
+    auto row2 = [&](int k, Term& z) {
+      Term s, c;
+      row(&sm.sgr.t2[k * kTabPitch + t.x], s, c);
 #pragma unroll
-    for (int i = 0; i < kLrMaxRun; i++) {
-      const int y = ya + i;
-      if (y >= yb) break;
-      const int32_t dg = s_win[(y + 3) * kWin + tx + 3];
-      const int32_t uu = dg << 4;
-      int32_t v = uu << 7;
-      if (R2) {
-        int32_t av, bv, shift;
-        if ((y & 1) == 0) {
-          if (i != 0) {
-            u2 = d2;
-            d2 = row2((y >> 1) + 1);
+      for (int i = 0; i < 2; i++) {
+        z.a[i] = 5 * s.a[i] + c.a[i];
+        z.b[i] = 5 * s.b[i] + c.b[i];
+      }
+    };
+    // Outer rows' term X = 3 S + C, the middle row's Y = 4 S with the constants.
+    auto row1 = [&](int k, Term& X, Term& Y) {
+      Term s, c;
+      row(&sm.sgr.t1[k * kTabPitch + t.x], s, c);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        X.a[i] = 3 * s.a[i] + c.a[i];
+        X.b[i] = 3 * s.b[i] + c.b[i];
+        Y.a[i] = 4 * s.a[i] + 32;
+        Y.b[i] = 4 * s.b[i] + 256;
+      }
+    };
+    Term z0, x0, x1, y1, skip;
+    if (R2) row2(t.ya >> 1, z0);
+    if (R1) {
+      row1(t.ya, x0, skip);
+      row1(t.ya + 1, x1, y1);
+    }
+#pragma unroll 1
+    for (int y = t.ya; y < t.yb; y += 2) {
+      Term z1;
+      if (R2) row2((y >> 1) + 1, z1);
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        if (r == 1 && y + 1 >= t.yb) break;
+        const uint32_t d2 = sm.win[(y + r + 3) * kWinWords + (t.x >> 1) + 2];
+        const int dg[2] = {(int)(d2 & 0xffff), (int)(d2 >> 16)};
+        Term x2, y2;
+        if (R1) row1(y + r + 2, x2, y2);
+        int v[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          int p = dg[i] * kd + 32768;
+          if (R2) {
+            const int f = r == 0 ? ((z0.a[i] + z1.a[i] + 32) * dg[i] + (z0.b[i] + z1.b[i] + 256)) >> 9
+                                 : ((z1.a[i] + 16) * dg[i] + (z1.b[i] + 128)) >> 8;
+            p += f * k0;
           }
-          av = 5 * (u2.sa + d2.sa) + u2.ca + d2.ca;
-          bv = 5 * (u2.sb + d2.sb) + u2.cb + d2.cb;
-          shift = 9;
-        } else {
-          av = 5 * d2.sa + d2.ca;
-          bv = 5 * d2.sb + d2.cb;
-          shift = 8;
+          if (R1) {
+            const int f = ((x0.a[i] + y1.a[i] + x2.a[i]) * dg[i] + (x0.b[i] + y1.b[i] + x2.b[i])) >> 9;
+            p += f * k1;
+          }
+          v[i] = __vimin_s32_relu(p >> 16, maxv);
         }
-        v += xq0 * (rpot(av * dg + bv, shift) - uu);
+        out(y + r, t.x, v[0], v[1]);
+        if (R1) {
+          x0 = x1;
+          x1 = x2;
+          y1 = y2;
+        }
       }
-      if (R1) {
-        const SC d1 = row1(y + 2);
-        const int32_t av = 4 * m1.sa + 3 * (u1.sa + d1.sa) + u1.ca + d1.ca;
-        const int32_t bv = 4 * m1.sb + 3 * (u1.sb + d1.sb) + u1.cb + d1.cb;
-        v += xq1 * (rpot(av * dg + bv, 9) - uu);
-        u1 = m1;
-        m1 = d1;
-      }
-      // restoration/selfguided.go:233-247: projection with the int16 wrap.
-      const int32_t wv = (int32_t)(int16_t)rpot(v, 11);
-      out(y, tx, imin(imax(wv, 0), maxv));
+      if (R2) z0 = z1;
     }
   }
   __syncthreads();
@@ -299,27 +394,70 @@ __device__ __forceinline__ void lr_sgr_window_t(LrSmem& sm, int w, int h, int bd
 // The self-guided filter with parameter set `set` and the coded xqd pair
 // (restoration/selfguided.go:111-127, DecodeSGRXQ), dispatched on which of
 // its two radii are on (r0 is 0 or 2, r1 is 0 or 1).
-template <class Out>
+template <bool k8, class Out>
 __device__ __forceinline__ void lr_sgr_window(LrSmem& sm, int w, int h, int bd, int set, int xqd0, int xqd1, int PW,
                                               Out&& out) {
   const int r0 = c_sgr_params[set][0], r1 = c_sgr_params[set][1];
   const int s0 = c_sgr_params[set][2], s1 = c_sgr_params[set][3];
   if (r0 == 0)
-    lr_sgr_window_t<false, true>(sm, w, h, bd, s0, s1, 0, 128 - xqd1, PW, out);
+    lr_sgr_window_t<false, true, k8>(sm, w, h, bd, s0, s1, 0, 128 - xqd1, PW, out);
   else if (r1 == 0)
-    lr_sgr_window_t<true, false>(sm, w, h, bd, s0, s1, xqd0, 0, PW, out);
+    lr_sgr_window_t<true, false, k8>(sm, w, h, bd, s0, s1, xqd0, 0, PW, out);
   else
-    lr_sgr_window_t<true, true>(sm, w, h, bd, s0, s1, xqd0, 128 - xqd0 - xqd1, PW, out);
+    lr_sgr_window_t<true, true, k8>(sm, w, h, bd, s0, s1, xqd0, 128 - xqd0 - xqd1, PW, out);
 }
 
-// One restoration tile: processing column j of stripe s of `plane`.
+// Stages rows [0, wh) of a window: row(r) is the source row r's pointer to
+// sample 0 of the plane (columns are clamped to 0 .. Wc - 1), x0 the tile's
+// first column, w its width.  A task is four columns of a row; loads go out
+// before the first is used.
+template <typename T, class Row>
+__device__ __forceinline__ void lr_stage(uint32_t* win, int x0, int w, int wh, int Wc, bool words, Row&& row) {
+  const int groups = (w + 11) >> 2;  // columns -4 .. w + 3 and up
+  const uint32_t inv = (65536u + (uint32_t)groups - 1) / (uint32_t)groups;  // i / groups for i < 1,260
+  const int total = groups * wh;
+  constexpr int kTasks = (18 * kWinRows + 255) / 256;
+  uint2 v[kTasks];
+#pragma unroll
+  for (int k = 0; k < kTasks; k++) {
+    const int i = threadIdx.x + 256 * k;
+    if (i >= total) continue;
+    const int r = (int)((i * inv) >> 16), g = i - r * groups;
+    const int x = x0 - 4 + 4 * g;
+    const T* src = row(r);
+    if (words && x >= 0 && x + 4 <= Wc) {
+      if constexpr (sizeof(T) == 1)
+        v[k].x = *reinterpret_cast<const uint32_t*>(src + x);
+      else
+        v[k] = *reinterpret_cast<const uint2*>(src + x);
+    } else {
+      uint32_t s[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) s[j] = src[iclip(x + j, 0, Wc - 1)];
+      if constexpr (sizeof(T) == 1)
+        v[k].x = s[0] | s[1] << 8 | s[2] << 16 | s[3] << 24;
+      else
+        v[k] = make_uint2(s[0] | s[1] << 16, s[2] | s[3] << 16);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kTasks; k++) {
+    const int i = threadIdx.x + 256 * k;
+    if (i >= total) continue;
+    const int r = (int)((i * inv) >> 16), g = i - r * groups;
+    uint2 o = v[k];
+    if constexpr (sizeof(T) == 1)
+      o = make_uint2(__byte_perm(v[k].x, 0, 0x4140), __byte_perm(v[k].x, 0, 0x4342));
+    *reinterpret_cast<uint2*>(&win[r * kWinWords + 2 * g]) = o;
+  }
+}
+
+// One restoration tile: column j of stripe s of `plane`, PW samples wide.
 template <typename T>
-__device__ void lr_tile(const DFrame& src, const DFrame& dst, const LrArgs& a, const int* aw, const int* ah,
-                        int enabled, int plane, int j, int s, LrSmem& sm) {
-  uint16_t* s_win = sm.win;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ssx = plane ? src.ssx : 0, ssy = plane ? src.ssy : 0;
-  const int PW = 64 >> ssx, SH = 64 >> ssy, off = 8 >> ssy;
+__device__ __forceinline__ void lr_tile(const DFrame& src, const DFrame& dst, const LrArgs& a, const int* aw,
+                                        const int* ah, int enabled, int plane, int j, int s, LrSmem& sm) {
+  const int ssy = plane ? src.ssy : 0;
+  const int PW = a.tile_w[plane], SH = 64 >> ssy, off = 8 >> ssy;
   const int Wa = aw[plane], Ha = ah[plane];
   const DPlane& sp = src.pl[plane];
   const DPlane& dp = dst.pl[plane];
@@ -329,7 +467,6 @@ __device__ void lr_tile(const DFrame& src, const DFrame& dst, const LrArgs& a, c
   if (x0 >= Wa || y0 >= Ha) return;
   const int x1 = imin(x0 + PW, Wa), y1 = imin((s + 1) * SH - off, Ha);
   const int tid = threadIdx.x;
-  const int tx = tid % PW, ty0 = tid / PW, rowStep = 256 / PW;
   const int bd = sizeof(T) == 1 ? 8 : src.bd;  // a constant for 8-bit: the rounding shifts fold
 
   // Which restoration unit (if any) covers this tile.
@@ -351,62 +488,52 @@ __device__ void lr_tile(const DFrame& src, const DFrame& dst, const LrArgs& a, c
   const int nominal = SH - (y0 == 0 ? off : 0);
   const bool copyAbove = y0 != 0, copyBelow = y0 + nominal < Hc;
   const int kAbove = s, kBelow = s + 1;  // boundary indices of the saved lines
-  const int ww = w + 6, wh = h + 6;
-  auto srcRow = [&](int r) -> const T* {
+  const bool words = ((reinterpret_cast<uintptr_t>(sp.ptr) | (uintptr_t)sp.stride) & (4 * sizeof(T) - 1)) == 0;
+  lr_stage<T>(sm.win, x0, w, h + 6, Wc, words, [&](int r) -> const T* {
     const int yy = y0 - 3 + r;
     if (yy < y0 && copyAbove)
       return reinterpret_cast<const T*>(a.lines[plane] + (int64_t)(kAbove * 4 + imax(yy - y0 + 2, 0)) * a.line_stride[plane]);
     if (yy >= yf1 && copyBelow)
       return reinterpret_cast<const T*>(a.lines[plane] + (int64_t)(kBelow * 4 + 2 + imin(yy - yf1, 1)) * a.line_stride[plane]);
     return row_ptr<T>(sp, iclip(yy, 0, Hc - 1));
-  };
-  // A warp's rows r and r+8 and each lane's three columns are loaded before
-  // any is stored: six loads in flight per lane (ww <= 70 < 96).
-  for (int r0 = warp; r0 < wh; r0 += 16) {
-    uint16_t v[2][3];
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const int r = r0 + 8 * q;
-      if (r < wh) {
-        const T* srow = srcRow(r);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          const int c = lane + 32 * k;
-          if (c < ww) v[q][k] = (uint16_t)srow[iclip(x0 - 3 + c, 0, Wc - 1)];
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 2; q++)
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-        if (r0 + 8 * q < wh && lane + 32 * k < ww) s_win[(r0 + 8 * q) * kWin + lane + 32 * k] = v[q][k];
-  }
-  for (int i = tid; i < 256; i += 256) sm.x_by_xplus1[i] = c_x_by_xplus1[i];
+  });
+  sm.xbx[tid] = c_xbx[tid];
   __syncthreads();
 
   // Pixels of the tile outside the cropped plane are copied through.
-  if ((x1 > Wc || y1 > Hc) && tx < x1 - x0)
-    for (int y = y0 + ty0; y < y1; y += rowStep)
-      if (x0 + tx >= Wc || y >= Hc) row_ptr<T>(dp, y)[x0 + tx] = row_ptr<T>(sp, y)[x0 + tx];
+  if (x1 > Wc || y1 > Hc)
+    for (int i = tid; i < (x1 - x0) * (y1 - y0); i += 256) {
+      const int y = y0 + i / (x1 - x0), x = x0 + i % (x1 - x0);
+      if (x >= Wc || y >= Hc) row_ptr<T>(dp, y)[x] = row_ptr<T>(sp, y)[x];
+    }
 
-  auto store = [&](int y, int x, int v) { row_ptr<T>(dp, y0 + y)[x0 + x] = (T)v; };
-  if (u->type == PF_LR_WIENER) {
-    const int hv0 = u->wiener_h[0], hv1 = u->wiener_h[1], hv2 = u->wiener_h[2];
-    const int hf[7] = {hv0, hv1, hv2, -2 * (hv0 + hv1 + hv2), hv2, hv1, hv0};
-    const int vv0 = u->wiener_v[0], vv1 = u->wiener_v[1], vv2 = u->wiener_v[2];
-    const int vf[7] = {vv0, vv1, vv2, -2 * (vv0 + vv1 + vv2), vv2, vv1, vv0};
-    lr_wiener_window(sm, w, h, bd, hf, vf, PW, store);
-    return;
-  }
-  // ---- SGRproj (restoration/selfguided.go:132-359) ----
-  lr_sgr_window(sm, w, h, bd, u->sgr_set, u->sgr_xqd[0], u->sgr_xqd[1], PW, store);
+  // Two neighbours go out as one word where the row allows it.
+  uint8_t* const ob = dp.ptr + (int64_t)y0 * dp.stride + (int64_t)x0 * (int)sizeof(T);
+  const int64_t os = dp.stride;
+  const bool pairs = ((reinterpret_cast<uintptr_t>(ob) | (uintptr_t)os) & (2 * sizeof(T) - 1)) == 0;
+  auto store = [&](int y, int x, int v0, int v1) {
+    T* o = reinterpret_cast<T*>(ob + y * os) + x;
+    if (pairs && x + 1 < w) {
+      if constexpr (sizeof(T) == 1)
+        *reinterpret_cast<uint16_t*>(o) = (uint16_t)(v0 | v1 << 8);
+      else
+        *reinterpret_cast<uint32_t*>(o) = (uint32_t)v0 | (uint32_t)v1 << 16;
+    } else {
+      o[0] = (T)v0;
+      if (x + 1 < w) o[1] = (T)v1;
+    }
+  };
+  if (u->type == PF_LR_WIENER)
+    lr_wiener_window(sm, w, h, bd, u->wiener_h, u->wiener_v, PW, store);
+  else
+    lr_sgr_window<sizeof(T) == 1>(sm, w, h, bd, u->sgr_set, u->sgr_xqd[0], u->sgr_xqd[1], PW, store);
 }
 
 cudaError_t lr_upload_tables() {
+  uint8_t xbx[256];
+  for (int z = 0; z < 256; z++) xbx[z] = (uint8_t)(pf_sgr_x_by_xplus1[z] - 1);
   cudaError_t e = cudaMemcpyToSymbol(c_sgr_params, pf_sgr_params, sizeof(pf_sgr_params));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_x_by_xplus1, pf_sgr_x_by_xplus1, sizeof(pf_sgr_x_by_xplus1));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_one_by_x, pf_sgr_one_by_x, sizeof(pf_sgr_one_by_x));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_xbx, xbx, sizeof(xbx));
   return e;
 }
 
@@ -449,8 +576,8 @@ __global__ void __launch_bounds__(256, 4) k_lr_batch(BatchArgs b) {
         // The tile's stripe of the CDEF output with its 3-sample halo.
         const LrTile t = lr_locate(b, base, item);
         const FrameJob& J = *t.J;
-        const int ssx = t.plane ? J.io.ssx : 0, ssy = t.plane ? J.io.ssy : 0;
-        const int PW = 64 >> ssx, SH = 64 >> ssy, off = 8 >> ssy;
+        const int ssy = t.plane ? J.io.ssy : 0;
+        const int PW = J.lr.tile_w[t.plane], SH = 64 >> ssy, off = 8 >> ssy;
         const int x0 = t.j * PW, y0 = t.s * SH - off;
         if (J.io.bd == 8)
           prefetch_block<uint8_t>(J.scr.pl[t.plane], x0 - 3, x0 + PW + 3, y0 - 3, y0 + SH + 3);
@@ -571,31 +698,15 @@ __device__ __forceinline__ void lrs_block_sum(uint32_t (&v)[N], uint32_t* red) {
 __device__ __forceinline__ void lrs_stage(const LrsArgs& a, LrsSmem& sm, int x0, int y0, int w, int h, bool tables,
                                           bool source) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Six loads in flight per lane, as in lr_tile.
-  for (int r0 = warp; r0 < h + 6; r0 += 16) {
-    uint8_t v[2][3];
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const int r = r0 + 8 * q;
-      if (r < h + 6) {
-        const uint8_t* row = a.rec + (int64_t)iclip(y0 - 3 + r, 0, a.H - 1) * a.rstride;
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-          if (lane + 32 * k < w + 6) v[q][k] = row[iclip(x0 - 3 + lane + 32 * k, 0, a.W - 1)];
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 2; q++)
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-        if (r0 + 8 * q < h + 6 && lane + 32 * k < w + 6) sm.lr.win[(r0 + 8 * q) * kWin + lane + 32 * k] = v[q][k];
-  }
+  const bool words = ((reinterpret_cast<uintptr_t>(a.rec) | (uintptr_t)a.rstride) & 3) == 0;
+  lr_stage<uint8_t>(sm.lr.win, x0, w, h + 6, a.W, words,
+                    [&](int r) { return a.rec + (int64_t)iclip(y0 - 3 + r, 0, a.H - 1) * a.rstride; });
   if (source)
     for (int r = warp; r < h; r += 8) {
       const uint8_t* row = a.src + (int64_t)(y0 + r) * a.sstride + x0;
       for (int c = lane; c < w; c += 32) sm.src[r * 64 + c] = row[c];
     }
-  if (tables) sm.lr.x_by_xplus1[threadIdx.x] = c_x_by_xplus1[threadIdx.x];
+  if (tables) sm.lr.xbx[threadIdx.x] = c_xbx[threadIdx.x];
   __syncthreads();
 }
 
@@ -622,14 +733,6 @@ __device__ __forceinline__ void lrs_hsse(uint32_t* acc, int s, int p06, int p15,
   if constexpr (C + 1 < PF_LR_WIENER_CANDIDATES) lrs_hsse<C + 1>(acc, s, p06, p15, p24, p3);
 }
 
-__device__ __forceinline__ void lrs_taps(int c, int* f) {
-  const int t0 = c_lrs_wiener[c][0], t1 = c_lrs_wiener[c][1], t2 = c_lrs_wiener[c][2];
-  f[0] = f[6] = t0;
-  f[1] = f[5] = t1;
-  f[2] = f[4] = t2;
-  f[3] = -2 * (t0 + t1 + t2);  // restoration/wiener.go:44-47 (NewWienerFilter)
-}
-
 // SearchWienerUnitU8's choice over the table (encoder/restoration.go:161-209).
 __device__ __forceinline__ int lrs_wiener_pick(const uint32_t* cand, uint32_t base, int area) {
   int pick = -1;
@@ -641,6 +744,19 @@ __device__ __forceinline__ int lrs_wiener_pick(const uint32_t* cand, uint32_t ba
         pick = c;
       }
   return pick;
+}
+
+// One exact filter's outputs of columns x and x + 1: their squared error
+// against the source, and into the candidate buffer (rows of 64).
+__device__ __forceinline__ uint32_t lrs_outcome(const LrsSmem& sm, uint8_t* keep, int w, int y, int x, int v0, int v1) {
+  const int d0 = (int)sm.src[y * 64 + x] - v0;
+  uint32_t e = (uint32_t)(d0 * d0);
+  if (x + 1 < w) {
+    const int d1 = (int)sm.src[y * 64 + x + 1] - v1;
+    e += (uint32_t)(d1 * d1);
+  }
+  if (keep) *reinterpret_cast<uint16_t*>(&keep[y * 64 + x]) = (uint16_t)(v0 | v1 << 8);  // x + 1 <= 63
+  return e;
 }
 
 __global__ void __launch_bounds__(256, 3) k_lr_search_sse(LrsArgs a) {
@@ -663,11 +779,8 @@ __global__ void __launch_bounds__(256, 3) k_lr_search_sse(LrsArgs a) {
     lrs_stage(a, sm, x0, y0, w, h, true, true);
     uint32_t acc[1] = {0};
     uint8_t* keep = a.cand ? lrs_cand(a, unit, job) : nullptr;
-    lr_sgr_window(sm.lr, w, h, 8, c_lrs_sgr[p][0], c_lrs_sgr[p][1], c_lrs_sgr[p][2], 64, [&](int y, int x, int v) {
-      const int d = (int)sm.src[y * 64 + x] - v;
-      acc[0] += (uint32_t)(d * d);
-      if (keep) keep[y * 64 + x] = (uint8_t)v;
-    });
+    lr_sgr_window<true>(sm.lr, w, h, 8, c_lrs_sgr[p][0], c_lrs_sgr[p][1], c_lrs_sgr[p][2], 64,
+                        [&](int y, int x, int v0, int v1) { acc[0] += lrs_outcome(sm, keep, w, y, x, v0, v1); });
     lrs_block_sum(acc, sm.red);
     if (tid == 0) T.sgr[p] = acc[0];
     return;
@@ -681,7 +794,7 @@ __global__ void __launch_bounds__(256, 3) k_lr_search_sse(LrsArgs a) {
     const int tx = tid & 63;
     if (tx < w)
       for (int y = tid >> 6; y < h; y += 4) {
-        const uint16_t* wr = &sm.lr.win[(y + 3) * kWin + tx];
+        const uint16_t* wr = reinterpret_cast<const uint16_t*>(sm.lr.win) + (y + 3) * 2 * kWinWords + tx + 1;
         const int s = sm.src[y * 64 + tx];
         const int d0 = s - (int)wr[3];
         acc[0] += (uint32_t)(d0 * d0);
@@ -707,15 +820,10 @@ __global__ void __launch_bounds__(256, 3) k_lr_search_sse(LrsArgs a) {
   uint32_t ex[1] = {kLrsNone};
   if (pick >= 0 && fits) {
     // The exact filter of the pick (keyframe_lossy.go:2344-2366).
-    int fv[7];
-    lrs_taps(pick, fv);
     ex[0] = 0;
     uint8_t* keep = a.cand ? lrs_cand(a, unit, 0) : nullptr;
-    lr_wiener_window(sm.lr, w, h, 8, fv, fv, 64, [&](int y, int x, int v) {
-      const int d = (int)sm.src[y * 64 + x] - v;
-      ex[0] += (uint32_t)(d * d);
-      if (keep) keep[y * 64 + x] = (uint8_t)v;
-    });
+    lr_wiener_window(sm.lr, w, h, 8, c_lrs_wiener[pick], c_lrs_wiener[pick], 64,
+                     [&](int y, int x, int v0, int v1) { ex[0] += lrs_outcome(sm, keep, w, y, x, v0, v1); });
     lrs_block_sum(ex, sm.red);
   }
   if (tid == 0) {
