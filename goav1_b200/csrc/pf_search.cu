@@ -20,11 +20,17 @@
 //   k_sel_greedy    finish (:886-945): jointStrengthSearchDual /
 //                   searchOneDual (:780-869) for one nb = 1 << cluster index,
 //                   all 5*nb greedy and refinement steps inside one launch.
-//                   Eight CTAs of a thread-block cluster each own a slice of
+//                   The CTAs of a thread-block cluster each own a slice of
 //                   the filter blocks (SSE rows in shared memory), compute
 //                   partial savings sav[j][k] = sum_i max(0, best_i -
-//                   m0[i][j] - m1[i][k]) (the reference's form), and reduce
-//                   them through distributed shared memory.
+//                   m0[i][j] - m1[i][k]) (the reference's form), and hand
+//                   them to the CTA that reduces the pair through
+//                   distributed shared memory.  The refinement ends once nb
+//                   steps in a row have changed nothing (no later one can).
+//                   Bound by the barriers of a step, two of the cluster
+//                   among them; 1080p: 303 us with all 40 steps of 8
+//                   presets run, 127 now; the learned search's 8 steps 62
+//                   (1,024 threads a CTA instead of 512: 152 and 75).
 //   k_sel_finish    the RD choice of nb and the per-block preset index.
 #include <cooperative_groups.h>
 #include <string.h>
@@ -431,14 +437,16 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(256, 3) k_cdef_searc
 // ---- greedy preset selection (finish) ----
 
 struct SelShared {
-  unsigned long long part[4096];       // this CTA's partial savings (or column sums)
+  // Partial savings of this CTA's slice of the pairs, a row from each CTA of
+  // the cluster (first pick: this CTA's column sums).
+  alignas(16) unsigned long long part[4096];
   unsigned long long col[128];
-  unsigned long long candV[2], candSB[2];
-  int candI[2];
+  unsigned long long candV[2][kSelMaxCluster], candSB[2][kSelMaxCluster];
+  int candI[2][kSelMaxCluster];
   unsigned long long redV[kSelThreads / 32];
   int redI[kSelThreads / 32];
   unsigned long long redS[kSelThreads / 32];
-  int lev0[8], lev1[8];
+  int lev0[8], lev1[8], drop[2];
   unsigned long long tot;
 };
 
@@ -484,7 +492,9 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
   int* s_sb = reinterpret_cast<int*>(smem + sizeof(SelShared));  // [nfb] non-skip blocks
   uint32_t* s_best = reinterpret_cast<uint32_t*>(s_sb + ((a.nfb + 3) & ~3));
   uint32_t* s_min1 = s_best + a.cap;
-  uint32_t* s_rows = s_min1 + a.cap;  // [cap][128] when kRows
+  // [cap][128] when kRows, on 16 bytes (the pool is, and sel_smem_bytes leaves room).
+  uint32_t* s_rows = s_min1 + a.cap;
+  s_rows += (4 - (((unsigned char*)s_rows - smem) >> 2 & 3)) & 3;
   cg::cluster_group cl = cg::this_cluster();
   const int CS = (int)cl.num_blocks();
   const int rank = (int)cl.block_rank();
@@ -525,8 +535,10 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
   if (t < 8) S.lev0[t] = S.lev1[t] = 0;
   __syncthreads();
   const int steps = a.refine ? 5 * nb : nb;
+  int same = 0;  // refinement steps in a row that took back the pick they had dropped
   for (int k = 0; k < steps; k++) {
     const int nbCur = k < nb ? k : nb - 1;
+    const int drop0 = S.drop[0], drop1 = S.drop[1];
     const int par = k & 1;
     if (nbCur == 0) {
       // First pick: the luma and chroma strengths with the least total SSE.
@@ -571,11 +583,11 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
       for (int o = 16; o > 0; o >>= 1) sb += __shfl_xor_sync(0xffffffffu, sb, o);
       if (lane == 0) S.redS[warp] = sb;
       __syncthreads();
+      unsigned long long sbAll = 0;  // warp 0's: the CTA's sum
       if (warp == 0) {
-        unsigned long long v = lane < kSelThreads / 32 ? S.redS[lane] : 0;
+        sbAll = lane < kSelThreads / 32 ? S.redS[lane] : 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) S.candSB[par] = v;
+        for (int o = 16; o > 0; o >>= 1) sbAll += __shfl_xor_sync(0xffffffffu, sbAll, o);
       }
       // Partial savings of this CTA's blocks: thread t owns (j, k0..k0+7).
       // A block saves below 2^29, so eight blocks sum exactly in 32 bits
@@ -590,12 +602,20 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
         for (int il = il0; il < il1; il++) {
           const uint32_t bi = s_best[il], a0 = row(il, 0, j);
           if (a0 + s_min1[il] >= bi) continue;  // no k can save anything
-          const uint32_t rem = bi - a0;
+          // Both are below 2^30 and a sentinel is 2^31 - 1, so the signed
+          // difference cannot overflow.
+          const int rem = (int)(bi - a0);
+          uint32_t v[8];
+          if (kRows) {
+            const uint4* r4 = reinterpret_cast<const uint4*>(&s_rows[il * 128 + 64 + k0]);
+            const uint4 x = r4[0], y = r4[1];
+            v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+          } else {
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            const uint32_t v = row(il, 1, k0 + q);
-            acc32[q] += v < rem ? rem - v : 0u;
+            for (int q = 0; q < 8; q++) v[q] = row(il, 1, k0 + q);
           }
+#pragma unroll
+          for (int q = 0; q < 8; q++) acc32[q] += (uint32_t)__viaddmax_s32(-(int)v[q], rem, 0);
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) {
@@ -603,22 +623,27 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
           acc32[q] = 0;
         }
       }
+      // Each CTA reduces a slice of the pairs: the eight sums go straight
+      // into their slice's CTA (rows of one sender each), so that only the
+      // barrier is waited for and every read after it is local.
+      {
+        const int e0 = t * 8, to = e0 / pairs;
+        ulonglong2* d = reinterpret_cast<ulonglong2*>(cl.map_shared_rank(&S.part[0], to) + rank * pairs + (e0 - to * pairs));
 #pragma unroll
-      for (int q = 0; q < 8; q++) S.part[j * 64 + k0 + q] = acc[q];
+        for (int q = 0; q < 4; q++) d[q] = make_ulonglong2(acc[2 * q], acc[2 * q + 1]);
+      }
       cl.sync();
-      // Reduce this CTA's slice across the cluster; first maximum wins.
+      // First maximum wins.  Two neighbouring threads share a pair.
       unsigned long long bv = 0;
       int bi = 0x7fffffff;
-      for (int e = rank * pairs + t; e < (rank + 1) * pairs; e += kSelThreads) {
-        // Four independent remote reads in flight (CS is a multiple of 4).
-        unsigned long long v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-        for (int r = 0; r < CS; r += 4) {
-          v0 += cl.map_shared_rank(&S.part[0], r)[e];
-          v1 += cl.map_shared_rank(&S.part[0], r + 1)[e];
-          v2 += cl.map_shared_rank(&S.part[0], r + 2)[e];
-          v3 += cl.map_shared_rank(&S.part[0], r + 3)[e];
-        }
-        argmax_merge(bv, bi, (v0 + v1) + (v2 + v3), e);
+      for (int e2 = t; e2 < 2 * pairs; e2 += kSelThreads) {
+        const int e = e2 >> 1, r0 = (e2 & 1) * (CS >> 1);
+        unsigned long long sum = 0;
+#pragma unroll
+        for (int r = 0; r < kSelMaxCluster / 2; r++)
+          if (r < (CS >> 1)) sum += S.part[(r0 + r) * pairs + e];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        argmax_merge(bv, bi, sum, rank * pairs + e);
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -644,21 +669,23 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
           const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
           argmax_merge(v, i, v2, i2);
         }
-        if (lane == 0) {
-          S.candV[par] = v;
-          S.candI[par] = i;
+        // Lane r hands this CTA's candidate and partial sum of best_i to
+        // rank r (alternate steps use alternate places).
+        if (lane < CS) {
+          SelShared* R = cl.map_shared_rank(&S, lane);
+          R->candV[par][rank] = v;
+          R->candI[par][rank] = i;
+          R->candSB[par][rank] = sbAll;
         }
       }
       cl.sync();
       if (warp == 0) {
-        // Lane r reads rank r's candidate and partial sum of best_i.
         unsigned long long v = 0, sbr = 0;
         int i = 0x7fffffff;
         if (lane < CS) {
-          const SelShared* R = cl.map_shared_rank(&S, lane);
-          v = R->candV[par];
-          i = R->candI[par];
-          sbr = R->candSB[par];
+          v = S.candV[par][lane];
+          i = S.candI[par][lane];
+          sbr = S.candSB[par][lane];
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -674,13 +701,29 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
         }
       }
     }
-    // Refinement passes drop the oldest pick (jointStrengthSearchDual).
-    if (t == 0 && k + 1 >= nb && k + 1 < steps)
-      for (int g = 0; g < nb - 1; g++) {
-        S.lev0[g] = S.lev0[g + 1];
-        S.lev1[g] = S.lev1[g + 1];
-      }
     __syncthreads();
+    // A pick depends only on the set of the other nb - 1, so once nb steps in
+    // a row have taken back what they dropped, every later one does: the
+    // remaining steps only turn the list, which is then done at once.
+    if (k >= nb) same = S.lev0[nb - 1] == drop0 && S.lev1[nb - 1] == drop1 ? same + 1 : 0;
+    const int turn = same == nb ? (steps - 1 - k) % nb : 1;
+    __syncthreads();
+    // Refinement passes drop the oldest pick (jointStrengthSearchDual).
+    if (t == 0 && k + 1 >= nb && k + 1 < steps) {
+      S.drop[0] = S.lev0[0];
+      S.drop[1] = S.lev1[0];
+      for (int q = 0; q < turn; q++) {
+        const int l0 = S.lev0[0], l1 = S.lev1[0];
+        for (int g = 0; g < nb - 1; g++) {
+          S.lev0[g] = S.lev0[g + 1];
+          S.lev1[g] = S.lev1[g + 1];
+        }
+        S.lev0[nb - 1] = l0;
+        S.lev1[nb - 1] = l1;
+      }
+    }
+    __syncthreads();
+    if (same == nb) break;
   }
   if (rank == 0 && t == 0) {
     for (int g = 0; g < 8; g++) {
@@ -755,7 +798,7 @@ __global__ void __launch_bounds__(256) k_sel_finish(SelArgs a, int maxCfg, unsig
 
 size_t sel_smem_bytes(int nfb, bool rows) {
   const int cap = (nfb + kSelMinCluster - 1) / kSelMinCluster;
-  return sizeof(SelShared) + (size_t)((nfb + 3) & ~3) * 4 + (size_t)cap * 8 + (rows ? (size_t)cap * 512 : 0);
+  return sizeof(SelShared) + (size_t)((nfb + 3) & ~3) * 4 + (size_t)cap * 8 + (rows ? (size_t)cap * 512 + 16 : 0);
 }
 
 cudaError_t launch_search(const SearchArgs& a, cudaStream_t st) {
