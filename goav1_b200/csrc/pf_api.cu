@@ -1842,6 +1842,13 @@ void* pf_internal_search_scratch(pf_ctx* c, size_t bytes) {
   return c->search.p;
 }
 void* pf_internal_stream(pf_ctx* c) { return (void*)c->stream; }
+// The context's second stream, made to wait for what its stream holds so far:
+// a copy there overlaps what is queued on the stream next.  Null on failure.
+void* pf_internal_fork(pf_ctx* c) {
+  if (cudaEventRecord(c->fork, c->stream) != cudaSuccess || cudaStreamWaitEvent(c->side, c->fork, 0) != cudaSuccess)
+    return nullptr;
+  return (void*)c->side;
+}
 // The context's stage events when it times stages (pf_config.timing), else null.
 cudaEvent_t* pf_internal_events(pf_ctx* c) { return c->timing ? c->ev : nullptr; }
 

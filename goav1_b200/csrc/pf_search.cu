@@ -888,6 +888,7 @@ void* pf_internal_search_scratch(pf_ctx* c, size_t bytes);  // pf_api.cu
 void* pf_internal_stream(pf_ctx* c);
 cudaEvent_t* pf_internal_events(pf_ctx* c);  // pf_api.cu: null unless the context times stages
 void* pf_internal_pinned(pf_ctx* c, size_t bytes);
+void* pf_internal_fork(pf_ctx* c);  // pf_api.cu
 void* pf_internal_cached_upload(pf_ctx* c, const void* host, size_t bytes, size_t extra, cudaStream_t st,
                                 int* changed);
 int pf_internal_wait(pf_ctx* c, void* stream);  // pf_api.cu: blocking or bounded by the context's deadline
@@ -935,7 +936,7 @@ struct Staged {
   uint8_t* idx;
   FinishOut* fo;
   uint8_t* extra;
-  uint8_t* pin;  // page-locked staging: noskip words up, then the results down
+  uint8_t* pin;  // page-locked staging: noskip words up, then the results down, then the SSE table
   int nfb, maxCfg;
   cudaStream_t st;
   pf_ctx* ctx;
@@ -960,9 +961,10 @@ static int check_search_frame(const pf_frame* f, const pf_frame* recon) {
 
 static void level1_trials(TrialList* t);
 
-// source may be null (features only: the source is never read).
+// source may be null (features only: the source is never read).  table: the
+// SSE table will be wanted.
 static int stage_search(pf_ctx* ctx, const pf_frame* source, const pf_frame* recon, const uint8_t* noskip,
-                        int damping, int maxCfg, size_t extra, Staged* S) {
+                        int damping, int maxCfg, size_t extra, bool table, Staged* S) {
   int stt = check_search_frame(recon, recon);
   if (stt == PF_OK && source) stt = check_search_frame(source, recon);
   if (stt != PF_OK) return stt;
@@ -1017,8 +1019,10 @@ static int stage_search(pf_ctx* ctx, const pf_frame* source, const pf_frame* rec
   // scratch either way; host words go through page-locked staging so the
   // copy does not hold the host.
   // One page-locked block for the call (requested once, so it never moves
-  // while a copy is queued): the noskip words, then the selection results.
-  uint8_t* pin = (uint8_t*)pf_internal_pinned(ctx, al((size_t)nfb * 8) + al(sizeof(FinishOut)) + al(nfb));
+  // while a copy is queued): the noskip words, the selection results, the SSE
+  // table.
+  uint8_t* pin = (uint8_t*)pf_internal_pinned(ctx, al((size_t)nfb * 8) + al(sizeof(FinishOut)) + al(nfb) +
+                                                       (table ? (size_t)2 * nfb * 64 * 8 : 0));
   if (!pin) return PF_ERR_DEVICE;
   S->pin = pin;
   const uint8_t* ns = nullptr;
@@ -1093,20 +1097,32 @@ static int search_finish(Staged& S, const pf_cdef_search_params* params, uint64_
   const cudaStream_t st = S.st;
   if (launch_search(S.a, st) != cudaSuccess) return PF_ERR_DEVICE;
   if (ev && cudaEventRecord(ev[3], st) != cudaSuccess) return PF_ERR_DEVICE;
-  if (launch_select(S.s, S.maxCfg, (unsigned long long)params->lambda, S.idx, S.fo, st) != cudaSuccess)
-    return PF_ERR_DEVICE;
-  if (ev && cudaEventRecord(ev[4], st) != cudaSuccess) return PF_ERR_DEVICE;
   // The small results come back through the page-locked block (a pageable
-  // destination would make each copy a staged, synchronous one).
+  // destination would make each copy a staged, synchronous one).  So does
+  // the SSE table (522 KB at 1080p, 58 us of the call as a pageable copy at
+  // its end): on the second stream and on to the caller beside the selection,
+  // which does not write it.
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   uint8_t* pfo = S.pin + al((size_t)S.nfb * 8);
   uint8_t* pidx = pfo + al(sizeof(FinishOut));
-  if (cudaMemcpyAsync(pfo, S.fo, sizeof(FinishOut), cudaMemcpyDeviceToHost, st) != cudaSuccess) return PF_ERR_DEVICE;
-  if (mse_out &&
-      cudaMemcpyAsync(mse_out, S.a.mse, (size_t)2 * S.nfb * 64 * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+  uint8_t* ptab = pidx + al(S.nfb);
+  const size_t tab = (size_t)2 * S.nfb * 64 * 8;
+  cudaStream_t side = nullptr;
+  if (mse_out) {
+    side = (cudaStream_t)pf_internal_fork(S.ctx);
+    if (!side || cudaMemcpyAsync(ptab, S.a.mse, tab, cudaMemcpyDeviceToHost, side) != cudaSuccess) return PF_ERR_DEVICE;
+  }
+  if (launch_select(S.s, S.maxCfg, (unsigned long long)params->lambda, S.idx, S.fo, st) != cudaSuccess)
     return PF_ERR_DEVICE;
+  if (ev && cudaEventRecord(ev[4], st) != cudaSuccess) return PF_ERR_DEVICE;
+  if (cudaMemcpyAsync(pfo, S.fo, sizeof(FinishOut), cudaMemcpyDeviceToHost, st) != cudaSuccess) return PF_ERR_DEVICE;
   if (fb_index_out && cudaMemcpyAsync(pidx, S.idx, S.nfb, cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return PF_ERR_DEVICE;
+  if (mse_out) {
+    const int w = pf_internal_wait(S.ctx, side);
+    if (w != PF_OK) return w;
+    memcpy(mse_out, ptab, tab);
+  }
   const int w = pf_internal_wait(S.ctx, st);
   if (w != PF_OK) return w;
   FinishOut fo;
@@ -1132,7 +1148,7 @@ extern "C" int pf_cdef_search(pf_ctx* ctx, const pf_frame* source, const pf_fram
                               pf_cdef_search_result* result) {
   if (!ctx || !source || !recon || !params) return PF_ERR_INVALID_ARG;
   Staged S;
-  const int stt = stage_search(ctx, source, recon, noskip, search_damping(params), search_max_cfg(params), 0, &S);
+  const int stt = stage_search(ctx, source, recon, noskip, search_damping(params), search_max_cfg(params), 0, mse_out != nullptr, &S);
   if (stt != PF_OK) return stt;
   return search_finish(S, params, mse_out, fb_index_out, result);
 }
@@ -1153,7 +1169,7 @@ extern "C" int pf_cdef_search_ex(pf_ctx* ctx, const pf_frame* source, const pf_f
   t.count = ctrls->count;
   t.ss = ctrls->subsampling < 4 ? ctrls->subsampling : 4;  // BLOCK_8X8 caps the luma step (searchRow, :694-699)
   Staged S;
-  const int stt = stage_search(ctx, source, recon, noskip, search_damping(params), search_max_cfg(params), 0, &S);
+  const int stt = stage_search(ctx, source, recon, noskip, search_damping(params), search_max_cfg(params), 0, mse_out != nullptr, &S);
   if (stt != PF_OK) return stt;
   S.a.trials = t;
   S.s.uvFromY = ctrls->uv_from_y ? 1 : 0;
@@ -1373,7 +1389,7 @@ extern "C" int pf_cdef_features(pf_ctx* ctx, const pf_frame* recon, const uint8_
   const int miCols = ((recon->width + 7) >> 3) << 1, miRows = ((recon->height + 7) >> 3) << 1;
   const int nfb = ((miCols + 15) / 16) * ((miRows + 15) / 16);
   const size_t xBytes = (size_t)nfb * PF_MLP_FEATURES * sizeof(float);
-  const int stt = stage_search(ctx, nullptr, recon, noskip, dmp, 0, xBytes, &S);
+  const int stt = stage_search(ctx, nullptr, recon, noskip, dmp, 0, xBytes, false, &S);
   if (stt != PF_OK) return stt;
   float* X = (float*)S.extra;
   if (launch_features(S.a, qindex, X, true, S.st) != cudaSuccess) return PF_ERR_DEVICE;
@@ -1398,7 +1414,7 @@ extern "C" int pf_cdef_search_learned(pf_ctx* ctx, const pf_frame* source, const
   const size_t dBytes = al((size_t)nfb * 128);
   Staged S;
   const int stt = stage_search(ctx, source, recon, noskip, search_damping(params), search_max_cfg(params),
-                               xBytes + mBytes + dBytes, &S);
+                               xBytes + mBytes + dBytes, mse_out != nullptr, &S);
   if (stt != PF_OK) return stt;
   float* X = (float*)S.extra;
   uint64_t* masks = (uint64_t*)(S.extra + xBytes);
