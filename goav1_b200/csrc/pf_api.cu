@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "pf_common.cuh"
+#include "pf_superres.cuh"
 #include "pf_wait.h"
 
 namespace pf {
@@ -34,11 +35,6 @@ cudaError_t launch_fg_apply_batch(const BatchArgs& b, int total, int grid, cudaS
 cudaError_t launch_extend_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
 cudaError_t lr_upload_tables();
 cudaError_t fg_upload_tables();
-cudaError_t launch_superres_frame(const uint8_t* const* src, const int64_t* sstride, uint8_t* const* dst,
-                                  const int64_t* dstride, const pf_frame* coded, int upW, cudaStream_t st);
-cudaError_t launch_superres_lines(const uint8_t* const* src, const int64_t* sstride, uint8_t* const* lines,
-                                  const int64_t* lstride, const int* nb, const pf_frame* coded, int upW,
-                                  cudaStream_t st);
 }  // namespace pf
 
 using namespace pf;
@@ -531,7 +527,7 @@ extern "C" pf_ctx* pf_create(const pf_config* cfg, int* status) {
   c->timing = cfg ? cfg->timing : 0;
   c->wait_timeout_us = cfg ? cfg->wait_timeout_us : 0;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess || lr_upload_tables() != cudaSuccess ||
-      fg_upload_tables() != cudaSuccess) {
+      fg_upload_tables() != cudaSuccess || superres_upload_tables() != cudaSuccess) {
     delete c;
     if (status) *status = PF_ERR_DEVICE;
     return nullptr;
@@ -616,6 +612,10 @@ struct FrameRef {
   // upscaled deblock rows); null: the CDEF pass saves them.
   uint8_t* ext_lines[3];
   int64_t ext_line_stride[3];
+  // The frame's samples do not exist yet: they are the upscale of `coded`
+  // (a super-resolved frame), made before the frame's stages run, into the
+  // CDEF output's place when the frame is restored and into the frame else.
+  const SrFrame* coded;
 };
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -716,6 +716,11 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
     const int xdec = p ? f->ss_x : 0, ydec = p ? f->ss_y : 0;
     J.aw[p] = ((f->width + 7) & ~7) >> xdec;
     J.ah[p] = ((f->height + 7) & ~7) >> ydec;
+    if (r.coded) {
+      // What lies around an upscaled crop is the caller's.
+      J.aw[p] = f->plane[p].width;
+      J.ah[p] = f->plane[p].height;
+    }
   }
   for (int k = 0; k < ST_COUNT; k++) counts[k] = 0;
 
@@ -812,14 +817,16 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
         l.line_stride[p] = a.line_stride[p];
       }
     }
-    counts[ST_CDEF] = ucols * urows;
+    counts[ST_CDEF] = r.coded ? 0 : ucols * urows;
     int tiles = 0;
     for (int p = 0; p < (f->mono ? 1 : 3); p++) {
       const int sx = p ? f->ss_x : 0, sy = p ? f->ss_y : 0;
       // Units are powers of two and tiles start at multiples of their width,
-      // so a tile no wider than a unit has one unit.
+      // so a tile no wider than a unit has one unit.  A plane that is only
+      // copied back takes four tiles' width at a time: 16 KB a CTA keep four
+      // 16-byte words of each thread in flight.
       const int SH = 64 >> sy, off = 8 >> sy;
-      const int PW = lrOn && s->lr.type[p] != PF_LR_NONE && J.lr.unit_size[p] < 64 ? 64 >> sx : 64;
+      const int PW = !lrOn || s->lr.type[p] == PF_LR_NONE ? 256 : J.lr.unit_size[p] < 64 ? 64 >> sx : 64;
       J.lr.tile_w[p] = PW;
       J.lr_cols[p] = (J.aw[p] + PW - 1) / PW;
       J.lr_rows[p] = (J.ah[p] + off + SH - 1) / SH;
@@ -1147,9 +1154,8 @@ static int prepare_batch(pf_ctx* c, const FrameRef* refs, int n, Bytes& hs, DevB
 
 static void add_stats(const pf_ctx* c, int n, uint32_t done, pf_stats* stats) {
   if (!stats) return;
-  auto total = [&](int k) { return c->hbase[(size_t)k * (n + 1) + n]; };
   stats->completed |= done;
-  stats->cdef_units += total(ST_CDEF);
+  for (int i = 0; i < n; i++) stats->cdef_units += c->hjobs[i].cdef.ucols * c->hjobs[i].cdef.urows;
   // Restoration units are counted as the reference's processing units (64
   // luma samples wide), whatever the tiles' width.
   for (int i = 0; i < n; i++) {
@@ -1173,6 +1179,19 @@ static int run_batch(pf_ctx* c, const FrameRef* refs, int n, pf_stats* stats, bo
   }
   int st = prepare_batch(c, refs, n, c->hside, c->sidebuf, &done, &fg);
   if (st != PF_OK) return st;
+  // Super-resolved frames: the upscales, where their stages will read them.
+  std::vector<SrFrame> sr;
+  for (int i = 0; i < n; i++)
+    if (refs[i].coded) {
+      SrFrame u = *refs[i].coded;
+      const DFrame& to = c->hjobs[i].do_lr ? c->hjobs[i].scr : c->hjobs[i].io;
+      for (int p = 0; p < 3; p++) {
+        u.dst[p] = to.pl[p].ptr;
+        u.dstride[p] = to.pl[p].stride;
+      }
+      sr.push_back(u);
+    }
+  if (!sr.empty()) CK(launch_superres(sr.data(), (int)sr.size(), false, c->stream));
   const int est = (useGraph && !c->timing)
                       ? replay_or_capture(c, n, fg)
                       : enqueue_batch(c, c->hjobs.data(), c->hbase.data(), c->hside.data(), c->hside.size(), n, fg);
@@ -1516,6 +1535,114 @@ static size_t superres_line_bytes(const pf_frame* up, const pf_frame_side* sb, i
   return total;
 }
 
+// A super-resolved frame's device planes and its two halves of side information.
+struct SrWork {
+  const pf_frame *coded, *up, *display;  // display: null without grain
+  const pf_frame_side *sa, *sb;
+  void *cio[3], *uio[3], *dio[3];
+  int64_t cst[3], ust[3], dst[3];
+};
+
+// The chain on n super-resolved frames, each stage one launch over every frame
+// that has it: deblocking of the coded frames, their stripe-boundary rows
+// upscaled into one buffer, CDEF, the upscales and the upscaled grid's stages.
+// A restored frame is upscaled straight into the place the restoration reads
+// from, so no pass copies it there.  *acc: all runs' statistics; *last: the
+// upscaled grid's.
+static int superres_chain(pf_ctx* c, const SrWork* w, int n, pf_stats* acc, pf_stats* last) {
+  auto run = [&](std::vector<FrameRef>& refs, pf_stats* one) {
+    if (refs.empty()) return (int)PF_OK;
+    const int st = run_batch(c, refs.data(), (int)refs.size(), one);
+    acc->completed |= one->completed;
+    acc->cdef_units += one->cdef_units;
+    acc->lr_units += one->lr_units;
+    acc->fg_rows += one->fg_rows;
+    return st;
+  };
+  auto coded_ref = [&](int i, const pf_frame_side* side) {
+    FrameRef x;
+    memset(&x, 0, sizeof(x));
+    x.f = w[i].coded;
+    x.s = side;
+    for (int p = 0; p < 3; p++) {
+      x.io[p] = w[i].cio[p];
+      x.ioStride[p] = w[i].cst[p];
+    }
+    return x;
+  };
+  std::vector<pf_frame_side> s1((size_t)n), s2((size_t)n);
+  std::vector<FrameRef> refs;
+  refs.reserve((size_t)n);
+  pf_stats one;
+  for (int i = 0; i < n; i++)
+    if (w[i].sa->stages & PF_STAGE_LOOP_FILTER) {
+      s1[i] = *w[i].sa;
+      s1[i].stages = PF_STAGE_LOOP_FILTER;
+      refs.push_back(coded_ref(i, &s1[i]));
+    }
+  int st = run(refs, &one);
+  if (st != PF_OK) return st;
+  std::vector<SrFrame> sr((size_t)n);
+  size_t ltotal = 0;
+  for (int i = 0; i < n; i++) {
+    SrFrame& f = sr[i];
+    memset(&f, 0, sizeof(f));
+    f.coded = w[i].coded;
+    f.up_width = w[i].up->width;
+    for (int p = 0; p < 3; p++) {
+      f.src[p] = (const uint8_t*)w[i].cio[p];
+      f.sstride[p] = w[i].cst[p];
+    }
+    ltotal += superres_line_bytes(w[i].up, w[i].sb, f.boundaries, f.dstride);
+  }
+  if (ltotal) CK(c->sr_lines.ensure(ltotal + 256));
+  size_t off = 0;
+  for (SrFrame& f : sr)
+    for (int p = 0; p < 3; p++)
+      if (f.boundaries[p]) {
+        f.dst[p] = (uint8_t*)c->sr_lines.p + off;
+        off += align256((size_t)f.boundaries[p] * 4 * f.dstride[p]);
+      }
+  CK(launch_superres(sr.data(), n, true, c->stream));
+  refs.clear();
+  for (int i = 0; i < n; i++)
+    if ((w[i].sa->stages & PF_STAGE_CDEF) && cdef_any(w[i].coded, w[i].sa)) {
+      s2[i] = *w[i].sa;
+      s2[i].stages = PF_STAGE_CDEF;
+      refs.push_back(coded_ref(i, &s2[i]));
+    }
+  if ((st = run(refs, &one)) != PF_OK) return st;
+  refs.clear();
+  std::vector<SrFrame> direct;  // frames with no stage after the upscale
+  for (int i = 0; i < n; i++) {
+    if (!w[i].sb->stages) {
+      direct.push_back(sr[i]);
+      for (int p = 0; p < 3; p++) {
+        direct.back().dst[p] = (uint8_t*)w[i].uio[p];
+        direct.back().dstride[p] = w[i].ust[p];
+      }
+      continue;
+    }
+    FrameRef x;
+    memset(&x, 0, sizeof(x));
+    x.f = w[i].up;
+    x.s = w[i].sb;
+    x.display = w[i].display;
+    x.coded = &sr[i];
+    for (int p = 0; p < 3; p++) {
+      x.io[p] = w[i].uio[p];
+      x.ioStride[p] = w[i].ust[p];
+      x.dp[p] = w[i].dio[p];
+      x.dStride[p] = w[i].dst[p];
+      x.ext_lines[p] = sr[i].boundaries[p] ? sr[i].dst[p] : nullptr;
+      x.ext_line_stride[p] = sr[i].boundaries[p] ? sr[i].dstride[p] : 0;
+    }
+    refs.push_back(x);
+  }
+  if (!direct.empty()) CK(launch_superres(direct.data(), (int)direct.size(), false, c->stream));
+  return run(refs, last);
+}
+
 extern "C" int pf_frame_apply_superres(pf_ctx* c, const pf_frame* coded, const pf_frame_side* s,
                                        const pf_frame* up, const pf_frame* display, pf_stats* stats) {
   if (!c) return PF_ERR_INVALID_ARG;
@@ -1557,59 +1684,25 @@ extern "C" int pf_frame_apply_superres(pf_ctx* c, const pf_frame* coded, const p
       }
     }
   }
-  auto ref_of = [](const pf_frame* f, const pf_frame_side* side, void* const* io, const int64_t* ios) {
-    FrameRef x;
-    memset(&x, 0, sizeof(x));
-    x.f = f;
-    x.s = side;
-    for (int p = 0; p < 3; p++) {
-      x.io[p] = io[p];
-      x.ioStride[p] = ios[p];
-    }
-    return x;
-  };
-  uint32_t done = 0;
-  if (sa.stages & PF_STAGE_LOOP_FILTER) {
-    pf_frame_side s1 = sa;
-    s1.stages = PF_STAGE_LOOP_FILTER;
-    const FrameRef x = ref_of(coded, &s1, cio, cst);
-    if ((st = run_batch(c, &x, 1, nullptr)) != PF_OK) return st;
-    done |= PF_STAGE_LOOP_FILTER;
+  SrWork w;
+  w.coded = coded;
+  w.up = up;
+  w.display = wantDisp ? display : nullptr;
+  w.sa = &sa;
+  w.sb = &sb;
+  for (int p = 0; p < 3; p++) {
+    w.cio[p] = cio[p];
+    w.cst[p] = cst[p];
+    w.uio[p] = uio[p];
+    w.ust[p] = ust[p];
+    w.dio[p] = dio[p];
+    w.dst[p] = dst3[p];
   }
-  // The deblocked coded rows around the stripe boundaries, upscaled.
-  uint8_t* lines[3] = {};
-  int64_t lstride[3] = {};
-  if (lr_any(&sb)) {
-    int nb[3];
-    const size_t total = superres_line_bytes(up, &sb, nb, lstride);
-    CK(c->sr_lines.ensure(total + 256));
-    size_t off = 0;
-    for (int p = 0; p < nplanes; p++)
-      if (nb[p]) {
-        lines[p] = (uint8_t*)c->sr_lines.p + off;
-        off += align256((size_t)nb[p] * 4 * lstride[p]);
-      }
-    CK(launch_superres_lines((const uint8_t* const*)cio, cst, lines, lstride, nb, coded, up->width, cs));
-  }
-  if ((sa.stages & PF_STAGE_CDEF) && cdef_any(coded, &sa)) {
-    pf_frame_side s2 = sa;
-    s2.stages = PF_STAGE_CDEF;
-    const FrameRef x = ref_of(coded, &s2, cio, cst);
-    if ((st = run_batch(c, &x, 1, nullptr)) != PF_OK) return st;
-    done |= PF_STAGE_CDEF;
-  }
-  CK(launch_superres_frame((const uint8_t* const*)cio, cst, (uint8_t* const*)uio, ust, coded, up->width, cs));
-  if (sb.stages) {
-    FrameRef x = ref_of(up, &sb, uio, ust);
-    x.display = wantDisp ? display : nullptr;
-    for (int p = 0; p < 3; p++) {
-      x.dp[p] = dio[p];
-      x.dStride[p] = dst3[p];
-      x.ext_lines[p] = lines[p];
-      x.ext_line_stride[p] = lstride[p];
-    }
-    if ((st = run_batch(c, &x, 1, stats)) != PF_OK) return st;
-  }
+  pf_stats acc;
+  memset(&acc, 0, sizeof(acc));
+  pf_stats last;
+  memset(&last, 0, sizeof(last));
+  if ((st = superres_chain(c, &w, 1, &acc, &last)) != PF_OK) return st;
   if (host) {
     auto down = [&](const pf_frame* f, void* const* dev, const int64_t* ds) -> cudaError_t {
       for (int p = 0; p < nplanes; p++) {
@@ -1626,7 +1719,9 @@ extern "C" int pf_frame_apply_superres(pf_ctx* c, const pf_frame* coded, const p
   }
   CKW(wait_stream(c, cs, __LINE__));
   if (stats) {
-    stats->completed |= done;
+    // The unit counts are those of the upscaled frame's stages.
+    *stats = last;
+    stats->completed = acc.completed;
     read_stage_times(c, stats);
   }
   CK(cudaGetLastError());
@@ -1664,102 +1759,28 @@ extern "C" int pf_batch_apply_superres(pf_ctx* c, const pf_superres_item* items,
     return PF_OK;
   }
   CK(cudaSetDevice(c->device));
-  const cudaStream_t cs = c->stream;
-  auto ref_of = [](const pf_frame* f, const pf_frame_side* side) {
-    FrameRef x;
-    memset(&x, 0, sizeof(x));
-    x.f = f;
-    x.s = side;
+  std::vector<SrWork> w((size_t)n);
+  for (int i = 0; i < n; i++) {
+    SrWork& x = w[i];
+    x.coded = items[i].coded;
+    x.up = items[i].up;
+    x.display = (sb[i].stages & PF_STAGE_FILM_GRAIN) ? items[i].display : nullptr;
+    x.sa = &sa[i];
+    x.sb = &sb[i];
     for (int p = 0; p < 3; p++) {
-      x.io[p] = f->plane[p].data;
-      x.ioStride[p] = f->plane[p].stride;
+      x.cio[p] = x.coded->plane[p].data;
+      x.cst[p] = x.coded->plane[p].stride;
+      x.uio[p] = x.up->plane[p].data;
+      x.ust[p] = x.up->plane[p].stride;
+      x.dio[p] = x.display ? x.display->plane[p].data : nullptr;
+      x.dst[p] = x.display ? x.display->plane[p].stride : 0;
     }
-    return x;
-  };
-  pf_stats acc;
+  }
+  pf_stats acc, last;
   memset(&acc, 0, sizeof(acc));
-  auto run = [&](std::vector<FrameRef>& refs) {
-    if (refs.empty()) return (int)PF_OK;
-    pf_stats one;
-    const int st = run_batch(c, refs.data(), (int)refs.size(), &one);
-    acc.completed |= one.completed;
-    acc.cdef_units += one.cdef_units;
-    acc.lr_units += one.lr_units;
-    acc.fg_rows += one.fg_rows;
-    return st;
-  };
-  std::vector<pf_frame_side> s1((size_t)n), s2((size_t)n);
-  std::vector<FrameRef> refs;
-  refs.reserve((size_t)n);
-  // Deblocking, every coded frame in one launch per pass.
-  for (int i = 0; i < n; i++)
-    if (sa[i].stages & PF_STAGE_LOOP_FILTER) {
-      s1[i] = sa[i];
-      s1[i].stages = PF_STAGE_LOOP_FILTER;
-      refs.push_back(ref_of(items[i].coded, &s1[i]));
-    }
-  int st = run(refs);
+  memset(&last, 0, sizeof(last));
+  const int st = superres_chain(c, w.data(), n, &acc, &last);
   if (st != PF_OK) return st;
-  // The deblocked rows around each frame's stripe boundaries, upscaled, into
-  // one buffer for the whole batch.
-  std::vector<int> nb((size_t)n * 3);
-  std::vector<int64_t> lstride((size_t)n * 3);
-  std::vector<size_t> loff((size_t)n);
-  size_t ltotal = 0;
-  for (int i = 0; i < n; i++) {
-    loff[i] = ltotal;
-    ltotal += superres_line_bytes(items[i].up, &sb[i], &nb[3 * i], &lstride[3 * i]);
-  }
-  if (ltotal) CK(c->sr_lines.ensure(ltotal + 256));
-  std::vector<uint8_t*> lines((size_t)n * 3, nullptr);
-  for (int i = 0; i < n; i++) {
-    if (!lr_any(&sb[i])) continue;
-    size_t off = loff[i];
-    for (int p = 0; p < 3; p++)
-      if (nb[3 * i + p]) {
-        lines[3 * i + p] = (uint8_t*)c->sr_lines.p + off;
-        off += align256((size_t)nb[3 * i + p] * 4 * lstride[3 * i + p]);
-      }
-    const pf_frame* cf = items[i].coded;
-    void* cio[3] = {cf->plane[0].data, cf->plane[1].data, cf->plane[2].data};
-    const int64_t cst[3] = {cf->plane[0].stride, cf->plane[1].stride, cf->plane[2].stride};
-    CK(launch_superres_lines((const uint8_t* const*)cio, cst, &lines[3 * i], &lstride[3 * i], &nb[3 * i], cf,
-                             items[i].up->width, cs));
-  }
-  // CDEF over the coded frames.
-  refs.clear();
-  for (int i = 0; i < n; i++)
-    if ((sa[i].stages & PF_STAGE_CDEF) && cdef_any(items[i].coded, &sa[i])) {
-      s2[i] = sa[i];
-      s2[i].stages = PF_STAGE_CDEF;
-      refs.push_back(ref_of(items[i].coded, &s2[i]));
-    }
-  if ((st = run(refs)) != PF_OK) return st;
-  // Upscale, then the upscaled-grid stages over every frame.
-  refs.clear();
-  for (int i = 0; i < n; i++) {
-    const pf_frame* cf = items[i].coded;
-    const pf_frame* uf = items[i].up;
-    void* cio[3] = {cf->plane[0].data, cf->plane[1].data, cf->plane[2].data};
-    const int64_t cst[3] = {cf->plane[0].stride, cf->plane[1].stride, cf->plane[2].stride};
-    void* uio[3] = {uf->plane[0].data, uf->plane[1].data, uf->plane[2].data};
-    const int64_t ust[3] = {uf->plane[0].stride, uf->plane[1].stride, uf->plane[2].stride};
-    CK(launch_superres_frame((const uint8_t* const*)cio, cst, (uint8_t* const*)uio, ust, cf, uf->width, cs));
-    if (!sb[i].stages) continue;
-    FrameRef x = ref_of(uf, &sb[i]);
-    const bool wantDisp = (sb[i].stages & PF_STAGE_FILM_GRAIN) && items[i].display;
-    x.display = wantDisp ? items[i].display : nullptr;
-    for (int p = 0; p < 3; p++) {
-      if (wantDisp) {
-        x.dp[p] = items[i].display->plane[p].data;
-        x.dStride[p] = items[i].display->plane[p].stride;
-      }
-      x.ext_lines[p] = lines[3 * i + p];
-      x.ext_line_stride[p] = lstride[3 * i + p];
-    }
-    refs.push_back(x);
-  }
-  if ((st = run(refs)) != PF_OK) return st;
   if (stats) *stats = acc;
   CK(cudaGetLastError());
   return PF_OK;

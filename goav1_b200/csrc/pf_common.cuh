@@ -55,13 +55,15 @@ __device__ __forceinline__ void copy_block(const DPlane& from, const DPlane& to,
   if (((reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(d0) | (uintptr_t)from.stride |
         (uintptr_t)to.stride | (uintptr_t)rowBytes) & 15) == 0) {
     const int wpr = rowBytes >> 4, total = (y1 - y0) * wpr;
+    const int lg = (wpr & (wpr - 1)) == 0 ? 31 - __clz(wpr) : -1;  // whole tiles: a power of two
+    auto row_of = [&](int i) { return lg >= 0 ? i >> lg : i / wpr; };
     for (int i0 = threadIdx.x; i0 < total; i0 += 4 * blockDim.x) {
       uint4 v[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         const int i = i0 + k * blockDim.x;
         if (i < total) {
-          const int r = i / wpr, c = i - r * wpr;
+          const int r = row_of(i), c = i - r * wpr;
           v[k] = *reinterpret_cast<const uint4*>(s0 + (int64_t)r * from.stride + c * 16);
         }
       }
@@ -69,7 +71,7 @@ __device__ __forceinline__ void copy_block(const DPlane& from, const DPlane& to,
       for (int k = 0; k < 4; k++) {
         const int i = i0 + k * blockDim.x;
         if (i < total) {
-          const int r = i / wpr, c = i - r * wpr;
+          const int r = row_of(i), c = i - r * wpr;
           *reinterpret_cast<uint4*>(d0 + (int64_t)r * to.stride + c * 16) = v[k];
         }
       }
