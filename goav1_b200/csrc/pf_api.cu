@@ -26,13 +26,13 @@
 #include "pf_wait.h"
 
 namespace pf {
-cudaError_t launch_deblock_batch(const BatchArgs& b, int total, int grid, int dir, cudaStream_t st);
-cudaError_t launch_cdef_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
-cudaError_t launch_lr_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
-cudaError_t launch_fg_templates_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
-cudaError_t launch_fg_offsets_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
-cudaError_t launch_fg_apply_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
-cudaError_t launch_extend_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
+cudaError_t launch_deblock(const StageLaunch& l, int dir);
+cudaError_t launch_cdef(const StageLaunch& l);
+cudaError_t launch_lr(const StageLaunch& l);
+cudaError_t launch_fg_templates(const StageLaunch& l);
+cudaError_t launch_fg_offsets(const StageLaunch& l);
+cudaError_t launch_fg_apply(const StageLaunch& l);
+cudaError_t launch_extend(const StageLaunch& l);
 cudaError_t lr_upload_tables();
 cudaError_t fg_upload_tables();
 }  // namespace pf
@@ -913,13 +913,23 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
   }
 }
 
+// Whether a batch is one frame under the default schedules, whose launches
+// carry the frame's job themselves (StageLaunch::one).
+static bool single_frame(const pf_ctx* c, int n) {
+  bool plain = n == 1 && (c->tile[ST_FG_APPLY] == 0 || c->tile[ST_FG_APPLY] == 3);
+  for (int k = 0; k < ST_COUNT; k++) plain &= c->persistent[k] == 0 && c->chunk[k] == 1 && c->ahead[k] == 0;
+  return plain;
+}
+
 // Queues the copies of the host tables (from the given host buffers) and
 // every stage's launch on the context's streams.
 // djobs / dbases: device copies of the tables when the caller uploaded them
 // already (null: copy hjobs / hbase / hside into the context's buffers here).
+// replayed: the launches are being captured and will run with other jobs.
 static int enqueue_batch(pf_ctx* c, const FrameJob* hjobs, const int* hbase, const uint8_t* hside, size_t nside,
-                         int n, bool fg, const void* djobs = nullptr, const void* dbases = nullptr) {
+                         int n, bool fg, bool replayed, const void* djobs = nullptr, const void* dbases = nullptr) {
   const cudaStream_t st = c->stream;
+  const FrameJob* one = !replayed && single_frame(c, n) ? hjobs : nullptr;
   if (!djobs) {
     if (nside) {
       CK(cudaMemcpyAsync(c->sidebuf.p, hside, nside, cudaMemcpyHostToDevice, st));
@@ -929,8 +939,10 @@ static int enqueue_batch(pf_ctx* c, const FrameJob* hjobs, const int* hbase, con
         c->side_pending = true;
       }
     }
-    CK(cudaMemcpyAsync(c->jobs.p, hjobs, sizeof(FrameJob) * n, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(c->bases.p, hbase, sizeof(int) * c->hbase.size(), cudaMemcpyHostToDevice, st));
+    if (!one) {
+      CK(cudaMemcpyAsync(c->jobs.p, hjobs, sizeof(FrameJob) * n, cudaMemcpyHostToDevice, st));
+      CK(cudaMemcpyAsync(c->bases.p, hbase, sizeof(int) * c->hbase.size(), cudaMemcpyHostToDevice, st));
+    }
     djobs = c->jobs.p;
     dbases = c->bases.p;
   }
@@ -957,33 +969,35 @@ static int enqueue_batch(pf_ctx* c, const FrameJob* hjobs, const int* hbase, con
   auto count = [&](int k, int f0, int f1) {
     return hbase[(size_t)k * (n + 1) + f1] - hbase[(size_t)k * (n + 1) + f0];
   };
-  auto args = [&](int k, int f0, int f1, int grp, int* grid) {
-    BatchArgs a = b;
-    a.f0 = f0;
-    a.f1 = f1;
-    const int t = count(k, f0, f1);
-    a.chunk = c->chunk[k];
-    a.ahead = c->ahead[k];
-    a.tile = c->tile[k];
-    const int chunks = (t + a.chunk - 1) / a.chunk;
+  // Stage k over the frames [f0, f1) of group grp on stream gs.
+  auto stage = [&](int k, int f0, int f1, int grp, cudaStream_t gs, bool dependent) {
+    StageLaunch l;
+    l.args = b;
+    l.args.f0 = f0;
+    l.args.f1 = f1;
+    l.one = one;
+    l.st = gs;
+    l.dependent = dependent;
+    l.total = count(k, f0, f1);
+    l.args.chunk = c->chunk[k];
+    l.args.ahead = c->ahead[k];
+    l.args.tile = c->tile[k];
+    const int chunks = (l.total + l.args.chunk - 1) / l.args.chunk;
     if (c->persistent[k] > 0 && chunks > c->persistent[k]) {
-      *grid = c->persistent[k];
-      a.counters = (int*)c->counters.p + grp * ST_COUNT;
+      l.grid = c->persistent[k];
+      l.args.counters = (int*)c->counters.p + grp * ST_COUNT;
     } else {
-      *grid = chunks;
-      a.counters = nullptr;
+      l.grid = chunks;
+      l.args.counters = nullptr;
     }
-    return a;
+    return l;
   };
-  int g;
   // Film-grain templates and offsets depend on nothing else: side stream.
   if (fg) {
     CK(cudaEventRecord(c->fork, st));
     CK(cudaStreamWaitEvent(c->side, c->fork, 0));
-    BatchArgs a = args(ST_FG_TEMPLATES, 0, n, 0, &g);
-    CK(launch_fg_templates_batch(a, count(ST_FG_TEMPLATES, 0, n), g, c->side));
-    a = args(ST_FG_OFFSETS, 0, n, 0, &g);
-    CK(launch_fg_offsets_batch(a, count(ST_FG_OFFSETS, 0, n), g, c->side));
+    CK(launch_fg_templates(stage(ST_FG_TEMPLATES, 0, n, 0, c->side, false)));
+    CK(launch_fg_offsets(stage(ST_FG_OFFSETS, 0, n, 0, c->side, false)));
     CK(cudaEventRecord(c->join, c->side));
   }
   // Stage events: per stage with one group; with two only the whole batch
@@ -997,20 +1011,27 @@ static int enqueue_batch(pf_ctx* c, const FrameJob* hjobs, const int* hbase, con
   for (int gi = 0; gi < groups; gi++) {
     const cudaStream_t gs = gi ? c->stream2 : st;
     const int f0 = gi ? fmid : 0, f1 = groups == 2 && gi == 0 ? fmid : n;
-    BatchArgs a = args(ST_DEBLOCK_V, f0, f1, gi, &g);
-    CK(launch_deblock_batch(a, count(ST_DEBLOCK_V, f0, f1), g, 0, gs));
-    a = args(ST_DEBLOCK_H, f0, f1, gi, &g);
-    CK(launch_deblock_batch(a, count(ST_DEBLOCK_H, f0, f1), g, 1, gs));
-    if (stageEv) CK(cudaEventRecord(c->ev[1], gs));
-    a = args(ST_CDEF, f0, f1, gi, &g);
-    CK(launch_cdef_batch(a, count(ST_CDEF, f0, f1), g, gs));
-    if (stageEv) CK(cudaEventRecord(c->ev[2], gs));
-    a = args(ST_LR, f0, f1, gi, &g);
-    CK(launch_lr_batch(a, count(ST_LR, f0, f1), g, gs));
-    if (stageEv) CK(cudaEventRecord(c->ev[3], gs));
-    a = args(ST_EXTEND, f0, f1, gi, &g);
-    CK(launch_extend_batch(a, count(ST_EXTEND, f0, f1), g, gs));
-    if (stageEv) CK(cudaEventRecord(c->ev[4], gs));
+    // A stage may overlap the drain of the one right before it on the stream
+    // (launch_stage); events in between rule that out.
+    bool after = false;
+    auto run = [&](int k, auto launch) {
+      const StageLaunch l = stage(k, f0, f1, gi, gs, after);
+      if (l.total > 0) after = true;
+      return launch(l);
+    };
+    auto mark = [&](int e) {
+      after = false;
+      return cudaEventRecord(c->ev[e], gs);
+    };
+    CK(run(ST_DEBLOCK_V, [](const StageLaunch& l) { return launch_deblock(l, 0); }));
+    CK(run(ST_DEBLOCK_H, [](const StageLaunch& l) { return launch_deblock(l, 1); }));
+    if (stageEv) CK(mark(1));
+    CK(run(ST_CDEF, launch_cdef));
+    if (stageEv) CK(mark(2));
+    CK(run(ST_LR, launch_lr));
+    if (stageEv) CK(mark(3));
+    CK(run(ST_EXTEND, launch_extend));
+    if (stageEv) CK(mark(4));
     if (c->mark_chain && gi == 0) {
       // While capturing, an external event node: each replay records it
       // for the copy stream that waits on it outside the graph.
@@ -1018,10 +1039,13 @@ static int enqueue_batch(pf_ctx* c, const FrameJob* hjobs, const int* hbase, con
       CK(cudaStreamIsCapturing(gs, &cap));
       CK(cap == cudaStreamCaptureStatusActive ? cudaEventRecordWithFlags(c->chain_done, gs, cudaEventRecordExternal)
                                                : cudaEventRecord(c->chain_done, gs));
+      after = false;
     }
-    if (fg) CK(cudaStreamWaitEvent(gs, c->join, 0));
-    a = args(ST_FG_APPLY, f0, f1, gi, &g);
-    CK(launch_fg_apply_batch(a, count(ST_FG_APPLY, f0, f1), g, gs));
+    if (fg) {
+      CK(cudaStreamWaitEvent(gs, c->join, 0));
+      after = false;
+    }
+    CK(run(ST_FG_APPLY, launch_fg_apply));
   }
   if (groups == 2) {
     CK(cudaEventRecord(c->gjoin, c->stream2));
@@ -1096,7 +1120,7 @@ static int replay_or_capture(pf_ctx* c, int n, bool fg) {
   if (!g.exec) {
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     const int est =
-        enqueue_batch(c, (const FrameJob*)g.pjobs, (const int*)g.pbase, (const uint8_t*)g.pside, ns, n, fg);
+        enqueue_batch(c, (const FrameJob*)g.pjobs, (const int*)g.pbase, (const uint8_t*)g.pside, ns, n, fg, true);
     const cudaError_t ce = cudaStreamEndCapture(st, &g.graph);
     cudaError_t ie = cudaSuccess;
     if (est == PF_OK && ce == cudaSuccess) ie = cudaGraphInstantiate(&g.exec, g.graph, 0);
@@ -1192,9 +1216,12 @@ static int run_batch(pf_ctx* c, const FrameRef* refs, int n, pf_stats* stats, bo
       sr.push_back(u);
     }
   if (!sr.empty()) CK(launch_superres(sr.data(), (int)sr.size(), false, c->stream));
-  const int est = (useGraph && !c->timing)
-                      ? replay_or_capture(c, n, fg)
-                      : enqueue_batch(c, c->hjobs.data(), c->hbase.data(), c->hside.data(), c->hside.size(), n, fg);
+  // A single frame's launches carry its job, which a captured graph could
+  // not: they go out directly (in less host time than a replay).
+  const int est =
+      (useGraph && !c->timing && !single_frame(c, n))
+          ? replay_or_capture(c, n, fg)
+          : enqueue_batch(c, c->hjobs.data(), c->hbase.data(), c->hside.data(), c->hside.size(), n, fg, false);
   if (est != PF_OK) return est;
   if (stats) {
     stats->completed = 0;
@@ -1470,7 +1497,7 @@ static int run_host_pipeline(pf_ctx* c, const pf_batch_item* items, int n, pf_st
     CK(cudaMemcpyAsync(h.dbases.p, h.pbase, nb, cudaMemcpyHostToDevice, c->h2d));
     CK(cudaEventRecord(h.up, c->h2d));
     CK(cudaStreamWaitEvent(c->stream, h.up, 0));
-    st = enqueue_batch(c, (const FrameJob*)h.pjobs, (const int*)h.pbase, nullptr, 0, m, fg, h.djobs.p, h.dbases.p);
+    st = enqueue_batch(c, (const FrameJob*)h.pjobs, (const int*)h.pbase, nullptr, 0, m, fg, false, h.djobs.p, h.dbases.p);
     if (st != PF_OK) return st;
     add_stats(c, m, done, stats);
     CK(cudaEventRecord(h.comp, c->stream));

@@ -530,31 +530,33 @@ __device__ __noinline__ int cdef_unit_planes(const FrameJob* J, int uc, int ur, 
   return cdef_unit<T, false, false>(*J, uc, ur, 0, *sm);
 }
 
+__device__ __forceinline__ void cdef_item(const FrameJob& J, int local, CdefSmem& sm) {
+  const int uc = local % J.cdef.ucols, ur = local / J.cdef.ucols;
+  const bool c420 = J.io.ssx && J.io.ssy;
+  if (J.io.bd == 8) {
+    if (c420)
+      cdef_unit<uint8_t, false, true>(J, uc, ur, 0, sm);
+    else
+      cdef_unit_planes<uint8_t>(&J, uc, ur, &sm);
+  } else {
+    int from = 0;
+    if (J.io.bd == 10)
+      from = c420 ? cdef_unit<uint16_t, false, true>(J, uc, ur, 0, sm) : cdef_unit_planes<uint16_t>(&J, uc, ur, &sm);
+    if (from < 3) cdef_unit_raw(&J, uc, ur, from, &sm);
+  }
+}
+
 // Batched CDEF: each work item is one 64x64 unit of one frame.
 template <bool kLoop>
 __global__ void __launch_bounds__(256, 4) k_cdef_batch(BatchArgs b) {
   __shared__ CdefSmem sm;
+  stage_begin();
   const int* base = b.base + ST_CDEF * (b.n + 1);
   for_each_item<kLoop>(
       b, ST_CDEF,
       [&](int item) {
         const int fi = find_frame(base, b.n, item);
-        const FrameJob& J = b.jobs[fi];
-        const int local = item - base[fi];
-        const int uc = local % J.cdef.ucols, ur = local / J.cdef.ucols;
-        const bool c420 = J.io.ssx && J.io.ssy;
-        if (J.io.bd == 8) {
-          if (c420)
-            cdef_unit<uint8_t, false, true>(J, uc, ur, 0, sm);
-          else
-            cdef_unit_planes<uint8_t>(&J, uc, ur, &sm);
-        } else {
-          int from = 0;
-          if (J.io.bd == 10)
-            from = c420 ? cdef_unit<uint16_t, false, true>(J, uc, ur, 0, sm)
-                        : cdef_unit_planes<uint16_t>(&J, uc, ur, &sm);
-          if (from < 3) cdef_unit_raw(&J, uc, ur, from, &sm);
-        }
+        cdef_item(b.jobs[fi], item - base[fi], sm);
       },
       [&](int item) {
         // Every plane's unit with its 8-column / 2-row halo.
@@ -573,14 +575,19 @@ __global__ void __launch_bounds__(256, 4) k_cdef_batch(BatchArgs b) {
       });
 }
 
-cudaError_t launch_cdef_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
+__global__ void __launch_bounds__(256, 4) k_cdef_one(const __grid_constant__ FrameJob J) {
+  __shared__ CdefSmem sm;
+  stage_begin();
+  cdef_item(J, blockIdx.x, sm);
+}
+
+cudaError_t launch_cdef(const StageLaunch& l) {
+  if (l.total <= 0) return cudaSuccess;
+  if (l.one) return launch_stage(k_cdef_one, l.total, 256, 0, l.st, l.dependent, *l.one);
   static int wave = 0;
-  if (batch_loops(b))
-    k_cdef_batch<true><<<grid, 256, 0, st>>>(b);
-  else
-    k_cdef_batch<false><<<grid, 256, 0, st>>>(with_wave(b, k_cdef_batch<false>, 256, 0, wave));
-  return cudaGetLastError();
+  if (batch_loops(l.args)) return launch_stage(k_cdef_batch<true>, l.grid, 256, 0, l.st, l.dependent, l.args);
+  return launch_stage(k_cdef_batch<false>, l.grid, 256, 0, l.st, l.dependent,
+                      with_wave(l.args, k_cdef_batch<false>, 256, 0, wave));
 }
 
 }  // namespace pf

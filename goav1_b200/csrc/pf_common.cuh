@@ -332,8 +332,48 @@ __device__ __forceinline__ void for_each_item(const BatchArgs& b, int stage, F f
   for_each_item<kLoop>(b, stage, f, none);
 }
 
+// Start of every stage kernel.  A stage's launch may be a programmatic
+// dependent of the stage before (launch_stage): its CTAs are placed while
+// that one drains and wait here until it has finished and its writes are
+// visible.  The next stage may in turn be placed as soon as all of this
+// one's CTAs have started.  Neither does anything in an ordinary launch.
+__device__ __forceinline__ void stage_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Whether a launch needs the looping form of for_each_item.
 inline bool batch_loops(const BatchArgs& b) { return b.counters != nullptr || b.chunk > 1; }
+
+// Launches a stage kernel; `dependent`: the work before it on the stream is a
+// stage kernel, which it may overlap up to stage_begin.
+template <class... P, class... A>
+inline cudaError_t launch_stage(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st,
+                                bool dependent, const A&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// How a stage is launched: over the job table (args), or, for a single frame
+// under the default schedules, with the frame's job itself as the kernel's
+// argument (`one`), which saves the table's copies and every CTA the way
+// through it.
+struct StageLaunch {
+  BatchArgs args;
+  const FrameJob* one;  // host pointer, or null
+  int total, grid;
+  cudaStream_t st;
+  bool dependent;
+};
 
 // CTAs of `kernel` the current device holds at once (SMs x CTAs per SM at
 // `threads` threads and `smem` dynamic shared bytes): a launch's wave.

@@ -264,58 +264,65 @@ __device__ __forceinline__ void deblock_unit(const DFrame& f, const LfArgs& a, i
 // of one frame (db_tile_w x db_tile_h units, 32x8 by default); 256 threads,
 // one edge unit each.
 struct DbTile {
-  const FrameJob* J;
   int plane, tx, ty;
 };
 
-__device__ __forceinline__ DbTile db_locate(const BatchArgs& b, const int* base, int item) {
-  const int fi = find_frame(base, b.n, item);
-  const FrameJob& J = b.jobs[fi];
-  int local = item - base[fi];
+__device__ __forceinline__ DbTile db_locate(const FrameJob& J, int local) {
   int plane = 0;
   while (plane < 2 && local >= J.db_tx[plane] * J.db_ty[plane]) {
     local -= J.db_tx[plane] * J.db_ty[plane];
     plane++;
   }
-  return DbTile{&J, plane, local % J.db_tx[plane], local / J.db_tx[plane]};
+  return DbTile{plane, local % J.db_tx[plane], local / J.db_tx[plane]};
+}
+
+__device__ __forceinline__ void db_tile(const FrameJob& J, int local, int dir) {
+  const DbTile t = db_locate(J, local);
+  const int tw = db_tile_w(J.db_tile), lg = 31 - __clz(tw);
+  const int c4 = t.tx * tw + (threadIdx.x & (tw - 1)), r4 = t.ty * (256 >> lg) + (threadIdx.x >> lg);
+  if (J.io.bd == 8)
+    deblock_unit<uint8_t>(J.io, J.lf, dir, t.plane, c4, r4);
+  else
+    deblock_unit<uint16_t>(J.io, J.lf, dir, t.plane, c4, r4);
 }
 
 template <bool kLoop>
 __global__ void __launch_bounds__(256, 4) k_deblock_batch(BatchArgs b, int dir) {
+  stage_begin();
   const int stage = dir == 0 ? ST_DEBLOCK_V : ST_DEBLOCK_H;
   const int* base = b.base + stage * (b.n + 1);
   for_each_item<kLoop>(
       b, stage,
       [&](int item) {
-        const DbTile t = db_locate(b, base, item);
-        const FrameJob& J = *t.J;
-        const int tw = db_tile_w(J.db_tile), lg = 31 - __clz(tw);
-        const int c4 = t.tx * tw + (threadIdx.x & (tw - 1)), r4 = t.ty * (256 >> lg) + (threadIdx.x >> lg);
-        if (J.io.bd == 8)
-          deblock_unit<uint8_t>(J.io, J.lf, dir, t.plane, c4, r4);
-        else
-          deblock_unit<uint16_t>(J.io, J.lf, dir, t.plane, c4, r4);
+        const int fi = find_frame(base, b.n, item);
+        db_tile(b.jobs[fi], item - base[fi], dir);
       },
       [&](int item) {
         // The tile's samples and the 8 on each side its edges can reach.
-        const DbTile t = db_locate(b, base, item);
-        const int tw = db_tile_w(t.J->db_tile), th = 256 / tw;
+        const int fi = find_frame(base, b.n, item);
+        const FrameJob& J = b.jobs[fi];
+        const DbTile t = db_locate(J, item - base[fi]);
+        const int tw = db_tile_w(J.db_tile), th = 256 / tw;
         const int x0 = t.tx * tw * 4, y0 = t.ty * th * 4;
-        if (t.J->io.bd == 8)
-          prefetch_block<uint8_t>(t.J->io.pl[t.plane], x0 - 8, x0 + tw * 4 + 8, y0 - 8, y0 + th * 4 + 8);
+        if (J.io.bd == 8)
+          prefetch_block<uint8_t>(J.io.pl[t.plane], x0 - 8, x0 + tw * 4 + 8, y0 - 8, y0 + th * 4 + 8);
         else
-          prefetch_block<uint16_t>(t.J->io.pl[t.plane], x0 - 8, x0 + tw * 4 + 8, y0 - 8, y0 + th * 4 + 8);
+          prefetch_block<uint16_t>(J.io.pl[t.plane], x0 - 8, x0 + tw * 4 + 8, y0 - 8, y0 + th * 4 + 8);
       });
 }
 
-cudaError_t launch_deblock_batch(const BatchArgs& b, int total, int grid, int dir, cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
+__global__ void __launch_bounds__(256, 4) k_deblock_one(const __grid_constant__ FrameJob J, int dir) {
+  stage_begin();
+  db_tile(J, blockIdx.x, dir);
+}
+
+cudaError_t launch_deblock(const StageLaunch& l, int dir) {
+  if (l.total <= 0) return cudaSuccess;
+  if (l.one) return launch_stage(k_deblock_one, l.total, 256, 0, l.st, l.dependent, *l.one, dir);
   static int wave = 0;
-  if (batch_loops(b))
-    k_deblock_batch<true><<<grid, 256, 0, st>>>(b, dir);
-  else
-    k_deblock_batch<false><<<grid, 256, 0, st>>>(with_wave(b, k_deblock_batch<false>, 256, 0, wave), dir);
-  return cudaGetLastError();
+  if (batch_loops(l.args)) return launch_stage(k_deblock_batch<true>, l.grid, 256, 0, l.st, l.dependent, l.args, dir);
+  return launch_stage(k_deblock_batch<false>, l.grid, 256, 0, l.st, l.dependent,
+                      with_wave(l.args, k_deblock_batch<false>, 256, 0, wave), dir);
 }
 
 }  // namespace pf

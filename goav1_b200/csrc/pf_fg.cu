@@ -16,8 +16,6 @@
 // t), one warp per template, rows in lanes, neighbours passed between lanes
 // by shuffles.  Offsets come from one thread per 32-row stripe.  The apply
 // is a thread per 4x4 samples, 64x64-sample tiles per CTA.
-#include <atomic>
-
 #include "pf_common.cuh"
 #include "pf_tables.h"
 
@@ -592,57 +590,65 @@ __device__ __forceinline__ void extend_px(const DFrame& f, int plane, int x, int
 
 // ---- batched kernels ----
 
+__device__ __forceinline__ void fg_templates_item(const FrameJob& J, TplSmem& S) {
+  fg_templates(J.fgt, J.fg.grain[0], J.fg.grain[1], J.fg.grain[2], S);
+}
+
 __global__ void __launch_bounds__(kFgTemplateThreads) k_fg_templates_batch(BatchArgs b) {
   extern __shared__ __align__(16) unsigned char s_tpl[];
   TplSmem& S = *reinterpret_cast<TplSmem*>(s_tpl);
   const int* base = b.base + ST_FG_TEMPLATES * (b.n + 1);
-  for_each_item(b, ST_FG_TEMPLATES, [&](int item) {
-    const FrameJob& J = b.jobs[find_frame(base, b.n, item)];
-    fg_templates(J.fgt, J.fg.grain[0], J.fg.grain[1], J.fg.grain[2], S);
-  });
+  for_each_item(b, ST_FG_TEMPLATES, [&](int item) { fg_templates_item(b.jobs[find_frame(base, b.n, item)], S); });
+}
+
+__global__ void __launch_bounds__(kFgTemplateThreads) k_fg_templates_one(const __grid_constant__ FrameJob J) {
+  extern __shared__ __align__(16) unsigned char s_tpl[];
+  fg_templates_item(J, *reinterpret_cast<TplSmem*>(s_tpl));
+}
+
+__device__ __forceinline__ void fg_offsets_item(const FrameJob& J, int local) {
+  if (J.io.bd > 8) {
+    // The first items of a frame of more than 8 bits build its scaling
+    // tables, 256 entries each.
+    const int per = 1 << (J.io.bd - 8);
+    if (local < 3 * per) {
+      const int pl = local / per, i0 = (local - pl * per) * 256;
+      for (int i = threadIdx.x; i < 256; i += 64)
+        J.fg.scale[pl * kFgScaleLen + i0 + i] = (uint8_t)scale_at(J.fg.lut[pl], i0 + i, J.io.bd);
+      return;
+    }
+    local -= 3 * per;
+  }
+  const int r = local * 64 + threadIdx.x;
+  if (r < J.fg.off_rows) fg_offsets_row(J.fgt.seed, r, J.fg.off_cols, const_cast<uint8_t*>(J.fg.offsets));
 }
 
 __global__ void __launch_bounds__(64) k_fg_offsets_batch(BatchArgs b) {
   const int* base = b.base + ST_FG_OFFSETS * (b.n + 1);
   for_each_item(b, ST_FG_OFFSETS, [&](int item) {
     const int fi = find_frame(base, b.n, item);
-    const FrameJob& J = b.jobs[fi];
-    int local = item - base[fi];
-    if (J.io.bd > 8) {
-      // The first items of a frame of more than 8 bits build its scaling
-      // tables, 256 entries each.
-      const int per = 1 << (J.io.bd - 8);
-      if (local < 3 * per) {
-        const int pl = local / per, i0 = (local - pl * per) * 256;
-        for (int i = threadIdx.x; i < 256; i += 64)
-          J.fg.scale[pl * kFgScaleLen + i0 + i] = (uint8_t)scale_at(J.fg.lut[pl], i0 + i, J.io.bd);
-        return;
-      }
-      local -= 3 * per;
-    }
-    const int r = local * 64 + threadIdx.x;
-    if (r < J.fg.off_rows) fg_offsets_row(J.fgt.seed, r, J.fg.off_cols, const_cast<uint8_t*>(J.fg.offsets));
+    fg_offsets_item(b.jobs[fi], item - base[fi]);
   });
+}
+
+__global__ void __launch_bounds__(64) k_fg_offsets_one(const __grid_constant__ FrameJob J) {
+  fg_offsets_item(J, blockIdx.x);
 }
 
 // Display frame: 64x64-sample tiles of each plane, 256 threads of four
 // columns by four rows.  The plane's scaling table is staged in shared memory
 // per tile.
 struct FgTile {
-  const FrameJob* J;
   int plane, tx, ty;
 };
 
-__device__ __forceinline__ FgTile fg_locate(const BatchArgs& b, const int* base, int item) {
-  const int fi = find_frame(base, b.n, item);
-  const FrameJob& J = b.jobs[fi];
-  int local = item - base[fi];
+__device__ __forceinline__ FgTile fg_locate(const FrameJob& J, int local) {
   int plane = 0;
   while (plane < 2 && local >= J.fg_tx[plane] * J.fg_ty[plane]) {
     local -= J.fg_tx[plane] * J.fg_ty[plane];
     plane++;
   }
-  return FgTile{&J, plane, local % J.fg_tx[plane], local / J.fg_tx[plane]};
+  return FgTile{plane, local % J.fg_tx[plane], local / J.fg_tx[plane]};
 }
 
 // A quad of a plane whose rows are not on word boundaries, or one that
@@ -666,8 +672,7 @@ __device__ __forceinline__ void fg_apply_plane(const FrameJob& J, const uint8_t*
 }
 
 template <typename T, int kRows>
-__device__ __forceinline__ void fg_tile(const FgTile& t, uint8_t* lut) {
-  const FrameJob& J = *t.J;
+__device__ __forceinline__ void fg_tile(const FrameJob& J, const FgTile& t, uint8_t* lut) {
   const int tid = threadIdx.x;
   if (sizeof(T) == 1) {
     lut[tid] = J.fg.lut[t.plane][tid];
@@ -704,21 +709,25 @@ __device__ __forceinline__ void fg_tile(const FgTile& t, uint8_t* lut) {
 template <bool kLoop, int kRows>
 __global__ void __launch_bounds__(256, 4) k_fg_apply_batch(BatchArgs b) {
   __shared__ __align__(16) uint8_t s_lut[kFgScaleLen];
+  stage_begin();
   const int* base = b.base + ST_FG_APPLY * (b.n + 1);
   for_each_item<kLoop>(
       b, ST_FG_APPLY,
       [&](int item) {
-        const FgTile t = fg_locate(b, base, item);
-        if (t.J->io.bd == 8)
-          fg_tile<uint8_t, kRows>(t, s_lut);
+        const int fi = find_frame(base, b.n, item);
+        const FrameJob& J = b.jobs[fi];
+        const FgTile t = fg_locate(J, item - base[fi]);
+        if (J.io.bd == 8)
+          fg_tile<uint8_t, kRows>(J, t, s_lut);
         else
-          fg_tile<uint16_t, kRows>(t, s_lut);
+          fg_tile<uint16_t, kRows>(J, t, s_lut);
         if (kLoop) __syncthreads();  // the table is rewritten by the next tile
       },
       [&](int item) {
         // The tile of the filtered frame (the grain's input).
-        const FgTile t = fg_locate(b, base, item);
-        const FrameJob& J = *t.J;
+        const int fi = find_frame(base, b.n, item);
+        const FrameJob& J = b.jobs[fi];
+        const FgTile t = fg_locate(J, item - base[fi]);
         const int x0 = t.tx * 64, y0 = t.ty * 64;
         if (J.io.bd == 8)
           prefetch_block<uint8_t>(J.io.pl[t.plane], x0, x0 + 64, y0, y0 + 64);
@@ -727,38 +736,56 @@ __global__ void __launch_bounds__(256, 4) k_fg_apply_batch(BatchArgs b) {
       });
 }
 
+__global__ void __launch_bounds__(256, 4) k_fg_apply_one(const __grid_constant__ FrameJob J) {
+  __shared__ __align__(16) uint8_t s_lut[kFgScaleLen];
+  stage_begin();
+  const FgTile t = fg_locate(J, blockIdx.x);
+  if (J.io.bd == 8)
+    fg_tile<uint8_t, 4>(J, t, s_lut);
+  else
+    fg_tile<uint16_t, 4>(J, t, s_lut);
+}
+
 // Border extension: 64x4-sample tiles of the right strip [w, aw) x [0, h)
 // then of the bottom strip [0, aw) x [h, ah), per plane.
+__device__ __forceinline__ void extend_item(const FrameJob& J, int local) {
+  for (int plane = 0; plane < 3; plane++) {
+    const int nr = J.ext_r[plane][0] * J.ext_r[plane][1], nb = J.ext_b[plane][0] * J.ext_b[plane][1];
+    if (local >= nr + nb) {
+      local -= nr + nb;
+      continue;
+    }
+    const DPlane& p = J.io.pl[plane];
+    int x, y;
+    if (local < nr) {
+      x = p.w + (local % J.ext_r[plane][0]) * 64 + (threadIdx.x & 63);
+      y = (local / J.ext_r[plane][0]) * 4 + (threadIdx.x >> 6);
+      if (y >= p.h) return;
+    } else {
+      local -= nr;
+      x = (local % J.ext_b[plane][0]) * 64 + (threadIdx.x & 63);
+      y = p.h + (local / J.ext_b[plane][0]) * 4 + (threadIdx.x >> 6);
+    }
+    if (J.io.bd == 8)
+      extend_px<uint8_t>(J.io, plane, x, y);
+    else
+      extend_px<uint16_t>(J.io, plane, x, y);
+    return;
+  }
+}
+
 __global__ void __launch_bounds__(256) k_extend_batch(BatchArgs b) {
+  stage_begin();
   const int* base = b.base + ST_EXTEND * (b.n + 1);
   for_each_item(b, ST_EXTEND, [&](int item) {
     const int fi = find_frame(base, b.n, item);
-    const FrameJob& J = b.jobs[fi];
-    int local = item - base[fi];
-    for (int plane = 0; plane < 3; plane++) {
-      const int nr = J.ext_r[plane][0] * J.ext_r[plane][1], nb = J.ext_b[plane][0] * J.ext_b[plane][1];
-      if (local >= nr + nb) {
-        local -= nr + nb;
-        continue;
-      }
-      const DPlane& p = J.io.pl[plane];
-      int x, y;
-      if (local < nr) {
-        x = p.w + (local % J.ext_r[plane][0]) * 64 + (threadIdx.x & 63);
-        y = (local / J.ext_r[plane][0]) * 4 + (threadIdx.x >> 6);
-        if (y >= p.h) return;
-      } else {
-        local -= nr;
-        x = (local % J.ext_b[plane][0]) * 64 + (threadIdx.x & 63);
-        y = p.h + (local / J.ext_b[plane][0]) * 4 + (threadIdx.x >> 6);
-      }
-      if (J.io.bd == 8)
-        extend_px<uint8_t>(J.io, plane, x, y);
-      else
-        extend_px<uint16_t>(J.io, plane, x, y);
-      return;
-    }
+    extend_item(b.jobs[fi], item - base[fi]);
   });
+}
+
+__global__ void __launch_bounds__(256) k_extend_one(const __grid_constant__ FrameJob J) {
+  stage_begin();
+  extend_item(J, blockIdx.x);
 }
 
 // LFSR step as a GF(2)^16 map, for the host-side jump tables.
@@ -766,6 +793,8 @@ static uint16_t lfsr_step_host(uint16_t reg) {
   const uint16_t bit = ((reg >> 0) ^ (reg >> 1) ^ (reg >> 3) ^ (reg >> 12)) & 1;
   return (uint16_t)((reg >> 1) | (bit << 15));
 }
+
+static cudaError_t fg_configure();
 
 cudaError_t fg_upload_tables() {
   static_assert(sizeof(pf_gaussian_sequence) == sizeof(g_gauss), "Gaussian sequence length");
@@ -787,56 +816,54 @@ cudaError_t fg_upload_tables() {
   }
   e = cudaMemcpyToSymbol(g_jump, jump, sizeof(jump));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_jump_len, lens, sizeof(lens));
+  if (e == cudaSuccess) e = fg_configure();
   return e;
 }
 
-cudaError_t launch_fg_templates_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
-  // The shared layout is above the default 48 KB: opt in once per device.
-  constexpr int kMaxDevices = 64;
-  static std::atomic<bool> configured[kMaxDevices];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-  if (!configured[dev].load(std::memory_order_acquire)) {
-    e = cudaFuncSetAttribute(k_fg_templates_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TplSmem));
-    if (e != cudaSuccess) return e;
-    configured[dev].store(true, std::memory_order_release);
-  }
-  k_fg_templates_batch<<<grid, kFgTemplateThreads, sizeof(TplSmem), st>>>(b);
-  return cudaGetLastError();
+static cudaError_t fg_configure() {
+  // The templates' shared layout is above the default 48 KB.
+  cudaError_t e = cudaFuncSetAttribute(k_fg_templates_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TplSmem));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_fg_templates_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TplSmem));
+  return e;
 }
 
-cudaError_t launch_fg_offsets_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
-  k_fg_offsets_batch<<<grid, 64, 0, st>>>(b);
-  return cudaGetLastError();
+cudaError_t launch_fg_templates(const StageLaunch& l) {
+  if (l.total <= 0) return cudaSuccess;
+  if (l.one)
+    return launch_stage(k_fg_templates_one, l.total, kFgTemplateThreads, sizeof(TplSmem), l.st, false, *l.one);
+  return launch_stage(k_fg_templates_batch, l.grid, kFgTemplateThreads, sizeof(TplSmem), l.st, false, l.args);
+}
+
+cudaError_t launch_fg_offsets(const StageLaunch& l) {
+  if (l.total <= 0) return cudaSuccess;
+  if (l.one) return launch_stage(k_fg_offsets_one, l.total, 64, 0, l.st, false, *l.one);
+  return launch_stage(k_fg_offsets_batch, l.grid, 64, 0, l.st, false, l.args);
 }
 
 template <int kRows>
-static void launch_fg_apply_rows(const BatchArgs& b, int grid, cudaStream_t st) {
+static cudaError_t launch_fg_apply_rows(const StageLaunch& l) {
   static int wave = 0;
-  if (batch_loops(b))
-    k_fg_apply_batch<true, kRows><<<grid, 256, 0, st>>>(b);
-  else
-    k_fg_apply_batch<false, kRows><<<grid, 256, 0, st>>>(with_wave(b, k_fg_apply_batch<false, kRows>, 256, 0, wave));
+  if (batch_loops(l.args))
+    return launch_stage(k_fg_apply_batch<true, kRows>, l.grid, 256, 0, l.st, l.dependent, l.args);
+  return launch_stage(k_fg_apply_batch<false, kRows>, l.grid, 256, 0, l.st, l.dependent,
+                      with_wave(l.args, k_fg_apply_batch<false, kRows>, 256, 0, wave));
 }
 
-cudaError_t launch_fg_apply_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
-  switch (b.tile) {
-    case 1: launch_fg_apply_rows<2>(b, grid, st); break;
-    case 2: launch_fg_apply_rows<1>(b, grid, st); break;
-    default: launch_fg_apply_rows<4>(b, grid, st);
+cudaError_t launch_fg_apply(const StageLaunch& l) {
+  if (l.total <= 0) return cudaSuccess;
+  if (l.one) return launch_stage(k_fg_apply_one, l.total, 256, 0, l.st, l.dependent, *l.one);
+  switch (l.args.tile) {
+    case 1: return launch_fg_apply_rows<2>(l);
+    case 2: return launch_fg_apply_rows<1>(l);
+    default: return launch_fg_apply_rows<4>(l);
   }
-  return cudaGetLastError();
 }
 
-cudaError_t launch_extend_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
-  k_extend_batch<<<grid, 256, 0, st>>>(b);
-  return cudaGetLastError();
+cudaError_t launch_extend(const StageLaunch& l) {
+  if (l.total <= 0) return cudaSuccess;
+  if (l.one) return launch_stage(k_extend_one, l.total, 256, 0, l.st, l.dependent, *l.one);
+  return launch_stage(k_extend_batch, l.grid, 256, 0, l.st, l.dependent, l.args);
 }
 
 }  // namespace pf

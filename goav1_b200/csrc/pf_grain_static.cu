@@ -13,11 +13,8 @@
 // holds until the process exits.
 //
 // The array is shared by every call on a device and keeps whatever the last
-// call left in it.  Nothing in it has to start at zero: each call rewrites the
-// job record, the stage table, all three templates and every offset it reads.
-// The job record and stage table reach the array through a one-CTA kernel
-// that takes them as its by-value argument, so no host buffer is read after
-// the call returns.  Calls whose work overlaps on the GPU (two streams, or two
+// call left in it.  Nothing in it has to start at zero: each call rewrites all
+// three templates, the scaling tables and every offset it reads.  Calls whose work overlaps on the GPU (two streams, or two
 // threads) race on the array; callers must order them, e.g. by issuing them
 // on one stream.
 #include <mutex>
@@ -29,24 +26,20 @@
 namespace pf {
 cudaError_t fg_upload_tables();
 void build_scaling_lut(uint8_t* dst, const uint8_t (*pts)[2], int n);
-cudaError_t launch_fg_templates_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
-cudaError_t launch_fg_offsets_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
-cudaError_t launch_fg_apply_batch(const BatchArgs& b, int total, int grid, cudaStream_t st);
+cudaError_t launch_fg_templates(const StageLaunch& l);
+cudaError_t launch_fg_offsets(const StageLaunch& l);
+cudaError_t launch_fg_apply(const StageLaunch& l);
 }  // namespace pf
 
 using namespace pf;
 
 namespace {
 
-// Scratch layout (bytes): [job record | stage table | 3 grain templates |
-// scaling tables | offsets].
-constexpr size_t kJobBytes = 8192;
-constexpr size_t kBaseOff = kJobBytes;
-constexpr size_t kGrainOff = kBaseOff + 256;
+// Scratch layout (bytes): [3 grain templates | scaling tables | offsets].
+constexpr size_t kGrainOff = 0;
 constexpr size_t kGrainBytes = (3 * kGrainLen * sizeof(int16_t) + 255) / 256 * 256;
 constexpr size_t kScaleOff = kGrainOff + kGrainBytes;
 constexpr size_t kOffsetsOff = kScaleOff + 3 * kFgScaleLen;
-static_assert(sizeof(FrameJob) <= kJobBytes, "job record does not fit its scratch slot");
 static_assert(kOffsetsOff + PF_GRAIN_STATIC_MAX_BLOCKS <= PF_GRAIN_STATIC_SCRATCH_BYTES, "scratch too small");
 
 }  // namespace
@@ -76,23 +69,6 @@ int setup_device(int dev, uint8_t** out) {
   }
   *out = (uint8_t*)p;
   return PF_OK;
-}
-
-// The job record and the stage prefix table, written into the scratch array
-// by one CTA from its kernel argument.
-struct StaticRecord {
-  FrameJob job;
-  int base[ST_COUNT * 2];
-};
-static_assert(sizeof(FrameJob) % 4 == 0, "record is copied as 32-bit words");
-static_assert(sizeof(StaticRecord) <= 4096, "record must fit the kernel parameter space");
-
-__global__ void k_grain_static_record(StaticRecord r, uint8_t* scratch) {
-  const uint32_t* job = (const uint32_t*)&r.job;
-  uint32_t* dj = (uint32_t*)scratch;
-  for (int i = threadIdx.x; i < (int)(sizeof(FrameJob) / 4); i += blockDim.x) dj[i] = job[i];
-  int* db = (int*)(scratch + kBaseOff);
-  for (int i = threadIdx.x; i < ST_COUNT * 2; i += blockDim.x) db[i] = r.base[i];
 }
 
 DFrame device_frame(const pf_frame* f) {
@@ -137,9 +113,8 @@ extern "C" int pf_film_grain_static(const pf_frame* ref, const pf_film_grain* fg
   if (st != PF_OK) return st;
 
   // The one-frame job: film grain only.
-  StaticRecord R;
-  memset(&R, 0, sizeof(R));
-  FrameJob& J = R.job;
+  FrameJob J;
+  memset(&J, 0, sizeof(J));
   J.io = device_frame(ref);
   J.disp = device_frame(display);
   FgArgs& a = J.fg;
@@ -201,27 +176,18 @@ extern "C" int pf_film_grain_static(const pf_frame* ref, const pf_film_grain* fg
     tiles += J.fg_tx[p] * J.fg_ty[p];
   }
   counts[ST_FG_APPLY] = tiles;
-  for (int k = 0; k < ST_COUNT; k++) {
-    R.base[2 * k] = 0;
-    R.base[2 * k + 1] = counts[k];
-  }
-  const cudaStream_t s = (cudaStream_t)stream;
-  k_grain_static_record<<<1, 128, 0, s>>>(R, scratch);
-  if (cudaGetLastError() != cudaSuccess) return PF_ERR_DEVICE;
-  BatchArgs b;
-  b.jobs = (const FrameJob*)scratch;
-  b.base = (const int*)(scratch + kBaseOff);
-  b.n = 1;
-  b.counters = nullptr;
-  b.chunk = 1;
-  b.ahead = 0;
-  b.tile = 0;
-  b.f0 = 0;
-  b.f1 = 1;
-  b.wave = 0;
-  if (launch_fg_templates_batch(b, counts[ST_FG_TEMPLATES], counts[ST_FG_TEMPLATES], s) != cudaSuccess ||
-      launch_fg_offsets_batch(b, counts[ST_FG_OFFSETS], counts[ST_FG_OFFSETS], s) != cudaSuccess ||
-      launch_fg_apply_batch(b, counts[ST_FG_APPLY], counts[ST_FG_APPLY], s) != cudaSuccess)
+  // The launches carry the job as their argument, so no host buffer is read
+  // after the call returns.
+  auto stage = [&](int k) {
+    StageLaunch l;
+    memset(&l, 0, sizeof(l));
+    l.one = &J;
+    l.total = l.grid = counts[k];
+    l.st = (cudaStream_t)stream;
+    return l;
+  };
+  if (launch_fg_templates(stage(ST_FG_TEMPLATES)) != cudaSuccess ||
+      launch_fg_offsets(stage(ST_FG_OFFSETS)) != cudaSuccess || launch_fg_apply(stage(ST_FG_APPLY)) != cudaSuccess)
     return PF_ERR_DEVICE;
   return PF_OK;
 }

@@ -529,53 +529,57 @@ __device__ __forceinline__ void lr_tile(const DFrame& src, const DFrame& dst, co
     lr_sgr_window<sizeof(T) == 1>(sm, w, h, bd, u->sgr_set, u->sgr_xqd[0], u->sgr_xqd[1], PW, store);
 }
 
+static cudaError_t lr_configure();
+
 cudaError_t lr_upload_tables() {
   uint8_t xbx[256];
   for (int z = 0; z < 256; z++) xbx[z] = (uint8_t)(pf_sgr_x_by_xplus1[z] - 1);
   cudaError_t e = cudaMemcpyToSymbol(c_sgr_params, pf_sgr_params, sizeof(pf_sgr_params));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_xbx, xbx, sizeof(xbx));
-  return e;
+  return e == cudaSuccess ? lr_configure() : e;
 }
 
 // Batched restoration: each work item is one (processing column, stripe)
 // tile of one plane of one frame.  Frames without restoration get the copy
 // of the CDEF output back into the frame.
 struct LrTile {
-  const FrameJob* J;
   int plane, j, s;
 };
 
-__device__ __forceinline__ LrTile lr_locate(const BatchArgs& b, const int* base, int item) {
-  const int fi = find_frame(base, b.n, item);
-  const FrameJob& J = b.jobs[fi];
-  int local = item - base[fi];
+__device__ __forceinline__ LrTile lr_locate(const FrameJob& J, int local) {
   int plane = 0;
   while (plane < 2 && local >= J.lr_cols[plane] * J.lr_rows[plane]) {
     local -= J.lr_cols[plane] * J.lr_rows[plane];
     plane++;
   }
-  return LrTile{&J, plane, local % J.lr_cols[plane], local / J.lr_cols[plane]};
+  return LrTile{plane, local % J.lr_cols[plane], local / J.lr_cols[plane]};
+}
+
+__device__ __forceinline__ void lr_item(const FrameJob& J, int local, LrSmem& sm) {
+  const LrTile t = lr_locate(J, local);
+  if (J.io.bd == 8)
+    lr_tile<uint8_t>(J.scr, J.io, J.lr, J.aw, J.ah, J.do_lr, t.plane, t.j, t.s, sm);
+  else
+    lr_tile<uint16_t>(J.scr, J.io, J.lr, J.aw, J.ah, J.do_lr, t.plane, t.j, t.s, sm);
 }
 
 template <bool kLoop>
 __global__ void __launch_bounds__(256, 4) k_lr_batch(BatchArgs b) {
   extern __shared__ __align__(16) uint8_t lr_smem_raw[];
   LrSmem& sm = *reinterpret_cast<LrSmem*>(lr_smem_raw);
+  stage_begin();
   const int* base = b.base + ST_LR * (b.n + 1);
   for_each_item<kLoop>(
       b, ST_LR,
       [&](int item) {
-        const LrTile t = lr_locate(b, base, item);
-        const FrameJob& J = *t.J;
-        if (J.io.bd == 8)
-          lr_tile<uint8_t>(J.scr, J.io, J.lr, J.aw, J.ah, J.do_lr, t.plane, t.j, t.s, sm);
-        else
-          lr_tile<uint16_t>(J.scr, J.io, J.lr, J.aw, J.ah, J.do_lr, t.plane, t.j, t.s, sm);
+        const int fi = find_frame(base, b.n, item);
+        lr_item(b.jobs[fi], item - base[fi], sm);
       },
       [&](int item) {
         // The tile's stripe of the CDEF output with its 3-sample halo.
-        const LrTile t = lr_locate(b, base, item);
-        const FrameJob& J = *t.J;
+        const int fi = find_frame(base, b.n, item);
+        const FrameJob& J = b.jobs[fi];
+        const LrTile t = lr_locate(J, item - base[fi]);
         const int ssy = t.plane ? J.io.ssy : 0;
         const int PW = J.lr.tile_w[t.plane], SH = 64 >> ssy, off = 8 >> ssy;
         const int x0 = t.j * PW, y0 = t.s * SH - off;
@@ -586,22 +590,32 @@ __global__ void __launch_bounds__(256, 4) k_lr_batch(BatchArgs b) {
       });
 }
 
-cudaError_t launch_lr_batch(const BatchArgs& b, int total, int grid, cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(k_lr_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LrSmem));
+__global__ void __launch_bounds__(256, 4) k_lr_one(const __grid_constant__ FrameJob J) {
+  extern __shared__ __align__(16) uint8_t lr_smem_raw[];
+  stage_begin();
+  lr_item(J, blockIdx.x, *reinterpret_cast<LrSmem*>(lr_smem_raw));
+}
+
+// The shared layout's size, on the current device.
+static cudaError_t lr_configure() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](auto* kernel) {
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_lr_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LrSmem));
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LrSmem));
+  };
+  set(k_lr_batch<true>);
+  set(k_lr_batch<false>);
+  set(k_lr_one);
+  return e;
+}
+
+cudaError_t launch_lr(const StageLaunch& l) {
+  if (l.total <= 0) return cudaSuccess;
+  if (l.one) return launch_stage(k_lr_one, l.total, 256, sizeof(LrSmem), l.st, l.dependent, *l.one);
   static int wave = 0;
-  if (batch_loops(b))
-    k_lr_batch<true><<<grid, 256, sizeof(LrSmem), st>>>(b);
-  else
-    k_lr_batch<false><<<grid, 256, sizeof(LrSmem), st>>>(with_wave(b, k_lr_batch<false>, 256, sizeof(LrSmem), wave));
-  return cudaGetLastError();
+  if (batch_loops(l.args)) return launch_stage(k_lr_batch<true>, l.grid, 256, sizeof(LrSmem), l.st, l.dependent, l.args);
+  return launch_stage(k_lr_batch<false>, l.grid, 256, sizeof(LrSmem), l.st, l.dependent,
+                      with_wave(l.args, k_lr_batch<false>, 256, sizeof(LrSmem), wave));
 }
 
 // ---- encoder loop-restoration unit search ----

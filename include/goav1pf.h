@@ -311,9 +311,10 @@ int pf_batch_apply(pf_ctx* ctx, const pf_batch_item* items, int32_t n, pf_stats*
  *     that signature replay it, with only their job tables refreshed.  Up to
  *     8 signatures are kept; a change of the context's scratch buffers
  *     recaptures.  Graphs are not used while the context times stages.
- *     The switch covers batches of device frames and single-frame calls
- *     (pf_frame_apply, a batch of one); host-frame batches pipeline their
- *     chunks without graphs.
+ *     The switch covers batches of device frames.  A single frame under the
+ *     default schedules needs no graph: its launches carry its job as their
+ *     argument and go out directly.  Host-frame batches pipeline their chunks
+ *     without graphs.
  *   - The schedule of each stage group (pf_schedule, pf_set_schedule):
  *       ctas           persistent CTAs draining the stage's items through an
  *                      atomic counter (0 = one CTA per chunk);
@@ -622,7 +623,7 @@ int pf_lf_build(pf_ctx* ctx, const pf_lf_record* records, int32_t mi_cols, int32
  * device, or an application whose device memory is already owned by another
  * allocator.  It writes display = ref with film grain applied, exactly as
  * pf_frame_apply with only PF_STAGE_FILM_GRAIN does, but allocates nothing:
- * its scratch (grain templates, block offsets, the job record) is one
+ * its scratch (grain templates, scaling tables, block offsets) is one
  * file-scope device array of PF_GRAIN_STATIC_SCRATCH_BYTES that every GPU
  * loading the library holds until the process exits.
  *   - ref and display are device frames (PF_MEM_DEVICE) of equal geometry on
@@ -637,8 +638,8 @@ int pf_lf_build(pf_ctx* ctx, const pf_lf_record* records, int32_t mi_cols, int32
  *     cannot use the symbol as an address).  The tables live in the library's
  *     module, so after cudaDeviceReset this entry point must not be called
  *     again on that device.
- *   - The job record reaches the array as a kernel argument: nothing the
- *     call reads from host memory is needed after it returns.
+ *   - The job record is the kernels' argument: nothing the call reads from
+ *     host memory is needed after it returns.
  *   - Work is queued on `stream` (a cudaStream_t, or NULL for the legacy
  *     default stream); the call returns without waiting for it.
  *   - Every call shares the one array and it keeps the last call's contents;
