@@ -1414,11 +1414,13 @@ static int run_host_pipeline(pf_ctx* c, const pf_batch_item* items, int n, pf_st
   if (!c->h2d) {
     CK(cudaStreamCreateWithFlags(&c->h2d, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&c->d2h, cudaStreamNonBlocking));
-    for (pf_ctx::HostSlot& h : c->hslot) {
-      CK(cudaEventCreateWithFlags(&h.up, cudaEventDisableTiming));
-      CK(cudaEventCreateWithFlags(&h.comp, cudaEventDisableTiming));
-      CK(cudaEventCreateWithFlags(&h.down, cudaEventDisableTiming));
-    }
+  }
+  // The copy streams may be an earlier single-frame call's; the slots' events
+  // are made here only.
+  for (pf_ctx::HostSlot& h : c->hslot) {
+    if (!h.up) CK(cudaEventCreateWithFlags(&h.up, cudaEventDisableTiming));
+    if (!h.comp) CK(cudaEventCreateWithFlags(&h.comp, cudaEventDisableTiming));
+    if (!h.down) CK(cudaEventCreateWithFlags(&h.down, cudaEventDisableTiming));
   }
   const int chunk = std::max(1, c->host_chunk);
   const int nchunks = (n + chunk - 1) / chunk;

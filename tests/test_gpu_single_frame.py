@@ -44,3 +44,25 @@ def test_single_frames(graphs, schedule):
                         assert np.array_equal(a, b), "call %d frame %d %s plane %d" % (call, i, name, p)
     finally:
         r.close()
+
+
+def test_host_batch_after_a_single_host_frame():
+    """A batch of host frames on a context whose copy streams an earlier
+    single-frame call made."""
+    import oracle_ctypes
+    from goav1_b200.postfilter import PostFilterRunner
+
+    r = PostFilterRunner()
+    try:
+        frames = [synth.make_frame(1, 80 + i, width=200, height=136) for i in range(6)]
+        fr, si = frames[0]
+        r.apply(fr.copy().pf(), si.side, fr.like().pf())
+        out = [(fr.copy(), fr.like()) for fr, _ in frames]
+        r.apply_batch([(o.pf(), si.side, d.pf()) for (o, d), (_, si) in zip(out, frames)])
+        for (fr, si), got in zip(frames, out):
+            ref, rdisp = fr.copy(), fr.like()
+            assert oracle_ctypes.frame_apply(ref.pf(), si.side, rdisp.pf()) == 0
+            for want, g in zip((ref, rdisp), got):
+                assert all(np.array_equal(a, b) for a, b in zip(want.planes, g.planes))
+    finally:
+        r.close()
