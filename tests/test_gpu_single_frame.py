@@ -56,7 +56,8 @@ def test_host_batch_after_a_single_host_frame():
     try:
         frames = [synth.make_frame(1, 80 + i, width=200, height=136) for i in range(6)]
         fr, si = frames[0]
-        r.apply(fr.copy().pf(), si.side, fr.like().pf())
+        one, one_disp = fr.copy(), fr.like()  # pf() does not own the planes
+        r.apply(one.pf(), si.side, one_disp.pf())
         out = [(fr.copy(), fr.like()) for fr, _ in frames]
         r.apply_batch([(o.pf(), si.side, d.pf()) for (o, d), (_, si) in zip(out, frames)])
         for (fr, si), got in zip(frames, out):
