@@ -122,12 +122,12 @@ struct pf_ctx {
   bool side_pending = false;
   // The schedule of each stage's launch (pf_schedule): persistent-CTA count
   // (0 = one CTA per chunk), work items per chunk, items prefetched ahead,
-  // and the deblocking tile shape.
+  // and the deblocking tile setting.
   int persistent[ST_COUNT] = {};
   int chunk[ST_COUNT] = {1, 1, 1, 1, 1, 1, 1, 1};
   int ahead[ST_COUNT] = {};
   int tile[ST_COUNT] = {};  // launch-level tile setting (grain apply: rows loaded together)
-  int db_tile = 0;          // deblocking tile shape (per job: it sets the tile counts)
+  int db_tile = 0;          // deblocking tile setting (db_units_log2)
   // Frame groups (pf_set_frame_groups): 2 runs the batch's two halves on the
   // main stream and stream2.
   int frame_groups = 1;
@@ -745,8 +745,8 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
       if (a.gate_chroma[p]) continue;
       const int sx = p ? f->ss_x : 0, sy = p ? f->ss_y : 0;
       const int w4 = (((f->width + sx) >> sx) + 3) >> 2, h4 = (((f->height + sy) >> sy) + 3) >> 2;
-      J.db_tx[p] = (w4 + db_tile_w(dbTile) - 1) / db_tile_w(dbTile);
-      J.db_ty[p] = (h4 + db_tile_h(dbTile) - 1) / db_tile_h(dbTile);
+      J.db_tx[p] = (w4 + 31) >> 5;
+      J.db_ty[p] = (h4 + (8 << dbTile) - 1) >> (3 + dbTile);
       tiles += J.db_tx[p] * J.db_ty[p];
     }
     counts[ST_DEBLOCK_V] = counts[ST_DEBLOCK_H] = tiles;
@@ -1157,9 +1157,17 @@ static int prepare_batch(pf_ctx* c, const FrameRef* refs, int n, Bytes& hs, DevB
   c->hbase.assign((size_t)ST_COUNT * (n + 1), 0);
   hs.clear();
   uint32_t done = 0;
+  int64_t units = 0;  // 4x4 units of the call's planes that are deblocked
+  for (int i = 0; i < n; i++) {
+    const pf_frame* f = refs[i].f;
+    if (!(refs[i].s->stages & PF_STAGE_LOOP_FILTER)) continue;
+    const int64_t px = (int64_t)f->width * f->height;
+    units += (px + (f->mono ? 0 : 2 * (px >> (f->ss_x + f->ss_y)))) >> 4;
+  }
+  const int dbTile = db_units_log2(c->db_tile, units);
   for (int i = 0; i < n; i++) {
     int counts[ST_COUNT];
-    fill_job(refs[i], arena, side, hs, c->hjobs[i], counts, c->db_tile);
+    fill_job(refs[i], arena, side, hs, c->hjobs[i], counts, dbTile);
     for (int k = 0; k < ST_COUNT; k++) c->hbase[(size_t)k * (n + 1) + i + 1] = c->hbase[(size_t)k * (n + 1) + i] + counts[k];
     const pf_frame_side* s = refs[i].s;
     if (counts[ST_DEBLOCK_V]) done |= PF_STAGE_LOOP_FILTER;

@@ -187,7 +187,7 @@ struct FrameJob {
   FgArgs fg;
   FgTemplateArgs fgt;
   int aw[3], ah[3];          // MI-aligned plane extents
-  int db_tile;               // deblocking tile shape (db_tile_w / db_tile_h)
+  int db_tile;               // deblocking tile height: 8 << db_tile units (db_units_log2)
   int db_tx[3], db_ty[3];    // deblock tiles per plane (0 = gated)
   int lr_cols[3], lr_rows[3];  // restoration tiles (processing column x stripe)
   int fg_tx[3], fg_ty[3];    // 64x64-sample tiles of the display planes
@@ -214,10 +214,19 @@ struct BatchArgs {
   int wave;
 };
 
-// Deblocking tile shapes (pf_schedule.tile): width x height in 4x4 edge
-// units, 256 units (one per thread) a tile.
-__host__ __device__ __forceinline__ int db_tile_w(int tile) { return tile == 1 ? 64 : tile == 2 ? 16 : tile == 3 ? 8 : 32; }
-__host__ __device__ __forceinline__ int db_tile_h(int tile) { return 256 / db_tile_w(tile); }
+// log2 of the 4x4 edge units a thread lists in a deblocking tile (32 units
+// wide, 256 threads): the tile setting (pf_schedule.tile) 1..3 gives it; 0
+// takes it from the units of the call's frames.  The device holds 592 CTAs
+// (four on each of 148 SMs).  One unit a thread while such tiles fit in one
+// wave (a 352x288 frame: 16.9 us for both directions against 17.9 with two);
+// four once tiles of that size make two waves or more (six 1920x1080 frames:
+// 9.3 us a frame against 9.9 with two and 12.9 with one; 60: 6.7, 8.1, 11.5);
+// two between (one frame: 20.6 against 23.5 with four and 25.8 with one; one
+// 3840x2160 10-bit frame: 40.8, 41.3, 52.5).
+inline int db_units_log2(int tile, int64_t units) {
+  if (tile > 0) return tile - 1;
+  return units >= (int64_t)2 * 592 * 1024 ? 2 : units > (int64_t)592 * 256 ? 1 : 0;
+}
 
 // Prefetches the samples [x0, x1) x [y0, y1) of a plane (clamped to its
 // allocation) into L2, one 128-byte line per thread at a time.  A hint only:

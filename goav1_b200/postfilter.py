@@ -142,7 +142,7 @@ class PostFilterRunner:
 
     def set_schedule(self, group, ctas=0, units_per_cta=1, staging=0, tile=0):
         """Schedule of a stage group (abi.PF_TUNE_*): persistent CTAs, work
-        items per CTA, items prefetched ahead, deblocking tile shape."""
+        items per CTA, items prefetched ahead, deblocking tile size."""
         s = abi.pf_schedule(ctas, units_per_cta, staging, tile)
         check(lib().pf_set_schedule(self._h, group, C.byref(s)))
 

@@ -327,9 +327,8 @@ int pf_batch_apply(pf_ctx* ctx, const pf_batch_item* items, int32_t n, pf_stats*
  *                      a CTA starting about when this one ends will take;
  *                      with larger chunks, the item that many places on
  *                      inside the chunk (then below units_per_cta);
- *       tile           deblocking: the tile shape, 0 = 32x8, 1 = 64x4,
- *                      2 = 16x16, 3 = 8x32 edge units a tile (one thread
- *                      each); grain apply: how many of a thread's four rows
+ *       tile           deblocking: the tile, 1 = 32x8, 2 = 32x16, 3 = 32x32
+ *                      edge units, 0 = by the call's size; grain apply: how many of a thread's four rows
  *                      have their loads issued together, 0 and 3 = four,
  *                      1 = two, 2 = one; 0 for the other groups.
  *     Work items are independent, so every schedule gives the same samples.

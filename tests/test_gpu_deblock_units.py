@@ -1,0 +1,97 @@
+"""Deblocking alone against the oracle at the edges of its forms: frames
+smaller than a tile and one unit past it, every chroma layout, smooth planes
+(the wide filters' flat tests pass) and noisy ones (the narrow filter and its
+clamps at both ends of the range), 8 and 10 bits (packed pairs of lines), 12
+bits, 10-bit frames holding longer samples and levels above 63 (line by line),
+and planes whose rows start on no 4-sample boundary.  Integer arithmetic:
+tolerance zero."""
+
+import numpy as np
+import pytest
+
+from goav1_b200 import abi, synth
+
+pytestmark = pytest.mark.gpu
+
+STAGES = abi.PF_STAGE_LOOP_FILTER
+
+
+@pytest.fixture(scope="module")
+def runner():
+    from goav1_b200.postfilter import PostFilterRunner
+
+    r = PostFilterRunner()
+    yield r
+    r.close()
+
+
+def frame(seed, w, h, bd, ss, content):
+    """A deblocking-only frame of one of three kinds of samples."""
+    fr, si = synth.make_frame(1, seed, width=w, height=h, bit_depth=bd, ss=ss, stages=STAGES)
+    rng = np.random.default_rng([seed, 5])
+    top = (1 << bd) - 1
+    for p in fr.planes:
+        if content == "smooth":  # flat blocks, small steps, noise within the flat bound
+            y, x = np.indices(p.shape)
+            step = rng.integers(0, 4 << (bd - 8), size=((p.shape[0] + 7) // 8, (p.shape[1] + 7) // 8))
+            v = (top >> 1) + step[y // 8, x // 8] + rng.integers(0, 2, p.shape)
+            p[:] = np.where(rng.random(p.shape) < 0.01, rng.integers(0, top + 1, p.shape), v)
+        elif content == "ends":  # both ends of the range, close together
+            y, x = np.indices(p.shape)
+            side = rng.integers(0, 2, size=((p.shape[0] + 15) // 16, (p.shape[1] + 15) // 16))
+            d = rng.integers(0, 6 << (bd - 8), p.shape)
+            p[:] = np.where(side[y // 16, x // 16] == 1, top - d, d)
+    return fr, si
+
+
+def check(runner, fr, si):
+    import oracle_ctypes
+
+    ref, out = fr.copy(), fr.copy()
+    assert oracle_ctypes.frame_apply(ref.pf(), si.side, None) == 0
+    runner.apply(out.pf(), si.side)
+    for p, (a, b) in enumerate(zip(ref.planes, out.planes)):
+        assert np.array_equal(a, b), "plane %d differs in %d samples" % (p, int((a != b).sum()))
+    return ref
+
+
+@pytest.mark.parametrize("w,h", [(8, 8), (64, 64), (132, 36), (200, 136)])
+@pytest.mark.parametrize("ss", [(1, 1), (1, 0), (0, 0), (0, 1)], ids=["420", "422", "444", "440"])
+@pytest.mark.parametrize("bd", [8, 10, 12])
+@pytest.mark.parametrize("content", ["texture", "smooth", "ends"])
+def test_units(runner, w, h, ss, bd, content):
+    for seed in range(4):
+        check(runner, *frame(w + 3 * h + bd + 1000 * seed, w, h, bd, ss, content))
+
+
+@pytest.mark.parametrize("plane", [0, 1, 2])
+def test_samples_longer_than_ten_bits(runner, plane):
+    for seed in range(4):
+        fr, si = frame(77 + plane + 10 * seed, 200, 136, 10, (1, 1), "smooth")
+        rng = np.random.default_rng(plane)
+        at = rng.random(fr.planes[plane].shape) < 0.02
+        fr.planes[plane][at] = rng.integers(1024, 1100, size=int(at.sum()))
+        check(runner, fr, si)
+
+
+@pytest.mark.parametrize("bd", [8, 10])
+def test_rows_off_word_boundaries(runner, bd):
+    import oracle_ctypes
+    import torch
+
+    fr, si = frame(91 + bd, 200, 136, bd, (1, 1), "smooth")
+    ref = fr.copy()
+    assert oracle_ctypes.frame_apply(ref.pf(), si.side, None) == 0
+    f, keep = fr.pf(memory=abi.PF_MEM_DEVICE, ptrs=[0, 0, 0]), []
+    for p, a in enumerate(fr.planes):
+        t = torch.zeros((a.shape[0], a.shape[1] + 3), dtype=torch.uint8 if bd == 8 else torch.int16, device="cuda")
+        t[:, 1:1 + a.shape[1]] = torch.from_numpy(a if bd == 8 else a.view(np.int16)).cuda()
+        keep.append(t)
+        f.plane[p].data = t.data_ptr() + t.element_size()
+        f.plane[p].stride = t.stride(0) * t.element_size()
+    torch.cuda.synchronize()
+    runner.apply(f, si.side)
+    runner.sync()
+    for p, a in enumerate(ref.planes):
+        got = keep[p][:, 1:1 + a.shape[1]].cpu().numpy()
+        assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
