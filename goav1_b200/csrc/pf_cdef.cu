@@ -31,8 +31,7 @@
 namespace pf {
 
 // What a luma block's filter needs, made once per block: the primary tap's
-// constants (PairTap; plain strength and shift for samples staged as
-// integers) and flags: bit 31 filtered, bit 4 odd strength (weights 3, 3
+// constants (PairTap) and flags: bit 31 filtered, bit 4 odd strength (weights 3, 3
 // instead of 4, 2), low bits the direction.
 struct CdefBlk {
   PairTap pri;
@@ -186,7 +185,7 @@ __device__ __forceinline__ uint32_t stage_any(const CdefPlane& p, const uint8_t*
 // the CTA and warps 0-3 of the third; 2 x (10 x 18) chroma tasks follow on
 // warps 4-7 and in a fourth.  All of a thread's loads are in flight together.
 // kIn: a whole 64x64 unit with its halo inside the frame.
-template <typename T, bool kIn>
+template <typename T, bool kIn, bool kRaw>
 __device__ __forceinline__ uint32_t stage_420(const CdefPlane& P, const CdefPlane& Q, const uint8_t* vsrc, bool y,
                                               bool c, CdefSmem& sm) {
   const int tid = threadIdx.x;
@@ -218,11 +217,11 @@ __device__ __forceinline__ uint32_t stage_420(const CdefPlane& P, const CdefPlan
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     if (!on[k]) continue;
-    over |= stage_over<T>(t[k]);
+    if (!kRaw) over |= stage_over<T>(t[k]);
     if (k == 3 || (k == 2 && c2))
-      stage_store<T, kIn, false, kPC>(Q, d[k], cg[k], t[k], sm.c[i[k] >= 180]);
+      stage_store<T, kIn, kRaw, kPC>(Q, d[k], cg[k], t[k], sm.c[i[k] >= 180]);
     else
-      stage_store<T, kIn, false, kPW>(P, d[k], cg[k], t[k], sm.y);
+      stage_store<T, kIn, kRaw, kPW>(P, d[k], cg[k], t[k], sm.y);
   }
   return over;
 }
@@ -233,7 +232,7 @@ __device__ __forceinline__ uint32_t stage_420(const CdefPlane& P, const CdefPlan
 // block's parameters.
 template <typename T, bool kRaw, bool kPri, bool kSec, int kBh, class B>
 __device__ __forceinline__ void filter_run(const uint32_t* c, int pitch, const int2* ofs, uint8_t* o, int64_t os,
-                                           int rows, const PairTap& st, int sec, int secShift, int coeffShift, B blk) {
+                                           int rows, const PairTap& st, B blk) {
 #pragma unroll 1
   for (int k = 0; k * kBh < rows; k++) {
     const CdefBlk b = blk(k);
@@ -248,14 +247,7 @@ __device__ __forceinline__ void filter_run(const uint32_t* c, int pitch, const i
         if (!kRaw) {
           v = pair_filter<kPri, kSec>(c, b.pri, w0, w1, st, po, s0, s1);
         } else {
-          const uint16_t* e = reinterpret_cast<const uint16_t*>(c);
-          const int2 p2 = make_int2(2 * po.x, 2 * po.y), q0 = make_int2(2 * s0.x, 2 * s0.y),
-                     q1 = make_int2(2 * s1.x, 2 * s1.y);
-          v = 0;
-#pragma unroll 1
-          for (int h = 1; h >= 0; h--)
-            v = v << 16 |
-                (cdef_filter_px(e + h, (int)b.pri.k, (int)b.pri.m, sec, secShift, p2, q0, q1, coeffShift) & 0xffff);
+          v = pair_filter_ints<kPri, kSec>(c, b.pri, odd ? 3 : 4, odd ? 3 : 2, st, po, s0, s1);
         }
       }
       if (sizeof(T) == 2 && !kRaw) v &= 0x03ff03ffu;
@@ -267,15 +259,15 @@ __device__ __forceinline__ void filter_run(const uint32_t* c, int pitch, const i
 
 template <typename T, bool kRaw, int kBh, class B>
 __device__ __forceinline__ void filter_plane(const uint32_t* c, int pitch, const int2* ofs, uint8_t* o, int64_t os,
-                                             int rows, int pri, int sec, int damping, int coeffShift, B blk) {
+                                             int rows, int pri, int sec, int damping, B blk) {
   const int secShift = constrain_shift(sec, damping);
-  const PairTap st = pair_tap(sec, secShift);
-  if (kRaw || (pri && sec))
-    filter_run<T, kRaw, true, true, kBh>(c, pitch, ofs, o, os, rows, st, sec, secShift, coeffShift, blk);
+  const PairTap st = kRaw ? pair_tap_ints(sec, secShift) : pair_tap(sec, secShift);
+  if (pri && sec)
+    filter_run<T, kRaw, true, true, kBh>(c, pitch, ofs, o, os, rows, st, blk);
   else if (pri)
-    filter_run<T, kRaw, true, false, kBh>(c, pitch, ofs, o, os, rows, st, sec, secShift, coeffShift, blk);
+    filter_run<T, kRaw, true, false, kBh>(c, pitch, ofs, o, os, rows, st, blk);
   else
-    filter_run<T, kRaw, false, true, kBh>(c, pitch, ofs, o, os, rows, st, sec, secShift, coeffShift, blk);
+    filter_run<T, kRaw, false, true, kBh>(c, pitch, ofs, o, os, rows, st, blk);
 }
 
 // The four rows b-2 .. b+1 around the restoration stripe boundary
@@ -368,9 +360,9 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
       Q.words &= ((reinterpret_cast<uintptr_t>(vsrc) | (uintptr_t)J.io.pl[2].stride) & (4 * sizeof(T) - 1)) == 0;
       Q.words &= J.io.pl[2].stride == Q.stride;
       if (P.inside && P.words && Q.inside && Q.words && P.w == 64 && P.h == 64 && actY && actC) {
-        over = stage_420<T, true>(P, Q, vsrc, true, true, sm);
+        over = stage_420<T, true, kRaw>(P, Q, vsrc, true, true, sm);
       } else if (J.io.pl[2].stride == Q.stride) {
-        over = stage_420<T, false>(P, Q, vsrc, actY, actC, sm);
+        over = stage_420<T, false, kRaw>(P, Q, vsrc, actY, actC, sm);
       } else {
         if (actY) over |= stage_any<T, kRaw, kPW>(P, P.src, sm.y);
         if (actC) {
@@ -426,7 +418,7 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
       const int strength = ypri ? adjust_strength(ypri, var) : 0;
       const int shift = constrain_shift(strength, ydamp);
       CdefBlk blk;
-      blk.pri = kRaw ? PairTap{(uint32_t)strength, (uint32_t)shift, 0} : pair_tap(strength, shift);
+      blk.pri = kRaw ? pair_tap_ints(strength, shift) : pair_tap(strength, shift);
       blk.flags = (strength | ysec ? 1u << 31 : 0u) | (((strength >> coeffShift) & 1) << 4) | (ypri ? best : 0);
       sm.blk[tid] = blk;
     } else if (!k420 && plane == 1 && actC && cpri && ssx != ssy && tid < 64 && ((listed >> tid) & 1)) {
@@ -447,7 +439,7 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
         if (tx < P.w && rows > 0)
           filter_plane<T, kRaw, 8>(&sm.y[(2 + ya) * kPW + kPX + tx], kPW, sm.ofs[0],
                                    ob + (int64_t)(P.y + ya) * os + (int64_t)(P.x + tx) * (int)sizeof(T), os, rows, ypri,
-                                   ysec, ydamp, coeffShift, [&](int k) {
+                                   ysec, ydamp, [&](int k) {
                                      const int b = ((ya >> 3) + k) * 8 + (tx >> 3);
                                      CdefBlk r = sm.blk[b];
                                      if (!((listed >> b) & 1)) r.flags = 0;
@@ -460,7 +452,7 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
     if (k420 ? nplanes > 1 : plane > 0) {
       const int cshift = constrain_shift(cpri, cdamp);
       CdefBlk cb;
-      cb.pri = kRaw ? PairTap{(uint32_t)cpri, (uint32_t)cshift, 0} : pair_tap(cpri, cshift);
+      cb.pri = kRaw ? pair_tap_ints(cpri, cshift) : pair_tap(cpri, cshift);
       cb.flags = 1u << 31 | (((cpri >> coeffShift) & 1) << 4);
       auto chroma_blk = [&](int b) {
         CdefBlk r = cb;
@@ -479,7 +471,7 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
         } else if (lane < Q.w && rows > 0) {
           filter_plane<T, kRaw, 4>(&sm.c[pl - 1][(2 + ya) * kPC + kPX + lane], kPC, sm.ofs[1],
                                    ob + (int64_t)(Q.y + ya) * os + (int64_t)(Q.x + lane) * (int)sizeof(T), os, rows,
-                                   cpri, csec, cdamp, coeffShift,
+                                   cpri, csec, cdamp,
                                    [&](int k) { return chroma_blk(((ya >> 2) + k) * 8 + (lane >> 2)); });
         }
       } else if (!actC) {
@@ -494,9 +486,9 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
         if (tx < P.w && rows > 0) {
           auto at = [&](int k) { return chroma_blk(((ya >> (3 - ssy)) + k) * 8 + (tx >> (3 - ssx))); };
           if (ssy)
-            filter_plane<T, kRaw, 4>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, coeffShift, at);
+            filter_plane<T, kRaw, 4>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, at);
           else
-            filter_plane<T, kRaw, 8>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, coeffShift, at);
+            filter_plane<T, kRaw, 8>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, at);
         }
       }
     }
@@ -521,7 +513,10 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
 // The unit from plane `plane` on, with samples staged as integers: 12-bit
 // frames, and 10-bit ones that hold longer samples.
 __device__ __noinline__ void cdef_unit_raw(const FrameJob* J, int uc, int ur, int plane, CdefSmem* sm) {
-  cdef_unit<uint16_t, true, false>(*J, uc, ur, plane, *sm);
+  if (J->io.ssx && J->io.ssy)
+    cdef_unit<uint16_t, true, true>(*J, uc, ur, plane, *sm);
+  else
+    cdef_unit<uint16_t, true, false>(*J, uc, ur, plane, *sm);
 }
 
 // 4:2:2, 4:4:4 and 4:4:0.
