@@ -335,10 +335,11 @@ __device__ __forceinline__ void fg_offsets_row(uint16_t seed, int r, int cols, u
 //
 // Bound by integer issue (57 % of the slots) and the wait for the grain
 // behind the block offset.  us per frame: 60 x 1080p 8-bit 12.6 before (one
-// column by 16 rows a thread, every sample by itself), 7.1 now, at 2.2 warp
-// instructions per luma sample instead of 5.0; 8 x 4K 10-bit 62.9 and 30.2;
-// one 1080p frame 25.6 and 17.  Two rows' or one row's loads at a time
-// measured 7.3 and 7.8; 5 or 6 CTAs per SM (48, 40 registers) 7.6 and 7.5.
+// column by 16 rows a thread, every sample by itself), 6.9 now, at 2.2 warp
+// instructions per luma sample instead of 5.0; 8 x 4K 10-bit 62.9 and 29.3;
+// one 1080p frame 25.6 and 17.  (With the neighbours' offsets and grains read
+// row by row, after the stores: 7.1 and 30.1.)  Two rows' or one row's loads
+// at a time measured 7.3 and 7.8; 3 or 5 CTAs per SM 8.1 and 7.2.
 
 template <typename T>
 struct FgQuad;
@@ -408,10 +409,10 @@ template <bool kSx>
 __device__ __forceinline__ uint2 grain4(const int16_t* row, int c) {
   if (!kSx) {
     const uint32_t* w = reinterpret_cast<const uint32_t*>(row + c);
-    return make_uint2(w[0], w[1]);
+    return make_uint2(__ldg(w), __ldg(w + 1));
   }
   const uint32_t* w = reinterpret_cast<const uint32_t*>(row + (c & ~1));
-  const uint32_t a = w[0], b = w[1], d = w[2];
+  const uint32_t a = __ldg(w), b = __ldg(w + 1), d = __ldg(w + 2);
   const int sh = (c & 1) * 16;
   return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, d, sh));
 }
@@ -463,7 +464,9 @@ __device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& d
   // Template column / row origins of the current, left, top and top-left blocks.
   auto gcol = [&](int offset, int bc) { return 3 + (ovl >> sx) * (3 + (offset >> 4)) + xi + bw * bc; };
   auto grow = [&](int offset, int br) { return 3 + (ovl >> sy) * (3 + (offset & 15)) + yi0 + bh * br; };
-  const int o00 = offs[0];
+  // The offsets at once: after a store they would be read again.
+  const int o00 = __ldg(offs), o10 = xStart ? __ldg(offs - 1) : 0, o01 = yStart ? __ldg(offs - a.off_cols) : 0;
+  const int o11 = xStart && yStart ? __ldg(offs - a.off_cols - 1) : 0;
   const int c00 = gcol(o00, 0);
   const int16_t* g00 = gr + grow(o00, 0) * kGW;
   const int shift = a.scaling_shift, rnd = 1 << (shift - 1);
@@ -515,24 +518,22 @@ __device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& d
             for (int j = 0; j < ovl; j++)
               if (j < xStart) {
                 const int hpw = sx ? 23 : (j == 1 ? 17 : 27), hcw = sx ? 22 : (j == 1 ? 27 : 17);
-                gv[j] = blend_w(gr[r10 * kGW + c10 + j], gv[j], hpw, hcw, bd);
+                gv[j] = blend_w(__ldg(&gr[r10 * kGW + c10 + j]), gv[j], hpw, hcw, bd);
               }
           }
-          if (k < yStart) {
+          if (k < ovl && k < yStart) {
             const int vpw = sy ? 23 : (k == 1 ? 17 : 27), vcw = sy ? 22 : (k == 1 ? 27 : 17);
-            const int o01 = offs[-a.off_cols];
             const uint2 t = grain4<kSx>(gr + (grow(o01, 1) + k) * kGW, gcol(o01, 0));
             int tv[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) tv[j] = grain_of(t, j);
             if (xStart) {
-              const int o11 = offs[-a.off_cols - 1];
               const int c11 = gcol(o11, 1), r11 = grow(o11, 1) + k;
 #pragma unroll
               for (int j = 0; j < ovl; j++)
                 if (j < xStart) {
                   const int hpw = sx ? 23 : (j == 1 ? 17 : 27), hcw = sx ? 22 : (j == 1 ? 27 : 17);
-                  tv[j] = blend_w(gr[r11 * kGW + c11 + j], tv[j], hpw, hcw, bd);
+                  tv[j] = blend_w(__ldg(&gr[r11 * kGW + c11 + j]), tv[j], hpw, hcw, bd);
                 }
             }
 #pragma unroll
