@@ -11,8 +11,8 @@
 // minimum of the two transforms either side (lfmask/mask.go:110-400).  That
 // rule depends only on the cells either side of an edge, so here each 4x4
 // cell decides its own edges: one CTA per 128x128 region and a thread per
-// cell.  A warp is one column of cells for the vertical edges and, after a
-// transpose through shared memory, one row for the horizontal edges; each
+// cell.  A warp is one row of cells for the horizontal edges and, after a
+// transpose through shared memory, one column for the vertical edges; each
 // strength lane of the mask is then one warp ballot, so every mask word is
 // written once, without atomics.
 //
@@ -24,9 +24,19 @@
 //
 // The errors the reference returns come from its level-cache walk, which
 // visits cells in a chain per MI row (an invalid cell steps one cell, a
-// valid one jumps to its MIColEnd).  k_lf_build's row CTAs find that chain
-// for each row by pointer doubling in shared memory and keep its first
-// error; the host takes the first row's.
+// valid one jumps to its MIColEnd).  A map without a cell that the walk would
+// refuse has none; k_lf_build, which reads every cell, reports whether there
+// is one.  Only then does k_lf_walk find each row's chain by pointer doubling
+// in shared memory and keep its first error; the host takes the first row's.
+//
+// Bound by latency: a 1920x1080 map is one CTA per SM, so the kernel takes
+// what its dependent loads and about 600 instructions a thread do; hence two
+// rounds of loads in all, rows of cells along the lanes (a record is 32
+// bytes: columns took four times the lines) and the record-indexed tables in
+// shared memory.  A 480 x 270 map: 19.3 us with columns along the lanes and
+// the chroma cell's loads after the luma ones, 10.7 now (its launch alone, by
+// the profiler); the whole call 38.2 us with a walk of every row in the same
+// launch and its result copied back, 29.2 now.
 #include <limits.h>
 #include <string.h>
 
@@ -37,7 +47,11 @@ namespace pf {
 
 constexpr int kLfBatch = 1, kLfFilter = 2;  // error kinds: INVALID_BATCH, INVALID_FILTER
 
+// What is indexed by a cell's own record: read from shared memory, where a
+// warp's different entries do not wait for one another.
 struct MapTables {
+  int16_t segDelta[8][4];
+  int8_t refDelta[8], modeDelta[2];
   uint8_t block[22][2];  // W4, H4
   uint8_t tx[19][5];     // W4, H4, Log2W, Log2H, Sub
 };
@@ -47,12 +61,11 @@ struct MapArgs {
   uint16_t* masks;
   uint32_t* levels;  // one 4-byte level cell per MI cell
   unsigned long long* rowErr;  // per MI row: first error (cell << 8 | kind) or all ones
-  int cols, rows, sbw, regions, ssx, ssy, mono, ccols, crows;
+  int* refused;  // page-locked host word: set when the walk would refuse a cell if it met it
+  int cols, rows, sbw, ssx, ssy, mono, ccols, crows;
   // ResolveBlockLevels inputs (loopfilter/level.go:86-118)
   uint8_t base[3][2];
   uint8_t lumaZero, deltaPresent, deltaMulti, segEnabled, modeRef;
-  int8_t refDelta[8], modeDelta[2];
-  int16_t segDelta[8][4];
   MapTables t;
 };
 
@@ -153,15 +166,15 @@ __device__ __forceinline__ LfRec load_head(const MapArgs& a, int x, int y, bool 
 // or bottom row (horizontal), read at map cell (x, y) whose record is `r`
 // (fillLeftLumaContext / fillAboveLumaContext, loop_filter_masks.go:553-646):
 // 2 when the cell holds no valid block.
-__device__ int luma_edge_ctx(const MapArgs& a, const LfRec& r, int x, int y, bool vertical) {
+__device__ int luma_edge_ctx(const MapArgs& a, const MapTables& t, const LfRec& r, int x, int y, bool vertical) {
   if (!r.valid() || r.bs() >= 22) return 2;
-  const int nbw = min(a.cols - r.col(), (int)a.t.block[r.bs()][0]);
-  const int nbh = min(a.rows - r.row(), (int)a.t.block[r.bs()][1]);
+  const int nbw = min(a.cols - r.col(), (int)t.block[r.bs()][0]);
+  const int nbh = min(a.rows - r.row(), (int)t.block[r.bs()][1]);
   if (nbw <= 0 || nbh <= 0) return 2;
   const int lx = vertical ? nbw - 1 : x - r.col();
   const int ly = vertical ? y - r.row() : nbh - 1;
   if (lx < 0 || lx >= nbw || ly < 0 || ly >= nbh) return 2;
-  const Leaf L = tx_leaf(a.t, safe_tx(r.txy()), uniform_tx(r), r.split(), lx, ly);
+  const Leaf L = tx_leaf(t, safe_tx(r.txy()), uniform_tx(r), r.split(), lx, ly);
   return vertical ? L.cw : L.ch;
 }
 
@@ -170,26 +183,29 @@ __device__ __forceinline__ int clamp_level(int v) { return v < 0 ? 0 : (v > 63 ?
 // ResolveBlockLevels (loopfilter/level.go:120-190) packed as the level cell
 // [Y vertical, Y horizontal, U, V].  Indices are masked so that a record the
 // check kernel rejects cannot read out of range.
-__device__ uint32_t block_levels(const MapArgs& a, const LfRec& r) {
+// kChroma: the last two, else the first two.
+template <bool kChroma>
+__device__ __forceinline__ uint32_t block_levels(const MapArgs& a, const MapTables& t, const LfRec& r) {
   if (a.lumaZero) return 0;
   if (!a.deltaPresent && !a.segEnabled && !a.modeRef)
-    return a.base[0][0] | a.base[0][1] << 8 | a.base[1][0] << 16 | a.base[2][0] << 24;
+    return kChroma ? a.base[1][0] << 16 | (uint32_t)a.base[2][0] << 24 : a.base[0][0] | a.base[0][1] << 8;
   const int nplanes = a.mono ? 1 : 3;
   const int ref = r.ref() & 7, seg = r.seg() & 7;
   uint32_t out = 0;
-  for (int k = 0; k < 4; k++) {  // (Y,V) (Y,H) (U,V) (V,V)
+#pragma unroll
+  for (int k = kChroma ? 2 : 0; k < (kChroma ? 4 : 2); k++) {  // (Y,V) (Y,H) (U,V) (V,V)
     const int plane = k < 2 ? 0 : k - 1, edge = k < 2 ? k : 0;
     if (plane >= nplanes) break;
     const int base = a.base[plane][edge];
     if (plane && base == 0) continue;
     int dl = 0;
     if (a.deltaPresent) dl = a.deltaMulti ? r.deltaMulti(plane ? plane + 1 : edge) : r.deltaFromBase();
-    const int sd = a.segEnabled ? a.segDelta[seg][plane ? plane + 1 : edge] : 0;
+    const int sd = a.segEnabled ? t.segDelta[seg][plane ? plane + 1 : edge] : 0;
     int lvl = clamp_level(base + dl);
     lvl = clamp_level(lvl + sd);
     if (a.modeRef) {
-      int d = a.refDelta[ref];
-      if (ref > 0) d += a.modeDelta[r.mode() & 1];
+      int d = t.refDelta[ref];
+      if (ref > 0) d += t.modeDelta[r.mode() & 1];
       lvl = clamp_level(lvl + d * (1 << (lvl >> 5)));
     }
     out |= (uint32_t)lvl << (8 * k);
@@ -201,65 +217,76 @@ __device__ uint32_t block_levels(const MapArgs& a, const LfRec& r) {
 // neighbours: the width class of the vertical edge on its left and of the
 // horizontal edge on its top (-1: no edge), and the luma bytes of its level
 // cell.
-__device__ void luma_cell(const MapArgs& a, int x, int y, const LfRec& r, const LfRec& left, const LfRec& above,
+__device__ void luma_cell(const MapArgs& a, const MapTables& t, int x, int y, const LfRec& r, const LfRec& left, const LfRec& above,
                           int& sv, int& sh, uint32_t& lv) {
   if (!r.valid() || r.bs() >= 22) return;
   const int bx = r.col(), by = r.row();
-  const int bw4 = min(a.cols - bx, (int)a.t.block[r.bs()][0]);
-  const int bh4 = min(a.rows - by, (int)a.t.block[r.bs()][1]);
+  const int bw4 = min(a.cols - bx, (int)t.block[r.bs()][0]);
+  const int bh4 = min(a.rows - by, (int)t.block[r.bs()][1]);
   const int lx = x - bx, ly = y - by;
   if (lx < 0 || ly < 0 || lx >= bw4 || ly >= bh4) return;
   const int tx = safe_tx(r.txy());
   const bool uni = uniform_tx(r);
   const bool inner = r.intra() || !r.skip();
-  const Leaf L = tx_leaf(a.t, tx, uni, r.split(), lx, ly);
+  const Leaf L = tx_leaf(t, tx, uni, r.split(), lx, ly);
   if (lx == 0)
-    sv = min(L.cw, bx > 0 ? luma_edge_ctx(a, left, x - 1, y, true) : 2);
+    sv = min(L.cw, bx > 0 ? luma_edge_ctx(a, t, left, x - 1, y, true) : 2);
   else if (L.left && inner)
-    sv = min(L.cw, tx_leaf(a.t, tx, uni, r.split(), lx - 1, ly).cw);
+    sv = min(L.cw, tx_leaf(t, tx, uni, r.split(), lx - 1, ly).cw);
   if (ly == 0)
-    sh = min(L.ch, by > 0 ? luma_edge_ctx(a, above, x, y - 1, false) : 2);
+    sh = min(L.ch, by > 0 ? luma_edge_ctx(a, t, above, x, y - 1, false) : 2);
   else if (L.top && inner)
-    sh = min(L.ch, tx_leaf(a.t, tx, uni, r.split(), lx, ly - 1).ch);
-  lv = block_levels(a, r) & 0xffff;
+    sh = min(L.ch, tx_leaf(t, tx, uni, r.split(), lx, ly - 1).ch);
+  lv = block_levels<false>(a, t, r);
 }
 
 // Chroma level bytes of chroma cell (x, y): the covering block last in raster
 // order of origin (the reference's walk writes each block's chroma rect), one
-// of the records at the cell's luma group.
-__device__ uint32_t chroma_levels(const MapArgs& a, int x, int y) {
-  // The group is 1, 2 or 4 cells: k = j * 2 + i with i <= ssx, j <= ssy.
-  uint32_t head0[4], head2[4];
+// of the records at the cell's luma group.  The group is 1, 2 or 4 cells: k =
+// j * 2 + i with i <= ssx, j <= ssy; chroma_heads reads what picks one.
+struct ChromaHeads {
+  uint32_t origin[4], size[4];  // words 0 and 2
+};
+
+__device__ __forceinline__ ChromaHeads chroma_heads(const MapArgs& a, int x, int y) {
+  ChromaHeads h;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const int i = k & 1, j = k >> 1;
-    head2[k] = 0;
+    h.origin[k] = h.size[k] = 0;
     if (i <= a.ssx && j <= a.ssy) {
       const uint4 u = __ldg(a.rec + 2 * ((size_t)((y << a.ssy) + j) * a.cols + (x << a.ssx) + i));
-      head0[k] = u.x, head2[k] = u.z;
+      h.origin[k] = u.x, h.size[k] = u.z;
     }
   }
+  return h;
+}
+
+// The group's cell that counts, -1 without one.
+__device__ __forceinline__ int chroma_pick(const ChromaHeads& h) {
   int best = -1;
   uint32_t bestKey = 0;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const bool valid = (head2[k] >> 8) & 0xff;
-    if (!valid || (head2[k] & 0xff) >= 22) continue;
-    const uint32_t key = head0[k];  // mi_row << 16 | mi_col: raster order of origin
+    const bool valid = (h.size[k] >> 8) & 0xff;
+    if (!valid || (h.size[k] & 0xff) >= 22) continue;
+    const uint32_t key = h.origin[k];  // mi_row << 16 | mi_col: raster order of origin
     if (best < 0 || key > bestKey) best = k, bestKey = key;
   }
-  if (best < 0) return 0;
-  return block_levels(a, load_rec(a, (x << a.ssx) + (best & 1), (y << a.ssy) + (best >> 1))) & 0xffff0000u;
+  return best;
 }
 
 // Chroma cell (cx, cy) with the record `r` at the bottom-right luma cell of
 // its luma group: the block carrying the shared chroma there (the has_chroma
 // gate of dav1d as BuildFromMap applies it, loop_filter_masks.go:508-533).
-__device__ void chroma_cell(const MapArgs& a, int cx, int cy, const LfRec& r, int& sv, int& sh) {
+// The two context records, read where the cell starts its block, depend only
+// on the block's origin.
+__device__ __forceinline__ void chroma_cell(const MapArgs& a, const MapTables& t, int cx, int cy, const LfRec& r,
+                                            const LfRec& nl, const LfRec& na, int& sv, int& sh) {
   const int lx = (cx << a.ssx) + a.ssx, ly = (cy << a.ssy) + a.ssy;
   if (!r.valid() || !r.hasUV() || r.bs() >= 22) return;
   const int bx = r.col(), by = r.row();
-  const int W4 = a.t.block[r.bs()][0], H4 = a.t.block[r.bs()][1];
+  const int W4 = t.block[r.bs()][0], H4 = t.block[r.bs()][1];
   if (!((W4 > a.ssx || (bx & 1)) && (H4 > a.ssy || (by & 1)))) return;
   const int bw4 = min(a.cols - bx, W4), bh4 = min(a.rows - by, H4);
   if (lx < bx || lx >= bx + bw4 || ly < by || ly >= by + bh4) return;
@@ -267,119 +294,123 @@ __device__ void chroma_cell(const MapArgs& a, int cx, int cy, const LfRec& r, in
   const int cbh4 = min(a.crows - (by >> a.ssy), (H4 + a.ssy) >> a.ssy);
   const int lcx = cx - (bx >> a.ssx), lcy = cy - (by >> a.ssy);
   if (lcx < 0 || lcy < 0 || lcx >= cbw4 || lcy >= cbh4) return;
-  const uint8_t* d = a.t.tx[safe_tx(r.txuv())];
+  const uint8_t* d = t.tx[safe_tx(r.txuv())];
   const int cw = d[2] != 0, ch = d[3] != 0;
   const bool inner = r.intra() || !r.skip();
-  // The two context loads depend only on the block origin: issue both.
-  const bool needL = lcx == 0 && bx > 0, needA = lcy == 0 && by > 0;
-  LfRec nl, na;
-  if (needL) nl = load_head(a, bx - 1, min((cy << a.ssy) + a.ssy, a.rows - 1), false);
-  if (needA) na = load_head(a, min((cx << a.ssx) + a.ssx, a.cols - 1), by - 1, false);
   if (lcx == 0) {
     int ctx = 1;
-    if (needL && nl.valid() && nl.hasUV()) ctx = a.t.tx[safe_tx(nl.txuv())][2] != 0;
+    if (bx > 0 && nl.valid() && nl.hasUV()) ctx = t.tx[safe_tx(nl.txuv())][2] != 0;
     sv = min(cw, ctx);
   } else if (inner && (lcx & (d[0] - 1)) == 0) {
     sv = cw;
   }
   if (lcy == 0) {
     int ctx = 1;
-    if (needA && na.valid() && na.hasUV()) ctx = a.t.tx[safe_tx(na.txuv())][3] != 0;
+    if (by > 0 && na.valid() && na.hasUV()) ctx = t.tx[safe_tx(na.txuv())][3] != 0;
     sh = min(ch, ctx);
   } else if (inner && (lcy & (d[1] - 1)) == 0) {
     sh = ch;
   }
 }
 
+// The error the reference's level-cache walk (postfilter_loopfilter_masks.go:
+// 146-224) meets if it visits cell (c, row) of record `r`: ResolveBlockLevels'
+// checks (level.go:126-175) come before the block-size check, as there.
+__device__ __forceinline__ int walk_error(const MapArgs& a, const LfRec& r, int c, int row) {
+  if (!r.valid()) return 0;
+  const int next = r.colEnd();
+  if (next <= c || next > a.cols) return kLfBatch;
+  if (r.col() != c || r.row() != row) return 0;
+  if (r.ref() >= 8 || r.mode() > 1 || (!a.lumaZero && a.segEnabled && r.seg() >= 8)) return kLfFilter;
+  return r.bs() >= 22 || r.txy() >= 19 || (!a.mono && r.hasUV() && r.txuv() >= 19) ? kLfBatch : 0;
+}
+
 // One 128x128 region (32x32 cells) per CTA, a thread per cell.
-__device__ void region_masks(const MapArgs& a, int region, int8_t (*s_t)[33], uint32_t (*s_lv)[33]) {
-  const int rx = region % a.sbw, ry = region / a.sbw;
+struct RegionSmem {
+  int8_t luma[32][33], chroma[32][33];  // vertical edges' classes
+  MapTables t;
+};
+
+__global__ void __launch_bounds__(1024) k_lf_build(MapArgs a) {
+  __shared__ RegionSmem S;
+  const int rx = blockIdx.x % a.sbw, ry = blockIdx.x / a.sbw;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t* M = (uint32_t*)(a.masks + (size_t)region * PF_LF_MASK_WORDS);
+  uint32_t* M = (uint32_t*)(a.masks + (size_t)blockIdx.x * PF_LF_MASK_WORDS);
 
   // Every record load that does not depend on another goes out first: the
   // cell's own record, its left and upper neighbours (read only when the
-  // cell starts its block), and the emitter of this thread's chroma cell.
-  const int x = rx * 32 + w, y = ry * 32 + lane;
+  // cell starts its block), the heads of its chroma cell's group (the level
+  // cell's chroma bytes) and the emitter of this thread's chroma cell.
+  const int x = rx * 32 + lane, y = ry * 32 + w;
   const bool in = x < a.cols && y < a.rows;
   const int cwid = 32 >> a.ssx, chgt = 32 >> a.ssy;
-  const int cx = rx * cwid + w, cy = ry * chgt + lane;
-  const bool cin = !a.mono && w < cwid && lane < chgt && cx < a.ccols && cy < a.crows;
-  LfRec own, left, above, em;
+  const int cx = rx * cwid + lane, cy = ry * chgt + w;
+  const bool cin = !a.mono && lane < cwid && w < chgt && cx < a.ccols && cy < a.crows;
+  const int ex = (cx << a.ssx) + a.ssx, ey = (cy << a.ssy) + a.ssy;  // the emitter
+  const bool clv = in && !a.mono && x < a.ccols && y < a.crows;
+  LfRec own, left, above, em, nl, na, cl;
+  ChromaHeads heads;
   if (in) own = load_rec(a, x, y);
+  if (cin) em = load_head(a, ex, ey, false);
+  if (clv) heads = chroma_heads(a, x, y);
   if (in && x > 0) left = load_head(a, x - 1, y, true);
   if (in && y > 0) above = load_head(a, x, y - 1, true);
-  if (cin) em = load_head(a, (cx << a.ssx) + a.ssx, (cy << a.ssy) + a.ssy, false);
+  if (threadIdx.x < sizeof(MapTables)) ((uint8_t*)&S.t)[threadIdx.x] = ((const uint8_t*)&a.t)[threadIdx.x];
+  __syncthreads();
+  // Then those that do: the chroma cell's contexts and level record.
+  // (An origin past its own cell belongs to a record that is not used.)
+  if (cin && em.col() > 0 && em.col() <= ex) nl = load_head(a, em.col() - 1, ey, false);
+  if (cin && em.row() > 0 && em.row() <= ey) na = load_head(a, ex, em.row() - 1, false);
+  const int best = clv ? chroma_pick(heads) : -1;
+  if (best >= 0) cl = load_rec(a, (x << a.ssx) + (best & 1), (y << a.ssy) + (best >> 1));
 
-  // Luma.  Warp = column w, lane = row: vertical edges of column w.
-  int sv = -1, sh = -1;
-  uint32_t lv = 0;
+  // Warp = row w, lane = column: horizontal edges and level cells of row w.
+  int sv = -1, sh = -1, cv = -1, chs = -1;
   if (in) {
-    luma_cell(a, x, y, own, left, above, sv, sh, lv);
-    if (!a.mono && x < a.ccols && y < a.crows) lv |= chroma_levels(a, x, y);
+    if (walk_error(a, own, x, y)) *(volatile int*)a.refused = 1;
+    uint32_t lv = 0;
+    luma_cell(a, S.t, x, y, own, left, above, sv, sh, lv);
+    if (best >= 0) lv |= block_levels<true>(a, S.t, cl);
+    a.levels[(size_t)y * a.cols + x] = lv;
   }
-  // Y[0][w][s] as one 32-bit word: bit = row within the region.
-#pragma unroll
-  for (int s = 0; s < 3; s++) {
-    const uint32_t b = __ballot_sync(0xffffffffu, sv == s);
-    if (lane == 0) M[w * 3 + s] = b;
-  }
-  s_t[lane][w] = (int8_t)sh;
-  s_lv[lane][w] = lv;
-  __syncthreads();
-  // Warp = row w, lane = column: horizontal edges of row w, and the level
-  // cells of row w stored coalesced.
-  {
-    const int s0 = s_t[w][lane];
-#pragma unroll
-    for (int s = 0; s < 3; s++) {
-      const uint32_t b = __ballot_sync(0xffffffffu, s0 == s);
-      if (lane == 0) M[(32 + w) * 3 + s] = b;
-    }
-    const int x2 = rx * 32 + lane, y2 = ry * 32 + w;
-    if (x2 < a.cols && y2 < a.rows) a.levels[(size_t)y2 * a.cols + x2] = s_lv[w][lane];
-  }
-  __syncthreads();
-
-  // Chroma: the region's (32 >> ssx) x (32 >> ssy) chroma cells.  UV[dir][pos][s]
-  // is two 16-bit halves split at 16 >> ss of the scanned direction.
-  int cv = -1, chs = -1;
-  if (cin) chroma_cell(a, cx, cy, em, cv, chs);
+  if (cin) chroma_cell(a, S.t, cx, cy, em, nl, na, cv, chs);
+  S.luma[w][lane] = (int8_t)sv;
+  S.chroma[w][lane] = (int8_t)cv;
+  // Y[dir][pos][s] as one 32-bit word: bit = column (row) within the region;
+  // UV[dir][pos][s] is two 16-bit halves split at 16 >> ss of the scanned
+  // direction.
   const int vsplit = 16 >> a.ssy, hsplit = 16 >> a.ssx;
 #pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const uint32_t b = __ballot_sync(0xffffffffu, cv == s);
-    if (lane == 0) M[192 + w * 2 + s] = (b & ((1u << vsplit) - 1)) | (b >> vsplit) << 16;
+  for (int s = 0; s < 3; s++) {
+    const uint32_t b = __ballot_sync(0xffffffffu, sh == s);
+    if (lane == 0) M[(32 + w) * 3 + s] = b;
   }
-  s_t[lane][w] = (int8_t)chs;
-  __syncthreads();
-  {
-    const int s0 = s_t[w][lane];
 #pragma unroll
-    for (int s = 0; s < 2; s++) {
-      const uint32_t b = __ballot_sync(0xffffffffu, s0 == s);
-      if (lane == 0) M[192 + (32 + w) * 2 + s] = (b & ((1u << hsplit) - 1)) | (b >> hsplit) << 16;
-    }
+  for (int s = 0; s < 2; s++) {
+    const uint32_t b = __ballot_sync(0xffffffffu, chs == s);
+    if (lane == 0) M[192 + (32 + w) * 2 + s] = (b & ((1u << hsplit) - 1)) | (b >> hsplit) << 16;
+  }
+  __syncthreads();
+  // Warp = column w, lane = row: vertical edges of column w.
+  const int l0 = S.luma[lane][w], c0 = S.chroma[lane][w];
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    const uint32_t b = __ballot_sync(0xffffffffu, l0 == s);
+    if (lane == 0) M[w * 3 + s] = b;
+  }
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    const uint32_t b = __ballot_sync(0xffffffffu, c0 == s);
+    if (lane == 0) M[192 + w * 2 + s] = (b & ((1u << vsplit) - 1)) | (b >> vsplit) << 16;
   }
 }
 
-// The reference's level-cache walk over one MI row (postfilter_loopfilter_masks
-// .go:146-224): each cell's successor in the chain and the error the walk
-// meets if it visits the cell; ResolveBlockLevels' checks (level.go:126-175)
-// come before the block-size check, as in the reference.
+// A cell's successor in the walk's chain and, above bit 20, its error.
 __device__ uint32_t walk_cell(const MapArgs& a, int c, int row) {
   const LfRec r = load_rec(a, c, row);
   if (!r.valid()) return c + 1;
-  const int next = r.colEnd();
-  if (next <= c || next > a.cols) return (uint32_t)c | (uint32_t)kLfBatch << 20;
-  uint32_t code = 0;
-  if (r.col() == c && r.row() == row) {
-    if (r.ref() >= 8 || r.mode() > 1 || (!a.lumaZero && a.segEnabled && r.seg() >= 8))
-      code = kLfFilter;
-    else if (r.bs() >= 22 || r.txy() >= 19 || (!a.mono && r.hasUV() && r.txuv() >= 19))
-      code = kLfBatch;
-  }
-  return (uint32_t)next | code << 20;
+  const int code = walk_error(a, r, c, row), next = r.colEnd();
+  return (uint32_t)(next <= c || next > a.cols ? c : next) | (uint32_t)code << 20;
 }
 
 struct WalkSmem {
@@ -435,16 +466,10 @@ __device__ void row_walk(const MapArgs& a, int row, WalkSmem& S) {
   }
 }
 
-// One launch: CTAs [0, regions) build the masks and level cache of one
-// 128x128 region each, the rest walk one MI row each for the status.
-__global__ void __launch_bounds__(1024) k_lf_build(MapArgs a) {
-  __shared__ int8_t s_t[32][33];
-  __shared__ uint32_t s_lv[32][33];
-  __shared__ WalkSmem s_walk;
-  if ((int)blockIdx.x < a.regions)
-    region_masks(a, blockIdx.x, s_t, s_lv);
-  else
-    row_walk(a, blockIdx.x - a.regions, s_walk);
+// One CTA per MI row, for the status of a map with a cell to refuse.
+__global__ void __launch_bounds__(1024) k_lf_walk(MapArgs a) {
+  __shared__ WalkSmem S;
+  row_walk(a, blockIdx.x, S);
 }
 
 }  // namespace pf
@@ -482,9 +507,9 @@ extern "C" int pf_lf_build(pf_ctx* ctx, const pf_lf_record* records, int32_t col
   a.lumaZero = lv->level_y[0] == 0 && lv->level_y[1] == 0;
   a.deltaPresent = lv->delta_lf_present != 0, a.deltaMulti = lv->delta_lf_multi != 0;
   a.segEnabled = lv->segmentation_enabled != 0, a.modeRef = lv->mode_ref_delta_enabled != 0;
-  memcpy(a.refDelta, lv->ref_delta, 8);
-  memcpy(a.modeDelta, lv->mode_delta, 2);
-  if (a.segEnabled) memcpy(a.segDelta, lv->segment_delta, sizeof(a.segDelta));
+  memcpy(a.t.refDelta, lv->ref_delta, 8);
+  memcpy(a.t.modeDelta, lv->mode_delta, 2);
+  if (a.segEnabled) memcpy(a.t.segDelta, lv->segment_delta, sizeof(a.t.segDelta));
   memcpy(a.t.block, pf_block_dims, sizeof(a.t.block));
   memcpy(a.t.tx, pf_tx_dims, sizeof(a.t.tx));
 
@@ -518,14 +543,21 @@ extern "C" int pf_lf_build(pf_ctx* ctx, const pf_lf_record* records, int32_t col
     a.levels = (uint32_t*)level_cache;
   }
   if (e != cudaSuccess) return PF_ERR_DEVICE;
-  a.regions = a.sbw * sbh;
-  k_lf_build<<<a.regions + rows, 1024, 0, st>>>(a);
+  a.refused = (int*)hostErr;
+  *a.refused = 0;
+  k_lf_build<<<a.sbw * sbh, 1024, 0, st>>>(a);
   e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hostErr, a.rowErr, (size_t)rows * 8, cudaMemcpyDeviceToHost, st);
   if (hostOut && e == cudaSuccess) e = cudaMemcpyAsync(masks, a.masks, maskB, cudaMemcpyDeviceToHost, st);
   if (hostOut && e == cudaSuccess) e = cudaMemcpyAsync(level_cache, a.levels, lcB, cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return PF_ERR_DEVICE;
-  const int w = pf_internal_wait(ctx, st);
+  int w = pf_internal_wait(ctx, st);
+  if (w != PF_OK) return w;
+  if (!*(volatile int*)a.refused) return PF_OK;
+  k_lf_walk<<<rows, 1024, 0, st>>>(a);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hostErr, a.rowErr, (size_t)rows * 8, cudaMemcpyDeviceToHost, st);
+  if (e != cudaSuccess) return PF_ERR_DEVICE;
+  w = pf_internal_wait(ctx, st);
   if (w != PF_OK) return w;
   unsigned long long err = ~0ull;
   for (int r = 0; r < rows; r++) err = hostErr[r] < err ? hostErr[r] : err;

@@ -137,6 +137,25 @@ def test_errors(runner):
     check(runner, rec, lv)
 
 
+@pytest.mark.parametrize("field,value", [("mi_col_end", 0), ("ref_frame", 8), ("block_size", 22)])
+def test_cells_the_walk_never_meets(runner, field, value):
+    """A cell that the walk would refuse, inside a block whose row it jumps
+    over, is no error.  (Masks and levels of a cell come from its own record,
+    the reference's from the block's origin: the same in a map whose blocks'
+    cells all hold the block's record, and for a field that neither reads.)"""
+    rec, _ = synth.make_lf_map(11, 64, 32, p_split=0.3)
+    rows, cols = np.nonzero((rec["mi_col"] != np.arange(64)[None, :]) & (rec["valid"] == 1))
+    assert len(rows)
+    bad = rec.copy()
+    for k in np.random.default_rng(3).integers(0, len(rows), 20):
+        bad[field][rows[k], cols[k]] = value
+    lv = synth.make_lf_levels(11, "deltas")
+    assert oracle(bad, lv)[0] == 0
+    runner.lf_build(bad, lv)
+    if field == "mi_col_end":
+        check(runner, bad, lv)
+
+
 def test_masks_drive_the_deblocking(runner):
     """The chain's deblocking stage on GPU-built masks and levels equals the
     oracle's chain on the oracle-built ones."""
