@@ -28,9 +28,11 @@
 //                   distributed shared memory.  The refinement ends once nb
 //                   steps in a row have changed nothing (no later one can).
 //                   Bound by the barriers of a step, two of the cluster
-//                   among them; 1080p: 303 us with all 40 steps of 8
-//                   presets run, 127 now; the learned search's 8 steps 62
-//                   (1,024 threads a CTA instead of 512: 152 and 75).
+//                   among them, hence maxima by warp reductions of one
+//                   key and one thread's bookkeeping a step; 1080p: 303 us
+//                   with all 40 steps of 8 presets run, 127 ended early, 120
+//                   now; the learned search's 8 steps 62 and 57 (1,024
+//                   threads a CTA instead of 512: 152 and 75).
 //   k_sel_finish    the RD choice of nb and the per-block preset index.
 #include <cooperative_groups.h>
 #include <string.h>
@@ -440,22 +442,26 @@ struct SelShared {
   // Partial savings of this CTA's slice of the pairs, a row from each CTA of
   // the cluster (first pick: this CTA's column sums).
   alignas(16) unsigned long long part[4096];
-  unsigned long long col[128];
-  unsigned long long candV[2][kSelMaxCluster], candSB[2][kSelMaxCluster];
-  int candI[2][kSelMaxCluster];
-  unsigned long long redV[kSelThreads / 32];
-  int redI[kSelThreads / 32];
-  unsigned long long redS[kSelThreads / 32];
-  int lev0[8], lev1[8], drop[2];
-  unsigned long long tot;
+  unsigned long long cand[2][kSelMaxCluster];
+  unsigned long long tot[kSelMaxCluster];  // rank 0's: every CTA's part of the total
+  unsigned long long red[kSelThreads / 32];
+  int wsum[kSelThreads / 32];
+  int lev0[8], lev1[8];
+  int done;
 };
 
-// First maximum wins: larger value, or equal value at a lower index.
-__device__ __forceinline__ void argmax_merge(unsigned long long& v, int& i, unsigned long long v2, int i2) {
-  if (i == 0x7fffffff || v2 > v || (v2 == v && i2 < i)) {
-    v = v2;
-    i = i2;
-  }
+// A pair's saving with the pair's number below it, turned: the largest key is
+// the first maximum.  A sum over the blocks (at most 2^16 of less than 2^31)
+// is below kSelSumMax, so what it lacks of that serves for the first minimum.
+constexpr unsigned long long kSelSumMax = 1ull << 50;
+__device__ __forceinline__ unsigned long long sel_key(unsigned long long saving, int pair) {
+  return saving << 12 | (unsigned long long)(4095 - pair);
+}
+
+// The warp's largest key, by its upper and then its lower word.
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
+  const uint32_t hi = (uint32_t)(v >> 32), top = __reduce_max_sync(~0u, hi);
+  return (unsigned long long)top << 32 | __reduce_max_sync(~0u, hi == top ? (uint32_t)v : 0u);
 }
 
 // The non-skip filter blocks in order (computeCDEFList's non-empty units):
@@ -501,7 +507,7 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
   const int cfg = blockIdx.x / CS;
   const int nb = 1 << cfg;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int n = compact_blocks(a.skip, a.nfb, s_sb, S.redI);
+  const int n = compact_blocks(a.skip, a.nfb, s_sb, S.wsum);
   SelOut* out = a.out;
   if (n == 0) {
     if (rank == 0 && t == 0) {
@@ -527,18 +533,16 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
       s_rows[e] = (uint32_t)(pl ? M1 : M0)[(size_t)fb * 64 + j];
     }
   __syncthreads();
-  for (int il = t; il < cnt; il += kSelThreads) {
-    uint32_t m = 0xffffffffu;
-    for (int k = 0; k < 64; k++) m = min(m, row(il, 1, k));
-    s_min1[il] = m;
+  for (int il = warp; il < cnt; il += kSelThreads / 32) {
+    const uint32_t m = __reduce_min_sync(~0u, min(row(il, 1, lane), row(il, 1, lane + 32)));
+    if (lane == 0) s_min1[il] = m;
   }
   if (t < 8) S.lev0[t] = S.lev1[t] = 0;
   __syncthreads();
   const int steps = a.refine ? 5 * nb : nb;
-  int same = 0;  // refinement steps in a row that took back the pick they had dropped
+  int same = 0, drop0 = 0, drop1 = 0;  // thread 0's: refinement steps in a row that took back the pick they had dropped
   for (int k = 0; k < steps; k++) {
     const int nbCur = k < nb ? k : nb - 1;
-    const int drop0 = S.drop[0], drop1 = S.drop[1];
     const int par = k & 1;
     if (nbCur == 0) {
       // First pick: the luma and chroma strengths with the least total SSE.
@@ -556,39 +560,25 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
           s2 += cl.map_shared_rank(&S.part[0], r + 2)[t];
           s3 += cl.map_shared_rank(&S.part[0], r + 3)[t];
         }
-        S.col[t] = (s0 + s1) + (s2 + s3);
+        const unsigned long long sum = (s0 + s1) + (s2 + s3);
+        // The first minimum of each plane's 64 sums, two warps a plane.
+        const unsigned long long best = warp_max(sel_key(kSelSumMax - sum, t & 63));
+        if (lane == 0) S.red[warp] = best;
       }
       __syncthreads();
       if (t == 0) {
-        int b0 = 0, b1 = 0;
-        for (int j = 1; j < 64; j++) {
-          if (S.col[j] < S.col[b0]) b0 = j;
-          if (S.col[64 + j] < S.col[64 + b1]) b1 = j;
-        }
-        S.lev0[0] = b0;
-        S.lev1[0] = b1;
-        S.tot = S.col[b0] + S.col[64 + b1];
+        S.lev0[0] = 4095 - (int)(max(S.red[0], S.red[1]) & 4095);
+        S.lev1[0] = 4095 - (int)(max(S.red[2], S.red[3]) & 4095);
       }
       cl.sync();  // every CTA has read the others' column sums
     } else {
-      // best_i over the strengths selected so far, and its sum.
-      unsigned long long sb = 0;
+      // best_i over the strengths selected so far.
       for (int il = t; il < cnt; il += kSelThreads) {
         uint32_t best = row(il, 0, S.lev0[0]) + row(il, 1, S.lev1[0]);
         for (int g = 1; g < nbCur; g++) best = min(best, row(il, 0, S.lev0[g]) + row(il, 1, S.lev1[g]));
         s_best[il] = best;
-        sb += best;
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sb += __shfl_xor_sync(0xffffffffu, sb, o);
-      if (lane == 0) S.redS[warp] = sb;
       __syncthreads();
-      unsigned long long sbAll = 0;  // warp 0's: the CTA's sum
-      if (warp == 0) {
-        sbAll = lane < kSelThreads / 32 ? S.redS[lane] : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sbAll += __shfl_xor_sync(0xffffffffu, sbAll, o);
-      }
       // Partial savings of this CTA's blocks: thread t owns (j, k0..k0+7).
       // A block saves below 2^29, so eight blocks sum exactly in 32 bits
       // before joining the 64-bit totals.
@@ -634,8 +624,7 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
       }
       cl.sync();
       // First maximum wins.  Two neighbouring threads share a pair.
-      unsigned long long bv = 0;
-      int bi = 0x7fffffff;
+      unsigned long long key = 0;
       for (int e2 = t; e2 < 2 * pairs; e2 += kSelThreads) {
         const int e = e2 >> 1, r0 = (e2 & 1) * (CS >> 1);
         unsigned long long sum = 0;
@@ -643,96 +632,78 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
         for (int r = 0; r < kSelMaxCluster / 2; r++)
           if (r < (CS >> 1)) sum += S.part[(r0 + r) * pairs + e];
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        argmax_merge(bv, bi, sum, rank * pairs + e);
+        key = max(key, sel_key(sum, rank * pairs + e));
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long v2 = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
-        argmax_merge(bv, bi, v2, i2);
-      }
-      if (lane == 0) {
-        S.redV[warp] = bv;
-        S.redI[warp] = bi;
-      }
+      key = warp_max(key);
+      if (lane == 0) S.red[warp] = key;
       __syncthreads();
       if (warp == 0) {
-        unsigned long long v = 0;
-        int i = 0x7fffffff;
-        if (lane < kSelThreads / 32) {
-          v = S.redV[lane];
-          i = S.redI[lane];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const unsigned long long v2 = __shfl_xor_sync(0xffffffffu, v, o);
-          const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-          argmax_merge(v, i, v2, i2);
-        }
-        // Lane r hands this CTA's candidate and partial sum of best_i to
-        // rank r (alternate steps use alternate places).
-        if (lane < CS) {
-          SelShared* R = cl.map_shared_rank(&S, lane);
-          R->candV[par][rank] = v;
-          R->candI[par][rank] = i;
-          R->candSB[par][rank] = sbAll;
-        }
+        key = warp_max(lane < kSelThreads / 32 ? S.red[lane] : 0);
+        // Lane r hands this CTA's candidate to rank r (alternate steps use
+        // alternate places).
+        if (lane < CS) cl.map_shared_rank(&S, lane)->cand[par][rank] = key;
       }
       cl.sync();
       if (warp == 0) {
-        unsigned long long v = 0, sbr = 0;
-        int i = 0x7fffffff;
-        if (lane < CS) {
-          v = S.candV[par][lane];
-          i = S.candI[par][lane];
-          sbr = S.candSB[par][lane];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const unsigned long long v2 = __shfl_xor_sync(0xffffffffu, v, o);
-          const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-          argmax_merge(v, i, v2, i2);
-          sbr += __shfl_xor_sync(0xffffffffu, sbr, o);
-        }
+        key = warp_max(lane < CS ? S.cand[par][lane] : 0);
         if (lane == 0) {
+          const int i = 4095 - (int)(key & 4095);
           S.lev0[nbCur] = i >> 6;
           S.lev1[nbCur] = i & 63;
-          S.tot = sbr - v;
         }
       }
     }
-    __syncthreads();
-    // A pick depends only on the set of the other nb - 1, so once nb steps in
-    // a row have taken back what they dropped, every later one does: the
-    // remaining steps only turn the list, which is then done at once.
-    if (k >= nb) same = S.lev0[nb - 1] == drop0 && S.lev1[nb - 1] == drop1 ? same + 1 : 0;
-    const int turn = same == nb ? (steps - 1 - k) % nb : 1;
-    __syncthreads();
-    // Refinement passes drop the oldest pick (jointStrengthSearchDual).
-    if (t == 0 && k + 1 >= nb && k + 1 < steps) {
-      S.drop[0] = S.lev0[0];
-      S.drop[1] = S.lev1[0];
-      for (int q = 0; q < turn; q++) {
-        const int l0 = S.lev0[0], l1 = S.lev1[0];
-        for (int g = 0; g < nb - 1; g++) {
-          S.lev0[g] = S.lev0[g + 1];
-          S.lev1[g] = S.lev1[g + 1];
+    if (t == 0) {
+      // A pick depends only on the set of the other nb - 1, so once nb steps
+      // in a row have taken back what they dropped, every later one does: the
+      // remaining steps only turn the list, which is then done at once.
+      if (k >= nb) same = S.lev0[nb - 1] == drop0 && S.lev1[nb - 1] == drop1 ? same + 1 : 0;
+      const int turn = same == nb ? (steps - 1 - k) % nb : 1;
+      // Refinement passes drop the oldest pick (jointStrengthSearchDual).
+      if (k + 1 >= nb && k + 1 < steps) {
+        drop0 = S.lev0[0];
+        drop1 = S.lev1[0];
+        for (int q = 0; q < turn; q++) {
+          const int l0 = S.lev0[0], l1 = S.lev1[0];
+          for (int g = 0; g < nb - 1; g++) {
+            S.lev0[g] = S.lev0[g + 1];
+            S.lev1[g] = S.lev1[g + 1];
+          }
+          S.lev0[nb - 1] = l0;
+          S.lev1[nb - 1] = l1;
         }
-        S.lev0[nb - 1] = l0;
-        S.lev1[nb - 1] = l1;
       }
+      S.done = same == nb;
     }
     __syncthreads();
-    if (same == nb) break;
+    if (S.done) break;
   }
+  // The total SSE with the picks.
+  unsigned long long tot = 0;
+  for (int il = t; il < cnt; il += kSelThreads) {
+    uint32_t best = row(il, 0, S.lev0[0]) + row(il, 1, S.lev1[0]);
+    for (int g = 1; g < nb; g++) best = min(best, row(il, 0, S.lev0[g]) + row(il, 1, S.lev1[g]));
+    tot += best;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+  if (lane == 0) S.red[warp] = tot;
+  __syncthreads();
+  if (t == 0) {
+    tot = 0;
+    for (int i = 0; i < kSelThreads / 32; i++) tot += S.red[i];
+    cl.map_shared_rank(&S, 0)->tot[rank] = tot;
+  }
+  cl.sync();
   if (rank == 0 && t == 0) {
     for (int g = 0; g < 8; g++) {
       out->lev0[cfg][g] = g < nb ? S.lev0[g] : 0;
       out->lev1[cfg][g] = g < nb ? S.lev1[g] : 0;
     }
-    out->tot[cfg] = S.tot;
+    tot = 0;
+    for (int r = 0; r < CS; r++) tot += S.tot[r];
+    out->tot[cfg] = tot;
   }
-  cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // RD choice of nb (finish, :914-931) and the per-block preset index.
