@@ -632,7 +632,11 @@ cudaError_t launch_lr(const StageLaunch& l) {
 // bytes, 10 MB at 1080p, so it stays in L2).  k_lr_search_decide: one CTA
 // per unit replays the reference's decisions over the table, writes the
 // unit record and copies the winner's samples (or the unfiltered ones) into
-// the output plane.
+// the output plane.  Bound by integer issue and the wait for the staged rows;
+// 1920x1080, by the profiler: 68 us for the measuring kernel with the source
+// read byte by byte at three CTAs per SM, 53 by words, 49 with four CTAs (five
+// and six: the same call time); 11.8 us for the decisions with the copy byte
+// by byte, 4.4 now.
 
 // The candidate tap sets and presets of encoder/restoration.go:166-173 and
 // :235-240, in the reference's order (first strictly better wins).
@@ -671,7 +675,7 @@ __device__ __forceinline__ uint8_t* lrs_cand(const LrsArgs& a, int unit, int job
 
 struct LrsSmem {
   LrSmem lr;
-  uint8_t src[64 * 64];
+  alignas(4) uint8_t src[64 * 64];
   uint32_t red[8 * 8];
 };
 
@@ -711,15 +715,21 @@ __device__ __forceinline__ void lrs_block_sum(uint32_t (&v)[N], uint32_t* red) {
 // `tables`; the unit's source samples into sm.src when `source`.
 __device__ __forceinline__ void lrs_stage(const LrsArgs& a, LrsSmem& sm, int x0, int y0, int w, int h, bool tables,
                                           bool source) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool words = ((reinterpret_cast<uintptr_t>(a.rec) | (uintptr_t)a.rstride) & 3) == 0;
   lr_stage<uint8_t>(sm.lr.win, x0, w, h + 6, a.W, words,
                     [&](int r) { return a.rec + (int64_t)iclip(y0 - 3 + r, 0, a.H - 1) * a.rstride; });
-  if (source)
-    for (int r = warp; r < h; r += 8) {
-      const uint8_t* row = a.src + (int64_t)(y0 + r) * a.sstride + x0;
-      for (int c = lane; c < w; c += 32) sm.src[r * 64 + c] = row[c];
+  if (source) {
+    // Four samples a load where the rows allow it (x0 is a multiple of 64).
+    const bool quads = ((reinterpret_cast<uintptr_t>(a.src) | (uintptr_t)a.sstride) & 3) == 0;
+    for (int i = threadIdx.x; i < h * 16; i += 256) {
+      const int r = i >> 4, c = (i & 15) * 4;
+      const uint8_t* p = a.src + (int64_t)(y0 + r) * a.sstride + x0 + c;
+      if (quads && c + 4 <= w)
+        *reinterpret_cast<uint32_t*>(&sm.src[r * 64 + c]) = *reinterpret_cast<const uint32_t*>(p);
+      else
+        for (int k = 0; k < 4 && c + k < w; k++) sm.src[r * 64 + c + k] = p[k];
     }
+  }
   if (tables) sm.lr.xbx[threadIdx.x] = c_xbx[threadIdx.x];
   __syncthreads();
 }
@@ -763,17 +773,15 @@ __device__ __forceinline__ int lrs_wiener_pick(const uint32_t* cand, uint32_t ba
 // One exact filter's outputs of columns x and x + 1: their squared error
 // against the source, and into the candidate buffer (rows of 64).
 __device__ __forceinline__ uint32_t lrs_outcome(const LrsSmem& sm, uint8_t* keep, int w, int y, int x, int v0, int v1) {
-  const int d0 = (int)sm.src[y * 64 + x] - v0;
+  const uint32_t s = *reinterpret_cast<const uint16_t*>(&sm.src[y * 64 + x]);  // x is even
+  const int d0 = (int)(s & 0xff) - v0, d1 = (int)(s >> 8) - v1;
   uint32_t e = (uint32_t)(d0 * d0);
-  if (x + 1 < w) {
-    const int d1 = (int)sm.src[y * 64 + x + 1] - v1;
-    e += (uint32_t)(d1 * d1);
-  }
+  if (x + 1 < w) e += (uint32_t)(d1 * d1);
   if (keep) *reinterpret_cast<uint16_t*>(&keep[y * 64 + x]) = (uint16_t)(v0 | v1 << 8);  // x + 1 <= 63
   return e;
 }
 
-__global__ void __launch_bounds__(256, 3) k_lr_search_sse(LrsArgs a) {
+__global__ void __launch_bounds__(256, 4) k_lr_search_sse(LrsArgs a) {
   extern __shared__ __align__(16) uint8_t lrs_smem_raw[];
   LrsSmem& sm = *reinterpret_cast<LrsSmem*>(lrs_smem_raw);
   const int unit = blockIdx.x, job = blockIdx.y;
@@ -905,15 +913,31 @@ __global__ void __launch_bounds__(256) k_lr_search_decide(LrsArgs a) {
   // measuring CTA; NONE units keep the reconstruction.
   const uint8_t* from = type == PF_LR_WIENER ? lrs_cand(a, unit, 0)
                         : type == PF_LR_SGRPROJ ? lrs_cand(a, unit, 1 + spick) : nullptr;
-  if (from) {
-    const int x = tid & 63;
-    if (x < w)
-      for (int y = tid >> 6; y < h; y += 4) a.dst[(int64_t)(y0 + y) * a.dstride + x0 + x] = from[y * 64 + x];
+  // Units of up to 64x64 whose rows allow it (x0 is a multiple of 64): a word
+  // of four rows a thread, all loads before the first store.
+  const uint8_t* src = from ? from : a.rec + (int64_t)y0 * a.rstride + x0;
+  const int64_t sstride = from ? 64 : a.rstride;
+  uint8_t* dst = a.dst + (int64_t)y0 * a.dstride + x0;
+  if (fits && ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)sstride | reinterpret_cast<uintptr_t>(dst) |
+                (uintptr_t)a.dstride) & 3) == 0) {
+    const int x = (tid & 15) * 4, r = tid >> 4;
+    uint32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (r + 16 * k < h && x + 4 <= w) v[k] = *reinterpret_cast<const uint32_t*>(src + (r + 16 * k) * sstride + x);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int y = r + 16 * k;
+      if (y >= h) break;
+      if (x + 4 <= w)
+        *reinterpret_cast<uint32_t*>(dst + y * a.dstride + x) = v[k];
+      else
+        for (int i = x; i < w; i++) dst[y * a.dstride + i] = src[y * sstride + i];
+    }
     return;
   }
   for (int y = tid >> 5; y < h; y += 8)
-    for (int x = tid & 31; x < w; x += 32)
-      a.dst[(int64_t)(y0 + y) * a.dstride + x0 + x] = a.rec[(int64_t)(y0 + y) * a.rstride + x0 + x];
+    for (int x = tid & 31; x < w; x += 32) dst[(int64_t)y * a.dstride + x] = src[(int64_t)y * sstride + x];
 }
 
 static int lrs_check(const pf_frame* f, const pf_frame* ref) {

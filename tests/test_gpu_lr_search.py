@@ -126,3 +126,30 @@ def test_arguments_are_checked(runner):
         from goav1_b200.postfilter import check
 
         check(lib().pf_lr_search(None, C.byref(src.pf()), C.byref(rec.pf()), None, None, 0))
+
+
+@pytest.mark.parametrize("w,h", [(200, 136), (67, 72)])
+@pytest.mark.parametrize("off", [1, 2], ids=["odd", "even"])
+def test_rows_off_word_boundaries(runner, w, h, off):
+    """Source, reconstruction and output rows that start on no 4-sample
+    boundary: the units are read and written byte by byte."""
+    import torch
+
+    src, rec, _ = synth.make_lr_search_pair(21 + off, w, h)
+    want, out = _oracle(src, rec)
+    frames, keep = [], []
+    for fr, fill in ((src, True), (rec, True), (rec, False)):
+        f = fr.pf(memory=abi.PF_MEM_DEVICE, ptrs=[0, 0, 0])
+        for p, a in enumerate(fr.planes):
+            t = torch.zeros((a.shape[0], a.shape[1] + 3), dtype=torch.uint8, device="cuda")
+            if fill:
+                t[:, off:off + a.shape[1]] = torch.from_numpy(a).cuda()
+            keep.append(t)
+            f.plane[p].data, f.plane[p].stride = t.data_ptr() + off, t.stride(0)
+        frames.append(f)
+    torch.cuda.synchronize()
+    got = runner.lr_search(*frames)
+    _assert_units(want, got)
+    res = keep[6][:, off:].cpu().numpy()
+    assert np.array_equal(res[:h, :w], out.planes[0][:h, :w])
+    assert not res[h:].any() and not res[:, w:].any()
