@@ -61,7 +61,7 @@ namespace pf {
 // taps instead of 64 x 12, and the rest of a trial is one addition, the
 // rounding, the clamp and the squared error of four samples at a time.
 // Bound by the packed instructions themselves.  1080p: all 64 luma and 64
-// chroma trials 113 us, trial by trial with constrain() tables about 1,500;
+// chroma trials 107 us, trial by trial with constrain() tables about 1,500;
 // the learned search's few trials a block 54 us, then 178.
 //
 // What a sample does not count for is settled once, before the trials: an

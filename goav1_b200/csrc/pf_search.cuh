@@ -86,13 +86,9 @@ __device__ __forceinline__ uint64_t fb_listed(const SearchArgs& a, int fb, int l
 #pragma unroll
     for (int i = 0; i < 8; i++) word |= (uint64_t)a.noskip[(size_t)fb * 8 + i] << (8 * i);
   }
-  uint64_t listed = 0;
-  for (int r = 0; r < imin(a.miRows - lr, 16); r += 2)
-    for (int c = 0; c < imin(a.miCols - lc, 16); c += 2) {
-      const int b = (r >> 1) * 8 + (c >> 1);
-      listed |= word & (1ull << b);
-    }
-  return listed;
+  // The 8x8 blocks whose first cell is inside the MI grid.
+  const int rows = (imin(a.miRows - lr, 16) + 1) >> 1, cols = (imin(a.miCols - lc, 16) + 1) >> 1;
+  return word & (0x0101010101010101ull * ((1u << cols) - 1)) & (rows == 8 ? ~0ull : (1ull << (8 * rows)) - 1);
 }
 
 // cdef/direction.go:37-79 (partial sums) and :469-501 (cost), 8-bit samples

@@ -75,6 +75,28 @@ def test_features_match_oracle(runner, oracle, w, h, use_ns):
     assert np.allclose(Xg, Xo, rtol=4e-7, atol=1e-7), np.abs(Xg - Xo).max()
 
 
+@pytest.mark.parametrize("w,h", [(65, 66), (67, 129), (70, 72), (133, 75)])
+@pytest.mark.parametrize("off", [0, 1], ids=["words", "bytes"])
+def test_features_of_ragged_blocks(runner, oracle, w, h, off):
+    """Blocks of one to a few columns and rows, and planes whose rows start on
+    no 4-sample boundary; the tolerance of the other sizes (the sums are exact
+    integers, the logarithms two roundings)."""
+    import torch
+
+    _, rec, ns = _pair(runner, 41 + w, w, h)
+    f, keep = rec.pf(memory=abi.PF_MEM_DEVICE, ptrs=[0, 0, 0]), []
+    for p, a in enumerate(rec.planes):
+        t = torch.zeros((a.shape[0], a.shape[1] + 8), dtype=torch.uint8, device="cuda")
+        t[:, off:off + a.shape[1]] = torch.from_numpy(a).cuda()
+        keep.append(t)
+        f.plane[p].data, f.plane[p].stride = t.data_ptr() + off, t.stride(0)
+    torch.cuda.synchronize()
+    Xg = runner.cdef_features(f, ns, 90)
+    Xo = np.zeros_like(Xg)
+    assert oracle.oracle_cdef_features(C.byref(rec.pf()), ns.ctypes.data, 90, 0, Xo.ctypes.data) == 0
+    assert np.allclose(Xg, Xo, rtol=4e-7, atol=1e-7), np.abs(Xg - Xo).max()
+
+
 def test_forward_matches_oracle(runner, oracle):
     m, X, _ = _rand_model(1, 100)
     Pg = runner.mlp_forward(m, X)
