@@ -782,6 +782,7 @@ __device__ __forceinline__ uint32_t lrs_outcome(const LrsSmem& sm, uint8_t* keep
 }
 
 __global__ void __launch_bounds__(256, 4) k_lr_search_sse(LrsArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(16) uint8_t lrs_smem_raw[];
   LrsSmem& sm = *reinterpret_cast<LrsSmem*>(lrs_smem_raw);
   const int unit = blockIdx.x, job = blockIdx.y;
@@ -859,6 +860,7 @@ __global__ void __launch_bounds__(256, 4) k_lr_search_sse(LrsArgs a) {
 // The unit's decision (keyframe_lossy.go:2338-2382) and, with a.dst, the
 // unit filtered by it (:2422-2453).
 __global__ void __launch_bounds__(256) k_lr_search_decide(LrsArgs a) {
+  stage_begin();
   const int unit = blockIdx.x, tid = threadIdx.x;
   int x0, y0, x1, y1;
   lrs_rect(a, unit % a.horz, unit / a.horz, x0, y0, x1, y1);
@@ -1034,7 +1036,7 @@ extern "C" int pf_lr_search(pf_ctx* ctx, const pf_frame* source, const pf_frame*
     configured = true;
   }
   k_lr_search_sse<<<dim3(n, 1 + PF_LR_SGR_PRESETS), 256, sizeof(LrsSmem), st>>>(a);
-  k_lr_search_decide<<<n, 256, 0, st>>>(a);
+  if (launch_stage(k_lr_search_decide, n, 256, 0, st, true, a) != cudaSuccess) return PF_ERR_DEVICE;
   e = cudaGetLastError();
   if (e == cudaSuccess && host && restored)
     e = cudaMemcpy2DAsync(restored->plane[0].data, restored->plane[0].stride, a.dst, W, W, H,

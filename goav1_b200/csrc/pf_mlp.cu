@@ -139,6 +139,7 @@ __device__ __forceinline__ void feat_quad(const uint8_t* blk, int pitch, int w, 
 }
 
 __global__ void __launch_bounds__(256, 4) k_cdef_features(SearchArgs a, int qindex, float* X) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ FeatAcc A;
   __shared__ int32_t s_cost[64 * 8];
   __shared__ __align__(8) uint8_t s_y[64 * kFeatY];     // the filter block's luma (allocated part)
@@ -398,17 +399,23 @@ __global__ void k_mlp_expand(const pf_cdef_mlp* M, float* W) {
     W[p] = reinterpret_cast<const float*>(&M->feat_shift[0])[p - kNP];  // shift, then scale
 }
 
+// The network's fp32 weights and biases, contiguous like the tile's: 16-byte
+// copies.
+template <int TILE>
+__device__ __forceinline__ void mlp_load(MlpTileT<TILE>& T, const float* Wf) {
+  const float4* src = reinterpret_cast<const float4*>(Wf);
+  float4* dst = reinterpret_cast<float4*>(&T.w1[0]);
+  for (int e = threadIdx.x; e < kNP / 4; e += kMlpThreads) dst[e] = src[e];
+}
+
 template <int TILE>
 __device__ void mlp_forward(MlpTileT<TILE>& T, const pf_cdef_mlp* M, const float* X, const int* rows, int first, int count,
-                            const float* means = nullptr, const float* Wf = nullptr) {
+                            const float* means = nullptr, const float* Wf = nullptr, bool loaded = false) {
   const int t = threadIdx.x;
   const float* shift = M ? M->feat_shift : Wf + kNP;
   const float* scale = M ? M->feat_scale : Wf + kNP + kF;
   if (Wf) {
-    // fp32 weights and biases, contiguous like the tile's: 16-byte copies.
-    const float4* src = reinterpret_cast<const float4*>(Wf);
-    float4* dst = reinterpret_cast<float4*>(&T.w1[0]);
-    for (int e = t; e < kNP / 4; e += kMlpThreads) dst[e] = src[e];
+    if (!loaded) mlp_load(T, Wf);
   } else {
     for (int e = t; e < kNW1; e += kMlpThreads) T.w1[e] = bf16_to_f(M->w1[e]);
     for (int e = t; e < kNW2; e += kMlpThreads) T.w2[e] = bf16_to_f(M->w2[e]);
@@ -493,8 +500,13 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_masks(const float* W, const
   __shared__ uint64_t s_m[kInferTile][2];
   __shared__ int s_conf[kInferTile][2];
   const int first = blockIdx.x * kInferTile, count = imin(kInferTile, nfb - first);
+  // The weights do not wait for the features: they are copied while the
+  // kernel before drains.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  mlp_load(T, W);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   frame_means(X, nfb, FM);  // features 33..39 (the features kernel leaves them unset)
-  mlp_forward(T, nullptr, X, nullptr, first, count, FM.mean, W);
+  mlp_forward(T, nullptr, X, nullptr, first, count, FM.mean, W, true);
   mlp_softmax(T, false);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int task = warp; task < 2 * kInferTile; task += kMlpThreads / 32) {
@@ -714,10 +726,15 @@ cudaError_t launch_mlp_masks(const pf_cdef_mlp* dmodel, float* W, bool expand, c
     if (e != cudaSuccess) return e;
     ready = dev;
   }
-  if (expand) k_mlp_expand<<<(kExpanded + 255) / 256, 256, 0, st>>>(dmodel, W);
-  k_mlp_masks<<<(nfb + kInferTile - 1) / kInferTile, kMlpThreads, sizeof(MlpInfer), st>>>(W, X, nfb, threshold,
-                                                                                       candidates, masks);
-  return cudaGetLastError();
+  if (expand) {
+    k_mlp_expand<<<(kExpanded + 255) / 256, 256, 0, st>>>(dmodel, W);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  // Placed while the features kernel drains, except when the weights have just
+  // been queued.
+  return launch_stage(k_mlp_masks, (nfb + kInferTile - 1) / kInferTile, kMlpThreads, sizeof(MlpInfer), st, !expand, (const float*)W, X,
+                      nfb, threshold, candidates, masks);
 }
 
 }  // namespace pf

@@ -147,6 +147,7 @@ __device__ __forceinline__ uint32_t search_err(uint32_t y4, uint32_t s4, uint32_
 }
 
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(256, 3) k_cdef_search(SearchArgs a) {
+  stage_begin();
   __shared__ SearchSmem sm;
   cg::cluster_group cl = cg::this_cluster();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -493,6 +494,7 @@ __device__ int compact_blocks(const uint8_t* skip, int nfb, int* list, int* wsum
 // 64x64 block's SSE is below 2^28) are copied into shared memory.
 template <bool kRows>
 __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
+  stage_begin();
   extern __shared__ __align__(16) unsigned char smem[];
   SelShared& S = *reinterpret_cast<SelShared*>(smem);
   int* s_sb = reinterpret_cast<int*>(smem + sizeof(SelShared));  // [nfb] non-skip blocks
@@ -709,6 +711,7 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
 // RD choice of nb (finish, :914-931) and the per-block preset index.
 __global__ void __launch_bounds__(256) k_sel_finish(SelArgs a, int maxCfg, unsigned long long lambda, uint8_t* fbIndex,
                                                     FinishOut* fo) {
+  stage_begin();
   __shared__ int s_best, s_n;
   const SelOut* st = a.out;
   if (threadIdx.x == 0) s_n = 0;
@@ -773,12 +776,14 @@ size_t sel_smem_bytes(int nfb, bool rows) {
 }
 
 cudaError_t launch_search(const SearchArgs& a, cudaStream_t st) {
-  k_cdef_search<<<3 * a.nhfb * a.nvfb, 256, 0, st>>>(a);
-  return cudaGetLastError();
+  // After the mask kernel (tmask) the CTAs are placed while that one drains.
+  return launch_stage(k_cdef_search, 3 * a.nhfb * a.nvfb, 256, 0, st, a.tmask != nullptr, a);
 }
 
 // Launches k_sel_greedy with 16-CTA clusters when the device can place one
-// with this much shared memory, else with 8-CTA clusters.
+// with this much shared memory, else with 8-CTA clusters.  Not as a
+// programmatic dependent: its clusters, placed while the search drains, took
+// the exhaustive 1080p call from 260 to 300 us.
 template <bool kRows>
 static cudaError_t launch_greedy(const SelArgs& s, int maxCfg, size_t bytes, cudaStream_t st) {
   const void* fn = (const void*)k_sel_greedy<kRows>;
@@ -843,8 +848,7 @@ cudaError_t launch_select(SelArgs s, int maxCfg, unsigned long long lambda, uint
   if (bytes > kSelMaxSmem) return cudaErrorInvalidValue;
   const cudaError_t e = rows ? launch_greedy<true>(s, maxCfg, bytes, st) : launch_greedy<false>(s, maxCfg, bytes, st);
   if (e != cudaSuccess) return e;
-  k_sel_finish<<<imax(1, (s.nfb + 255) / 256), 256, 0, st>>>(s, maxCfg, lambda, fbIndex, fo);
-  return cudaGetLastError();
+  return launch_stage(k_sel_finish, imax(1, (s.nfb + 255) / 256), 256, 0, st, true, s, maxCfg, lambda, fbIndex, fo);
 }
 
 }  // namespace pf
