@@ -464,16 +464,15 @@ def measure_issue_peaks():
 
 
 # Per-frame counters of the batched chain kernels at the 1080p 8-bit 4:2:0
-# workload, from one ncu capture of a 60-frame launch of each kernel as the
-# autotuner sets them on this batch (deblocking 16x16 tiles, grain apply four
-# columns a thread; profiles/postfilter_chain_counters_1080p8_60frames.md has
+# workload, from one ncu capture of a 60-frame launch of each kernel under the
+# default schedule (profiles/postfilter_chain_counters_1080p8_60frames.md has
 # the command and the raw figures): DRAM bytes read + written and warp
 # instructions executed (deblocking: both passes).
 KERNEL_COUNTERS_1080P8 = {
-    "deblock": {"dram_bytes": (443.94e6 + 176.06e6) / 60, "warp_inst": 571.48e6 / 60},
-    "cdef": {"dram_bytes": (187.19e6 + 164.21e6) / 60, "warp_inst": 1097.56e6 / 60},
-    "restoration": {"dram_bytes": (205.87e6 + 152.76e6) / 60, "warp_inst": 943.62e6 / 60},
-    "film_grain": {"dram_bytes": (189.65e6 + 151.37e6) / 60, "warp_inst": 500.34e6 / 60},
+    "deblock": {"dram_bytes": (446.61e6 + 192.33e6) / 60, "warp_inst": 240.54e6 / 60},
+    "cdef": {"dram_bytes": (187.69e6 + 166.32e6) / 60, "warp_inst": 580.50e6 / 60},
+    "restoration": {"dram_bytes": (205.83e6 + 152.40e6) / 60, "warp_inst": 540.98e6 / 60},
+    "film_grain": {"dram_bytes": (189.61e6 + 143.97e6) / 60, "warp_inst": 288.63e6 / 60},
 }
 
 
@@ -634,7 +633,7 @@ def main():
         reset()
         step()
     torch.cuda.synchronize()
-    launches_per_step = 7  # one launch per stage for the whole batch
+    launches_per_step = 8  # one launch per stage for the whole batch, deblocking two, grain three
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
     dist.barrier(world)
     torch.cuda.synchronize()
