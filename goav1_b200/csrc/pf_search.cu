@@ -30,9 +30,12 @@
 //                   Bound by the barriers of a step, two of the cluster
 //                   among them, hence maxima by warp reductions of one
 //                   key and one thread's bookkeeping a step; 1080p: 303 us
-//                   with all 40 steps of 8 presets run, 127 ended early, 120
-//                   now; the learned search's 8 steps 62 and 57 (1,024
-//                   threads a CTA instead of 512: 152 and 75).
+//                   with all 40 steps of 8 presets run, 127 ended early, 95
+//                   now; the learned search's 8 steps 62 and 47 (1,024
+//                   threads a CTA instead of 512: 152 and 75).  Of a step's
+//                   11,500 cycles the partial savings take 4,800, handing
+//                   them over 2,600 (9,000 as 64-bit sums of eight
+//                   neighbouring pairs a thread).
 //   k_sel_finish    the RD choice of nb and the per-block preset index.
 #include <cooperative_groups.h>
 #include <string.h>
@@ -443,6 +446,7 @@ struct SelShared {
   // Partial savings of this CTA's slice of the pairs, a row from each CTA of
   // the cluster (first pick: this CTA's column sums).
   alignas(16) unsigned long long part[4096];
+  int narrow[kSelMaxCluster];  // whether a CTA's partial savings fit 32 bits
   unsigned long long cand[2][kSelMaxCluster];
   unsigned long long tot[kSelMaxCluster];  // rank 0's: every CTA's part of the total
   unsigned long long red[kSelThreads / 32];
@@ -535,12 +539,24 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
       s_rows[e] = (uint32_t)(pl ? M1 : M0)[(size_t)fb * 64 + j];
     }
   __syncthreads();
+  unsigned long long most = 0;
   for (int il = warp; il < cnt; il += kSelThreads / 32) {
-    const uint32_t m = __reduce_min_sync(~0u, min(row(il, 1, lane), row(il, 1, lane + 32)));
+    const uint32_t a0 = row(il, 1, lane), a1 = row(il, 1, lane + 32);
+    const uint32_t m = __reduce_min_sync(~0u, min(a0, a1));
     if (lane == 0) s_min1[il] = m;
+    // No block saves more than its largest SSEs (places past the trial list
+    // hold 2^31 - 1 and are never picked).
+    auto held = [](uint32_t v) { return v == kNotATrial ? 0u : v; };
+    most += __reduce_max_sync(~0u, max(held(a0), held(a1)));
+    most += __reduce_max_sync(~0u, max(held(row(il, 0, lane)), held(row(il, 0, lane + 32))));
   }
+  if (lane == 0) S.red[warp] = most;
   if (t < 8) S.lev0[t] = S.lev1[t] = 0;
   __syncthreads();
+  if (t < CS) {
+    most = 0;
+    for (int i = 0; i < kSelThreads / 32; i++) most += S.red[i];
+  }
   const int steps = a.refine ? 5 * nb : nb;
   int same = 0, drop0 = 0, drop1 = 0;  // thread 0's: refinement steps in a row that took back the pick they had dropped
   for (int k = 0; k < steps; k++) {
@@ -553,7 +569,8 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
         for (int il = 0; il < cnt; il++) s += row(il, t >> 6, t & 63);
         S.part[t] = s;
       }
-      cl.sync();
+      cl.sync();  // (the first: every CTA of the cluster has started)
+      if (t < CS) cl.map_shared_rank(&S, t)->narrow[rank] = most < 1ull << 32;
       if (t < 128) {
         unsigned long long s0 = 0, s1 = 0, s2 = 0, s3 = 0;
         for (int r = 0; r < CS; r += 4) {
@@ -581,10 +598,13 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
         s_best[il] = best;
       }
       __syncthreads();
-      // Partial savings of this CTA's blocks: thread t owns (j, k0..k0+7).
-      // A block saves below 2^29, so eight blocks sum exactly in 32 bits
-      // before joining the 64-bit totals.
-      const int j = t >> 3, k0 = (t & 7) * 8;
+      // Partial savings of this CTA's blocks: thread t owns (j, k) for the
+      // strengths k = 32 m + 4 (t & 7) + 0..3, so that eight neighbours' sums
+      // are 128 bytes of a row when they are handed over.  A block saves
+      // below 2^29, so eight blocks sum exactly in 32 bits before joining the
+      // 64-bit totals; all of them do where the CTA's narrow flag says so.
+      const bool narrow = S.narrow[rank];
+      const int j = t >> 3, k0 = (t & 7) * 4;
       unsigned long long acc[8];
       uint32_t acc32[8];
 #pragma unroll
@@ -599,16 +619,19 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
           const int rem = (int)(bi - a0);
           uint32_t v[8];
           if (kRows) {
-            const uint4* r4 = reinterpret_cast<const uint4*>(&s_rows[il * 128 + 64 + k0]);
-            const uint4 x = r4[0], y = r4[1];
-            v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+              const uint4 x = *reinterpret_cast<const uint4*>(&s_rows[il * 128 + 64 + 32 * m + k0]);
+              v[4 * m] = x.x, v[4 * m + 1] = x.y, v[4 * m + 2] = x.z, v[4 * m + 3] = x.w;
+            }
           } else {
 #pragma unroll
-            for (int q = 0; q < 8; q++) v[q] = row(il, 1, k0 + q);
+            for (int q = 0; q < 8; q++) v[q] = row(il, 1, 32 * (q >> 2) + k0 + (q & 3));
           }
 #pragma unroll
           for (int q = 0; q < 8; q++) acc32[q] += (uint32_t)__viaddmax_s32(-(int)v[q], rem, 0);
         }
+        if (narrow) continue;
 #pragma unroll
         for (int q = 0; q < 8; q++) {
           acc[q] += acc32[q];
@@ -619,10 +642,20 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
       // into their slice's CTA (rows of one sender each), so that only the
       // barrier is waited for and every read after it is local.
       {
-        const int e0 = t * 8, to = e0 / pairs;
-        ulonglong2* d = reinterpret_cast<ulonglong2*>(cl.map_shared_rank(&S.part[0], to) + rank * pairs + (e0 - to * pairs));
+        const int e0 = j * 64 + k0, to = e0 / pairs;
+        unsigned long long* d = cl.map_shared_rank(&S.part[0], to) + rank * pairs;  // the sender's row
+        const int at = e0 - to * pairs;
+        if (narrow) {
+          uint32_t* d32 = reinterpret_cast<uint32_t*>(d) + at;
 #pragma unroll
-        for (int q = 0; q < 4; q++) d[q] = make_ulonglong2(acc[2 * q], acc[2 * q + 1]);
+          for (int m = 0; m < 2; m++)
+            *reinterpret_cast<uint4*>(d32 + 32 * m) =
+                make_uint4(acc32[4 * m], acc32[4 * m + 1], acc32[4 * m + 2], acc32[4 * m + 3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 8; q += 2)
+            *reinterpret_cast<ulonglong2*>(d + at + 32 * (q >> 2) + (q & 3)) = make_ulonglong2(acc[q], acc[q + 1]);
+        }
       }
       cl.sync();
       // First maximum wins.  Two neighbouring threads share a pair.
@@ -632,7 +665,10 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
         unsigned long long sum = 0;
 #pragma unroll
         for (int r = 0; r < kSelMaxCluster / 2; r++)
-          if (r < (CS >> 1)) sum += S.part[(r0 + r) * pairs + e];
+          if (r < (CS >> 1)) {
+            const unsigned long long* from = &S.part[(r0 + r) * pairs];
+            sum += S.narrow[r0 + r] ? reinterpret_cast<const uint32_t*>(from)[e] : from[e];
+          }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         key = max(key, sel_key(sum, rank * pairs + e));
       }

@@ -64,6 +64,27 @@ def test_search_all_blocks_without_noskip(runner):
     assert list(r0.y_strength) == list(r1.y_strength) and r0.bits == r1.bits
 
 
+@pytest.mark.parametrize("blocks", ["all", "some"])
+def test_selection_of_sums_past_32_bits(runner, blocks):
+    """240 blocks, most of them as far from their source as samples go: a
+    cluster CTA's share of the savings no longer fits 32 bits and is handed
+    over in 64 ("some": of part of the CTAs only)."""
+    src, rec, _, _ = synth.make_search_pair(5, 1280, 768)
+    rng = np.random.default_rng(11)
+    for s, r in zip(src.planes, rec.planes):
+        far = rng.random(s.shape) < 0.5
+        rows = s.shape[0] if blocks == "all" else s.shape[0] // 2
+        r[:rows][far[:rows]] = 255
+        r[:rows][~far[:rows]] = 0
+        s[:rows] = 255 - r[:rows]
+    r0, m0, i0 = _oracle(src, rec, None, 128, 4000.0, 8)
+    r1, m1, i1 = runner.cdef_search(src.pf(), rec.pf(), None, 128, 4000.0)
+    assert m0.max(axis=2).sum(axis=0)[:15].sum() >= 1 << 32  # one CTA's 15 blocks
+    assert np.array_equal(m0, m1) and np.array_equal(i0, i1)
+    assert (r0.bits, r0.cost) == (r1.bits, r1.cost)
+    assert list(r0.y_strength) == list(r1.y_strength) and list(r0.uv_strength) == list(r1.uv_strength)
+
+
 def test_search_rejects_unsupported_formats(runner):
     from goav1_b200.postfilter import ErrUnsupportedPostFilter
 
