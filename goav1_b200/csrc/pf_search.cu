@@ -30,10 +30,11 @@
 //                   Bound by the barriers of a step, two of the cluster
 //                   among them, hence maxima by warp reductions of one
 //                   key and one thread's bookkeeping a step; 1080p: 303 us
-//                   with all 40 steps of 8 presets run, 127 ended early, 95
-//                   now; the learned search's 8 steps 62 and 47 (1,024
+//                   with all 40 steps of 8 presets run, 127 ended early, 84
+//                   now; the learned search's 8 steps 62 and 43 (1,024
 //                   threads a CTA instead of 512: 152 and 75).  Of a step's
-//                   11,500 cycles the partial savings take 4,800, handing
+//                   cycles the partial savings took 4,800 of 11,500 block by
+//                   block (two at a time now, chroma rows negated), handing
 //                   them over 2,600 (9,000 as 64-bit sums of eight
 //                   neighbouring pairs a thread).
 //   k_sel_finish    the RD choice of nb and the per-block preset index.
@@ -495,7 +496,8 @@ __device__ int compact_blocks(const uint8_t* skip, int nfb, int* list, int* wsum
 // One cluster per configuration nb = 1 << (blockIdx.x / cluster size); the
 // cluster size (16, or 8 where a 16-CTA cluster cannot be placed) is read at
 // run time.  kRows: the filter blocks' SSE rows (as 32-bit values; an 8-bit
-// 64x64 block's SSE is below 2^28) are copied into shared memory.
+// 64x64 block's SSE is below 2^28) are copied into shared memory, chroma's
+// negated.
 template <bool kRows>
 __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
   stage_begin();
@@ -528,7 +530,7 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
   const uint64_t* M0 = a.mse;
   const uint64_t* M1 = a.mse + (size_t)a.nfb * 64;
   auto row = [&](int il, int pl, int j) -> uint32_t {
-    if (kRows) return s_rows[il * 128 + pl * 64 + j];
+    if (kRows) return pl ? 0u - s_rows[il * 128 + 64 + j] : s_rows[il * 128 + j];
     const int fb = s_sb[i0 + il];
     return (uint32_t)(pl ? M1 : M0)[(size_t)fb * 64 + j];
   };
@@ -536,7 +538,8 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
     for (int e = t; e < cnt * 128; e += kSelThreads) {
       const int il = e >> 7, pl = (e >> 6) & 1, j = e & 63;
       const int fb = s_sb[i0 + il];
-      s_rows[e] = (uint32_t)(pl ? M1 : M0)[(size_t)fb * 64 + j];
+      const uint32_t v = (uint32_t)(pl ? M1 : M0)[(size_t)fb * 64 + j];
+      s_rows[e] = pl ? 0u - v : v;  // chroma's negated: a term of the savings as it stands
     }
   __syncthreads();
   unsigned long long most = 0;
@@ -611,25 +614,34 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_greedy(SelArgs a) {
       for (int q = 0; q < 8; q++) acc[q] = acc32[q] = 0;
       for (int il0 = 0; il0 < cnt; il0 += 8) {
         const int il1 = imin(cnt, il0 + 8);
-        for (int il = il0; il < il1; il++) {
-          const uint32_t bi = s_best[il], a0 = row(il, 0, j);
-          if (a0 + s_min1[il] >= bi) continue;  // no k can save anything
-          // Both are below 2^30 and a sentinel is 2^31 - 1, so the signed
-          // difference cannot overflow.
-          const int rem = (int)(bi - a0);
-          uint32_t v[8];
-          if (kRows) {
+        for (int il = il0; il < il1; il += 2) {
+          // Two blocks a pass (the odd last one twice, the second time with
+          // nothing left to save).
+          const int ih = imin(il + 1, cnt - 1);
+          const uint32_t b0 = s_best[il], b1 = s_best[ih], a0 = row(il, 0, j), a1 = row(ih, 0, j);
+          const bool on0 = a0 + s_min1[il] < b0, on1 = ih > il && a1 + s_min1[ih] < b1;
+          if (!on0 && !on1) continue;  // no k can save anything
+          // Saved so far without chroma.  Both are below 2^30 where on and a
+          // sentinel is 2^31 - 1, so no difference can overflow.
+          const int rem0 = on0 ? (int)(b0 - a0) : 0, rem1 = on1 ? (int)(b1 - a1) : 0;
+          uint32_t v0[8], v1[8];
+          auto load = [&](int i, uint32_t (&v)[8]) {
+            if (kRows) {
 #pragma unroll
-            for (int m = 0; m < 2; m++) {
-              const uint4 x = *reinterpret_cast<const uint4*>(&s_rows[il * 128 + 64 + 32 * m + k0]);
-              v[4 * m] = x.x, v[4 * m + 1] = x.y, v[4 * m + 2] = x.z, v[4 * m + 3] = x.w;
+              for (int m = 0; m < 2; m++) {
+                const uint4 x = *reinterpret_cast<const uint4*>(&s_rows[i * 128 + 64 + 32 * m + k0]);
+                v[4 * m] = x.x, v[4 * m + 1] = x.y, v[4 * m + 2] = x.z, v[4 * m + 3] = x.w;
+              }
+            } else {
+#pragma unroll
+              for (int q = 0; q < 8; q++) v[q] = 0u - row(i, 1, 32 * (q >> 2) + k0 + (q & 3));
             }
-          } else {
+          };
+          load(il, v0);
+          load(ih, v1);
 #pragma unroll
-            for (int q = 0; q < 8; q++) v[q] = row(il, 1, 32 * (q >> 2) + k0 + (q & 3));
-          }
-#pragma unroll
-          for (int q = 0; q < 8; q++) acc32[q] += (uint32_t)__viaddmax_s32(-(int)v[q], rem, 0);
+          for (int q = 0; q < 8; q++)
+            acc32[q] += (uint32_t)__viaddmax_s32((int)v0[q], rem0, 0) + (uint32_t)__viaddmax_s32((int)v1[q], rem1, 0);
         }
         if (narrow) continue;
 #pragma unroll
