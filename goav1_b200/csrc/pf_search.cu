@@ -30,8 +30,8 @@
 //                   Bound by the barriers of a step, two of the cluster
 //                   among them, hence maxima by warp reductions of one
 //                   key and one thread's bookkeeping a step; 1080p: 303 us
-//                   with all 40 steps of 8 presets run, 127 ended early, 84
-//                   now; the learned search's 8 steps 62 and 43 (1,024
+//                   with all 40 steps of 8 presets run, 127 ended early, 85
+//                   now; the learned search's 8 steps 62 and 42 (1,024
 //                   threads a CTA instead of 512: 152 and 75).  Of a step's
 //                   cycles the partial savings took 4,800 of 11,500 block by
 //                   block (two at a time now, chroma rows negated), handing

@@ -85,6 +85,22 @@ def test_selection_of_sums_past_32_bits(runner, blocks):
     assert list(r0.y_strength) == list(r1.y_strength) and list(r0.uv_strength) == list(r1.uv_strength)
 
 
+def test_selection_of_more_blocks_than_shared_memory_holds(runner):
+    """2,916 filter blocks, of which about 150 count: the SSE rows are read
+    from the table instead of shared memory."""
+    w = h = 3456
+    src, rec, _, _ = synth.make_search_pair(9, w, h)
+    rng = np.random.default_rng(2)
+    ns = np.zeros((54 * 54, 8), np.uint8)
+    ns[rng.random(54 * 54) < 0.05] = 0xFF
+    ns = ns.reshape(-1)
+    r0, m0, i0 = _oracle(src, rec, ns, 100, 2000.0, 8)
+    r1, m1, i1 = runner.cdef_search(src.pf(), rec.pf(), ns, 100, 2000.0)
+    assert np.array_equal(m0, m1) and np.array_equal(i0, i1)
+    assert (r0.bits, r0.cost) == (r1.bits, r1.cost)
+    assert list(r0.y_strength) == list(r1.y_strength) and list(r0.uv_strength) == list(r1.uv_strength)
+
+
 def test_search_rejects_unsupported_formats(runner):
     from goav1_b200.postfilter import ErrUnsupportedPostFilter
 
