@@ -476,7 +476,7 @@ __device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& d
     maxV = (kLuma ? 235 : (a.matrix_identity ? 235 : 240)) << (bd - 8);
   }
   const bool cfl = a.cfl, edge = x + 4 > sp.w;
-  const int oddCol = a.odd_luma ? sp.w - 1 - x : -1;  // the column whose luma has no right neighbour
+  const int oddCol = a.odd_luma ? sp.w - 1 - x : -1;  // the column whose luma has no right neighbour (4 and up: another quad's)
   const int lumaMult = a.luma_mult[plane] - 128, mult = a.mult[plane] - 128;
   const int offs0 = (a.offset[plane] << (bd - 8)) - (1 << bd);
   const int top = (1 << bd) - 1;
@@ -552,7 +552,7 @@ __device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& d
               const typename Q::W& lw = l[r][j >> 1];
               const int b0 = Q::get(lw, 2 * (j & 1)), b1 = Q::get(lw, 2 * (j & 1) + 1);
               avg = (b0 + b1 + 1) >> 1;
-              if (edge && j == oddCol) avg = b0;
+              if (j == oddCol) avg = b0;
             } else {
               avg = Q::get(l[r][0], j);
             }

@@ -4,6 +4,8 @@ depth, scaling from luma, restricted range, no overlap, inactive planes, and
 planes whose rows start on no word boundary.  Integer arithmetic: tolerance
 zero."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -83,3 +85,33 @@ def test_rows_off_word_boundaries(runner, bd, ss):
     for p, a in enumerate(want.planes):
         got = keep[1][p][:, 1:1 + a.shape[1]].cpu().numpy()
         assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
+
+
+@pytest.mark.parametrize("w", [7, 63, 71])
+@pytest.mark.parametrize("ss", [(1, 1), (1, 0)], ids=["420", "422"])
+@pytest.mark.parametrize("bd", [8, 10, 12])
+def test_last_chroma_column_without_a_right_luma_neighbour(runner, w, ss, bd):
+    """Odd widths whose chroma width is a multiple of four: the last quad ends
+    at the crop and its last column's scaling index is one luma sample's.  The
+    luma padding holds other values than the last column, and no border
+    extension makes it alike."""
+    import goav1_b200
+    from goav1_b200.postfilter import DeviceFrame
+
+    fr, si = synth.make_frame(1, 3 * w + bd, width=w, height=34, bit_depth=bd, ss=ss, stages=abi.PF_STAGE_FILM_GRAIN)
+    luma = fr.planes[0]
+    luma[:, w:] = ((1 << bd) - 1) - luma[:, w - 1:w]
+    for name, fields in OPTIONS.items():
+        saved = {k: getattr(si.side.fg, k) for k in fields}
+        for k, v in fields.items():
+            setattr(si.side.fg, k, v)
+        want, out, disp = oracle(fr, si), fr.copy(), fr.like()
+        runner.apply(out.pf(), si.side, disp.pf())
+        dev, still = DeviceFrame(fr), DeviceFrame(fr.like())
+        assert goav1_b200.lib().pf_film_grain_static(C.byref(dev.pf()), C.byref(si.side.fg), C.byref(still.pf()),
+                                                     None) == abi.PF_OK
+        for p, (a, b, c) in enumerate(zip(want.planes, disp.planes, still.download().planes)):
+            assert np.array_equal(a, b), "%s: plane %d differs in %d samples" % (name, p, int((a != b).sum()))
+            assert np.array_equal(a, c), "%s, static: plane %d differs in %d samples" % (name, p, int((a != c).sum()))
+        for k, v in saved.items():
+            setattr(si.side.fg, k, v)
