@@ -30,6 +30,11 @@
 
 namespace pf {
 
+// How a unit's samples are staged and filtered: fp16 pairs (8 bits, 10-bit
+// words of at most 10 bits), packed 16-bit integers (words of at most 12
+// bits), one by one in 32-bit integers.
+enum CdefForm { kPairs, kInts, kWide };
+
 // What a luma block's filter needs, made once per block: the primary tap's
 // constants (PairTap) and flags: bit 31 filtered, bit 4 odd strength (weights 3, 3
 // instead of 4, 2), low bits the direction.
@@ -68,7 +73,7 @@ struct Quad<uint8_t> {
   static __device__ __forceinline__ uint32_t pair(W a, W b) {
     return __byte_perm(a, b, 0x0400 + 0x0101 * k) & 0x00ff00ffu;
   }
-  static __device__ __forceinline__ uint32_t over(W) { return 0; }
+  static __device__ __forceinline__ uint32_t bits(W) { return 0; }
 };
 template <>
 struct Quad<uint16_t> {
@@ -82,8 +87,7 @@ struct Quad<uint16_t> {
   static __device__ __forceinline__ uint32_t pair(W a, W b) {
     return __byte_perm(k < 2 ? a.x : a.y, k < 2 ? b.x : b.y, k & 1 ? 0x7632 : 0x5410);
   }
-  // Bits that a sample of 10 bits does not have.
-  static __device__ __forceinline__ uint32_t over(W a) { return (a.x | a.y) & 0xfc00fc00u; }
+  static __device__ __forceinline__ uint32_t bits(W a) { return a.x | a.y; }
 };
 
 // One plane of a unit: where its samples are and what of them there is.
@@ -134,11 +138,11 @@ __device__ __forceinline__ void stage_load(const CdefPlane& p, const uint8_t* sr
   }
 }
 
-// kRaw: plain integers instead of biased fp16 values.
-template <typename T, bool kIn, bool kRaw, int kPitch>
+// Pairs as biased fp16 values, the other forms as plain integers.
+template <typename T, bool kIn, CdefForm kForm, int kPitch>
 __device__ __forceinline__ void stage_store(const CdefPlane& p, int d, int cg, const typename Quad<T>::W (&v)[3],
                                             uint32_t* buf) {
-  constexpr uint32_t kBias = kRaw ? 0u : kPairBias, kNone = kRaw ? kPairRawNone : kPairNone;
+  constexpr uint32_t kBias = kForm == kPairs ? kPairBias : 0u, kNone = kForm == kPairs ? kPairNone : kPairRawNone;
   uint32_t* o = buf + 2 * d * kPitch + 4 * cg;
 #pragma unroll
   for (int j = 0; j < 2; j++) {
@@ -158,13 +162,15 @@ __device__ __forceinline__ void stage_store(const CdefPlane& p, int d, int cg, c
   }
 }
 
-template <typename T>
+// Bits that no sample of the form has.
+template <typename T, CdefForm kForm>
 __device__ __forceinline__ uint32_t stage_over(const typename Quad<T>::W (&v)[3]) {
-  return Quad<T>::over(v[0]) | Quad<T>::over(v[1]) | Quad<T>::over(v[2]);
+  constexpr uint32_t kOver = kForm == kPairs ? 0xfc00fc00u : kForm == kInts ? 0xf000f000u : 0u;
+  return (Quad<T>::bits(v[0]) | Quad<T>::bits(v[1]) | Quad<T>::bits(v[2])) & kOver;
 }
 
 // One plane's tasks one by one, any unit.
-template <typename T, bool kRaw, int kPitch>
+template <typename T, CdefForm kForm, int kPitch>
 __device__ __forceinline__ uint32_t stage_any(const CdefPlane& p, const uint8_t* src, uint32_t* buf) {
   const int cgs = (p.w + 8) >> 2;
   const uint32_t inv = (65536u + (uint32_t)cgs - 1) / (uint32_t)cgs;  // i / cgs for i < 612
@@ -175,8 +181,8 @@ __device__ __forceinline__ uint32_t stage_any(const CdefPlane& p, const uint8_t*
     typename Quad<T>::W t[3];
     const int d = (int)((i * inv) >> 16), cg = i - d * cgs;
     stage_load<T, false>(p, src, d, cg, t);
-    if (!kRaw) over |= stage_over<T>(t);
-    stage_store<T, false, kRaw, kPitch>(p, d, cg, t, buf);
+    over |= stage_over<T, kForm>(t);
+    stage_store<T, false, kForm, kPitch>(p, d, cg, t, buf);
   }
   return over;
 }
@@ -185,7 +191,7 @@ __device__ __forceinline__ uint32_t stage_any(const CdefPlane& p, const uint8_t*
 // the CTA and warps 0-3 of the third; 2 x (10 x 18) chroma tasks follow on
 // warps 4-7 and in a fourth.  All of a thread's loads are in flight together.
 // kIn: a whole 64x64 unit with its halo inside the frame.
-template <typename T, bool kIn, bool kRaw>
+template <typename T, bool kIn, CdefForm kForm>
 __device__ __forceinline__ uint32_t stage_420(const CdefPlane& P, const CdefPlane& Q, const uint8_t* vsrc, bool y,
                                               bool c, CdefSmem& sm) {
   const int tid = threadIdx.x;
@@ -217,11 +223,11 @@ __device__ __forceinline__ uint32_t stage_420(const CdefPlane& P, const CdefPlan
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     if (!on[k]) continue;
-    if (!kRaw) over |= stage_over<T>(t[k]);
+    over |= stage_over<T, kForm>(t[k]);
     if (k == 3 || (k == 2 && c2))
-      stage_store<T, kIn, kRaw, kPC>(Q, d[k], cg[k], t[k], sm.c[i[k] >= 180]);
+      stage_store<T, kIn, kForm, kPC>(Q, d[k], cg[k], t[k], sm.c[i[k] >= 180]);
     else
-      stage_store<T, kIn, kRaw, kPW>(P, d[k], cg[k], t[k], sm.y);
+      stage_store<T, kIn, kForm, kPW>(P, d[k], cg[k], t[k], sm.y);
   }
   return over;
 }
@@ -230,7 +236,7 @@ __device__ __forceinline__ uint32_t stage_420(const CdefPlane& P, const CdefPlan
 // at a time, so that a block's parameters are read once per block.  c: the
 // run's first word; o: its first output sample; blk(k): the run's k-th
 // block's parameters.
-template <typename T, bool kRaw, bool kPri, bool kSec, int kBh, class B>
+template <typename T, CdefForm kForm, bool kPri, bool kSec, int kBh, class B>
 __device__ __forceinline__ void filter_run(const uint32_t* c, int pitch, const int2* ofs, uint8_t* o, int64_t os,
                                            int rows, const PairTap& st, B blk) {
 #pragma unroll 1
@@ -244,30 +250,36 @@ __device__ __forceinline__ void filter_run(const uint32_t* c, int pitch, const i
     for (int y = 0; y < kBh; y += 2, c += 2 * pitch, o += 2 * os) {
       uint32_t v = c[0];
       if (filt) {
-        if (!kRaw) {
+        if (kForm == kPairs) {
           v = pair_filter<kPri, kSec>(c, b.pri, w0, w1, st, po, s0, s1);
-        } else {
+        } else if (kForm == kInts) {
           v = pair_filter_ints<kPri, kSec>(c, b.pri, odd ? 3 : 4, odd ? 3 : 2, st, po, s0, s1);
+        } else {
+          v = pair_filter_wide<kPri, kSec>(c, b.pri, odd ? 3 : 4, odd ? 3 : 2, st, po, s0, s1);
         }
       }
-      if (sizeof(T) == 2 && !kRaw) v &= 0x03ff03ffu;
+      if (sizeof(T) == 2 && kForm == kPairs) v &= 0x03ff03ffu;
       *reinterpret_cast<T*>(o) = (T)v;
       *reinterpret_cast<T*>(o + os) = (T)(v >> 16);
     }
   }
 }
 
-template <typename T, bool kRaw, int kBh, class B>
+template <CdefForm kForm>
+__device__ __forceinline__ PairTap cdef_tap(int thr, int shift) {
+  return kForm == kPairs ? pair_tap(thr, shift) : kForm == kInts ? pair_tap_ints(thr, shift) : pair_tap_wide(thr, shift);
+}
+
+template <typename T, CdefForm kForm, int kBh, class B>
 __device__ __forceinline__ void filter_plane(const uint32_t* c, int pitch, const int2* ofs, uint8_t* o, int64_t os,
                                              int rows, int pri, int sec, int damping, B blk) {
-  const int secShift = constrain_shift(sec, damping);
-  const PairTap st = kRaw ? pair_tap_ints(sec, secShift) : pair_tap(sec, secShift);
+  const PairTap st = cdef_tap<kForm>(sec, constrain_shift(sec, damping));
   if (pri && sec)
-    filter_run<T, kRaw, true, true, kBh>(c, pitch, ofs, o, os, rows, st, blk);
+    filter_run<T, kForm, true, true, kBh>(c, pitch, ofs, o, os, rows, st, blk);
   else if (pri)
-    filter_run<T, kRaw, true, false, kBh>(c, pitch, ofs, o, os, rows, st, blk);
+    filter_run<T, kForm, true, false, kBh>(c, pitch, ofs, o, os, rows, st, blk);
   else
-    filter_run<T, kRaw, false, true, kBh>(c, pitch, ofs, o, os, rows, st, blk);
+    filter_run<T, kForm, false, true, kBh>(c, pitch, ofs, o, os, rows, st, blk);
 }
 
 // The four rows b-2 .. b+1 around the restoration stripe boundary
@@ -300,15 +312,15 @@ __device__ __forceinline__ void cdef_save_lines(const CdefArgs& a, const DPlane&
 // instructions spends its time on.  Other layouts' chroma is as large as
 // luma or half of it and takes luma's place in shared memory, plane by
 // plane.  Starts at plane `plane` (0 for k420) and returns 3, or the plane it
-// stopped at, before writing it, because a 10-bit sample there has more than
-// 10 bits (kRaw off); the raw form takes over from that plane.
-template <typename T, bool kRaw, bool k420>
+// stopped at, before writing it, because a sample there has more bits than the
+// form takes; the next form goes on from that plane.
+template <typename T, CdefForm kForm, bool k420>
 __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int plane, CdefSmem& sm) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const CdefArgs& a = J.cdef;
   const int ssx = k420 ? 1 : J.io.ssx, ssy = k420 ? 1 : J.io.ssy;
-  const int coeffShift = sizeof(T) == 1 ? 0 : (kRaw ? J.io.bd - 8 : 2);
-  constexpr uint32_t kSample = kRaw ? 0xffffu : 0x3ffu;
+  const int coeffShift = sizeof(T) == 1 ? 0 : (kForm == kPairs ? 2 : J.io.bd - 8);
+  constexpr uint32_t kSample = kForm == kPairs ? 0x3ffu : 0xffffu;
   if (tid < 24) sm.ofs[tid / 12][tid % 12] = make_int2(pair_off(tid % 12, 0, tid < 12 ? kPW : kPC),
                                                        pair_off(tid % 12, 1, tid < 12 ? kPW : kPC));
   // ---- what the unit filters, postfilter_cdef.go:936-956 ----
@@ -360,22 +372,22 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
       Q.words &= ((reinterpret_cast<uintptr_t>(vsrc) | (uintptr_t)J.io.pl[2].stride) & (4 * sizeof(T) - 1)) == 0;
       Q.words &= J.io.pl[2].stride == Q.stride;
       if (P.inside && P.words && Q.inside && Q.words && P.w == 64 && P.h == 64 && actY && actC) {
-        over = stage_420<T, true, kRaw>(P, Q, vsrc, true, true, sm);
+        over = stage_420<T, true, kForm>(P, Q, vsrc, true, true, sm);
       } else if (J.io.pl[2].stride == Q.stride) {
-        over = stage_420<T, false, kRaw>(P, Q, vsrc, actY, actC, sm);
+        over = stage_420<T, false, kForm>(P, Q, vsrc, actY, actC, sm);
       } else {
-        if (actY) over |= stage_any<T, kRaw, kPW>(P, P.src, sm.y);
+        if (actY) over |= stage_any<T, kForm, kPW>(P, P.src, sm.y);
         if (actC) {
-          over |= stage_any<T, kRaw, kPC>(Q, Q.src, sm.c[0]);
+          over |= stage_any<T, kForm, kPC>(Q, Q.src, sm.c[0]);
           CdefPlane V = Q;
           V.stride = J.io.pl[2].stride;
-          over |= stage_any<T, kRaw, kPC>(V, vsrc, sm.c[1]);
+          over |= stage_any<T, kForm, kPC>(V, vsrc, sm.c[1]);
         }
       }
     } else if (actP) {
-      over = stage_any<T, kRaw, kPW>(P, P.src, sm.y);
+      over = stage_any<T, kForm, kPW>(P, P.src, sm.y);
     }
-    if (sizeof(T) == 1 || kRaw)
+    if (sizeof(T) == 1 || kForm == kWide)
       __syncthreads();
     else if (__syncthreads_or((int)(over != 0)))
       return plane;
@@ -384,9 +396,14 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
       // A pair of warps takes two directions of the 64 blocks, so a warp
       // runs one code without divergence.
       const int b = tid & 63;
-      if ((listed >> b) & 1)
-        dir_costs_vert(tid >> 6, &sm.y[(2 + (b >> 3) * 8) * kPW + kPX + (b & 7) * 8], kRaw ? coeffShift : (sizeof(T) == 1 ? 0 : 2),
-                       kRaw ? (0xffffu >> coeffShift) * 0x10001u : 0x00ff00ffu, &sm.cost[b * 8]);
+      const uint32_t* blk = &sm.y[(2 + (b >> 3) * 8) * kPW + kPX + (b & 7) * 8];
+      if (!((listed >> b) & 1)) {
+      } else if (kForm == kWide) {
+        for (int d = tid >> 6; d < 8; d += 4) sm.cost[b * 8 + d] = dir_cost_wide_any(d, blk, coeffShift);
+      } else {
+        dir_costs_vert(tid >> 6, blk, kForm == kInts ? coeffShift : (sizeof(T) == 1 ? 0 : 2),
+                       kForm == kInts ? (0xffffu >> coeffShift) * 0x10001u : 0x00ff00ffu, &sm.cost[b * 8]);
+      }
       __syncthreads();
     }
     // ---- block parameters (cdef/filter.go:490-543): the adjusted luma
@@ -416,9 +433,8 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
       sm.dir[tid] = (uint8_t)best;
       // lumaAdjust holds whenever ypri is not zero: needDir does then.
       const int strength = ypri ? adjust_strength(ypri, var) : 0;
-      const int shift = constrain_shift(strength, ydamp);
       CdefBlk blk;
-      blk.pri = kRaw ? pair_tap_ints(strength, shift) : pair_tap(strength, shift);
+      blk.pri = cdef_tap<kForm>(strength, constrain_shift(strength, ydamp));
       blk.flags = (strength | ysec ? 1u << 31 : 0u) | (((strength >> coeffShift) & 1) << 4) | (ypri ? best : 0);
       sm.blk[tid] = blk;
     } else if (!k420 && plane == 1 && actC && cpri && ssx != ssy && tid < 64 && ((listed >> tid) & 1)) {
@@ -437,7 +453,7 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
         const int64_t os = J.scr.pl[0].stride;
         const int tx = tid & 63, ya = (tid >> 6) * 16, rows = imin(16, P.h - ya);
         if (tx < P.w && rows > 0)
-          filter_plane<T, kRaw, 8>(&sm.y[(2 + ya) * kPW + kPX + tx], kPW, sm.ofs[0],
+          filter_plane<T, kForm, 8>(&sm.y[(2 + ya) * kPW + kPX + tx], kPW, sm.ofs[0],
                                    ob + (int64_t)(P.y + ya) * os + (int64_t)(P.x + tx) * (int)sizeof(T), os, rows, ypri,
                                    ysec, ydamp, [&](int k) {
                                      const int b = ((ya >> 3) + k) * 8 + (tx >> 3);
@@ -450,9 +466,8 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
       }
     }
     if (k420 ? nplanes > 1 : plane > 0) {
-      const int cshift = constrain_shift(cpri, cdamp);
       CdefBlk cb;
-      cb.pri = kRaw ? pair_tap_ints(cpri, cshift) : pair_tap(cpri, cshift);
+      cb.pri = cdef_tap<kForm>(cpri, constrain_shift(cpri, cdamp));
       cb.flags = 1u << 31 | (((cpri >> coeffShift) & 1) << 4);
       auto chroma_blk = [&](int b) {
         CdefBlk r = cb;
@@ -469,7 +484,7 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
           copy_block<T>(J.io.pl[1], J.scr.pl[1], Q.x, Q.x + Q.w, Q.y, Q.y + Q.h);
           copy_block<T>(J.io.pl[2], J.scr.pl[2], Q.x, Q.x + Q.w, Q.y, Q.y + Q.h);
         } else if (lane < Q.w && rows > 0) {
-          filter_plane<T, kRaw, 4>(&sm.c[pl - 1][(2 + ya) * kPC + kPX + lane], kPC, sm.ofs[1],
+          filter_plane<T, kForm, 4>(&sm.c[pl - 1][(2 + ya) * kPC + kPX + lane], kPC, sm.ofs[1],
                                    ob + (int64_t)(Q.y + ya) * os + (int64_t)(Q.x + lane) * (int)sizeof(T), os, rows,
                                    cpri, csec, cdamp,
                                    [&](int k) { return chroma_blk(((ya >> 2) + k) * 8 + (lane >> 2)); });
@@ -486,9 +501,9 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
         if (tx < P.w && rows > 0) {
           auto at = [&](int k) { return chroma_blk(((ya >> (3 - ssy)) + k) * 8 + (tx >> (3 - ssx))); };
           if (ssy)
-            filter_plane<T, kRaw, 4>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, at);
+            filter_plane<T, kForm, 4>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, at);
           else
-            filter_plane<T, kRaw, 8>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, at);
+            filter_plane<T, kForm, 8>(c, kPW, sm.ofs[0], o, os, rows, cpri, csec, cdamp, at);
         }
       }
     }
@@ -512,17 +527,16 @@ __device__ __forceinline__ int cdef_unit(const FrameJob& J, int uc, int ur, int 
 
 // The unit from plane `plane` on, with samples staged as integers: 12-bit
 // frames, and 10-bit ones that hold longer samples.
-__device__ __noinline__ void cdef_unit_raw(const FrameJob* J, int uc, int ur, int plane, CdefSmem* sm) {
-  if (J->io.ssx && J->io.ssy)
-    cdef_unit<uint16_t, true, true>(*J, uc, ur, plane, *sm);
-  else
-    cdef_unit<uint16_t, true, false>(*J, uc, ur, plane, *sm);
+template <CdefForm kForm>
+__device__ __noinline__ int cdef_unit_ints(const FrameJob* J, int uc, int ur, int plane, CdefSmem* sm) {
+  if (J->io.ssx && J->io.ssy) return cdef_unit<uint16_t, kForm, true>(*J, uc, ur, plane, *sm);
+  return cdef_unit<uint16_t, kForm, false>(*J, uc, ur, plane, *sm);
 }
 
 // 4:2:2, 4:4:4 and 4:4:0.
 template <typename T>
 __device__ __noinline__ int cdef_unit_planes(const FrameJob* J, int uc, int ur, CdefSmem* sm) {
-  return cdef_unit<T, false, false>(*J, uc, ur, 0, *sm);
+  return cdef_unit<T, kPairs, false>(*J, uc, ur, 0, *sm);
 }
 
 __device__ __forceinline__ void cdef_item(const FrameJob& J, int local, CdefSmem& sm) {
@@ -530,14 +544,15 @@ __device__ __forceinline__ void cdef_item(const FrameJob& J, int local, CdefSmem
   const bool c420 = J.io.ssx && J.io.ssy;
   if (J.io.bd == 8) {
     if (c420)
-      cdef_unit<uint8_t, false, true>(J, uc, ur, 0, sm);
+      cdef_unit<uint8_t, kPairs, true>(J, uc, ur, 0, sm);
     else
       cdef_unit_planes<uint8_t>(&J, uc, ur, &sm);
   } else {
     int from = 0;
     if (J.io.bd == 10)
-      from = c420 ? cdef_unit<uint16_t, false, true>(J, uc, ur, 0, sm) : cdef_unit_planes<uint16_t>(&J, uc, ur, &sm);
-    if (from < 3) cdef_unit_raw(&J, uc, ur, from, &sm);
+      from = c420 ? cdef_unit<uint16_t, kPairs, true>(J, uc, ur, 0, sm) : cdef_unit_planes<uint16_t>(&J, uc, ur, &sm);
+    if (from < 3) from = cdef_unit_ints<kInts>(&J, uc, ur, from, &sm);
+    if (from < 3) cdef_unit_ints<kWide>(&J, uc, ur, from, &sm);
   }
 }
 

@@ -26,7 +26,9 @@ constexpr int kVeryLarge = 0x4000;
 // exactly: the result is the same integer as the reference's
 // (tests/test_cdef_pair_arithmetic.py runs through every difference,
 // strength and shift).  12-bit samples do not fit: they are staged as plain
-// integers (absent: kVeryLarge) and filtered by packed 16-bit integers.
+// integers (absent: kVeryLarge) and filtered by packed 16-bit integers.  Words
+// that hold more than 12 bits, which no bitstream has, are staged the same way
+// and filtered one by one in 32-bit integers.
 constexpr int kPH = 68;  // rows -2 .. 65 of a unit
 constexpr int kPX = 4;   // words left of the unit's first column
 constexpr int kPW = 96;  // words a row: a multiple of the 32 banks, so a tap's row offset moves no lane's bank
@@ -140,6 +142,27 @@ __host__ __device__ constexpr int dir_count(int D, int k) {
   return n;
 }
 
+// The cost of a direction's partial sums (direction.go:469-501).
+template <int D>
+__host__ __device__ __forceinline__ int32_t dir_cost_sums(const int32_t (&p)[15]) {
+  if (D == 2 || D == 6) {
+    int32_t s = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) s += p[i] * p[i];
+    return s * 105;
+  }
+  if (D == 0 || D == 4) {
+    const int32_t div[8] = {840, 420, 280, 210, 168, 140, 120, 105};
+    int32_t s = 0;
+#pragma unroll
+    for (int i = 0; i < 7; i++) s += (p[i] * p[i] + p[14 - i] * p[14 - i]) * div[i];
+    return s + p[7] * p[7] * 105;
+  }
+  return (p[3] * p[3] + p[4] * p[4] + p[5] * p[5] + p[6] * p[6] + p[7] * p[7]) * 105 +
+         (p[0] * p[0] + p[10] * p[10]) * 420 + (p[1] * p[1] + p[9] * p[9]) * 210 +
+         (p[2] * p[2] + p[8] * p[8]) * 140;
+}
+
 // The direction cost on packed sample pairs: w[i][m] holds samples (i, 2m) and
 // (i, 2m + 1) of the block in its low and high halves, shifted to 8 bits.  Each pair is
 // added as one 32-bit word into the accumulator of its even sample's index
@@ -148,8 +171,8 @@ __host__ __device__ constexpr int dir_count(int D, int k) {
 // by +128: a half never sums more than eight values below 256, so it never
 // carries into the other.  The halves are then split into the partial sums,
 // the bias taken off by each sum's sample count, and the cost formed from
-// them (direction.go:469-501), so the result is the same integer as summing
-// the shifted, unbiased samples one by one.
+// them, so the result is the same integer as summing the shifted, unbiased
+// samples one by one.
 template <int D>
 __host__ __device__ __forceinline__ int32_t dir_cost_pairs(const uint32_t (&w)[8][4]) {
   constexpr int kDelta = dir_k(D, 0, 1) - dir_k(D, 0, 0);
@@ -167,22 +190,7 @@ __host__ __device__ __forceinline__ int32_t dir_cost_pairs(const uint32_t (&w)[8
     if (k - kDelta >= 0 && k - kDelta < 15) v += (int32_t)(acc[k - kDelta] >> 16);
     p[k] = v - 128 * dir_count(D, k);
   }
-  if (D == 2 || D == 6) {
-    int32_t s = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) s += p[i] * p[i];
-    return s * 105;
-  }
-  if (D == 0 || D == 4) {
-    const int32_t div[8] = {840, 420, 280, 210, 168, 140, 120, 105};
-    int32_t s = 0;
-#pragma unroll
-    for (int i = 0; i < 7; i++) s += (p[i] * p[i] + p[14 - i] * p[14 - i]) * div[i];
-    return s + p[7] * p[7] * 105;
-  }
-  return (p[3] * p[3] + p[4] * p[4] + p[5] * p[5] + p[6] * p[6] + p[7] * p[7]) * 105 +
-         (p[0] * p[0] + p[10] * p[10]) * 420 + (p[1] * p[1] + p[9] * p[9]) * 210 +
-         (p[2] * p[2] + p[8] * p[8]) * 140;
+  return dir_cost_sums<D>(p);
 }
 
 // Two of the eight direction costs of a block staged as vertical pairs (blk:
@@ -301,6 +309,68 @@ __device__ __forceinline__ uint32_t pair_filter_ints(const uint32_t* c, const Pa
   uint32_t y = __viaddmax_s16x2(x + add + kOne, ~sub, kLeast);
   if (kPri && kSec) y = __vmins2(__vmaxs2(y, lo), hi);
   return y;
+}
+
+// The same one sample after the other in 32-bit integers, for any 16-bit
+// samples, with absent ones as the reference has them: a tap of kVeryLarge
+// that the clamp's maximum masks.  Packed integers cannot hold the differences
+// of samples of 0x4000 and more, nor tell them from an absent one; the line
+// lies at 12 bits, far enough below that no absent tap counts.  8 x 4K at 12
+// bits with such a sample in every unit: 166 us a frame (91 without).
+__device__ __forceinline__ PairTap pair_tap_wide(int thr, int shift) { return PairTap{(uint32_t)thr, (uint32_t)shift, 0}; }
+
+template <bool kPri, bool kSec>
+__device__ __forceinline__ uint32_t pair_filter_wide(const uint32_t* c, const PairTap& pri, int w0, int w1,
+                                                     const PairTap& sec, int2 po, int2 s0, int2 s1) {
+  uint32_t y2 = 0;
+#pragma unroll 1
+  for (int h = 0; h < 32; h += 16) {
+    const int x = (c[0] >> h) & 0xffff;
+    int lo = x, hi = x;
+    auto tap = [&](int o, const PairTap& t) {
+      const int v = (c[o] >> h) & 0xffff, d = v - x, m = abs(d);
+      lo = imin(lo, v);
+      hi = imax(hi, v & (kVeryLarge - 1));
+      const int l = imin(imax((int)t.k - (m >> t.m), 0), m);
+      return d < 0 ? -l : l;
+    };
+    int sum = 0;
+    if (kPri) sum += w0 * (tap(po.x, pri) + tap(-po.x, pri)) + w1 * (tap(po.y, pri) + tap(-po.y, pri));
+    if (kSec)
+      sum += 2 * (tap(s0.x, sec) + tap(-s0.x, sec) + tap(s1.x, sec) + tap(-s1.x, sec)) + tap(s0.y, sec) +
+             tap(-s0.y, sec) + tap(s1.y, sec) + tap(-s1.y, sec);
+    int y = x + ((8 + sum - (sum < 0)) >> 4);
+    // By the block's own strength: a masked sample can lie outside its taps' range.
+    if (kPri && kSec && pri.k) y = imin(imax(y, lo), hi);
+    y2 |= (uint32_t)(y & 0xffff) << h;
+  }
+  return y2;
+}
+
+// One direction's cost of a block staged as vertical pairs, any samples.
+template <int D>
+__device__ __forceinline__ int32_t dir_cost_wide(const uint32_t* blk, int shift) {
+  int32_t p[15];
+#pragma unroll
+  for (int k = 0; k < 15; k++) p[k] = -128 * dir_count(D, k);
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) p[dir_k(D, i, j)] += (int32_t)((blk[i * kPW + j] & 0xffffu) >> shift);
+  return dir_cost_sums<D>(p);
+}
+
+__device__ __forceinline__ int32_t dir_cost_wide_any(int d, const uint32_t* blk, int shift) {
+  switch (d) {
+    case 0: return dir_cost_wide<0>(blk, shift);
+    case 1: return dir_cost_wide<1>(blk, shift);
+    case 2: return dir_cost_wide<2>(blk, shift);
+    case 3: return dir_cost_wide<3>(blk, shift);
+    case 4: return dir_cost_wide<4>(blk, shift);
+    case 5: return dir_cost_wide<5>(blk, shift);
+    case 6: return dir_cost_wide<6>(blk, shift);
+    default: return dir_cost_wide<7>(blk, shift);
+  }
 }
 
 }  // namespace pf

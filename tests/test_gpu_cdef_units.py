@@ -76,3 +76,35 @@ def test_rows_off_word_boundaries(runner, bd, ss):
     for p, a in enumerate(ref.planes):
         got = keep[p][:, 1:1 + a.shape[1]].cpu().numpy()
         assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
+
+
+@pytest.mark.parametrize("plane", [0, 1, 2])
+@pytest.mark.parametrize("ss", [(1, 1), (1, 0), (0, 0)], ids=["420", "422", "444"])
+@pytest.mark.parametrize("bd", [10, 12])
+def test_samples_longer_than_twelve_bits(runner, plane, ss, bd):
+    """16-bit words that hold more than 12 bits, in units with and without a
+    frame border.  Luma's stay where the direction costs of a block with one
+    of them fit 32 bits; with secondary strengths only, and in chroma, which
+    have no direction search of their own, they take the whole range."""
+    for secondary in (False, True):
+        fr, si = synth.make_frame(1, 31 + plane, width=264, height=200, bit_depth=bd, ss=ss, stages=STAGES)
+        whole = secondary or plane > 0
+        if secondary:
+            for i in range(8):
+                si.side.cdef.y_strength[i] = 1 + i % 3
+                si.side.cdef.uv_strength[i] = 1 + (i + 1) % 3
+        rng = np.random.default_rng([plane, bd])
+        px = fr.planes[plane]
+        at = rng.random(px.shape) < (0.02 if whole else 0.002)
+        n = int(at.sum())
+        if whole:
+            long = rng.integers(1 << 12, 1 << 16, size=n)
+            edge = rng.integers(0x3f00, 0x4100, size=n)  # around the value that stands for an absent sample
+            px[at] = np.where(rng.random(n) < 0.5, long, edge)
+        else:
+            px[at] = rng.integers(1 << 12, 0x1400 if bd == 10 else 0x4100, size=n)
+        ref, out = oracle(fr, si), fr.copy()
+        runner.apply(out.pf(), si.side)
+        for p, (a, b) in enumerate(zip(ref.planes, out.planes)):
+            assert np.array_equal(a, b), "secondary %s: plane %d differs in %d samples" % (
+                secondary, p, int((a != b).sum()))
