@@ -49,8 +49,8 @@ constexpr int kTabPitch = 68;  // SGR tables: column x at x + 1, x = -1 .. 64
 struct LrSmem {
   alignas(16) uint32_t win[kWinRows * kWinWords];
   union {
-    // SGR a and b of one box in one word, (a - 1) << 22 | b (a - 1 <= 255, b
-    // <= 256 * 4095), so that the sum of three neighbours is one addition
+    // SGR a and b of one box in one word, (a - 1) << 22 | b (a - 1 <= 255; b,
+    // a 32-bit product shifted by 12, below 2^20), so that the sum of three neighbours is one addition
     // chain: radius 1 for rows -1..h, radius 2 for the rows -1, 1, 3, ... it
     // is computed on.
     struct {
@@ -188,8 +188,8 @@ __device__ __forceinline__ uint32_t sgr_ab(uint32_t sum, uint32_t sq, int bd, ui
   if (k8) {
     p = sq * N - sum * sum;
   } else {
-    const int32_t av = rpot((int32_t)sq, 2 * (bd - 8)), bv = rpot((int32_t)sum, bd - 8);
-    p = (uint32_t)imax(av * N - bv * bv, 0);
+    const uint32_t av = (uint32_t)rpot((int32_t)sq, 2 * (bd - 8)), bv = (uint32_t)rpot((int32_t)sum, bd - 8);
+    p = max(av * N, bv * bv) - bv * bv;  // words beyond 12 bits reach above 2^31
   }
   uint32_t z = (p * sv + (1u << 19)) >> 20;
   z = z < 255u ? z : 255u;

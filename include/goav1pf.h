@@ -99,7 +99,9 @@ enum {
 };
 
 /* One plane of a frame.  data points at sample (0,0); 10/12-bit samples are
- * little-endian uint16 (frame/buffer.go, cdef/filter.go:366). */
+ * little-endian uint16 (frame/buffer.go, cdef/filter.go:366).  Words beyond
+ * the frame's depth, which no bitstream has, are filtered as the reference
+ * filters them, more slowly. */
 typedef struct pf_plane {
   void* data;
   int64_t stride;        /* bytes between rows */

@@ -97,3 +97,26 @@ def test_rows_off_word_boundaries(runner, bd, kind):
     for p, a in enumerate(ref.planes):
         got = keep[p][:, 1:1 + a.shape[1]].cpu().numpy()
         assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
+
+
+@pytest.mark.parametrize("w,h", [(63, 61), (141, 130)])
+@pytest.mark.parametrize("ss", [(1, 1), (0, 0)], ids=["420", "444"])
+@pytest.mark.parametrize("bd", [10, 12])
+@pytest.mark.parametrize("kind", ["wiener", "sgr"])
+@pytest.mark.parametrize("content", ["spots", "level"])
+def test_samples_longer_than_twelve_bits(runner, w, h, ss, bd, kind, content):
+    """16-bit words that hold more than 12 bits: single ones, at most one in a
+    box (none on a row or column that a border repeats), and whole planes of
+    them.  Every box's sum of squares fits 32 bits."""
+    fr, si = frame(w, h, bd, ss, kind, 64)
+    rng = np.random.default_rng([w, bd])
+    for p in fr.planes:
+        if content == "spots":
+            spots = p[3::8, 3::8]
+            spots[:] = rng.integers(1 << 12, 45000 if bd == 10 else 40000, size=spots.shape)
+        else:
+            p[:] = 8000 + p // (1 << (bd - 9))
+    ref, out = oracle(fr, si), fr.copy()
+    runner.apply(out.pf(), si.side)
+    for p, (a, b) in enumerate(zip(ref.planes, out.planes)):
+        assert np.array_equal(a, b), "plane %d differs in %d samples" % (p, int((a != b).sum()))
