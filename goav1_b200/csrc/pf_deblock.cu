@@ -557,6 +557,9 @@ __device__ __forceinline__ bool deblock_unit(const DFrame& f, const LfArgs& a, i
   // Those hold for the samples and levels of a bitstream; a 10-bit frame's
   // 16-bit words can hold more.
   if (L > 63) return false;
+  // The outer samples' word q4..q7: q7, which no filter needs, can be past the
+  // allocated row (a malformed mask again).
+  if (kWd == 16 && dir == 0 && c4 * 4 + 8 > pl.aw) return false;
   if constexpr (sizeof(T) == 2) {
     uint32_t over = 0;
 #pragma unroll

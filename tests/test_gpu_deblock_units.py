@@ -95,3 +95,40 @@ def test_rows_off_word_boundaries(runner, bd):
     for p, a in enumerate(ref.planes):
         got = keep[p][:, 1:1 + a.shape[1]].cpu().numpy()
         assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
+
+
+@pytest.mark.parametrize("bd", [8, 10])
+def test_wide_edge_that_ends_with_the_allocated_row(runner, bd):
+    """A 14-tap edge (from a malformed mask: its transforms are too narrow)
+    whose last tap is the last sample of the allocated row, in a buffer that
+    ends there: filtered without touching the word's fourth sample."""
+    import oracle_ctypes
+    import torch
+
+    w, h, aw, pitch = 16, 16, 19, 20
+    fr, si = frame(5, w, h, bd, (1, 1), "smooth")
+    fr.planes[0] = np.ascontiguousarray(fr.planes[0][:, :aw])
+    fr.planes[0][:] = (1 << (bd - 1)) + np.random.default_rng(bd).integers(0, 2, fr.planes[0].shape)
+    masks = np.zeros(abi.PF_LF_MASK_WORDS, np.uint16)
+    masks[(3 * 3 + 2) * 2] = 0xf  # vertical edges at column 12, widest class, the four unit rows
+    levels = np.full((h // 4, w // 4, 4), 40, np.uint8)
+    si.side.lf.masks, si.side.lf.level_cache = masks.ctypes.data, levels.ctypes.data
+    ref = fr.copy()
+    assert oracle_ctypes.frame_apply(ref.pf(), si.side, None) == 0
+    assert not np.array_equal(ref.planes[0], fr.planes[0])
+    f, keep = fr.pf(memory=abi.PF_MEM_DEVICE, ptrs=[0, 0, 0]), []
+    for p, a in enumerate(fr.planes):
+        rows, cols = a.shape
+        n = pitch if p == 0 else cols
+        flat = torch.zeros(n * (rows - 1) + cols, dtype=torch.uint8 if bd == 8 else torch.int16, device="cuda")
+        t = flat.as_strided((rows, cols), (n, 1))
+        t.copy_(torch.from_numpy(a if bd == 8 else a.view(np.int16)))
+        keep.append(t)
+        f.plane[p].data = t.data_ptr()
+        f.plane[p].stride = n * t.element_size()
+    torch.cuda.synchronize()
+    runner.apply(f, si.side)
+    runner.sync()
+    for p, a in enumerate(ref.planes):
+        got = keep[p].cpu().numpy()
+        assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
