@@ -335,11 +335,14 @@ __device__ __forceinline__ void fg_offsets_row(uint16_t seed, int r, int cols, u
 //
 // Bound by integer issue (57 % of the slots) and the wait for the grain
 // behind the block offset.  us per frame: 60 x 1080p 8-bit 12.6 before (one
-// column by 16 rows a thread, every sample by itself), 6.9 now, at 2.2 warp
-// instructions per luma sample instead of 5.0; 8 x 4K 10-bit 62.9 and 29.3;
-// one 1080p frame 25.6 and 17.  (With the neighbours' offsets and grains read
-// row by row, after the stores: 7.1 and 30.1.)  Two rows' or one row's loads
-// at a time measured 7.3 and 7.8; 3 or 5 CTAs per SM 8.1 and 7.2.
+// column by 16 rows a thread, every sample by itself), 6.8 now, at 2.2 warp
+// instructions per luma sample instead of 5.0; 8 x 4K 10-bit 62.9 and 28.8;
+// one 1080p frame 25.6 and 16.  The neighbouring blocks' offsets are read
+// ahead of the stores, their grains row by row through the read-only path
+// (the left block's offset read row by row, too: 6.84 and 29.4; all offsets,
+// and the grains by plain loads: 7.1 and 30.1).  With the last, two rows' or
+// one row's loads at a time measured 7.3 and 7.8, 3 or 5 CTAs per SM 8.1 and
+// 7.2.
 
 template <typename T>
 struct FgQuad;
@@ -512,7 +515,6 @@ __device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& d
           // Overlap (apply.go:301-343): horizontal weights 27/17 then 17/27
           // (subsampled 23/22), vertical ones the same by row.
           if (xStart) {
-            const int o10 = offs[-1];
             const int c10 = gcol(o10, 1), r10 = grow(o10, 0) + k;
 #pragma unroll
             for (int j = 0; j < ovl; j++)
