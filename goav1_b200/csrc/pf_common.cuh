@@ -239,13 +239,15 @@ __device__ __forceinline__ void prefetch_block(const DPlane& p, int x0, int x1, 
   y1 = y1 > p.ah ? p.ah : y1;
   if (x1 <= x0 || y1 <= y0) return;
   const uintptr_t row0 = reinterpret_cast<uintptr_t>(p.ptr) + (uintptr_t)x0 * sizeof(T);
-  const uintptr_t l0 = row0 & ~(uintptr_t)127;
-  const int lines = (int)(((row0 + (uintptr_t)(x1 - x0) * sizeof(T) - 1) >> 7) - (l0 >> 7)) + 1;
-  const int n = lines * (y1 - y0);
+  const uintptr_t bytes = (uintptr_t)(x1 - x0) * sizeof(T);
+  // Lines of a row that starts anywhere in its first one.
+  const int lines = (int)((bytes + 126) >> 7) + 1, n = lines * (y1 - y0);
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const int r = i / lines, l = i - r * lines;
-    const uintptr_t a = ((row0 + (uintptr_t)(y0 + r) * (uintptr_t)p.stride) & ~(uintptr_t)127) + (uintptr_t)l * 128;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+    const uintptr_t row = row0 + (uintptr_t)(y0 + r) * (uintptr_t)p.stride;
+    const uintptr_t a = (row & ~(uintptr_t)127) + (uintptr_t)l * 128;
+    // The row's own lines only: another may lie past the allocation.
+    if (a < row + bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
   }
 }
 
