@@ -132,3 +132,90 @@ def test_wide_edge_that_ends_with_the_allocated_row(runner, bd):
     for p, a in enumerate(ref.planes):
         got = keep[p].cpu().numpy()
         assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
+
+
+@pytest.fixture(params=[1, 2, 3], ids=["32x8", "32x16", "32x32"])
+def tiled(request):
+    """A runner for each tile size (a small frame takes the smallest by itself)."""
+    from goav1_b200.postfilter import PostFilterRunner
+
+    r = PostFilterRunner()
+    r.set_schedule(abi.PF_TUNE_DEBLOCK, tile=request.param)
+    yield r
+    r.close()
+
+
+@pytest.mark.parametrize("w,h", [(132, 36), (200, 136), (264, 330)])
+@pytest.mark.parametrize("ss", [(1, 1), (1, 0), (0, 0), (0, 1)], ids=["420", "422", "444", "440"])
+@pytest.mark.parametrize("bd", [8, 10, 12])
+def test_tile_sizes(tiled, w, h, ss, bd):
+    """One, two and four units a thread on tiles that the frame ends inside:
+    shared mask words, the class lists filled from both ends, the level rows."""
+    for content in ("texture", "smooth", "ends"):
+        check(tiled, *frame(w + 3 * h + bd, w, h, bd, ss, content))
+
+
+@pytest.mark.parametrize("plane", [0, 1, 2])
+def test_tile_sizes_with_samples_longer_than_ten_bits(tiled, plane):
+    fr, si = frame(77 + plane, 264, 330, 10, (1, 1), "smooth")
+    rng = np.random.default_rng(plane)
+    at = rng.random(fr.planes[plane].shape) < 0.02
+    fr.planes[plane][at] = rng.integers(1024, 1 << 16, size=int(at.sum()))
+    check(tiled, fr, si)
+
+
+def on_device(fr, bd, gap):
+    """A device copy of a frame, each row `gap` samples past a 4-sample boundary."""
+    import torch
+
+    f, keep = fr.pf(memory=abi.PF_MEM_DEVICE, ptrs=[0, 0, 0]), []
+    for p, a in enumerate(fr.planes):
+        t = torch.zeros((a.shape[0], a.shape[1] + 4), dtype=torch.uint8 if bd == 8 else torch.int16, device="cuda")
+        t[:, gap:gap + a.shape[1]] = torch.from_numpy(a if bd == 8 else a.view(np.int16)).cuda()
+        keep.append(t)
+        f.plane[p].data = t.data_ptr() + gap * t.element_size()
+        f.plane[p].stride = t.stride(0) * t.element_size()
+    torch.cuda.synchronize()
+    return f, keep
+
+
+@pytest.mark.parametrize("bd", [8, 10])
+def test_tile_sizes_with_rows_off_word_boundaries(tiled, bd):
+    import oracle_ctypes
+
+    fr, si = frame(91 + bd, 264, 330, bd, (1, 1), "smooth")
+    ref = fr.copy()
+    assert oracle_ctypes.frame_apply(ref.pf(), si.side, None) == 0
+    f, keep = on_device(fr, bd, 1)
+    tiled.apply(f, si.side)
+    tiled.sync()
+    for p, a in enumerate(ref.planes):
+        got = keep[p][:, 1:1 + a.shape[1]].cpu().numpy()
+        assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
+
+
+@pytest.mark.parametrize("bd", [8, 10])
+@pytest.mark.parametrize("content", ["smooth", "ends"])
+def test_levels_above_63(tiled, bd, content):
+    """A device-side level cache is not looked over: cells above 63 (no
+    bitstream has them) go line by line beside others that do not."""
+    import ctypes as C
+
+    import oracle_ctypes
+    from goav1_b200.postfilter import device_side
+
+    fr, si = frame(19 + bd, 200, 136, bd, (1, 1), content)
+    lf = si.side.lf
+    levels = np.ctypeslib.as_array(C.cast(lf.level_cache, C.POINTER(C.c_uint8)), (4 * lf.mi_cols * lf.mi_rows,)).copy()
+    rng = np.random.default_rng(bd)
+    at = rng.random(levels.size) < 0.2
+    levels[at] = rng.integers(64, 256, size=int(at.sum()))
+    lf.level_cache = levels.ctypes.data
+    ref = fr.copy()
+    assert oracle_ctypes.lib().oracle_loop_filter(C.byref(ref.pf()), C.byref(si.side)) == 0
+    f, keep = on_device(fr, bd, 0)
+    tiled.apply(f, device_side(si, fr).side)
+    tiled.sync()
+    for p, a in enumerate(ref.planes):
+        got = keep[p][:, :a.shape[1]].cpu().numpy()
+        assert np.array_equal(a, got if bd == 8 else got.view(np.uint16)), "plane %d" % p
