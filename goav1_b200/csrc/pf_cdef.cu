@@ -52,7 +52,6 @@ struct CdefSmem {
   alignas(16) uint32_t c[2][36 * kPC];
   alignas(16) int32_t cost[64 * 8];
   alignas(16) CdefBlk blk[64];
-  int32_t var[64];
   int2 ofs[2][12];  // direction tap offsets in words (cdef/filter.go:53-66), pitch kPW and kPC
   uint8_t dir[64];
 };

@@ -27,21 +27,6 @@ __device__ __forceinline__ T* row_ptr(const DPlane& p, int y) {
   return reinterpret_cast<T*>(p.ptr + (int64_t)y * p.stride);
 }
 
-// Copies column x of rows y, y+step, ... < yEnd from one plane to another,
-// four rows' loads issued before their stores (the planes may not alias).
-template <typename T>
-__device__ __forceinline__ void copy_column(const DPlane& from, const DPlane& to, int x, int y, int yEnd, int step) {
-  for (; y < yEnd; y += 4 * step) {
-    T v[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (y + k * step < yEnd) v[k] = row_ptr<T>(from, y + k * step)[x];
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (y + k * step < yEnd) row_ptr<T>(to, y + k * step)[x] = v[k];
-  }
-}
-
 // Copies the block [x0, x1) x [y0, y1) of one plane to another (the planes
 // may not alias) with the whole CTA: 16-byte words, up to four per thread in
 // flight, when both rows' starts and strides are 16-byte aligned and a row is

@@ -59,7 +59,6 @@ struct SrArgs {
   SrPlane pl[kSrFrames][3];
   int base[kSrFrames * 3 + 1];  // prefix of the planes' CTAs
   uint8_t deep[kSrFrames], maxv_bits[kSrFrames];
-  int n;
   int lines;
 };
 
@@ -146,13 +145,13 @@ cudaError_t launch_superres(const SrFrame* frames, int n, bool lines, cudaStream
   for (int at = 0; at < n; at += kSrFrames) {
     SrArgs a;
     memset(&a, 0, sizeof(a));
-    a.n = imin(kSrFrames, n - at);
+    const int frames_here = imin(kSrFrames, n - at);
     a.lines = lines;
     int total = 0;
     for (int i = 0; i < kSrFrames; i++)
       for (int p = 0; p < 3; p++) {
         a.base[3 * i + p] = total;
-        if (i >= a.n) continue;
+        if (i >= frames_here) continue;
         const SrFrame& F = frames[at + i];
         const pf_frame* c = F.coded;
         a.deep[i] = c->bit_depth > 8;
