@@ -126,8 +126,8 @@ struct pf_ctx {
   int persistent[ST_COUNT] = {};
   int chunk[ST_COUNT] = {1, 1, 1, 1, 1, 1, 1, 1};
   int ahead[ST_COUNT] = {};
-  int tile[ST_COUNT] = {};  // launch-level tile setting (grain apply: rows loaded together)
-  int db_tile = 0;          // deblocking tile setting (db_units_log2)
+  int db_tile = 0;  // deblocking tile setting (db_units_log2)
+  int fg_tile = 0;  // grain's: accepted and given back, it changes nothing
   // Frame groups (pf_set_frame_groups): 2 runs the batch's two halves on the
   // main stream and stream2.
   int frame_groups = 1;
@@ -916,7 +916,7 @@ static void fill_job(const FrameRef& r, Cursor& arena, Cursor& side, Bytes& hs, 
 // Whether a batch is one frame under the default schedules, whose launches
 // carry the frame's job themselves (StageLaunch::one).
 static bool single_frame(const pf_ctx* c, int n) {
-  bool plain = n == 1 && (c->tile[ST_FG_APPLY] == 0 || c->tile[ST_FG_APPLY] == 3);
+  bool plain = n == 1;
   for (int k = 0; k < ST_COUNT; k++) plain &= c->persistent[k] == 0 && c->chunk[k] == 1 && c->ahead[k] == 0;
   return plain;
 }
@@ -981,7 +981,6 @@ static int enqueue_batch(pf_ctx* c, const FrameJob* hjobs, const int* hbase, con
     l.total = count(k, f0, f1);
     l.args.chunk = c->chunk[k];
     l.args.ahead = c->ahead[k];
-    l.args.tile = c->tile[k];
     const int chunks = (l.total + l.args.chunk - 1) / l.args.chunk;
     if (c->persistent[k] > 0 && chunks > c->persistent[k]) {
       l.grid = c->persistent[k];
@@ -1070,7 +1069,6 @@ static std::vector<int64_t> batch_key(const pf_ctx* c, int n, bool fg) {
     k.push_back(c->persistent[i]);
     k.push_back(c->chunk[i]);
     k.push_back(c->ahead[i]);
-    k.push_back(c->tile[i]);
   }
   k.push_back(c->db_tile);
   k.push_back(c->frame_groups);
@@ -1983,9 +1981,9 @@ extern "C" int pf_set_schedule(pf_ctx* c, int32_t group, const pf_schedule* s) {
       c->persistent[k] = s->ctas;
       c->chunk[k] = s->units_per_cta;
       c->ahead[k] = s->staging;
-      c->tile[k] = group == PF_TUNE_DEBLOCK ? 0 : s->tile;
     }
   if (group == PF_TUNE_DEBLOCK) c->db_tile = s->tile;
+  if (group == PF_TUNE_FILM_GRAIN) c->fg_tile = s->tile;
   return PF_OK;
 }
 
@@ -1995,7 +1993,7 @@ extern "C" int pf_get_schedule(const pf_ctx* c, int32_t group, pf_schedule* s) {
   s->ctas = c->persistent[k];
   s->units_per_cta = c->chunk[k];
   s->staging = c->ahead[k];
-  s->tile = group == PF_TUNE_DEBLOCK ? c->db_tile : c->tile[k];
+  s->tile = group == PF_TUNE_DEBLOCK ? c->db_tile : group == PF_TUNE_FILM_GRAIN ? c->fg_tile : 0;
   return PF_OK;
 }
 
@@ -2047,7 +2045,7 @@ extern "C" int pf_autotune(pf_ctx* c, const pf_batch_item* items, int32_t n, int
         best = cand;
       }
     };
-    for (int t = 1; t <= 3; t++) {  // tile settings the group has (schedule_ok)
+    for (int t = 1; t <= 3 && gi == PF_TUNE_DEBLOCK; t++) {  // tile sizes
       pf_schedule s = best;
       s.tile = t;
       tryOne(s);

@@ -190,7 +190,6 @@ struct BatchArgs {
   // and how many items ahead of the current one the CTA prefetches into L2.
   int chunk;
   int ahead;
-  int tile;  // the stage's tile setting (pf_schedule.tile; deblocking reads it from the job)
   // The frames [f0, f1) this launch covers (a frame group of the batch;
   // items base[f0] .. base[f1] - 1 of each stage).
   int f0, f1;

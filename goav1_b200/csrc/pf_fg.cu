@@ -427,7 +427,8 @@ __device__ __forceinline__ int grain_of(uint2 g, int k) {
 
 // Columns x .. x + 3, rows y0 .. y0 + 3 of one display plane (x and y0
 // multiples of 4).  kLuma / kSx: the plane is luma / horizontally subsampled
-// chroma.  kRows rows' loads are issued before their first store.  word: four
+// chroma.  kRows rows' loads (four, or one where words do not fit) are issued
+// before their first store.  word: four
 // samples of a row move as one word.
 template <typename T, bool kLuma, bool kSx, int kRows>
 __device__ __forceinline__ void fg_apply_quad(const DFrame& ref, const DFrame& disp, const FgArgs& a,
@@ -661,7 +662,7 @@ __device__ __noinline__ void fg_apply_any(const FrameJob* J, const uint8_t* lut,
   fg_apply_quad<T, kLuma, kSx, 1>(J->io, J->disp, J->fg, lut, plane, x, y0, false);
 }
 
-template <typename T, bool kLuma, bool kSx, int kRows>
+template <typename T, bool kLuma, bool kSx>
 __device__ __forceinline__ void fg_apply_plane(const FrameJob& J, const uint8_t* lut, int plane, int x, int y0) {
   const DPlane &sp = J.io.pl[plane], &dp = J.disp.pl[plane], &lp = J.io.pl[0];
   if (x >= sp.aw || y0 >= sp.ah) return;
@@ -669,12 +670,12 @@ __device__ __forceinline__ void fg_apply_plane(const FrameJob& J, const uint8_t*
       ((reinterpret_cast<uintptr_t>(sp.ptr) | (uintptr_t)sp.stride | reinterpret_cast<uintptr_t>(dp.ptr) |
         (uintptr_t)dp.stride | reinterpret_cast<uintptr_t>(lp.ptr) | (uintptr_t)lp.stride) &
        (4 * sizeof(T) - 1)) == 0)
-    fg_apply_quad<T, kLuma, kSx, kRows>(J.io, J.disp, J.fg, lut, plane, x, y0, true);
+    fg_apply_quad<T, kLuma, kSx, 4>(J.io, J.disp, J.fg, lut, plane, x, y0, true);
   else
     fg_apply_any<T, kLuma, kSx>(&J, lut, plane, x, y0);
 }
 
-template <typename T, int kRows>
+template <typename T>
 __device__ __forceinline__ void fg_tile(const FrameJob& J, const FgTile& t, uint8_t* lut) {
   const int tid = threadIdx.x;
   if (sizeof(T) == 1) {
@@ -700,16 +701,14 @@ __device__ __forceinline__ void fg_tile(const FrameJob& J, const FgTile& t, uint
   }
   const int x = t.tx * 64 + 4 * q, y0 = t.ty * 64 + 4 * rg;
   if (t.plane == 0)
-    fg_apply_plane<T, true, false, kRows>(J, lut, 0, x, y0);
+    fg_apply_plane<T, true, false>(J, lut, 0, x, y0);
   else if (sx)
-    fg_apply_plane<T, false, true, kRows>(J, lut, t.plane, x, y0);
+    fg_apply_plane<T, false, true>(J, lut, t.plane, x, y0);
   else
-    fg_apply_plane<T, false, false, kRows>(J, lut, t.plane, x, y0);
+    fg_apply_plane<T, false, false>(J, lut, t.plane, x, y0);
 }
 
-// kRows: rows of a thread's four whose loads go out together (the grain
-// group's tile setting).
-template <bool kLoop, int kRows>
+template <bool kLoop>
 __global__ void __launch_bounds__(256, 4) k_fg_apply_batch(BatchArgs b) {
   __shared__ __align__(16) uint8_t s_lut[kFgScaleLen];
   stage_begin();
@@ -721,9 +720,9 @@ __global__ void __launch_bounds__(256, 4) k_fg_apply_batch(BatchArgs b) {
         const FrameJob& J = b.jobs[fi];
         const FgTile t = fg_locate(J, item - base[fi]);
         if (J.io.bd == 8)
-          fg_tile<uint8_t, kRows>(J, t, s_lut);
+          fg_tile<uint8_t>(J, t, s_lut);
         else
-          fg_tile<uint16_t, kRows>(J, t, s_lut);
+          fg_tile<uint16_t>(J, t, s_lut);
         if (kLoop) __syncthreads();  // the table is rewritten by the next tile
       },
       [&](int item) {
@@ -744,9 +743,9 @@ __global__ void __launch_bounds__(256, 4) k_fg_apply_one(const __grid_constant__
   stage_begin();
   const FgTile t = fg_locate(J, blockIdx.x);
   if (J.io.bd == 8)
-    fg_tile<uint8_t, 4>(J, t, s_lut);
+    fg_tile<uint8_t>(J, t, s_lut);
   else
-    fg_tile<uint16_t, 4>(J, t, s_lut);
+    fg_tile<uint16_t>(J, t, s_lut);
 }
 
 // Border extension: 64x4-sample tiles of the right strip [w, aw) x [0, h)
@@ -844,23 +843,13 @@ cudaError_t launch_fg_offsets(const StageLaunch& l) {
   return launch_stage(k_fg_offsets_batch, l.grid, 64, 0, l.st, false, l.args);
 }
 
-template <int kRows>
-static cudaError_t launch_fg_apply_rows(const StageLaunch& l) {
-  static int wave = 0;
-  if (batch_loops(l.args))
-    return launch_stage(k_fg_apply_batch<true, kRows>, l.grid, 256, 0, l.st, l.dependent, l.args);
-  return launch_stage(k_fg_apply_batch<false, kRows>, l.grid, 256, 0, l.st, l.dependent,
-                      with_wave(l.args, k_fg_apply_batch<false, kRows>, 256, 0, wave));
-}
-
 cudaError_t launch_fg_apply(const StageLaunch& l) {
   if (l.total <= 0) return cudaSuccess;
   if (l.one) return launch_stage(k_fg_apply_one, l.total, 256, 0, l.st, l.dependent, *l.one);
-  switch (l.args.tile) {
-    case 1: return launch_fg_apply_rows<2>(l);
-    case 2: return launch_fg_apply_rows<1>(l);
-    default: return launch_fg_apply_rows<4>(l);
-  }
+  static int wave = 0;
+  if (batch_loops(l.args)) return launch_stage(k_fg_apply_batch<true>, l.grid, 256, 0, l.st, l.dependent, l.args);
+  return launch_stage(k_fg_apply_batch<false>, l.grid, 256, 0, l.st, l.dependent,
+                      with_wave(l.args, k_fg_apply_batch<false>, 256, 0, wave));
 }
 
 cudaError_t launch_extend(const StageLaunch& l) {

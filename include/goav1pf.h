@@ -330,12 +330,12 @@ int pf_batch_apply(pf_ctx* ctx, const pf_batch_item* items, int32_t n, pf_stats*
  *                      with larger chunks, the item that many places on
  *                      inside the chunk (then below units_per_cta);
  *       tile           deblocking: the tile, 1 = 32x8, 2 = 32x16, 3 = 32x32
- *                      edge units, 0 = by the call's size; grain apply: how many of a thread's four rows
- *                      have their loads issued together, 0 and 3 = four,
- *                      1 = two, 2 = one; 0 for the other groups.
+ *                      edge units, 0 = by the call's size; grain apply:
+ *                      0..3 are accepted and are the same; 0 for the other
+ *                      groups.
  *     Work items are independent, so every schedule gives the same samples.
  * pf_autotune searches the schedule of each group on a given batch, one
- * dimension at a time (tile setting, units per CTA, staging depth, persistent
+ * dimension at a time (deblocking tile, units per CTA, staging depth, persistent
  * CTAs at 0, 1, 2, 4, 8 and 16 per SM), keeping after each the candidate
  * with the lowest median stage time over reps timed runs (one untimed run
  * first), then the frame-group count (1 or 2) by the whole batch's median
