@@ -1905,6 +1905,13 @@ void* pf_internal_fork(pf_ctx* c) {
     return nullptr;
   return (void*)c->side;
 }
+// Makes the context's stream wait for what its second one holds so far, so
+// that a wait for the stream (pf_sync after a timeout among them) covers both.
+bool pf_internal_join(pf_ctx* c) {
+  return cudaEventRecord(c->join, c->side) == cudaSuccess && cudaStreamWaitEvent(c->stream, c->join, 0) == cudaSuccess;
+}
+// Whether the context's waits have a deadline (pf_config.wait_timeout_us).
+bool pf_internal_bounded(const pf_ctx* c) { return c->wait_timeout_us > 0; }
 // The context's stage events when it times stages (pf_config.timing), else null.
 cudaEvent_t* pf_internal_events(pf_ctx* c) { return c->timing ? c->ev : nullptr; }
 

@@ -912,6 +912,8 @@ void* pf_internal_stream(pf_ctx* c);
 cudaEvent_t* pf_internal_events(pf_ctx* c);  // pf_api.cu: null unless the context times stages
 void* pf_internal_pinned(pf_ctx* c, size_t bytes);
 void* pf_internal_fork(pf_ctx* c);  // pf_api.cu
+bool pf_internal_join(pf_ctx* c);
+bool pf_internal_bounded(const pf_ctx* c);
 void* pf_internal_cached_upload(pf_ctx* c, const void* host, size_t bytes, size_t extra, cudaStream_t st,
                                 int* changed);
 int pf_internal_wait(pf_ctx* c, void* stream);  // pf_api.cu: blocking or bounded by the context's deadline
@@ -1141,13 +1143,17 @@ static int search_finish(Staged& S, const pf_cdef_search_params* params, uint64_
   if (cudaMemcpyAsync(pfo, S.fo, sizeof(FinishOut), cudaMemcpyDeviceToHost, st) != cudaSuccess) return PF_ERR_DEVICE;
   if (fb_index_out && cudaMemcpyAsync(pidx, S.idx, S.nfb, cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return PF_ERR_DEVICE;
-  if (mse_out) {
+  if (mse_out && !pf_internal_join(S.ctx)) return PF_ERR_DEVICE;
+  // A context with a deadline waits once, for both streams.
+  const bool early = mse_out && !pf_internal_bounded(S.ctx);
+  if (early) {
     const int w = pf_internal_wait(S.ctx, side);
     if (w != PF_OK) return w;
     memcpy(mse_out, ptab, tab);
   }
   const int w = pf_internal_wait(S.ctx, st);
   if (w != PF_OK) return w;
+  if (mse_out && !early) memcpy(mse_out, ptab, tab);
   FinishOut fo;
   memcpy(&fo, pfo, sizeof(fo));
   if (fb_index_out) memcpy(fb_index_out, pidx, S.nfb);

@@ -107,3 +107,40 @@ def test_search_rejects_unsupported_formats(runner):
     fr = synth.HostFrame.alloc(64, 64, 10)
     with pytest.raises(ErrUnsupportedPostFilter):
         runner.cdef_search(fr.pf(), fr.pf(), None, 100, 1000.0)
+
+
+def test_search_under_a_deadline():
+    """A context with a wait limit: a search that meets it gives the oracle's
+    table; one that gives up leaves work that pf_sync waits for, the table's
+    copy on the second stream included, after which another search is right."""
+    import time
+
+    from goav1_b200.postfilter import ErrTimeout, PostFilterRunner
+
+    big = synth.make_search_pair(6, 1920, 1080)
+    src, rec, side, _ = synth.make_search_pair(7, 256, 192)
+    ns = _noskip(side, rec)
+    r0, m0, i0 = _oracle(src, rec, ns, 100, 2000.0, 8)
+    hasty, patient = PostFilterRunner(wait_timeout_us=1), PostFilterRunner(wait_timeout_us=10_000_000)
+
+    def finished(f):
+        for _ in range(20000):  # bounded: the work takes less than a millisecond
+            try:
+                return f()
+            except ErrTimeout:
+                time.sleep(0.0005)
+        pytest.fail("still waiting")
+
+    try:
+        for _ in range(3):
+            with pytest.raises(ErrTimeout):
+                hasty.cdef_search(big[0].pf(), big[1].pf(), None, 128, 4000.0)
+            finished(hasty.sync)
+            with pytest.raises(ErrTimeout):
+                hasty.cdef_search(src.pf(), rec.pf(), ns, 100, 2000.0)
+            finished(hasty.sync)
+            r1, m1, i1 = patient.cdef_search(src.pf(), rec.pf(), ns, 100, 2000.0)
+            assert np.array_equal(m0, m1) and np.array_equal(i0, i1) and r0.cost == r1.cost
+    finally:
+        hasty.close()
+        patient.close()
