@@ -469,10 +469,10 @@ def measure_issue_peaks():
 # the command and the raw figures): DRAM bytes read + written and warp
 # instructions executed (deblocking: both passes).
 KERNEL_COUNTERS_1080P8 = {
-    "deblock": {"dram_bytes": (446.61e6 + 192.33e6) / 60, "warp_inst": 240.54e6 / 60},
-    "cdef": {"dram_bytes": (187.69e6 + 166.32e6) / 60, "warp_inst": 580.50e6 / 60},
-    "restoration": {"dram_bytes": (205.83e6 + 152.40e6) / 60, "warp_inst": 540.98e6 / 60},
-    "film_grain": {"dram_bytes": (189.61e6 + 143.97e6) / 60, "warp_inst": 288.63e6 / 60},
+    "deblock": {"dram_bytes": (446.61e6 + 192.33e6) / 60, "warp_inst": 240.36e6 / 60},
+    "cdef": {"dram_bytes": (187.70e6 + 165.06e6) / 60, "warp_inst": 581.21e6 / 60},
+    "restoration": {"dram_bytes": (205.82e6 + 152.08e6) / 60, "warp_inst": 540.49e6 / 60},
+    "film_grain": {"dram_bytes": (191.14e6 + 145.60e6) / 60, "warp_inst": 269.47e6 / 60},
 }
 
 

@@ -1766,7 +1766,7 @@ extern "C" int pf_frame_apply_superres(pf_ctx* c, const pf_frame* coded, const p
 // A batch of super-resolved frames: each stage of the chain runs as one
 // launch over every frame that has it (deblocking over the coded frames,
 // then CDEF, then restoration / extension / grain over the upscaled ones);
-// the boundary-line upscale and the frame upscale are launched per frame
+// the boundary-line upscale and the frame upscale, eight frames a launch, go
 // between them, in the decoder's order.  Device frames: returns once the
 // work is queued; host frames: one pf_frame_apply_superres per item.
 extern "C" int pf_batch_apply_superres(pf_ctx* c, const pf_superres_item* items, int32_t n, pf_stats* stats) {

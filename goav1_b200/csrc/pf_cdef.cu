@@ -24,7 +24,7 @@
 // shared reads) and the three 4:2:0 planes staged and filtered in one pass.
 // Per frame, 60 x 1080p 8-bit: 22.4 us before, 12.0 now (5.6 of it the taps,
 // 1.5 the directions, 1.0 the staging); 8 x 4K 10-bit: 103.2 and 49.4; one
-// 1080p frame alone: 44.8 and 24.3.  64 registers and 4 CTAs per SM: 48 (5
+// 1080p frame alone: 44.8 and 22.3.  64 registers and 4 CTAs per SM: 48 (5
 // CTAs, with spills) and 80 (3 CTAs) measured 4 % slower.
 #include "pf_cdef_dev.cuh"
 

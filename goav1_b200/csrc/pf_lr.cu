@@ -27,7 +27,7 @@
 // cost a CTA's set-up for a quarter of the samples.  us per frame: 60 x 1080p
 // 8-bit, a third of the units of each kind, 18.9 before, 10.4 now (7.6 and
 // 4.4 warp instructions per luma sample); 8 x 4K 10-bit 78.9 and 44.9; one
-// 1080p frame 28.7 and 20.6.  The encoder's search at 1080p: 144 and 68 us.
+// 1080p frame 28.7 and 19.5.  The encoder's search at 1080p: 144 and 68 us.
 #include "pf_common.cuh"
 #include "pf_tables.h"
 
